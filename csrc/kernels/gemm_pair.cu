@@ -1,0 +1,773 @@
+// gemm_pair.cu - bf16 GEMM on CTA pairs (tcgen05 cta_group::2), the plain (single GPU) products.
+//
+//   C[M,N] = alpha * sum_k A(m,k) * B(n,k)   (+ epilogue)
+//
+// Two CTAs on neighbouring SMs (a cluster of two) compute one 256 x BN tile. Each loads its own 128 rows of A and its own
+// BN / 2 rows of B into its own shared memory; the MMA, issued by one thread of the even CTA, reads both halves of B from
+// both SMs. What bounds the one-CTA kernel (gemm_tcgen05.cu) is shared-memory bandwidth: a 128 x 256 x 16 MMA takes 128
+// cycles and reads 12 KB (96 B / cycle) while TMA writes the next 12 KB (96 B / cycle) against 128 B / cycle per SM. The pair
+// reads and writes 8 KB per SM for the same arithmetic, and L2 delivers a third less.
+//
+// Warp 0 feeds a ring of shared-memory stages with TMA (no multicast: every CTA loads its own part), warp 1 of the even CTA
+// issues the MMAs, warps 2-9 drain the accumulator. Two accumulators per CTA in TMEM let the epilogue of a tile overlap the
+// main loop of the next. The epilogue goes through shared memory and leaves by TMA: full 128-byte rows instead of 16 bytes per
+// lane, edges clipped by the tensor map, the fp32 accumulation into C as a TMA reduction in L2 (one rounding, like a load and
+// an add); the residual is read into registers while the main loop still runs. (bf16 stores straight from the registers, a
+// 32-byte sector per lane, measured the same on aligned rows and up to 20 % slower on rows of 2000 bytes.)
+//
+// Measured against the one-CTA kernel (L2 flushed): 8192^3 812 -> 706 us (1556 TFLOP/s), 16384 x 2048 x 16384 1062 -> 712 us,
+// 16384 x 16384 x 2048 with SwiGLU 1026 -> 773 us, weight gradient 16384 x 2048 x 16384 1117 -> 794 us. One barrier round trip per
+// 64 k-elements instead of 128 held it at 1430 TFLOP/s: with data present, the issuing thread spends some 300 cycles between a
+// satisfied wait and its first MMA.
+#include "../plan/formats.h"
+#include "cai_kernels.h"
+#include "gemm_common.h"
+#include "host_common.h"
+#include "sm100.cuh"
+
+namespace cai {
+
+namespace pair {
+constexpr int kBM = 256;              // rows of a tile (128 per CTA)
+constexpr int kBK = 64;               // k-elements of a block (one 128-byte row of a K-major operand)
+constexpr int kPerStage = 2;          // blocks of a stage: one barrier round trip of the issuing thread per 128 k-elements
+constexpr int kUmmaK = 16;
+constexpr int kThreads = 320;         // warp 0 TMA, warp 1 MMA, warps 2-9 epilogue
+constexpr int kEpiWarps = 8;
+constexpr int kABytes = 128 * kBK * 2;
+constexpr int kBox = 4096;            // an epilogue box: 32 rows x 128 bytes
+template <int BN> constexpr int kBBytes = BN / 2 * kBK * 2;
+template <int BN> constexpr int kBlock = kABytes + kBBytes<BN>;
+template <int BN> constexpr int kStages = BN == 256 ? 3 : 4;
+template <int BN> constexpr int kSmem = kStages<BN> * kPerStage * kBlock<BN> + kEpiWarps * kBox + 512 + 1024;
+}  // namespace pair
+
+struct PairParams {
+    int M, N, K;
+    int a_mn, b_mn;
+    int epi;
+    float alpha;
+    int tiles_m, tiles_n, group_m, groups;
+    const int* seg_counts;
+    int seg_rows, seg_mode, grp_seg;
+    void* C;                      // split form: results leave through registers
+    const __nv_bfloat16* R;       // residual, read row by row
+    long long ldc, ldr, grp_c;    // grp_c: rows between the groups of C and R
+    int* status;
+};
+
+__device__ __forceinline__ bool pair_seg_live(const PairParams& p, int g, int row0) {
+    const int slab = row0 / p.seg_rows;
+    return row0 - slab * p.seg_rows < p.seg_counts[g * p.grp_seg + slab];
+}
+// Is the 128-row half that starts at row `row0` of group g computed and written?
+__device__ __forceinline__ bool pair_half_live(const PairParams& p, int g, int row0) {
+    return row0 < p.M && (p.seg_mode != 1 || pair_seg_live(p, g, row0));
+}
+
+// Which blocks of stage `ks` hold data (bit per block): all inside K, and under seg_mode 2 only live ones.
+__device__ __forceinline__ uint32_t pair_live_blocks(const PairParams& p, int g, int ks, int num_kb) {
+    uint32_t live = 0;
+#pragma unroll
+    for (int b = 0; b < pair::kPerStage; ++b) {
+        const int kb = ks * pair::kPerStage + b;
+        if (kb < num_kb && (p.seg_mode != 2 || pair_seg_live(p, g, kb * pair::kBK))) live |= 1u << b;
+    }
+    return live;
+}
+
+__device__ __forceinline__ void pair_tile_coords(const PairParams& p, int tile_all, int& tm, int& tn, int& grp) {
+    const int per_product = p.tiles_m * p.tiles_n;
+    grp = tile_all / per_product;
+    const int tile = tile_all - grp * per_product;
+    const int per_group = p.group_m * p.tiles_n;
+    const int g = tile / per_group;
+    const int first_m = g * p.group_m;
+    const int gsz = min(p.tiles_m - first_m, p.group_m);
+    const int in = tile - g * per_group;
+    tm = first_m + in % gsz;
+    tn = in / gsz;
+}
+
+// One stage of operands into this CTA's ring slot: rows m0.. of A and n0.. of B, k from ks * 128; `bar` is the pair's barrier.
+template <int BN>
+__device__ __forceinline__ void pair_load_stage(const CUtensorMap* tmA, const CUtensorMap* tmB, uint8_t* a_slot, uint8_t* b_slot,
+                                                uint32_t bar, const PairParams& p, int ks, uint32_t live, int m0, int n0, int grp) {
+    using namespace pair;
+#pragma unroll
+    for (int b = 0; b < kPerStage; ++b) {
+        if (!(live >> b & 1)) continue;
+        const int k0 = (ks * kPerStage + b) * kBK;
+        uint8_t* a_dst = a_slot + b * kABytes;
+        uint8_t* b_dst = b_slot + b * kBBytes<BN>;
+        if (!p.a_mn) {
+            tma_load_3d_pair(a_dst, tmA, bar, k0, m0, grp);
+        } else {
+#pragma unroll
+            for (int c = 0; c < 2; ++c) tma_load_3d_pair(a_dst + c * (kBK * 128), tmA, bar, m0 + c * 64, k0, grp);
+        }
+        if (!p.b_mn) {
+            tma_load_3d_pair(b_dst, tmB, bar, k0, n0, grp);
+        } else {
+#pragma unroll
+            for (int c = 0; c < BN / 128; ++c) tma_load_3d_pair(b_dst + c * (kBK * 128), tmB, bar, n0 + c * 64, k0, grp);
+        }
+    }
+}
+
+// What the issuing warp needs to turn a ring slot into MMAs. The whole warp walks the loop, so that descriptors stay in
+// uniform registers; one elected lane issues.
+template <int BN>
+struct PairMma {
+    uint64_t a_first, b_first;   // descriptors of the ring's first block
+    uint32_t a_step, b_step;     // descriptor distance of 16 k-elements
+    uint32_t idesc;
+    uint16_t pair_mask;
+    bool leader;
+    __device__ __forceinline__ PairMma(const PairParams& p, const uint8_t* sA, const uint8_t* sB, uint32_t rank) {
+        using namespace pair;
+        a_first = umma_smem_desc_sw128(smem_u32(sA), p.a_mn ? kBK * 128 : 0, 1024);
+        b_first = umma_smem_desc_sw128(smem_u32(sB), p.b_mn ? kBK * 128 : 0, 1024);
+        a_step = (p.a_mn ? kUmmaK * 128 : kUmmaK * 2) >> 4;
+        b_step = (p.b_mn ? kUmmaK * 128 : kUmmaK * 2) >> 4;
+        idesc = umma_idesc_bf16(kBM, BN, p.a_mn, p.b_mn);
+        pair_mask = static_cast<uint16_t>(3u << rank);
+        leader = elect_one();
+    }
+    // The live blocks of slot s into the accumulator; `started` is 0 before the first MMA of a tile, which overwrites it.
+    __device__ __forceinline__ void stage(uint32_t d_tmem, int s, uint32_t live, uint32_t& started, uint64_t* empty) {
+        using namespace pair;
+#pragma unroll
+        for (int b = 0; b < kPerStage; ++b) {
+            if (!(live >> b & 1)) continue;
+            const uint64_t adesc = a_first + static_cast<uint32_t>((s * kPerStage + b) * (kABytes >> 4));
+            const uint64_t bdesc = b_first + static_cast<uint32_t>((s * kPerStage + b) * (kBBytes<BN> >> 4));
+            if (leader) {
+#pragma unroll
+                for (int k = 0; k < kBK / kUmmaK; ++k)
+                    umma_f16_ss_pair(d_tmem, adesc + k * a_step, bdesc + k * b_step, idesc, k == 0 ? started : 1u);
+            }
+            started = 1;
+        }
+        if (leader) umma_commit_pair(empty, pair_mask);
+    }
+};
+
+template <int BN>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair::kThreads, 1)
+gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                 const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmR, const PairParams p) {
+    using namespace pair;
+    constexpr int STAGES = kStages<BN>;
+    constexpr int HALF = BN / 2;          // columns of the tile one epilogue warp drains; rows of B one CTA loads
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    uint8_t* sA = smem;
+    uint8_t* sB = smem + STAGES * kPerStage * kABytes;
+    uint8_t* sE = smem + STAGES * kPerStage * kBlock<BN>;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sE + kEpiWarps * kBox);
+    uint64_t* full = bars;                      // [STAGES] used in the even CTA: both CTAs' operands of a stage have landed
+    uint64_t* empty = bars + STAGES;            // [STAGES] in each CTA: the MMAs that read the stage are done
+    uint64_t* tmem_full = bars + 2 * STAGES;    // [2] in each CTA
+    uint64_t* tmem_empty = tmem_full + 2;       // [2] used in the even CTA: both CTAs' epilogue warps have read the accumulator
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty + 2);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+    const int warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
+    const uint32_t rank = cluster_ctarank();
+
+    if (warp == 0) {
+        // one barrier per lane: in turn they took as long as the TMEM allocation next door
+        if (lane < 2 * STAGES + 2) mbar_init(&bars[lane], 1);
+        else if (lane < 2 * STAGES + 4) mbar_init(&bars[lane], 2 * kEpiWarps);
+        if (lane == 31) *abort_flag = 0;
+        mbar_fence_init();
+    } else if (warp == 2 && lane == 0) {
+        tma_prefetch_desc(&tmA);
+        tma_prefetch_desc(&tmB);
+        tma_prefetch_desc(&tmC);
+    }
+    if (warp == 1) {
+        tmem_alloc_pair(tmem_slot, 2 * BN);
+        tmem_relinquish_pair();
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync();      // the other CTA's barriers are initialised before anything arrives on them
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+
+    const int num_tiles = p.tiles_m * p.tiles_n * p.groups;
+    const int num_kb = (p.K + kBK - 1) / kBK;
+    const int num_ks = (num_kb + kPerStage - 1) / kPerStage;
+    const int first = static_cast<int>(blockIdx.x >> 1), stride = static_cast<int>(gridDim.x >> 1);
+
+    if (warp == 0) {
+        if (lane == 0) {
+            // ---------------- TMA producer (both CTAs)
+            int s = 0;
+            uint32_t ph = 0;
+            bool ok = true;
+            for (int tile = first; tile < num_tiles && ok; tile += stride) {
+                int tm, tn, grp;
+                pair_tile_coords(p, tile, tm, tn, grp);
+                if (p.seg_mode == 1 && !pair_half_live(p, grp, tm * kBM) && !pair_half_live(p, grp, tm * kBM + 128)) continue;
+                const int m0 = tm * kBM + static_cast<int>(rank) * 128;
+                // SwiGLU: the even CTA brings the gate rows of the weight, the odd one the up rows of the same features
+                const int n0 = p.epi == CAI_EPI_SWIGLU ? tn * HALF + static_cast<int>(rank) * (p.N >> 1) : tn * BN + static_cast<int>(rank) * HALF;
+                for (int ks = 0; ks < num_ks; ++ks) {
+                    const uint32_t live = pair_live_blocks(p, grp, ks, num_kb);
+                    if (!live) continue;
+                    if (!mbar_wait(&empty[s], ph ^ 1, abort_flag, p.status, CAI_DEV_TIMEOUT_TMA_EMPTY)) {
+                        ok = false;
+                        break;
+                    }
+                    if (rank == 0) mbar_expect_tx(&full[s], 2 * kBlock<BN> * __popc(live));
+                    const uint32_t bar = map_to_cta(smem_u32(&full[s]), 0);
+                    pair_load_stage<BN>(&tmA, &tmB, sA + s * kPerStage * kABytes, sB + s * kPerStage * kBBytes<BN>, bar, p, ks, live, m0, n0, grp);
+                    if (++s == STAGES) {
+                        s = 0;
+                        ph ^= 1;
+                    }
+                }
+            }
+            if (ok) {
+                // every stage has been handed back: no arrival of the other CTA is still on its way when this CTA ends
+                for (int i = 0; i < STAGES && ok; ++i) {
+                    ok = mbar_wait(&empty[s], ph ^ 1, abort_flag, p.status, CAI_DEV_TIMEOUT_TMA_EMPTY);
+                    if (++s == STAGES) {
+                        s = 0;
+                        ph ^= 1;
+                    }
+                }
+            }
+            if (!ok) {
+                // Give copies still in flight time to land before the CTA's memory is released.
+                for (int i = 0; i < 32; ++i) __nanosleep(50000);
+            }
+        }
+    } else if (warp == 1) {
+        if (rank == 0) {
+            // ---------------- MMA issuer (even CTA)
+            PairMma<BN> mma(p, sA, sB, 0);
+            int s = 0;
+            uint32_t ph = 0;
+            bool ok = true;
+            int t = 0;
+            for (int tile = first; tile < num_tiles && ok; tile += stride) {
+                int grp = 0;
+                if (p.seg_mode) {
+                    int tm, tn;
+                    pair_tile_coords(p, tile, tm, tn, grp);
+                    if (p.seg_mode == 1 && !pair_half_live(p, grp, tm * kBM) && !pair_half_live(p, grp, tm * kBM + 128)) continue;
+                }
+                const int acc = t & 1;
+                const uint32_t acc_ph = (t >> 1) & 1;
+                ++t;
+                if (!mbar_wait_warp(&tmem_empty[acc], acc_ph ^ 1, abort_flag, p.status, CAI_DEV_TIMEOUT_TMEM_EMPTY)) {
+                    ok = false;
+                    break;
+                }
+                tc_fence_after();
+                const uint32_t d_tmem = tmem_base + acc * BN;
+                uint32_t started = 0;   // 0 for the first MMA of a tile, which overwrites the accumulator
+                for (int ks = 0; ks < num_ks; ++ks) {
+                    const uint32_t live = pair_live_blocks(p, grp, ks, num_kb);
+                    if (!live) continue;
+                    if (!mbar_wait_warp(&full[s], ph, abort_flag, p.status, CAI_DEV_TIMEOUT_TMA_FULL)) {
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after();
+                    mma.stage(d_tmem, s, live, started, &empty[s]);
+                    if (++s == STAGES) {
+                        s = 0;
+                        ph ^= 1;
+                    }
+                }
+                if (ok && mma.leader) umma_commit_pair(&tmem_full[acc], mma.pair_mask);
+            }
+        }
+    } else {
+        // ---------------- epilogue warps: TMEM -> registers -> shared memory -> TMA
+        const int q = warp & 3;              // TMEM lane quarter this warp may read
+        const int half = (warp - 2) >> 2;    // which half of the tile's columns
+        const int we = warp - 2;
+        uint8_t* box = sE + we * kBox;
+        const uint32_t box_row = smem_u32(box) + lane * 128;
+        const uint32_t sw = static_cast<uint32_t>(lane & 7);
+        const uint32_t lane_bits = static_cast<uint32_t>(q * 32) << 16;
+        const uint32_t release[2] = {map_to_cta(smem_u32(&tmem_empty[0]), 0), map_to_cta(smem_u32(&tmem_empty[1]), 0)};
+        int t = 0;
+        bool ok = true;
+        for (int tile = first; tile < num_tiles && ok; tile += stride) {
+            int tm, tn, grp;
+            pair_tile_coords(p, tile, tm, tn, grp);
+            const int half0 = tm * kBM + static_cast<int>(rank) * 128;
+            const bool mine = pair_half_live(p, grp, half0);
+            if (p.seg_mode == 1 && !mine && !pair_half_live(p, grp, tm * kBM + (1 - static_cast<int>(rank)) * 128)) continue;
+            const int acc = t & 1;
+            const uint32_t acc_ph = (t >> 1) & 1;
+            ++t;
+            // a weight-gradient tile whose every k-block was skipped has an undefined accumulator: it counts as zero
+            bool acc_valid = true;
+            if (p.seg_mode == 2) {
+                acc_valid = false;
+                for (int kb = 0; kb < num_kb && !acc_valid; ++kb) acc_valid = pair_seg_live(p, grp, kb * kBK);
+            }
+            const int row0 = half0 + q * 32;
+            const bool live = mine && row0 < p.M;
+            const int col_first = tn * BN + half * HALF;
+            const bool residual = p.epi == CAI_EPI_BF16_RESIDUAL;
+            // this lane's row of the residual: the first 64 columns come in while the main loop runs
+            const bool res_ok = residual && mine && row0 + lane < p.M;
+            const __nv_bfloat16* rrow = p.R + (static_cast<long long>(grp) * p.grp_c + row0 + lane) * p.ldr;
+            uint4 res[8];
+            auto fetch = [&](int col) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    if (res_ok && col + j * 8 < p.N) res[j] = *reinterpret_cast<const uint4*>(rrow + col + j * 8);
+            };
+            if (residual) fetch(col_first);
+            if (!mbar_wait_warp(&tmem_full[acc], acc_ph, abort_flag, p.status, CAI_DEV_TIMEOUT_TMEM_FULL)) {
+                ok = false;
+                break;
+            }
+            tc_fence_after();
+            const uint32_t tacc = tmem_base + lane_bits + acc * BN;
+            if (live) {
+                if (p.epi == CAI_EPI_SWIGLU) {
+                    // columns [0, HALF) are gate, [HALF, BN) up, of features tn * HALF ...; this warp's share is HALF / 2 of each
+                    const int F = p.N >> 1;
+#pragma unroll 1
+                    for (int c = 0; c < HALF / 2; c += 64) {
+                        uint32_t g[32], u[32], a[32];
+                        const int f0 = half * (HALF / 2) + c, j = tn * HALF + f0;
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            uint32_t rg[32], ru[32];
+                            tmem_ld_32x32(tacc + f0 + h * 32, rg);
+                            tmem_ld_32x32(tacc + HALF + f0 + h * 32, ru);
+                            tmem_ld_wait();
+#pragma unroll
+                            for (int e = 0; e < 16; ++e) {
+                                // round to bf16 first: the activation is computed from the values the backward will read
+                                const uint32_t pg = pack_bf16(__uint_as_float(rg[2 * e]) * p.alpha, __uint_as_float(rg[2 * e + 1]) * p.alpha);
+                                const uint32_t pu = pack_bf16(__uint_as_float(ru[2 * e]) * p.alpha, __uint_as_float(ru[2 * e + 1]) * p.alpha);
+                                const float g0 = bf16_lo(pg), g1 = bf16_hi(pg), u0 = bf16_lo(pu), u1 = bf16_hi(pu);
+                                g[h * 16 + e] = pg;
+                                u[h * 16 + e] = pu;
+                                a[h * 16 + e] = pack_bf16(g0 * (1.f / (1.f + __expf(-g0))) * u0, g1 * (1.f / (1.f + __expf(-g1))) * u1);
+                            }
+                        }
+                        if (j >= F) continue;
+#pragma unroll
+                        for (int o = 0; o < 3; ++o) {
+                            const uint32_t* v = o == 0 ? g : o == 1 ? u : a;
+                            if (lane == 0) tma_store_wait_read0();
+                            __syncwarp();
+#pragma unroll
+                            for (int k = 0; k < 8; ++k)
+                                st_shared_v4(box_row + ((k ^ sw) << 4), v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+                            fence_proxy_async_smem();
+                            __syncwarp();
+                            if (lane == 0) {
+                                if (o == 2) tma_store_3d(&tmR, box, j, row0, grp);
+                                else tma_store_3d(&tmC, box, o == 0 ? j : F + j, row0, grp);
+                                tma_store_commit();
+                            }
+                        }
+                    }
+                } else if (p.epi == CAI_EPI_BF16 || residual) {
+#pragma unroll 1
+                    for (int c = 0; c < HALF; c += 64) {
+                        const int col = col_first + c;
+                        if (col >= p.N) break;
+                        uint32_t r[2][32];
+                        tmem_ld_32x32(tacc + half * HALF + c, r[0]);
+                        tmem_ld_32x32(tacc + half * HALF + c + 32, r[1]);
+                        tmem_ld_wait();
+                        if (!acc_valid) {
+#pragma unroll
+                            for (int e = 0; e < 32; ++e) r[0][e] = r[1][e] = 0u;
+                        }
+                        if (lane == 0) tma_store_wait_read0();
+                        __syncwarp();
+#pragma unroll
+                        for (int k = 0; k < 8; ++k) {
+                            float v[8];
+#pragma unroll
+                            for (int e = 0; e < 8; ++e) v[e] = __uint_as_float(r[k >> 2][(k & 3) * 8 + e]) * p.alpha;
+                            const uint32_t at = box_row + ((k ^ sw) << 4);
+                            if (residual) {
+                                const uint4 rv = res[k];
+                                v[0] += bf16_lo(rv.x); v[1] += bf16_hi(rv.x);
+                                v[2] += bf16_lo(rv.y); v[3] += bf16_hi(rv.y);
+                                v[4] += bf16_lo(rv.z); v[5] += bf16_hi(rv.z);
+                                v[6] += bf16_lo(rv.w); v[7] += bf16_hi(rv.w);
+                            }
+                            st_shared_v4(at, pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
+                        }
+                        if (residual && c + 64 < HALF) fetch(col + 64);
+                        fence_proxy_async_smem();
+                        __syncwarp();
+                        if (lane == 0) {
+                            tma_store_3d(&tmC, box, col, row0, grp);
+                            tma_store_commit();
+                        }
+                    }
+                } else {
+                    const bool accum = p.epi == CAI_EPI_F32_ACCUM;
+#pragma unroll 1
+                    for (int c = 0; c < HALF; c += 32) {
+                        const int col = col_first + c;
+                        if (col >= p.N) break;
+                        uint32_t r[32];
+                        tmem_ld_32x32(tacc + half * HALF + c, r);
+                        tmem_ld_wait();
+                        if (lane == 0) tma_store_wait_read0();
+                        __syncwarp();
+#pragma unroll
+                        for (int k = 0; k < 8; ++k) {
+                            uint32_t v[4];
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) v[e] = acc_valid ? __float_as_uint(__uint_as_float(r[4 * k + e]) * p.alpha) : 0u;
+                            st_shared_v4(box_row + ((k ^ sw) << 4), v[0], v[1], v[2], v[3]);
+                        }
+                        fence_proxy_async_smem();
+                        __syncwarp();
+                        if (lane == 0) {
+                            if (accum) tma_reduce_add_3d(&tmC, box, col, row0, grp);
+                            else tma_store_3d(&tmC, box, col, row0, grp);
+                            tma_store_commit();
+                        }
+                    }
+                }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(release[acc]);
+        }
+        if (lane == 0) tma_store_wait0();
+    }
+
+    tc_fence_before();
+    __syncthreads();
+    __syncwarp();
+    cluster_sync();
+    if (warp == 1) {
+        tc_fence_after();
+        tmem_dealloc_pair(tmem_base, 2 * BN);
+    }
+}
+
+// ---------------------------------------------------------------------------- split along K
+// Few output tiles (short batches, the weight gradients of narrow layers): S pairs, one cluster of 2 S CTAs, share a 256 x 128
+// tile, each taking a slice of K. What bounds such a product is how fast one SM can be fed: a CTA of this tile takes in 48 KB
+// per 128 k-elements at about 54 B / cycle, twice as long as the MMAs need. The partial accumulators meet in shared memory:
+// every CTA leaves its 128 x 128 fp32 partial in its own (the operand ring is free by then), and after a cluster barrier each
+// adds up, always in the order of the slices, a 128 / S column slab of all partials of its rows through distributed shared
+// memory and writes it. No workspace, no atomics, the same result in every run.
+namespace pair {
+constexpr int kSplitBN = 128;
+constexpr int kSplitSmem = kStages<kSplitBN> * kPerStage * kBlock<kSplitBN> + 512 + 1024;
+}  // namespace pair
+
+template <int S>
+__global__ void __launch_bounds__(pair::kThreads, 1)
+gemm_pair_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const PairParams p) {
+    using namespace pair;
+    constexpr int BN = kSplitBN, STAGES = kStages<BN>, HALF = BN / 2;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    uint8_t* sA = smem;
+    uint8_t* sB = smem + STAGES * kPerStage * kABytes;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * kPerStage * kBlock<BN>);
+    uint64_t* full = bars;
+    uint64_t* empty = bars + STAGES;
+    uint64_t* tmem_full = bars + 2 * STAGES;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_full + 1);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t rank = cluster_ctarank();
+    const uint32_t even = rank & ~1u;          // the CTA of my pair that issues
+    const int slice = static_cast<int>(rank >> 1), side = static_cast<int>(rank & 1);
+
+    if (warp == 0) {
+        if (lane < 2 * STAGES + 1) mbar_init(&bars[lane], 1);
+        if (lane == 31) *abort_flag = 0;
+        mbar_fence_init();
+    } else if (warp == 2 && lane == 0) {
+        tma_prefetch_desc(&tmA);
+        tma_prefetch_desc(&tmB);
+    }
+    if (warp == 1) {
+        tmem_alloc_pair(tmem_slot, BN);
+        tmem_relinquish_pair();
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync();
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+
+    int tm, tn, grp;
+    pair_tile_coords(p, static_cast<int>(blockIdx.x) / (2 * S), tm, tn, grp);
+    const int num_kb = (p.K + kBK - 1) / kBK;
+    const int num_ks = (num_kb + kPerStage - 1) / kPerStage;
+    const int ks0 = num_ks * slice / S, ks1 = num_ks * (slice + 1) / S;
+    const int row_half = tm * kBM + side * 128;
+
+    if (warp == 0) {
+        if (lane == 0) {
+            // ---------------- TMA producer
+            int s = 0;
+            uint32_t ph = 0;
+            bool ok = true;
+            const uint32_t full0 = map_to_cta(smem_u32(full), even);
+            for (int ks = ks0; ks < ks1; ++ks) {
+                const uint32_t live = pair_live_blocks(p, grp, ks, num_kb);
+                if (!mbar_wait(&empty[s], ph ^ 1, abort_flag, p.status, CAI_DEV_TIMEOUT_TMA_EMPTY)) {
+                    ok = false;
+                    break;
+                }
+                if (side == 0) mbar_expect_tx(&full[s], 2 * kBlock<BN> * __popc(live));
+                pair_load_stage<BN>(&tmA, &tmB, sA + s * kPerStage * kABytes, sB + s * kPerStage * kBBytes<BN>, full0 + s * 8, p, ks, live,
+                                    row_half, tn * BN + side * HALF, grp);
+                if (++s == STAGES) {
+                    s = 0;
+                    ph ^= 1;
+                }
+            }
+            // every stage handed back: no arrival is still on its way when the CTA ends
+            for (int i = 0; i < STAGES && ok; ++i) {
+                ok = mbar_wait(&empty[s], ph ^ 1, abort_flag, p.status, CAI_DEV_TIMEOUT_TMA_EMPTY);
+                if (++s == STAGES) {
+                    s = 0;
+                    ph ^= 1;
+                }
+            }
+            if (!ok)
+                for (int i = 0; i < 32; ++i) __nanosleep(50000);   // let copies in flight land
+        }
+    } else if (warp == 1) {
+        if (side == 0) {
+            // ---------------- MMA issuer (even CTA of each pair)
+            PairMma<BN> mma(p, sA, sB, even);
+            int s = 0;
+            uint32_t ph = 0, started = 0;
+            bool ok = true;
+            for (int ks = ks0; ks < ks1; ++ks) {
+                const uint32_t live = pair_live_blocks(p, grp, ks, num_kb);
+                if (!mbar_wait_warp(&full[s], ph, abort_flag, p.status, CAI_DEV_TIMEOUT_TMA_FULL)) {
+                    ok = false;
+                    break;
+                }
+                tc_fence_after();
+                mma.stage(tmem_base, s, live, started, &empty[s]);
+                if (++s == STAGES) {
+                    s = 0;
+                    ph ^= 1;
+                }
+            }
+            if (ok && mma.leader) umma_commit_pair(tmem_full, mma.pair_mask);
+        }
+    } else if (row_half < p.M) {
+        // ---------------- partial accumulator -> shared memory: row r, 16-byte chunk c at r * 512 + (c ^ (r & 7)) * 16
+        const int q = warp & 3, half = (warp - 2) >> 2;
+        const uint32_t dst = smem_u32(smem) + (q * 32 + lane) * (BN * 4);
+        const uint32_t tacc = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + half * HALF;
+        if (mbar_wait_warp(tmem_full, 0, abort_flag, p.status, CAI_DEV_TIMEOUT_TMEM_FULL)) {
+            tc_fence_after();
+            uint32_t r[2][32];
+            tmem_ld_32x32(tacc, r[0]);
+            tmem_ld_32x32(tacc + 32, r[1]);
+            tmem_ld_wait();
+#pragma unroll
+            for (int c = 0; c < HALF / 4; ++c)
+                st_shared_v4(dst + (((half * (HALF / 4) + c) ^ (lane & 7)) << 4), r[c >> 3][(c & 7) * 4], r[c >> 3][(c & 7) * 4 + 1],
+                             r[c >> 3][(c & 7) * 4 + 2], r[c >> 3][(c & 7) * 4 + 3]);
+        }
+    }
+    tc_fence_before();
+    __syncwarp();
+    cluster_sync_memory();     // every partial of the cluster is in place
+    if (row_half < p.M && !*abort_flag) {
+        constexpr int W = BN / S / 4;          // 16-byte chunks of my slab per row
+        const int col0 = tn * BN + slice * (BN / S);
+        uint32_t src[S];
+#pragma unroll
+        for (int i = 0; i < S; ++i) src[i] = map_to_cta(smem_u32(smem), 2 * i + side);
+#pragma unroll 2
+        for (int it = threadIdx.x; it < 128 * W; it += kThreads) {
+            const int r = it / W, c = it % W;
+            const int row_in = row_half + r, col = col0 + c * 4;
+            const uint32_t at = r * (BN * 4) + (((slice * W + c) ^ (r & 7)) << 4);
+            float4 part[S];
+#pragma unroll
+            for (int i = 0; i < S; ++i) part[i] = ld_cluster_f4(src[i] + at);
+            if (row_in >= p.M || col >= p.N) continue;
+            float4 v = part[0];
+#pragma unroll
+            for (int i = 1; i < S; ++i) {
+                v.x += part[i].x; v.y += part[i].y; v.z += part[i].z; v.w += part[i].w;
+            }
+            v.x *= p.alpha; v.y *= p.alpha; v.z *= p.alpha; v.w *= p.alpha;
+            const long long row = row_in + static_cast<long long>(grp) * p.grp_c;
+            if (p.epi == CAI_EPI_F32 || p.epi == CAI_EPI_F32_ACCUM) {
+                float4* dst = reinterpret_cast<float4*>(static_cast<float*>(p.C) + row * p.ldc + col);
+                if (p.epi == CAI_EPI_F32_ACCUM) {
+                    const float4 old = *dst;
+                    v.x += old.x; v.y += old.y; v.z += old.z; v.w += old.w;
+                }
+                *dst = v;
+            } else {
+                if (p.epi == CAI_EPI_BF16_RESIDUAL) {
+                    const uint2 rv = *reinterpret_cast<const uint2*>(p.R + row * p.ldr + col);
+                    v.x += bf16_lo(rv.x); v.y += bf16_hi(rv.x); v.z += bf16_lo(rv.y); v.w += bf16_hi(rv.y);
+                }
+                *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(p.C) + row * p.ldc + col) = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
+            }
+        }
+    }
+    __syncwarp();
+    cluster_sync();            // nobody leaves while another CTA may still read its partial
+    if (warp == 1) {
+        tc_fence_after();
+        tmem_dealloc_pair(tmem_base, BN);
+    }
+}
+
+template <int S>
+static void split_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, unsigned grid, cudaStream_t st) {
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(pair::kThreads);
+    cfg.dynamicSmemBytes = pair::kSplitSmem;
+    cfg.stream = st;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2 * S;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+}
+
+// Tensor map of rows x cols per group, the groups `apart` rows apart.
+static bool pair_map(CUtensorMap* m, const GemmShape& g, const void* base, int rows, int cols, long long ld, long long apart, int box_cols,
+                     int box_rows, int bytes) {
+    return encode_tmap_3d(m, base, cols, rows, g.groups, ld, (g.groups > 1 ? apart : rows) * ld, box_cols, box_rows, bytes);
+}
+static bool pair_operand_maps(CUtensorMap* tmA, CUtensorMap* tmB, const void* A, const void* B, const GemmShape& g, int bn) {
+    const bool ok = !g.a_mn ? pair_map(tmA, g, A, g.M, g.K, g.lda, g.grp_a, 64, 128, 2) : pair_map(tmA, g, A, g.K, g.M, g.lda, g.grp_a, 64, pair::kBK, 2);
+    return ok && (!g.b_mn ? pair_map(tmB, g, B, g.N, g.K, g.ldb, g.grp_b, 64, bn / 2, 2)
+                          : pair_map(tmB, g, B, g.K, g.N, g.ldb, g.grp_b, 64, pair::kBK, 2));
+}
+
+// Split clusters of S pairs the device can hold at once (0: this form cannot run there).
+template <int S>
+static int split_clusters(int dev) {
+    static int count[64];   // value + 1, 0 = not asked yet
+    if (dev < 0 || dev >= 64) return 0;
+    if (!count[dev]) {
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute attr[1];
+        split_config<S>(cfg, attr, 2 * S, nullptr);
+        int n = 0;
+        if (cudaFuncSetAttribute(gemm_pair_split_kernel<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, pair::kSplitSmem) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&n, gemm_pair_split_kernel<S>, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            n = 0;
+        }
+        count[dev] = n + 1;
+    }
+    return count[dev] - 1;
+}
+
+template <int S>
+static int launch_split(const void* A, const void* B, const GemmShape& g, PairParams& p, cudaStream_t st) {
+    constexpr int BN = pair::kSplitBN;
+    CUtensorMap tmA, tmB;
+    if (!pair_operand_maps(&tmA, &tmB, A, B, g, BN)) return CAI_K_BAD_ARG;
+    p.tiles_m = (p.M + pair::kBM - 1) / pair::kBM;
+    p.tiles_n = (p.N + BN - 1) / BN;
+    p.group_m = 8;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    split_config<S>(cfg, attr, static_cast<unsigned>(2 * S * p.tiles_m * p.tiles_n * p.groups), st);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_pair_split_kernel<S>, tmA, tmB, p);
+    if (e != cudaSuccess) {
+        set_last_error("gemm_pair_split launch failed: %s", cudaGetErrorString(e));
+        return CAI_K_CUDA;
+    }
+    return CAI_K_OK;
+}
+
+template <int BN>
+static int launch_pair(const void* A, const void* B, const GemmShape& g, PairParams& p, int pairs, cudaStream_t st) {
+    CUtensorMap tmA, tmB, tmC, tmR;
+    bool ok = pair_operand_maps(&tmA, &tmB, A, B, g, BN);
+    const bool f32 = p.epi == CAI_EPI_F32 || p.epi == CAI_EPI_F32_ACCUM;
+    ok = ok && pair_map(&tmC, g, g.C, p.M, p.N, g.ldc, g.grp_c, f32 ? 32 : 64, 32, f32 ? 4 : 2);
+    tmR = tmC;
+    if (ok && p.epi == CAI_EPI_SWIGLU) ok = pair_map(&tmR, g, g.R, p.M, p.N / 2, g.ldr, g.grp_c, 64, 32, 2);
+    if (!ok) return CAI_K_BAD_ARG;
+    static bool configured[64] = {};
+    const int dev = current_device();
+    if (!configured[dev & 63]) {
+        if (cudaFuncSetAttribute(gemm_pair_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, pair::kSmem<BN>) != cudaSuccess) {
+            set_last_error("cudaFuncSetAttribute(gemm_pair) failed: %s", cudaGetErrorString(cudaGetLastError()));
+            return CAI_K_CUDA;
+        }
+        configured[dev & 63] = true;
+    }
+    p.tiles_m = (p.M + pair::kBM - 1) / pair::kBM;
+    p.tiles_n = (p.N + BN - 1) / BN;
+    p.group_m = 8;
+    const int tiles = p.tiles_m * p.tiles_n * p.groups;
+    const int grid = 2 * (tiles < pairs ? tiles : pairs);
+    gemm_pair_kernel<BN><<<grid, pair::kThreads, pair::kSmem<BN>, st>>>(tmA, tmB, tmC, tmR, p);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) {
+        set_last_error("gemm_pair launch failed: %s", cudaGetErrorString(e));
+        return CAI_K_CUDA;
+    }
+    return CAI_K_OK;
+}
+
+int gemm_pair(const void* A, const void* B, const GemmShape& g, cudaStream_t st) {
+    PairParams p;
+    p.M = g.M; p.N = g.N; p.K = g.K;
+    p.a_mn = g.a_mn; p.b_mn = g.b_mn;
+    p.epi = g.epi; p.alpha = g.alpha;
+    p.groups = g.groups;
+    p.seg_counts = g.seg_counts; p.seg_rows = g.seg_rows; p.seg_mode = g.seg_mode; p.grp_seg = g.grp_seg;
+    p.C = g.C;
+    p.R = static_cast<const __nv_bfloat16*>(g.R);
+    p.ldc = g.ldc; p.ldr = g.ldr; p.grp_c = g.grp_c;
+    const int dev = current_device();
+    p.status = status_words(dev);
+    const int pairs = sm_count(dev) / 2;
+    const int usable = g.sm_limit > 1 && g.sm_limit / 2 < pairs ? g.sm_limit / 2 : pairs;
+    // Which form: the smallest estimate in SM cycles. A stage of 128 k-elements takes a CTA about 1150 cycles in the 256-wide
+    // tile (1024 of MMA) and 850 in the 128-wide one (48 KB at 54 B / cycle; 512 of MMA); a wave of tiles adds the part of its
+    // epilogue that nothing hides, the split form the exchange of its partials. Measured, 256-wide / 128-wide / 2 / 4 slices:
+    // 3840 x 1000 x 2728 29.0 / 35.4 / 55.2 / 80.6 us, 333 x 3000 x 1024 16.6 / 12.5 / 18.8 / 27.0 us, 333 x 1024 x 3000
+    // 20.7 / 18.6 / 14.5 / 16.6 us (one-CTA kernel: 39.7, 16.2, 24.7 us). The rule looks at the shape only, so that a limit on the
+    // SMs does not change the order of summation.
+    const long long ks = (g.K + 127) / 128, tm = (g.M + pair::kBM - 1) / pair::kBM;
+    const long long t256 = tm * ((g.N + 255) / 256) * g.groups, t128 = tm * ((g.N + 127) / 128) * g.groups;
+    const double wide = static_cast<double>((t256 + pairs - 1) / pairs) * (ks * 1150.0 + 2500.0);
+    const double narrow = static_cast<double>((t128 + pairs - 1) / pairs) * (ks * 850.0 + 1500.0);
+    if (p.epi != CAI_EPI_SWIGLU && !p.seg_mode) {
+        // clusters of 4 and 8 that fit at once (33 and 15 on a GPU whose 148 SMs sit in groups of 16 to 20)
+        const bool fits2 = ks >= 2 && t128 <= split_clusters<2>(dev), fits4 = ks >= 4 && t128 <= split_clusters<4>(dev);
+        const double two = fits2 ? (ks + 1) / 2 * 850.0 + 4500.0 : 1e30, four = fits4 ? (ks + 3) / 4 * 850.0 + 4500.0 : 1e30;
+        if (four < two && four < wide && four < narrow) return launch_split<4>(A, B, g, p, st);
+        if (two < wide && two < narrow) return launch_split<2>(A, B, g, p, st);
+    }
+    if (p.epi == CAI_EPI_SWIGLU || wide <= narrow) return launch_pair<256>(A, B, g, p, usable, st);
+    return launch_pair<128>(A, B, g, p, usable, st);
+}
+
+}  // namespace cai

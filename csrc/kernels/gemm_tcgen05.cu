@@ -20,6 +20,7 @@
 #include "../comm/peer.cuh"
 #include "../plan/formats.h"
 #include "cai_kernels.h"
+#include "gemm_common.h"
 #include "host_common.h"
 #include "sm100.cuh"
 
@@ -878,6 +879,25 @@ static int gemm_dispatch(const void* A, const void* B, long long lda, long long 
     return launch_gemm<128, 6, false>(tmA, tmB, tmA2, p, sms, st);
 }
 
+// The product as the other kernels' launchers take it.
+static GemmShape shape_of(const GemmParams& p, long long lda, long long ldb, int sm_limit) {
+    GemmShape g;
+    g.M = p.M; g.N = p.N; g.K = p.K;
+    g.a_mn = p.a_mn; g.b_mn = p.b_mn;
+    g.epi = p.epi; g.alpha = p.alpha;
+    g.C = p.C; g.R = p.R;
+    g.lda = lda; g.ldb = ldb; g.ldc = p.ldc; g.ldr = p.ldr;
+    g.seg_counts = p.seg_counts; g.seg_rows = p.seg_rows; g.seg_mode = p.seg_mode; g.grp_seg = p.grp_seg;
+    g.groups = p.groups; g.grp_a = p.grp_a; g.grp_b = p.grp_b; g.grp_c = p.grp_c;
+    g.sm_limit = sm_limit;
+    return g;
+}
+// Plain products (no collective in the kernel) run on CTA pairs; the SwiGLU backward epilogue exists in this file only.
+static int gemm_plain(const void* A, const void* B, long long lda, long long ldb, GemmParams& p, int sm_limit, cudaStream_t st) {
+    if (p.epi == CAI_EPI_SWIGLU_BWD) return gemm_dispatch(A, B, lda, ldb, p, sm_limit, st);
+    return gemm_pair(A, B, shape_of(p, lda, ldb, sm_limit), st);
+}
+
 static void plain_params(GemmParams& p) {
     p.mode = kGemmPlain;
     p.group_kind = 0; p.n_copy = 0; p.rows_per_rank = 0; p.m_rot = 0;
@@ -940,7 +960,7 @@ CAI_API int cai_gemm_bf16_seg(const void* A, const void* B, void* C, const void*
     p.C = C; p.R = R;
     p.ldc = ldc; p.ldr = ldr;
     p.seg_counts = seg_counts; p.seg_rows = seg_rows; p.seg_mode = seg_mode;
-    return gemm_dispatch(A, B, lda, ldb, p, sm_limit, reinterpret_cast<cudaStream_t>(stream));
+    return gemm_plain(A, B, lda, ldb, p, sm_limit, reinterpret_cast<cudaStream_t>(stream));
 }
 
 CAI_API int cai_gemm_bf16_grouped(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
@@ -963,7 +983,7 @@ CAI_API int cai_gemm_bf16_grouped(const void* A, const void* B, void* C, int M, 
     p.C = C; p.ldc = ldc;
     p.seg_counts = seg_counts; p.seg_rows = seg_rows; p.seg_mode = seg_mode;
     p.groups = groups; p.grp_a = grp_a; p.grp_b = grp_b; p.grp_c = grp_c; p.grp_seg = grp_seg;
-    return gemm_dispatch(A, B, lda, ldb, p, 0, reinterpret_cast<cudaStream_t>(stream));
+    return gemm_plain(A, B, lda, ldb, p, 0, reinterpret_cast<cudaStream_t>(stream));
 }
 
 // y[T,N] = concat_rows(x_local of every member)[T,K] * op(B); also leaves the gathered rows in a_full.

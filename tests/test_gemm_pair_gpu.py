@@ -1,0 +1,52 @@
+"""GEMM on CTA pairs and its split along K: edges of the 256 x 256 / 256 x 128 tiles, of a stage and of the K slices."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+# M, N, K: one row, half tiles, one past a tile, K of a fraction of a block, of an odd number of blocks, fewer slices than
+# blocks; few tiles (split), one wave and several waves of tiles (persistent)
+SHAPES = [(1, 8, 8), (128, 128, 64), (129, 136, 72), (256, 256, 128), (257, 264, 1000), (333, 1024, 3000), (40, 3000, 512),
+          (1000, 1152, 3840), (513, 120, 4104), (4096, 5000, 200), (2500, 4104, 136)]
+
+
+@pytest.mark.parametrize("ta,tb", [(False, False), (False, True), (True, True), (True, False)])
+@pytest.mark.parametrize("M,N,K", SHAPES)
+def test_pair_gemm_edges(M, N, K, ta, tb):
+    from cai_b200 import ops
+    torch.manual_seed(0)
+    M = (M + 7) // 8 * 8 if ta else M                      # a contiguous M has to be a multiple of 8
+    a = torch.randn((K, M) if ta else (M, K), device="cuda").to(torch.bfloat16)
+    b = torch.randn((K, N) if tb else (N, K), device="cuda").to(torch.bfloat16)
+    A, B = (a.t() if ta else a).float(), (b if tb else b.t()).float()
+    ref = A @ B
+    # products of bf16 are exact in fp32; two sums of K terms in different orders differ by at most 2 K 2^-24 sum |a b|
+    bound = 2 * K * 2.0 ** -24 * (A.abs() @ B.abs()) + 1e-6
+    out = torch.full((M, N), 2.0, device="cuda")
+    ops.gemm(a, b, trans_a=ta, trans_b=tb, out=out, accumulate=True, alpha=0.5)
+    assert ((out - (2.0 + 0.5 * ref)).abs() <= bound + 2.0 ** -23 * (2.0 + ref.abs())).all()
+    wide = torch.full((M, N + 16), 7.0, device="cuda")     # a pitch wider than the row: nothing outside may be touched
+    ops.gemm(a, b, trans_a=ta, trans_b=tb, out=wide[:, :N])
+    assert ((wide[:, :N] - ref).abs() <= bound).all() and bool((wide[:, N:] == 7.0).all())
+    res = torch.randn(M, N, device="cuda").to(torch.bfloat16)
+    c = ops.gemm(a, b, trans_a=ta, trans_b=tb, residual=res)
+    want = ref + res.float()
+    assert ((c.float() - want).abs() <= bound + 2.0 ** -8 * want.abs() + 1e-6).all()    # and one rounding to bf16
+    assert torch.equal(c, ops.gemm(a, b, trans_a=ta, trans_b=tb, residual=res))         # the order of summation is fixed
+    from cai_b200.ops import _lib
+    assert _lib.device_status(clear=True) == 0
+
+
+@pytest.mark.parametrize("M,N", [(200, 72), (256, 136), (130, 256)])
+def test_pair_gemm_groups_do_not_touch_each_other(M, N):
+    """Group sizes that are no multiple of a tile or of the 32-row boxes: rows past a group belong to the next one."""
+    from cai_b200 import ops
+    torch.manual_seed(1)
+    G, K = 3, 192
+    a = torch.randn(G * M, K, device="cuda").to(torch.bfloat16)
+    b = torch.randn(G * N, K, device="cuda").to(torch.bfloat16)
+    out = torch.zeros(G * M, N, device="cuda")
+    ops.gemm_grouped(a, b, out, M, N, K, groups=G)
+    for g in range(G):
+        A, B = a[g * M:(g + 1) * M].float(), b[g * N:(g + 1) * N].float()
+        assert ((out[g * M:(g + 1) * M] - A @ B.t()).abs() <= 2 * K * 2.0 ** -24 * (A.abs() @ B.abs().t()) + 1e-6).all()
