@@ -14,17 +14,26 @@
 // both as a K-major operand (for the score products) and as an MN-major operand (for the
 // gradient products) through different UMMA descriptors, so nothing is transposed in memory.
 //
-// Roles per CTA: warp 0 issues TMA, warp 1 issues the MMAs, sixteen warps do the exponentials (four groups of four;
-// a warp owns 32 TMEM lanes, a group 32 of the step's 128 score columns). A thread turns 16 fp32 columns at a time
-// into 8 packed bf16 columns and writes them over the first half of what it has just read, so the groups never
-// touch each other's columns and need no barrier inside a step; the MMA reads its A operand in 8-column pieces,
-// 16 columns apart. Every warp arrives once (not every thread) on the barrier that releases the gradient MMAs. The
-// softmax scale is applied once to the finished dK / dQ, and only diagonal tiles run the code path with the mask.
-// Measured on a B200 (what shaped this layout): the issuing thread runs at most about one MMA ahead of the tensor
-// pipe, a barrier wait that is already satisfied still costs it 110-240 cycles because its shared-memory access
-// queues behind the operand reads of the MMAs, and 128 x 64 score products run at 58 cycles per MMA against 64 for
-// 128 x 128 ones; splitting a step into two 64-column half steps to overlap exponentials and MMAs therefore lost
-// to the plain 128-column step with more warps on the exponentials.
+// Roles per CTA: warp 0 issues TMA, warps 1 and 2 issue the MMAs, sixteen warps do the exponentials (four groups of
+// four; a warp owns 32 TMEM lanes, a group 32 of the step's 128 score columns). What bounds a step is the latency chain
+// of the compute warps, not the tensor pipe, so as little of that pipe's time as possible is left on the chain:
+//   dK / dV: S^T(i+1) is computed as soon as the warps hold the scores of step i in registers. P^T leaves through shared
+//            memory (in place of S^T it would hold up S^T(i+1) until dV(i) is done), before dP^T is looked at; dS^T goes
+//            over dP^T in TMEM. Warp 1 issues S^T and dV, warp 2 dP^T and dK.
+//   dQ:      warp 1 runs S ahead in two buffers, warp 2 alternates dP(j) and dQ(j).
+// Two issuing warps because a wait costs the issuing thread 110-300 cycles even when it is already satisfied (its
+// shared-memory access queues behind the operand reads of the MMAs): the other warp's MMAs run meanwhile. Each warp's MMAs
+// execute in the order of issue, which is what protects dP / dS (one overwrites the other); the two warps share no
+// operand that either writes. A thread keeps its 32 probabilities in fp32 registers until dP arrives. bf16 results in TMEM
+// go over the first half of the 32 columns they came from, so the groups never touch each other's columns and need
+// no barrier inside a step; a warp keeps the statistics of its queries in 32 words of its own. Every warp arrives once (not
+// every thread) on a barrier. The softmax scale is applied once to the finished dK / dQ, and only diagonal tiles run the
+// code path with the mask.
+// Measured on a B200, before (one step at a time: scores, exponentials, gradients) and now, both back to back on one GPU:
+// 8192 tokens, 32 / 8 heads: dK / dV 5390 -> 3700 cycles per 128 x 128 step and SM (1279 -> 1010 us: at 990 W the clock falls
+// from 1900 to 1640 MHz), dQ 4240 -> 3030 cycles (986 -> 800 us). 4096 tokens, 16 / 8 heads: 203 -> 140 and 170 -> 111 us.
+// P^T over S^T in TMEM, with S^T(i+1) behind dV(i): 8 % slower. Asking the barriers early without blocking, and fetching
+// the next scores before dS^T is handed over: 2-10 % slower.
 //
 // Replaces the reference's one-thread-per-query backward, which recomputes dp twice, scatters
 // dK/dV with atomicAdd and never zeroes dq/dk/dv (src/cuda/cai_kernels.cu:110-143).
@@ -84,7 +93,7 @@ __global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ out, const _
 // Sixteen compute warps: every scheduler has four of them to hide the TMEM and shared-memory latencies.
 constexpr int kAttnGroups = 4;
 constexpr int kAttnComputeThreads = kAttnGroups * 128;
-constexpr int kAttnBwdThreads = 128 + kAttnComputeThreads;  // warp 0 TMA, warp 1 MMA, warps 4-19 compute
+constexpr int kAttnBwdThreads = 128 + kAttnComputeThreads;  // warp 0 TMA, warps 1-2 MMA, warps 4-19 compute
 
 __device__ __forceinline__ void bar_sync_compute() { asm volatile("bar.sync 1, 512;" ::: "memory"); }
 
@@ -114,103 +123,90 @@ __device__ __forceinline__ void put_acc_chunk(uint32_t tacc, __nv_bfloat16* dst_
     }
 }
 
-// dK / dV work of one thread on 16 query columns: S^T / dP^T (dP^T `dp_off` columns behind S^T) -> P^T, dS^T
-// (unscaled) as bf16 over the first 8 of the 16 columns read.
-template <bool kDiag>
-__device__ __forceinline__ void dkdv_pass16(uint32_t tS, uint32_t dp_off, const float* L, const float* D,
-                                               float scale_log2, int r, int qb) {
-    const uint32_t tdP = tS + dp_off;
-    uint32_t sv[16], dp[16], pk[8], dk[8];
-    tmem_ld_32x16(tS, sv);
-    tmem_ld_32x16(tdP, dp);
-    const float4* L4 = reinterpret_cast<const float4*>(L);
-    const float4* D4 = reinterpret_cast<const float4*>(D);
-    float4 l[4], d[4];
+// Probabilities of one thread's 32 score columns, in place: exp2(s * scale_log2 - lse2). In the transposed form (dK / dV)
+// a column is a query with its own lse2; in the other (dQ) the thread's row is the query. One half (16 columns) per call.
+template <bool kDiag, int kHalf>
+__device__ __forceinline__ void prob_cols(uint32_t (&v)[32], const float4 (&ls)[4], float scale_log2, int r, int qb) {
 #pragma unroll
     for (int e4 = 0; e4 < 4; ++e4) {
-        l[e4] = L4[e4];
-        d[e4] = D4[e4];
-    }
-    tmem_ld_wait();
-#pragma unroll
-    for (int e4 = 0; e4 < 4; ++e4) {
-        const float ls[4] = {l[e4].x, l[e4].y, l[e4].z, l[e4].w}, ds[4] = {d[e4].x, d[e4].y, d[e4].z, d[e4].w};
-        float pr[4], dsv[4];
+        const float l[4] = {ls[e4].x, ls[e4].y, ls[e4].z, ls[e4].w};
 #pragma unroll
         for (int t = 0; t < 4; ++t) {
-            const int e = e4 * 4 + t;
-            float pv = fast_exp2(__uint_as_float(sv[e]) * scale_log2 - ls[t]);
+            const int e = kHalf * 16 + e4 * 4 + t;
+            float pv = fast_exp2(__uint_as_float(v[e]) * scale_log2 - l[t]);
             if constexpr (kDiag) {
                 if (r > qb + e) pv = 0.f;  // key (row r) may not lie after the query (column)
             }
-            pr[t] = pv;
-            dsv[t] = pv * (__uint_as_float(dp[e]) - ds[t]);
+            v[e] = __float_as_uint(pv);
         }
-        pk[e4 * 2] = pack_bf16(pr[0], pr[1]);
-        pk[e4 * 2 + 1] = pack_bf16(pr[2], pr[3]);
-        dk[e4 * 2] = pack_bf16(dsv[0], dsv[1]);
-        dk[e4 * 2 + 1] = pack_bf16(dsv[2], dsv[3]);
     }
-    tmem_st_32x8(tS, pk);
-    tmem_st_32x8(tdP, dk);
-    tmem_st_wait();
 }
-
-// dQ work of one thread on 16 key columns: S / dP (dP `dp_off` columns behind S) -> dS (unscaled) as bf16 over the
-// first 8 of the 16 dP columns read.
 template <bool kDiag>
-__device__ __forceinline__ void dq_pass16(uint32_t tS, uint32_t dp_off, float lse2, float dl, float scale_log2, int r,
-                                             int kb) {
-    const uint32_t tdP = tS + dp_off;
-    uint32_t sv[16], dp[16], dk[8];
-    tmem_ld_32x16(tS, sv);
-    tmem_ld_32x16(tdP, dp);
-    tmem_ld_wait();
+__device__ __forceinline__ void prob_rows(uint32_t (&v)[32], float lse2, float scale_log2, int r, int kb) {
 #pragma unroll
-    for (int e = 0; e < 16; e += 2) {
-        float p0 = fast_exp2(__uint_as_float(sv[e]) * scale_log2 - lse2);
-        float p1 = fast_exp2(__uint_as_float(sv[e + 1]) * scale_log2 - lse2);
+    for (int e = 0; e < 32; ++e) {
+        float pv = fast_exp2(__uint_as_float(v[e]) * scale_log2 - lse2);
         if constexpr (kDiag) {
-            if (kb + e > r) p0 = 0.f;
-            if (kb + e + 1 > r) p1 = 0.f;
+            if (kb + e > r) pv = 0.f;
         }
-        dk[e >> 1] = pack_bf16(p0 * (__uint_as_float(dp[e]) - dl), p1 * (__uint_as_float(dp[e + 1]) - dl));
+        v[e] = __float_as_uint(pv);
     }
-    tmem_st_32x8(tdP, dk);
-    tmem_st_wait();
 }
 
 // D[128,hd] (+)= A[128,128](TMEM, bf16 pairs) * B[128,hd] with B MN-major in two 16 KiB sub-tiles; the A operand sits in
-// eight pieces of 8 columns, 16 columns apart.
-__device__ __forceinline__ void issue_pv_g8(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_smem, uint32_t idesc,
-                                            bool accumulate) {
+// four pieces of 16 columns, 32 columns apart (each where one warp group read its 32 fp32 columns from).
+__device__ __forceinline__ void issue_pv_g16(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, bool accumulate) {
 #pragma unroll
-    for (int k = 0; k < kAttnTile / 16; ++k) {
-        umma_f16_ts(d_tmem, a_tmem + k * 16, umma_smem_desc_sw128(b_smem + k * 2048, kAttnSub, 1024), idesc,
-                    (accumulate || k > 0) ? 1u : 0u);
+    for (int k = 0; k < kAttnTile / 16; ++k)
+        umma_f16_ts(d_tmem, a_tmem + (k >> 1) * 32 + (k & 1) * 8, b_desc + k * (2048 >> 4), idesc, (accumulate || k > 0) ? 1u : 0u);
+}
+// S[128,128] = A[128,hd] * B[128,hd]^T, both K-major in two 64-column sub-tiles, from ready-made descriptors.
+__device__ __forceinline__ void issue_kk(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc) {
+#pragma unroll
+    for (int k = 0; k < kAttnHD / 16; ++k) {
+        const uint32_t off = ((k >> 2) * kAttnSub + (k & 3) * 32) >> 4;
+        umma_f16_ss(d_tmem, a_desc + off, b_desc + off, idesc, k > 0 ? 1u : 0u);
     }
 }
+// D[128,hd] (+)= A[128,128] * B[128,hd], both in shared memory: A K-major, B MN-major.
+__device__ __forceinline__ void issue_pd_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, bool accumulate) {
+#pragma unroll
+    for (int k = 0; k < kAttnTile / 16; ++k)
+        umma_f16_ss(d_tmem, a_desc + (((k >> 2) * kAttnSub + (k & 3) * 32) >> 4), b_desc + k * (2048 >> 4), idesc,
+                    (accumulate || k > 0) ? 1u : 0u);
+}
+constexpr uint32_t kTileDesc = kAttnTileBytes >> 4;   // descriptor distance of two tiles
 
-// ---------------------------------------------------------------------------- dK / dV, one 128 x 128 step in flight
+// ---------------------------------------------------------------------------- dK / dV
 __global__ void __launch_bounds__(kAttnBwdThreads, 1)
 attn_dkdv_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant__ CUtensorMap tm_do,
                  const AttnBwdParams p) {
-    extern __shared__ uint8_t smem_raw[];
-    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    // no room to round the base up: tiles start on swizzle boundaries only if the shared window does (checked)
+    extern __shared__ __align__(1024) uint8_t smem[];
+    if (smem_u32(smem) & 1023) {
+        if (threadIdx.x == 0) atomicCAS(p.status, 0, CAI_DEV_BAD_ARG);
+        return;
+    }
     uint8_t* sK = smem;
     uint8_t* sV = smem + kAttnTileBytes;
     uint8_t* sQ = smem + 2 * kAttnTileBytes;   // 2 stages
     uint8_t* sdO = smem + 4 * kAttnTileBytes;  // 2 stages
-    float* sL = reinterpret_cast<float*>(smem + 6 * kAttnTileBytes);  // [2][128] lse * log2e
-    float* sD = sL + 256;                                              // [2][128] delta
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sD + 256);
+    uint8_t* sP = smem + 6 * kAttnTileBytes;   // P^T, the A operand of dV
+    float* sStat = reinterpret_cast<float*>(smem + 7 * kAttnTileBytes);  // [16 warps][32] lse * log2e, later delta, of its columns
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sStat + kAttnComputeThreads);
     uint64_t* kv_full = bars;
-    uint64_t* qdo_full = bars + 1;
-    uint64_t* qdo_empty = bars + 3;
-    uint64_t* sdp_full = bars + 5;
-    uint64_t* pds_ready = bars + 6;
-    uint64_t* final_bar = bars + 7;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 8);
+    uint64_t* q_full = bars + 1;      // [2]
+    uint64_t* q_empty = bars + 3;     // [2] dK has read the tile (S^T long before)
+    uint64_t* do_full = bars + 5;     // [2]
+    uint64_t* do_empty = bars + 7;    // [2] dV and dP^T have read the tile
+    uint64_t* s_full = bars + 9;
+    uint64_t* s_empty = bars + 10;    // the compute warps have the scores in registers
+    uint64_t* dp_full = bars + 11;
+    uint64_t* p_ready = bars + 12;
+    uint64_t* p_free = bars + 13;     // dV has read P^T
+    uint64_t* ds_ready = bars + 14;
+    uint64_t* final_bar = bars + 15;  // both issuing warps' last MMAs
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -235,12 +231,18 @@ attn_dkdv_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
         tma_prefetch_desc(&tm_do);
         mbar_init(kv_full, 1);
         for (int i = 0; i < 2; ++i) {
-            mbar_init(&qdo_full[i], 1);
-            mbar_init(&qdo_empty[i], 1);
+            mbar_init(&q_full[i], 1);
+            mbar_init(&q_empty[i], 1);
+            mbar_init(&do_full[i], 1);
+            mbar_init(&do_empty[i], 2);
         }
-        mbar_init(sdp_full, 1);
-        mbar_init(pds_ready, kAttnComputeThreads / 32);
-        mbar_init(final_bar, 1);
+        mbar_init(s_full, 1);
+        mbar_init(s_empty, kAttnComputeThreads / 32);
+        mbar_init(dp_full, 1);
+        mbar_init(p_ready, kAttnComputeThreads / 32);
+        mbar_init(p_free, 1);
+        mbar_init(ds_ready, kAttnComputeThreads / 32);
+        mbar_init(final_bar, 2);
         *abort_flag = 0;
         mbar_fence_init();
     }
@@ -268,71 +270,163 @@ attn_dkdv_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
                 const uint32_t ph = (it >> 1) & 1;
                 const int h = h_first + it / per_head;
                 const int q_row = row_base + (j + it % per_head) * kAttnTile;
-                if (!mbar_wait(&qdo_empty[slot], ph ^ 1, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN)) { ok = false; break; }
-                mbar_expect_tx(&qdo_full[slot], 2 * kAttnTileBytes);
+                if (!mbar_wait(&q_empty[slot], ph ^ 1, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN)) { ok = false; break; }
+                mbar_expect_tx(&q_full[slot], kAttnTileBytes);
                 uint8_t* q = sQ + slot * kAttnTileBytes;
+                tma_load_2d(q, &tm_qkv, &q_full[slot], h * kAttnHD, q_row);
+                tma_load_2d(q + kAttnSub, &tm_qkv, &q_full[slot], h * kAttnHD + 64, q_row);
+                if (!mbar_wait(&do_empty[slot], ph ^ 1, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN)) { ok = false; break; }
+                mbar_expect_tx(&do_full[slot], kAttnTileBytes);
                 uint8_t* d = sdO + slot * kAttnTileBytes;
-                tma_load_2d(q, &tm_qkv, &qdo_full[slot], h * kAttnHD, q_row);
-                tma_load_2d(q + kAttnSub, &tm_qkv, &qdo_full[slot], h * kAttnHD + 64, q_row);
-                tma_load_2d(d, &tm_do, &qdo_full[slot], h * kAttnHD, q_row);
-                tma_load_2d(d + kAttnSub, &tm_do, &qdo_full[slot], h * kAttnHD + 64, q_row);
+                tma_load_2d(d, &tm_do, &do_full[slot], h * kAttnHD, q_row);
+                tma_load_2d(d + kAttnSub, &tm_do, &do_full[slot], h * kAttnHD + 64, q_row);
             }
             if (!ok)
                 for (int i = 0; i < 32; ++i) __nanosleep(50000);
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            const uint32_t idesc_kk = umma_idesc_bf16(128, 128, 0, 0);
-            const uint32_t idesc_mn = umma_idesc_bf16(128, 128, 0, 1);
-            const uint32_t aK = smem_u32(sK), aV = smem_u32(sV), aQ = smem_u32(sQ), aD = smem_u32(sdO);
-            bool ok = mbar_wait(kv_full, 0, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN);
-            for (int it = 0; it < iters && ok; ++it) {
+        // ---------------- S^T = K Q^T, a step ahead of the compute warps; dV += P^T dO. The whole warp walks the loop
+        // (descriptors in uniform registers).
+        const uint32_t idesc_kk = umma_idesc_bf16(128, 128, 0, 0), idesc_mn = umma_idesc_bf16(128, 128, 0, 1);
+        const uint64_t kd = umma_smem_desc_sw128(smem_u32(sK), 0, 1024), qd = umma_smem_desc_sw128(smem_u32(sQ), 0, 1024);
+        const uint64_t pd = umma_smem_desc_sw128(smem_u32(sP), 0, 1024), dod = umma_smem_desc_sw128(smem_u32(sdO), kAttnSub, 1024);
+        const bool leader = elect_one();
+        bool ok = mbar_wait_warp(kv_full, 0, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN);
+        for (int it = 0; it <= iters && ok; ++it) {
+            if (it < iters) {
                 const int slot = it & 1;
-                const uint32_t ph = (it >> 1) & 1;
-                if (!mbar_wait(&qdo_full[slot], ph, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN)) { ok = false; break; }
+                if (!mbar_wait_warp(s_empty, (it & 1) ^ 1, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN) ||
+                    !mbar_wait_warp(&q_full[slot], (it >> 1) & 1, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN)) { ok = false; break; }
                 tc_fence_after();
-                issue_qk(tS, aK, aQ + slot * kAttnTileBytes, idesc_kk);    // S^T  = K Q^T
-                issue_qk(tdP, aV, aD + slot * kAttnTileBytes, idesc_kk);   // dP^T = V dO^T
-                umma_commit(sdp_full);
-                if (!mbar_wait(pds_ready, it & 1, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN)) { ok = false; break; }
-                tc_fence_after();
-                issue_pv_g8(tdV, tS, aD + slot * kAttnTileBytes, idesc_mn, it > 0);   // dV += P^T dO
-                issue_pv_g8(tdK, tdP, aQ + slot * kAttnTileBytes, idesc_mn, it > 0);  // dK += dS^T Q (unscaled)
-                umma_commit(&qdo_empty[slot]);
+                if (leader) {
+                    issue_kk(tS, kd, qd + slot * kTileDesc, idesc_kk);
+                    umma_commit(s_full);
+                }
             }
-            if (ok) umma_commit(final_bar);
+            if (it > 0) {
+                const int slot = (it - 1) & 1;
+                if (!mbar_wait_warp(&do_full[slot], ((it - 1) >> 1) & 1, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN) ||
+                    !mbar_wait_warp(p_ready, (it - 1) & 1, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN)) { ok = false; break; }
+                tc_fence_after();
+                if (leader) {
+                    issue_pd_ss(tdV, pd, dod + slot * kTileDesc, idesc_mn, it > 1);
+                    umma_commit(p_free);
+                    umma_commit(&do_empty[slot]);
+                    if (it == iters) umma_commit(final_bar);
+                }
+            }
+        }
+    } else if (warp == 2) {
+        // ---------------- dP^T = V dO^T, dK += dS^T Q (unscaled). dK(i) comes after S^T(i), which the compute warps saw before
+        // they gave dS^T(i): the commit that frees Q(i) covers both its readers.
+        const uint32_t idesc_kk = umma_idesc_bf16(128, 128, 0, 0), idesc_mn = umma_idesc_bf16(128, 128, 0, 1);
+        const uint64_t vd = umma_smem_desc_sw128(smem_u32(sV), 0, 1024), dod = umma_smem_desc_sw128(smem_u32(sdO), 0, 1024);
+        const uint64_t qd = umma_smem_desc_sw128(smem_u32(sQ), kAttnSub, 1024);
+        const bool leader = elect_one();
+        bool ok = mbar_wait_warp(kv_full, 0, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN);
+        for (int it = 0; it <= iters && ok; ++it) {
+            if (it > 0) {
+                const int slot = (it - 1) & 1;
+                if (!mbar_wait_warp(&q_full[slot], ((it - 1) >> 1) & 1, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN) ||
+                    !mbar_wait_warp(ds_ready, (it - 1) & 1, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN)) { ok = false; break; }
+                tc_fence_after();
+                if (leader) {
+                    issue_pv_g16(tdK, tdP, qd + slot * kTileDesc, idesc_mn, it > 1);
+                    umma_commit(&q_empty[slot]);
+                    if (it == iters) umma_commit(final_bar);
+                }
+            }
+            if (it < iters) {
+                const int slot = it & 1;
+                if (!mbar_wait_warp(&do_full[slot], (it >> 1) & 1, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN)) { ok = false; break; }
+                tc_fence_after();
+                if (leader) {
+                    issue_kk(tdP, vd, dod + slot * kTileDesc, idesc_kk);
+                    umma_commit(dp_full);
+                    umma_commit(&do_empty[slot]);
+                }
+            }
         }
     } else if (warp >= 4) {
         const int r = (warp & 3) * 32 + lane;  // kv row inside the tile == TMEM lane
         const int grp = (warp - 4) >> 2;       // which 32 of the step's 128 query columns
         const uint32_t lane_bits = static_cast<uint32_t>((warp & 3) * 32) << 16;
+        const int qb = grp * 32;               // first of this warp's 32 query columns
+        const uint32_t tSg = tS + lane_bits + qb, tdPg = tdP + lane_bits + qb;
+        float* stat = sStat + (warp - 4) * 32;
+        // P^T row r, its 16-byte chunk c (8 queries) at chunk c ^ (r & 7) of the 128-byte row, 64 queries per sub-tile
+        const uint32_t prow = smem_u32(sP) + (grp >> 1) * kAttnSub + r * 128;
+        const uint32_t pchunk = (grp & 1) * 4, psw = r & 7;
         bool ok = true;
-        // per-row statistics of the query tile (lse from group 0, delta from group 1), fetched one step ahead
-        const float* stat = grp == 0 ? p.lse : p.delta;
-        auto stat_at = [&](int it) {
+        // statistics of this warp's queries (a lane holds one), fetched a step ahead; shared through the warp's own 32 words
+        auto stat_at = [&](const float* v, int it) {
             const int h = h_first + it / per_head;
             const int i = j + it % per_head;
-            return stat[(static_cast<long long>(b) * p.nh + h) * p.S + i * kAttnTile + r];
+            return v[(static_cast<long long>(b) * p.nh + h) * p.S + i * kAttnTile + qb + lane];
         };
-        float stat_next = grp < 2 ? stat_at(0) : 0.f;
-        for (int it = 0; it < iters; ++it) {
-            const int i = j + it % per_head;
-            const int buf = it & 1;
-            if (grp == 0) sL[buf * 128 + r] = stat_next * 1.4426950408889634f;
-            else if (grp == 1) sD[buf * 128 + r] = stat_next;
-            if (grp < 2 && it + 1 < iters) stat_next = stat_at(it + 1);
-            bar_sync_compute();
-            if (!mbar_wait_warp(sdp_full, it & 1, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN)) { ok = false; break; }
-            tc_fence_after();
+        float lse_next = stat_at(p.lse, 0), delta_next = stat_at(p.delta, 0);
 #pragma unroll 1
-            for (int cc = 0; cc < 2; ++cc) {
-                const int qb = grp * 32 + cc * 16;  // first query column of this pass
-                const uint32_t t = tS + lane_bits + qb;
-                if (i == j) dkdv_pass16<true>(t, 128, sL + buf * 128 + qb, sD + buf * 128 + qb, p.scale_log2, r, qb);
-                else dkdv_pass16<false>(t, 128, sL + buf * 128 + qb, sD + buf * 128 + qb, p.scale_log2, r, qb);
+        for (int it = 0; it < iters; ++it) {
+            const bool diag = it % per_head == 0;
+            const float delta = delta_next;
+            if (!mbar_wait_warp(s_full, it & 1, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN)) { ok = false; break; }
+            tc_fence_after();
+            uint32_t pr[32];
+            tmem_ld_32x32(tSg, pr);
+            __syncwarp();
+            stat[lane] = lse_next * 1.4426950408889634f;
+            if (it + 1 < iters) {
+                lse_next = stat_at(p.lse, it + 1);
+                delta_next = stat_at(p.delta, it + 1);
             }
+            __syncwarp();
+            float4 ls[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) ls[e] = reinterpret_cast<const float4*>(stat)[e];
+            tmem_ld_wait();
             tc_fence_before();
-            mbar_arrive_warp(pds_ready);
+            mbar_arrive_warp(s_empty);
+            if (diag) prob_cols<true, 0>(pr, ls, p.scale_log2, r, qb);
+            else prob_cols<false, 0>(pr, ls, p.scale_log2, r, qb);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) ls[e] = reinterpret_cast<const float4*>(stat)[4 + e];
+            if (diag) prob_cols<true, 1>(pr, ls, p.scale_log2, r, qb);
+            else prob_cols<false, 1>(pr, ls, p.scale_log2, r, qb);
+            __syncwarp();
+            stat[lane] = delta;
+            if (it > 0 && !mbar_wait_warp(p_free, (it - 1) & 1, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN)) { ok = false; break; }
+            auto give_p = [&]() {
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    uint32_t o[4];
+#pragma unroll
+                    for (int t = 0; t < 4; ++t)
+                        o[t] = pack_bf16(__uint_as_float(pr[c * 8 + 2 * t]), __uint_as_float(pr[c * 8 + 2 * t + 1]));
+                    st_shared_v4(prow + (((pchunk + c) ^ psw) << 4), o[0], o[1], o[2], o[3]);
+                }
+                fence_proxy_async_smem();
+                mbar_arrive_warp(p_ready);
+            };
+            give_p();
+            if (!mbar_wait_warp(dp_full, it & 1, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN)) { ok = false; break; }
+            tc_fence_after();
+            uint32_t dp[32];
+            tmem_ld_32x32(tdPg, dp);
+            tmem_ld_wait();
+            uint32_t dk[16];
+#pragma unroll
+            for (int e4 = 0; e4 < 8; ++e4) {
+                const float4 d = reinterpret_cast<const float4*>(stat)[e4];
+                const int e = e4 * 4;
+                dk[e4 * 2] = pack_bf16(__uint_as_float(pr[e]) * (__uint_as_float(dp[e]) - d.x),
+                                       __uint_as_float(pr[e + 1]) * (__uint_as_float(dp[e + 1]) - d.y));
+                dk[e4 * 2 + 1] = pack_bf16(__uint_as_float(pr[e + 2]) * (__uint_as_float(dp[e + 2]) - d.z),
+                                           __uint_as_float(pr[e + 3]) * (__uint_as_float(dp[e + 3]) - d.w));
+            }
+            tmem_st_32x16(tdPg, dk);
+            tmem_st_wait();
+            tc_fence_before();
+            mbar_arrive_warp(ds_ready);
         }
         if (ok && mbar_wait_warp(final_bar, 0, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN)) {
             tc_fence_after();
@@ -387,24 +481,31 @@ attn_dkdv_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
     }
 }
 
-// ---------------------------------------------------------------------------- dQ, one 128 x 128 step in flight
+// ---------------------------------------------------------------------------- dQ
 __global__ void __launch_bounds__(kAttnBwdThreads, 1)
 attn_dq_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant__ CUtensorMap tm_do,
                const AttnBwdParams p) {
-    extern __shared__ uint8_t smem_raw[];
-    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    extern __shared__ __align__(1024) uint8_t smem[];
+    if (smem_u32(smem) & 1023) {
+        if (threadIdx.x == 0) atomicCAS(p.status, 0, CAI_DEV_BAD_ARG);
+        return;
+    }
     uint8_t* sQ = smem;
     uint8_t* sdO = smem + kAttnTileBytes;
-    uint8_t* sK = smem + 2 * kAttnTileBytes;  // 2 stages
-    uint8_t* sV = smem + 4 * kAttnTileBytes;  // 2 stages
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 6 * kAttnTileBytes);
+    uint8_t* sK = smem + 2 * kAttnTileBytes;  // 3 stages: S runs a step ahead of the dQ that still needs the tile
+    uint8_t* sV = smem + 5 * kAttnTileBytes;  // 2 stages
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 7 * kAttnTileBytes);
     uint64_t* q_full = bars;
-    uint64_t* kv_full = bars + 1;
-    uint64_t* kv_empty = bars + 3;
-    uint64_t* sdp_full = bars + 5;
-    uint64_t* ds_ready = bars + 6;
-    uint64_t* final_bar = bars + 7;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 8);
+    uint64_t* k_full = bars + 1;     // [3]
+    uint64_t* k_empty = bars + 4;    // [3] dQ has read the tile
+    uint64_t* v_full = bars + 7;     // [2]
+    uint64_t* v_empty = bars + 9;    // [2]
+    uint64_t* s_full = bars + 11;    // [2]
+    uint64_t* s_empty = bars + 13;   // [2] the compute warps have read the scores
+    uint64_t* dp_full = bars + 15;
+    uint64_t* ds_ready = bars + 16;
+    uint64_t* final_bar = bars + 17;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 18);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -421,11 +522,17 @@ attn_dq_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant
         tma_prefetch_desc(&tm_qkv);
         tma_prefetch_desc(&tm_do);
         mbar_init(q_full, 1);
-        for (int k = 0; k < 2; ++k) {
-            mbar_init(&kv_full[k], 1);
-            mbar_init(&kv_empty[k], 1);
+        for (int k = 0; k < 3; ++k) {
+            mbar_init(&k_full[k], 1);
+            mbar_init(&k_empty[k], 1);
         }
-        mbar_init(sdp_full, 1);
+        for (int k = 0; k < 2; ++k) {
+            mbar_init(&v_full[k], 1);
+            mbar_init(&v_empty[k], 1);
+            mbar_init(&s_full[k], 1);
+            mbar_init(&s_empty[k], kAttnComputeThreads / 32);
+        }
+        mbar_init(dp_full, 1);
         mbar_init(ds_ready, kAttnComputeThreads / 32);
         mbar_init(final_bar, 1);
         *abort_flag = 0;
@@ -439,7 +546,7 @@ attn_dq_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    const uint32_t tS = tmem_base, tdP = tmem_base + 128, tdQ = tmem_base + 256;
+    const uint32_t tS = tmem_base, tdP = tmem_base + 256, tdQ = tmem_base + 384;   // two score buffers
 
     if (warp == 0) {
         if (lane == 0) {
@@ -450,42 +557,87 @@ attn_dq_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant
             tma_load_2d(sdO, &tm_do, q_full, col_q, q_row);
             tma_load_2d(sdO + kAttnSub, &tm_do, q_full, col_q + 64, q_row);
             bool ok = true;
+            int ks = 0;
+            uint32_t kph = 0;
             for (int j = 0; j < n && ok; ++j) {
                 const int slot = j & 1;
                 const uint32_t ph = (j >> 1) & 1;
                 const int kv_row = row_base + j * kAttnTile;
-                if (!mbar_wait(&kv_empty[slot], ph ^ 1, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN)) { ok = false; break; }
-                mbar_expect_tx(&kv_full[slot], 2 * kAttnTileBytes);
-                uint8_t* k = sK + slot * kAttnTileBytes;
+                if (!mbar_wait(&k_empty[ks], kph ^ 1, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN)) { ok = false; break; }
+                mbar_expect_tx(&k_full[ks], kAttnTileBytes);
+                uint8_t* k = sK + ks * kAttnTileBytes;
+                tma_load_2d(k, &tm_qkv, &k_full[ks], col_k, kv_row);
+                tma_load_2d(k + kAttnSub, &tm_qkv, &k_full[ks], col_k + 64, kv_row);
+                if (!mbar_wait(&v_empty[slot], ph ^ 1, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN)) { ok = false; break; }
+                mbar_expect_tx(&v_full[slot], kAttnTileBytes);
                 uint8_t* v = sV + slot * kAttnTileBytes;
-                tma_load_2d(k, &tm_qkv, &kv_full[slot], col_k, kv_row);
-                tma_load_2d(k + kAttnSub, &tm_qkv, &kv_full[slot], col_k + 64, kv_row);
-                tma_load_2d(v, &tm_qkv, &kv_full[slot], col_v, kv_row);
-                tma_load_2d(v + kAttnSub, &tm_qkv, &kv_full[slot], col_v + 64, kv_row);
+                tma_load_2d(v, &tm_qkv, &v_full[slot], col_v, kv_row);
+                tma_load_2d(v + kAttnSub, &tm_qkv, &v_full[slot], col_v + 64, kv_row);
+                if (++ks == 3) {
+                    ks = 0;
+                    kph ^= 1;
+                }
             }
             if (!ok)
                 for (int k = 0; k < 32; ++k) __nanosleep(50000);
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            const uint32_t idesc_kk = umma_idesc_bf16(128, 128, 0, 0);
-            const uint32_t idesc_mn = umma_idesc_bf16(128, 128, 0, 1);
-            const uint32_t aQ = smem_u32(sQ), aD = smem_u32(sdO), aK = smem_u32(sK), aV = smem_u32(sV);
-            bool ok = mbar_wait(q_full, 0, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN);
-            for (int j = 0; j < n && ok; ++j) {
-                const int slot = j & 1;
-                const uint32_t ph = (j >> 1) & 1;
-                if (!mbar_wait(&kv_full[slot], ph, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN)) { ok = false; break; }
-                tc_fence_after();
-                issue_qk(tS, aQ, aK + slot * kAttnTileBytes, idesc_kk);    // S  = Q K^T
-                issue_qk(tdP, aD, aV + slot * kAttnTileBytes, idesc_kk);   // dP = dO V^T
-                umma_commit(sdp_full);
-                if (!mbar_wait(ds_ready, j & 1, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN)) { ok = false; break; }
-                tc_fence_after();
-                issue_pv_g8(tdQ, tdP, aK + slot * kAttnTileBytes, idesc_mn, j > 0);  // dQ += dS K (unscaled)
-                umma_commit(&kv_empty[slot]);
+        // ---------------- S = Q K^T, up to two steps ahead of the compute warps
+        const uint32_t idesc_kk = umma_idesc_bf16(128, 128, 0, 0);
+        const uint64_t qd = umma_smem_desc_sw128(smem_u32(sQ), 0, 1024), kd = umma_smem_desc_sw128(smem_u32(sK), 0, 1024);
+        const bool leader = elect_one();
+        bool ok = mbar_wait_warp(q_full, 0, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN);
+        int ks = 0;
+        uint32_t kph = 0;
+        for (int j = 0; j < n && ok; ++j) {
+            const int buf = j & 1;
+            if (!mbar_wait_warp(&k_full[ks], kph, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN) ||
+                !mbar_wait_warp(&s_empty[buf], ((j >> 1) & 1) ^ 1, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN)) { ok = false; break; }
+            tc_fence_after();
+            if (leader) {
+                issue_kk(tS + buf * 128, qd, kd + ks * kTileDesc, idesc_kk);
+                umma_commit(&s_full[buf]);
             }
-            if (ok) umma_commit(final_bar);
+            if (++ks == 3) {
+                ks = 0;
+                kph ^= 1;
+            }
+        }
+    } else if (warp == 2) {
+        // ---------------- dP = dO V^T, dQ += dS K (unscaled). Ordered behind S(j) by ds_ready(j), which the compute warps
+        // give after they have seen S(j): the commit that frees K(j) therefore covers both its readers.
+        const uint32_t idesc_kk = umma_idesc_bf16(128, 128, 0, 0), idesc_mn = umma_idesc_bf16(128, 128, 0, 1);
+        const uint64_t dod = umma_smem_desc_sw128(smem_u32(sdO), 0, 1024), vd = umma_smem_desc_sw128(smem_u32(sV), 0, 1024);
+        const uint64_t kd = umma_smem_desc_sw128(smem_u32(sK), kAttnSub, 1024);
+        const bool leader = elect_one();
+        bool ok = mbar_wait_warp(q_full, 0, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN);
+        int ks = 0;            // ring slot and phase of the K tile of step j - 1
+        uint32_t kph = 0;
+        for (int j = 0; j <= n && ok; ++j) {
+            const int slot = j & 1;
+            if (j > 0) {
+                if (!mbar_wait_warp(&k_full[ks], kph, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN) ||
+                    !mbar_wait_warp(ds_ready, (j - 1) & 1, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN)) { ok = false; break; }
+                tc_fence_after();
+                if (leader) {
+                    issue_pv_g16(tdQ, tdP, kd + ks * kTileDesc, idesc_mn, j > 1);
+                    umma_commit(&k_empty[ks]);
+                    if (j == n) umma_commit(final_bar);
+                }
+                if (++ks == 3) {
+                    ks = 0;
+                    kph ^= 1;
+                }
+            }
+            if (j < n) {
+                if (!mbar_wait_warp(&v_full[slot], (j >> 1) & 1, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN)) { ok = false; break; }
+                tc_fence_after();
+                if (leader) {
+                    issue_kk(tdP, dod, vd + slot * kTileDesc, idesc_kk);
+                    umma_commit(dp_full);
+                    umma_commit(&v_empty[slot]);
+                }
+            }
         }
     } else if (warp >= 4) {
         const int r = (warp & 3) * 32 + lane;  // q row inside the tile
@@ -494,18 +646,32 @@ attn_dq_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant
         const long long vec = (static_cast<long long>(b) * p.nh + h) * p.S + i * kAttnTile + r;
         const float lse2 = p.lse[vec] * 1.4426950408889634f;
         const float dl = p.delta[vec];
+        const int kb = grp * 32;   // first of this warp's 32 key columns
+        const uint32_t tdPg = tdP + lane_bits + kb;
         bool ok = true;
 #pragma unroll 1
         for (int j = 0; j < n; ++j) {
-            if (!mbar_wait_warp(sdp_full, j & 1, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN)) { ok = false; break; }
+            const int buf = j & 1;
+            if (!mbar_wait_warp(&s_full[buf], (j >> 1) & 1, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN)) { ok = false; break; }
             tc_fence_after();
-#pragma unroll 1
-            for (int cc = 0; cc < 2; ++cc) {
-                const int kb = grp * 32 + cc * 16;  // first key column of this pass
-                const uint32_t t = tS + lane_bits + kb;
-                if (j == i) dq_pass16<true>(t, 128, lse2, dl, p.scale_log2, r, kb);
-                else dq_pass16<false>(t, 128, lse2, dl, p.scale_log2, r, kb);
-            }
+            uint32_t pr[32];
+            tmem_ld_32x32(tS + buf * 128 + lane_bits + kb, pr);
+            tmem_ld_wait();
+            tc_fence_before();
+            mbar_arrive_warp(&s_empty[buf]);
+            if (j == i) prob_rows<true>(pr, lse2, p.scale_log2, r, kb);
+            else prob_rows<false>(pr, lse2, p.scale_log2, r, kb);
+            if (!mbar_wait_warp(dp_full, j & 1, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN)) { ok = false; break; }
+            tc_fence_after();
+            uint32_t dp[32], dk[16];
+            tmem_ld_32x32(tdPg, dp);
+            tmem_ld_wait();
+#pragma unroll
+            for (int e = 0; e < 32; e += 2)
+                dk[e >> 1] = pack_bf16(__uint_as_float(pr[e]) * (__uint_as_float(dp[e]) - dl),
+                                       __uint_as_float(pr[e + 1]) * (__uint_as_float(dp[e + 1]) - dl));
+            tmem_st_32x16(tdPg, dk);
+            tmem_st_wait();
             tc_fence_before();
             mbar_arrive_warp(ds_ready);
         }
@@ -547,7 +713,7 @@ CAI_API int cai_flash_attn_bwd_parts(const void* qkv, const void* out, const voi
     CUtensorMap tm_qkv, tm_do;
     if (!encode_tmap_2d(&tm_qkv, qkv, static_cast<uint64_t>(B) * S, ld, ld, 64, kAttnTile, 2)) return CAI_K_BAD_ARG;
     if (!encode_tmap_2d(&tm_do, dout, static_cast<uint64_t>(B) * S, ldo, ldo, 64, kAttnTile, 2)) return CAI_K_BAD_ARG;
-    constexpr int smem_bytes = 6 * kAttnTileBytes + 2048 + 1024 + 256;
+    constexpr int smem_bytes = 7 * kAttnTileBytes + 2048 + 256;
     static bool configured[64] = {};
     const int dev = current_device();
     if (!configured[dev & 63]) {
