@@ -260,6 +260,62 @@ quant_rows_1x128_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, __nv
     if (lane == 0) scale[r * kb_n + kb] = s;
 }
 
+__device__ __forceinline__ uint32_t abs_bf16x2(uint32_t v) { return v & 0x7FFF7FFFu; }
+__device__ __forceinline__ uint32_t max_bf16x2(uint32_t a, uint32_t b) {
+    const __nv_bfloat162 m = __hmax2(*reinterpret_cast<const __nv_bfloat162*>(&a), *reinterpret_cast<const __nv_bfloat162*>(&b));
+    return *reinterpret_cast<const uint32_t*>(&m);
+}
+// Largest magnitude (as two bf16, the larger one counts) of eight.
+__device__ __forceinline__ uint32_t amax8(const uint4& v) {
+    return max_bf16x2(max_bf16x2(abs_bf16x2(v.x), abs_bf16x2(v.y)), max_bf16x2(abs_bf16x2(v.z), abs_bf16x2(v.w)));
+}
+__device__ __forceinline__ float amax_of(uint32_t m) { return fmaxf(bf16_lo(m), bf16_hi(m)); }
+// Eight bf16 times inv as e4m3.
+__device__ __forceinline__ uint2 quant8(const uint4& v, float inv) {
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    uint32_t h[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        h[k] = __nv_cvt_float2_to_fp8x2(make_float2(bf16_lo(w[k]) * inv, bf16_hi(w[k]) * inv), __NV_SATFINITE, __NV_E4M3);
+    return make_uint2(h[0] | (h[1] << 16), h[2] | (h[3] << 16));
+}
+
+// The same by 16 lanes per 128-column block, 16 bytes a lane, four blocks in flight per thread. What bounds this is bytes in
+// flight (the kernel above has 256 per warp, behind a division of 64-bit numbers). Measured, 8192 x 14336: 144 -> 62 us (2.4
+// -> 5.6 TB/s), 2000 x 14336: 36 -> 20 us. Rows of 16-byte aligned pieces only; the kernel above takes the rest.
+constexpr int kQuantUnroll = 4;
+__global__ void __launch_bounds__(256)
+quant_rows_vec_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, __nv_fp8_storage_t* __restrict__ q, long long ldq,
+                      float* __restrict__ scale, unsigned blocks, unsigned kb_n) {
+    const int sub = threadIdx.x & 15;
+    // half-warps of a CTA take consecutive blocks, kQuantUnroll times over
+    const unsigned b0 = blockIdx.x * (16u * kQuantUnroll) + (threadIdx.x >> 4);
+    uint4 v[kQuantUnroll];
+    long long row[kQuantUnroll];
+    unsigned col[kQuantUnroll];
+#pragma unroll
+    for (int i = 0; i < kQuantUnroll; ++i) {
+        const unsigned b = b0 + 16u * i, r = b / kb_n;
+        row[i] = r;
+        col[i] = (b - r * kb_n) * 128u + sub * 8;
+        v[i] = make_uint4(0, 0, 0, 0);
+        if (b < blocks) v[i] = *reinterpret_cast<const uint4*>(x + row[i] * ldx + col[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < kQuantUnroll; ++i) {
+        const unsigned b = b0 + 16u * i;
+        uint32_t m = amax8(v[i]);
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) m = max_bf16x2(m, __shfl_xor_sync(0xffffffffu, m, o));
+        const float amax = amax_of(m);
+        const float s = amax > 0.f ? amax / 448.f : 1.f;
+        if (b < blocks) {
+            *reinterpret_cast<uint2*>(q + row[i] * ldq + col[i]) = quant8(v[i], 1.f / s);
+            if (sub == 0) scale[b] = s;
+        }
+    }
+}
+
 // One CTA per 128x128 block of a weight [rows, cols]: a common scale; optionally also writes the
 // transposed quantised block (qt [cols, rows], for the input-gradient GEMM that contracts over rows).
 __global__ void __launch_bounds__(256)
@@ -306,6 +362,81 @@ quant_blocks_128x128_kernel(const __nv_bfloat16* __restrict__ w, long long ldw, 
                 qt[static_cast<long long>(gc) * ldqt + gr] = __nv_cvt_float_to_fp8(__bfloat162float(tile[r][c]) * inv, __NV_SATFINITE, __NV_E4M3);
         }
 }
+
+// The same with 16-byte loads kept in registers, 8-byte stores, and the transposed block turned in shared memory: a thread
+// reads a 16 x 4 patch of bytes, transposes it by byte permutations and writes 16 bytes to each of four rows of qt, eight
+// lanes filling a 128-byte line. One byte per store bound the kernel above. Word w of row r sits at w ^ (r / 16 * 4), which
+// keeps both sides free of bank conflicts. Measured with the transposed copy: 28672 x 4096 373 -> 76 us (1.3 -> 6.2 TB/s),
+// 4096 x 14336 203 -> 41 us. Needs cols % 8 == 0 and, for the transposed block, rows % 16 == 0, with the leading dimensions and
+// pointers to match; the kernel above takes the rest.
+__global__ void __launch_bounds__(256)
+quant_blocks_vec_kernel(const __nv_bfloat16* __restrict__ w, long long ldw, __nv_fp8_storage_t* __restrict__ q, long long ldq,
+                        __nv_fp8_storage_t* __restrict__ qt, long long ldqt, float* __restrict__ scale,
+                        float* __restrict__ scale_t, int rows, int cols) {
+    __shared__ __align__(16) uint32_t tile[128 * 32];
+    __shared__ float red[8];
+    const int bc = blockIdx.x, br = blockIdx.y;
+    const int nbc = gridDim.x, nbr = gridDim.y;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int r_in = threadIdx.x >> 4, c8 = threadIdx.x & 15;   // rows r_in + 16 i, columns c8 * 8 ...
+    const int gc = bc * 128 + c8 * 8;
+    uint4 v[8];
+    uint32_t m = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const long long gr = static_cast<long long>(br) * 128 + r_in + 16 * i;
+        v[i] = make_uint4(0, 0, 0, 0);
+        if (gr < rows && gc < cols) v[i] = *reinterpret_cast<const uint4*>(w + gr * ldw + gc);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) m = max_bf16x2(m, amax8(v[i]));
+    float amax = warp_max(amax_of(m));
+    if (lane == 0) red[warp] = amax;
+    __syncthreads();
+    amax = red[0];
+#pragma unroll
+    for (int k = 1; k < 8; ++k) amax = fmaxf(amax, red[k]);
+    const float s = amax > 0.f ? amax / 448.f : 1.f;
+    const float inv = 1.f / s;
+    if (threadIdx.x == 0) {
+        scale[static_cast<long long>(br) * nbc + bc] = s;
+        if (scale_t) scale_t[static_cast<long long>(bc) * nbr + br] = s;
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int r = r_in + 16 * i;
+        const long long gr = static_cast<long long>(br) * 128 + r;
+        const uint2 o = quant8(v[i], inv);
+        if (gr < rows && gc < cols) *reinterpret_cast<uint2*>(q + gr * ldq + gc) = o;
+        if (qt) *reinterpret_cast<uint2*>(&tile[r * 32 + ((c8 * 2) ^ (i * 4))]) = o;   // r / 16 == i
+    }
+    if (!qt) return;
+    __syncthreads();
+    const int rg = lane & 7, cw = warp * 4 + (lane >> 3);   // rows rg * 16 ..., columns cw * 4 ...
+    uint32_t out[4][4];                                     // [column][four rows each]
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        uint32_t a[4];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) a[t] = tile[(rg * 16 + k * 4 + t) * 32 + (cw ^ (rg * 4))];
+        const uint32_t lo01 = __byte_perm(a[0], a[1], 0x5140), hi01 = __byte_perm(a[0], a[1], 0x7362);
+        const uint32_t lo23 = __byte_perm(a[2], a[3], 0x5140), hi23 = __byte_perm(a[2], a[3], 0x7362);
+        out[0][k] = __byte_perm(lo01, lo23, 0x5410);
+        out[1][k] = __byte_perm(lo01, lo23, 0x7632);
+        out[2][k] = __byte_perm(hi01, hi23, 0x5410);
+        out[3][k] = __byte_perm(hi01, hi23, 0x7632);
+    }
+    const long long gr = static_cast<long long>(br) * 128 + rg * 16;
+    if (gr >= rows) return;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int c = bc * 128 + cw * 4 + j;
+        if (c < cols)
+            *reinterpret_cast<uint4*>(qt + static_cast<long long>(c) * ldqt + gr) = make_uint4(out[j][0], out[j][1], out[j][2], out[j][3]);
+    }
+}
+
+static bool aligned_to(const void* p, uintptr_t n) { return (reinterpret_cast<uintptr_t>(p) & (n - 1)) == 0; }
 
 }  // namespace cai
 
@@ -357,6 +488,13 @@ CAI_API int cai_quant_rows_1x128(const void* x, long long ldx, void* q, long lon
     }
     const long long warps = static_cast<long long>(rows) * (cols / 128);
     if (warps == 0) return CAI_K_OK;
+    if (warps < (1ll << 31) && !(ldx & 7) && !(ldq & 7) && aligned_to(x, 16) && aligned_to(q, 8)) {
+        constexpr unsigned per_cta = 16u * kQuantUnroll;
+        quant_rows_vec_kernel<<<static_cast<unsigned>((warps + per_cta - 1) / per_cta), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+            static_cast<const __nv_bfloat16*>(x), ldx, static_cast<__nv_fp8_storage_t*>(q), ldq, scale, static_cast<unsigned>(warps),
+            static_cast<unsigned>(cols / 128));
+        return cudaGetLastError() == cudaSuccess ? 0 : CAI_K_CUDA;
+    }
     quant_rows_1x128_kernel<<<static_cast<unsigned>((warps * 32 + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
         static_cast<const __nv_bfloat16*>(x), ldx, static_cast<__nv_fp8_storage_t*>(q), ldq, scale, rows, cols);
     return cudaGetLastError() == cudaSuccess ? 0 : CAI_K_CUDA;
@@ -366,6 +504,13 @@ CAI_API int cai_quant_blocks_128x128(const void* w, long long ldw, void* q, long
                                      float* scale_t, int rows, int cols, void* stream) {
     if (rows <= 0 || cols <= 0) return CAI_K_OK;
     dim3 grid((cols + 127) / 128, (rows + 127) / 128);
+    if (!(cols & 7) && !(ldw & 7) && !(ldq & 7) && aligned_to(w, 16) && aligned_to(q, 8) &&
+        (!qt || (!(rows & 15) && !(ldqt & 15) && aligned_to(qt, 16)))) {
+        quant_blocks_vec_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+            static_cast<const __nv_bfloat16*>(w), ldw, static_cast<__nv_fp8_storage_t*>(q), ldq, static_cast<__nv_fp8_storage_t*>(qt),
+            ldqt, scale, scale_t, rows, cols);
+        return cudaGetLastError() == cudaSuccess ? 0 : CAI_K_CUDA;
+    }
     quant_blocks_128x128_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
         static_cast<const __nv_bfloat16*>(w), ldw, static_cast<__nv_fp8_storage_t*>(q), ldq, static_cast<__nv_fp8_storage_t*>(qt),
         ldqt, scale, scale_t, rows, cols);

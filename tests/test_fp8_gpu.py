@@ -75,3 +75,44 @@ def test_training_with_fp8_linear_layers_tracks_bf16():
     assert b[-1] < b[0] - 0.3, b
     for x, y in zip(a, b):
         assert abs(x - y) < 0.03 * max(1.0, x), (a, b)
+
+
+def _strided(t, pad):
+    big = torch.zeros(t.shape[0], t.shape[1] + pad, device=t.device, dtype=t.dtype)
+    big[:, :t.shape[1]] = t
+    return big
+
+
+# The quantisers' wide form (16-byte pieces) against their narrow one, which takes rows at odd pitches: the same bytes.
+@pytest.mark.parametrize("rows,cols", [(1, 128), (63, 384), (65, 128), (300, 1152)])
+def test_quant_rows_forms_agree(rows, cols):
+    import ctypes
+    from cai_b200 import ops
+    torch.manual_seed(4)
+    x = (torch.randn(rows, cols, device="cuda") * 3).to(torch.bfloat16)
+    x[rows // 2, :128] = 0
+    q, s = ops.quant_rows_1x128(x)
+    xp = _strided(x, 4)
+    q2, s2 = torch.zeros_like(q), torch.zeros_like(s)
+    p = lambda t: ctypes.c_void_p(t.data_ptr())
+    assert ops.lib().cai_quant_rows_1x128(p(xp), ctypes.c_longlong(cols + 4), p(q2), ctypes.c_longlong(cols), p(s2), rows, cols,
+                                          ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+    assert torch.equal(q.view(torch.uint8), q2.view(torch.uint8)) and torch.equal(s, s2)
+
+
+@pytest.mark.parametrize("rows,cols", [(16, 8), (128, 128), (144, 392), (400, 264)])
+def test_quant_blocks_forms_agree(rows, cols):
+    import ctypes
+    from cai_b200 import ops
+    torch.manual_seed(5)
+    w = torch.randn(rows, cols, device="cuda").to(torch.bfloat16)
+    q, s, qt, st = ops.quant_blocks_128x128(w, transposed=True)
+    wp = _strided(w, 3)
+    q2, s2, qt2, st2 = torch.zeros_like(q), torch.zeros_like(s), torch.zeros_like(qt), torch.zeros_like(st)
+    p = lambda t: ctypes.c_void_p(t.data_ptr())
+    n = ctypes.c_longlong
+    assert ops.lib().cai_quant_blocks_128x128(p(wp), n(cols + 3), p(q2), n(q.stride(0)), p(qt2), n(qt.stride(0)), p(s2), p(st2), rows, cols,
+                                              ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+    for a, b in ((q, q2), (qt, qt2)):
+        assert torch.equal(a.view(torch.uint8), b.view(torch.uint8))
+    assert torch.equal(s, s2) and torch.equal(st, st2)
