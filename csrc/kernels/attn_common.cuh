@@ -36,4 +36,20 @@ __device__ __forceinline__ void issue_pv(uint32_t d_tmem, uint32_t p_tmem, uint3
     }
 }
 
+constexpr uint32_t kTileDesc = kAttnTileBytes >> 4;   // descriptor distance of two tiles
+// S[128,128] = A[128,hd] * B[128,hd]^T, both K-major in two 64-column sub-tiles, from ready-made descriptors.
+__device__ __forceinline__ void issue_kk(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc) {
+#pragma unroll
+    for (int k = 0; k < kAttnHD / 16; ++k) {
+        const uint32_t off = ((k >> 2) * kAttnSub + (k & 3) * 32) >> 4;
+        umma_f16_ss(d_tmem, a_desc + off, b_desc + off, idesc, k > 0 ? 1u : 0u);
+    }
+}
+// The same product as issue_pv with V's descriptor ready-made.
+__device__ __forceinline__ void issue_pv_desc(uint32_t d_tmem, uint32_t p_tmem, uint64_t v_desc, uint32_t idesc, bool accumulate) {
+#pragma unroll
+    for (int k = 0; k < kAttnTile / 16; ++k)
+        umma_f16_ts(d_tmem, p_tmem + k * 8, v_desc + k * (2048 >> 4), idesc, (accumulate || k > 0) ? 1u : 0u);
+}
+
 }  // namespace cai

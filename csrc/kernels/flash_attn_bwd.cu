@@ -160,14 +160,6 @@ __device__ __forceinline__ void issue_pv_g16(uint32_t d_tmem, uint32_t a_tmem, u
     for (int k = 0; k < kAttnTile / 16; ++k)
         umma_f16_ts(d_tmem, a_tmem + (k >> 1) * 32 + (k & 1) * 8, b_desc + k * (2048 >> 4), idesc, (accumulate || k > 0) ? 1u : 0u);
 }
-// S[128,128] = A[128,hd] * B[128,hd]^T, both K-major in two 64-column sub-tiles, from ready-made descriptors.
-__device__ __forceinline__ void issue_kk(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc) {
-#pragma unroll
-    for (int k = 0; k < kAttnHD / 16; ++k) {
-        const uint32_t off = ((k >> 2) * kAttnSub + (k & 3) * 32) >> 4;
-        umma_f16_ss(d_tmem, a_desc + off, b_desc + off, idesc, k > 0 ? 1u : 0u);
-    }
-}
 // D[128,hd] (+)= A[128,128] * B[128,hd], both in shared memory: A K-major, B MN-major.
 __device__ __forceinline__ void issue_pd_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, bool accumulate) {
 #pragma unroll
@@ -175,7 +167,6 @@ __device__ __forceinline__ void issue_pd_ss(uint32_t d_tmem, uint64_t a_desc, ui
         umma_f16_ss(d_tmem, a_desc + (((k >> 2) * kAttnSub + (k & 3) * 32) >> 4), b_desc + k * (2048 >> 4), idesc,
                     (accumulate || k > 0) ? 1u : 0u);
 }
-constexpr uint32_t kTileDesc = kAttnTileBytes >> 4;   // descriptor distance of two tiles
 
 // ---------------------------------------------------------------------------- dK / dV
 __global__ void __launch_bounds__(kAttnBwdThreads, 1)

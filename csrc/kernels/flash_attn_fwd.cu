@@ -2,7 +2,8 @@
 //
 // One CTA owns two adjacent 128-row query tiles (A and B) of one head and sweeps the key/value
 // tiles they may attend to. Warp 0 streams Q, K and V tiles with TMA straight out of the packed
-// QKV activation; warp 1 issues the tcgen05 MMAs; warps 4-7 and 8-11 are the softmax groups of
+// QKV activation; warps 1 and 2 issue the tcgen05 MMAs of tile A and tile B (one issuer for both left a tile waiting behind
+// the other's barriers: 3 x 640 tokens, 9 / 3 heads 26.0 -> 23.7 us, 8192 tokens, 32 / 8 heads 615 -> 581 us); warps 4-7 and 8-11 are the softmax groups of
 // tile A and tile B, one thread per query row. Scores live in tensor memory: S = Q K^T lands in
 // TMEM, the softmax group reads it with tcgen05.ld, writes the bf16 probabilities back over the
 // same columns with tcgen05.st, and O += P V consumes P directly from TMEM as the A operand.
@@ -73,10 +74,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm, const AttnFwdParams p) {
         tma_prefetch_desc(&tm);
         mbar_init(q_full, 1);
         for (int i = 0; i < 2; ++i) {
+            // both tiles' issuers hand a stage back. (Tile A, a key tile shorter, leaves the last one out: nobody waits for it.)
             mbar_init(&k_full[i], 1);
-            mbar_init(&k_empty[i], 1);
+            mbar_init(&k_empty[i], nB ? 2 : 1);
             mbar_init(&v_full[i], 1);
-            mbar_init(&v_empty[i], 1);
+            mbar_init(&v_empty[i], nB ? 2 : 1);
             mbar_init(&s_full[i], 1);
             mbar_init(&p_full[i], 4);
             mbar_init(&o_final[i], 1);
@@ -120,51 +122,43 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm, const AttnFwdParams p) {
             if (!ok)
                 for (int i = 0; i < 32; ++i) __nanosleep(50000);
         }
-    } else if (warp == 1) {
-        if (lane == 0) {
-            // ---------------- MMA issuer
-            const uint32_t idesc_qk = umma_idesc_bf16(128, 128, 0, 0);
-            const uint32_t idesc_pv = umma_idesc_bf16(128, 128, 0, 1);
-            const uint32_t sQa = smem_u32(sQ), sQb = smem_u32(sQ + kAttnTileBytes);
-            const uint32_t sK0 = smem_u32(sK), sV0 = smem_u32(sV);
-            const uint32_t tS[2] = {tmem_base, tmem_base + 128};
-            const uint32_t tO[2] = {tmem_base + 256, tmem_base + 384};
-            const uint32_t sQx[2] = {sQa, sQb};
-            const int nX[2] = {nA, nB};
-            bool ok = mbar_wait(q_full, 0, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN) &&
-                      mbar_wait(&k_full[0], 0, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN);
-            if (ok) {
-                tc_fence_after();
-                for (int X = 0; X < 2; ++X)
-                    if (nX[X] > 0) {
-                        issue_qk(tS[X], sQx[X], sK0, idesc_qk);
-                        umma_commit(&s_full[X]);
-                    }
+    } else if (warp == 1 || warp == 2) {
+        // ---------------- MMA issuers: warp 1 for tile A, warp 2 for tile B. The whole warp walks the loop (descriptors in
+        // uniform registers), one lane issues. P is waited for last: the loads are normally there, so that P V(j) and
+        // S(j+1) go out back to back once it arrives.
+        const int X = warp - 1, nx = X ? nB : nA;
+        const uint32_t idesc_qk = umma_idesc_bf16(128, 128, 0, 0), idesc_pv = umma_idesc_bf16(128, 128, 0, 1);
+        const uint64_t qd = umma_smem_desc_sw128(smem_u32(sQ + X * kAttnTileBytes), 0, 1024);
+        const uint64_t kd = umma_smem_desc_sw128(smem_u32(sK), 0, 1024), vd = umma_smem_desc_sw128(smem_u32(sV), kAttnSub, 1024);
+        const uint32_t tS = tmem_base + X * 128, tO = tmem_base + 256 + X * 128;
+        const bool leader = elect_one();
+        if (nx > 0 && mbar_wait_warp(q_full, 0, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN) &&
+            mbar_wait_warp(&k_full[0], 0, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN)) {
+            tc_fence_after();
+            if (leader) {
+                issue_kk(tS, qd, kd, idesc_qk);
+                umma_commit(&s_full[X]);
                 umma_commit(&k_empty[0]);
             }
-            for (int j = 0; j < n && ok; ++j) {
-                const int slot = j & 1;
-                const uint32_t ph = (j >> 1) & 1;
-                if (!mbar_wait(&v_full[slot], ph, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN)) { ok = false; break; }
-                const int ns = (j + 1) & 1;
-                const uint32_t nph = ((j + 1) >> 1) & 1;
-                for (int X = 0; X < 2 && ok; ++X) {
-                    if (j >= nX[X]) continue;
-                    if (!mbar_wait(&p_full[X], j & 1, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN)) { ok = false; break; }
-                    tc_fence_after();
-                    issue_pv(tO[X], tS[X], sV0 + slot * kAttnTileBytes, idesc_pv, j > 0);
-                    if (j + 1 < nX[X]) {
-                        if (!mbar_wait(&k_full[ns], nph, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN)) { ok = false; break; }
-                        tc_fence_after();
-                        issue_qk(tS[X], sQx[X], sK0 + ns * kAttnTileBytes, idesc_qk);
+            for (int j = 0; j < nx; ++j) {
+                const int slot = j & 1, ns = slot ^ 1;
+                const bool more = j + 1 < nx;
+                if (!mbar_wait_warp(&v_full[slot], (j >> 1) & 1, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN) ||
+                    (more && !mbar_wait_warp(&k_full[ns], ((j + 1) >> 1) & 1, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN)) ||
+                    !mbar_wait_warp(&p_full[X], j & 1, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN))
+                    break;
+                tc_fence_after();
+                if (leader) {
+                    issue_pv_desc(tO, tS, vd + slot * kTileDesc, idesc_pv, j > 0);
+                    if (more) {
+                        issue_kk(tS, qd, kd + ns * kTileDesc, idesc_qk);
                         umma_commit(&s_full[X]);
+                        umma_commit(&k_empty[ns]);
                     } else {
                         umma_commit(&o_final[X]);
                     }
+                    umma_commit(&v_empty[slot]);
                 }
-                if (!ok) break;
-                umma_commit(&v_empty[slot]);
-                if (j + 1 < n) umma_commit(&k_empty[ns]);
             }
         }
     } else if (warp >= 4) {
