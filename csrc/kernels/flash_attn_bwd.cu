@@ -69,24 +69,50 @@ struct AttnBwdParams {
 constexpr size_t kAttnChainSlots = 65536;
 __device__ unsigned int g_attn_chain[kAttnChainSlots];
 
-__global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ dout,
-                                  float* __restrict__ delta, int B, int S, int nh) {
-    const long long w = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    const long long total = static_cast<long long>(B) * S * nh;
-    if (w >= total) return;
-    const int h = w % nh;
-    const long long row = w / nh;  // b*S + s
-    const long long off = row * (static_cast<long long>(nh) * kAttnHD) + h * kAttnHD + lane * 4;
-    const uint2 a = *reinterpret_cast<const uint2*>(out + off);
-    const uint2 d = *reinterpret_cast<const uint2*>(dout + off);
-    float s = bf16_lo(a.x) * bf16_lo(d.x) + bf16_hi(a.x) * bf16_hi(d.x) + bf16_lo(a.y) * bf16_lo(d.y) +
-              bf16_hi(a.y) * bf16_hi(d.y);
+// Sixteen lanes per (token, head), 16 bytes a lane from each tensor, kDeltaUnroll of them in flight per thread: what bounds this is
+// bytes in flight (one pair of 8-byte loads per thread and a 64-bit division in front: 8192 tokens of
+// 32 heads 47 -> 29 us, 3 x 640 tokens of 9 heads 7.6 -> 4.5 us). The tensors are walked as one array of
+// 128-element rows. (dO starts on 16 bytes, or its tensor map is refused; O may start on 8.)
+constexpr int kDeltaUnroll = 2;
+__global__ void __launch_bounds__(256)
+attn_delta_kernel(const __nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ dout, float* __restrict__ delta,
+                  unsigned total, unsigned S, unsigned nh, bool out16) {
+    const unsigned w0 = blockIdx.x * (16u * kDeltaUnroll) + (threadIdx.x >> 4);
+    const int sub = threadIdx.x & 15;
+    uint4 a[kDeltaUnroll], d[kDeltaUnroll];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) {
-        const int b = row / S, sidx = row % S;
-        delta[(static_cast<long long>(b) * nh + h) * S + sidx] = s;
+    for (int i = 0; i < kDeltaUnroll; ++i) {
+        const unsigned w = w0 + 16u * i;
+        a[i] = d[i] = make_uint4(0, 0, 0, 0);
+        if (w < total) {
+            const size_t off = static_cast<size_t>(w) * kAttnHD + sub * 8;
+            if (out16) {
+                a[i] = *reinterpret_cast<const uint4*>(out + off);
+            } else {
+                const uint2 lo = *reinterpret_cast<const uint2*>(out + off), hi = *reinterpret_cast<const uint2*>(out + off + 4);
+                a[i] = make_uint4(lo.x, lo.y, hi.x, hi.y);
+            }
+            d[i] = *reinterpret_cast<const uint4*>(dout + off);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < kDeltaUnroll; ++i) {
+        // two quads of elements per lane, added last: the tree of sums over quads 16, 8, 4, 2 and 1 apart
+        float s0 = bf16_lo(a[i].x) * bf16_lo(d[i].x) + bf16_hi(a[i].x) * bf16_hi(d[i].x) + bf16_lo(a[i].y) * bf16_lo(d[i].y) +
+                   bf16_hi(a[i].y) * bf16_hi(d[i].y);
+        float s1 = bf16_lo(a[i].z) * bf16_lo(d[i].z) + bf16_hi(a[i].z) * bf16_hi(d[i].z) + bf16_lo(a[i].w) * bf16_lo(d[i].w) +
+                   bf16_hi(a[i].w) * bf16_hi(d[i].w);
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) {
+            s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+            s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+        }
+        const float s = s0 + s1;
+        const unsigned w = w0 + 16u * i;
+        if (sub == 0 && w < total) {
+            const unsigned row = w / nh, h = w - row * nh, b = row / S, at = row - b * S;
+            delta[(static_cast<size_t>(b) * nh + h) * S + at] = s;
+        }
     }
 }
 
@@ -715,10 +741,13 @@ CAI_API int cai_flash_attn_bwd_parts(const void* qkv, const void* out, const voi
         }
         configured[dev & 63] = true;
     }
-    const long long warps = static_cast<long long>(B) * S * nh;
-    if (parts & 1)
-        attn_delta_kernel<<<static_cast<unsigned>((warps * 32 + 255) / 256), 256, 0, st>>>(
-        static_cast<const __nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(dout), delta, B, S, nh);
+    const long long rows = static_cast<long long>(B) * S * nh;
+    if (parts & 1) {
+        constexpr unsigned per_cta = 16u * kDeltaUnroll;
+        attn_delta_kernel<<<static_cast<unsigned>((rows + per_cta - 1) / per_cta), 256, 0, st>>>(
+            static_cast<const __nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(dout), delta, static_cast<unsigned>(rows),
+            static_cast<unsigned>(S), static_cast<unsigned>(nh), (reinterpret_cast<uintptr_t>(out) & 15) == 0);
+    }
     AttnBwdParams p;
     p.B = B; p.S = S; p.nh = nh; p.nkv = nkv;
     p.scale = scale;
