@@ -155,3 +155,22 @@ def test_adamw_matches_reference_rule():
         pr = pr - lr * (mh / (vh.sqrt() + eps) + wd * pr)
     assert torch.allclose(p.double(), pr, atol=1e-5, rtol=1e-5)
     assert torch.equal(pb, p.to(torch.bfloat16))
+
+
+# Rows handled by 1, 2, 4 and 8 warps; fewer rows than warps, ragged last chunks, an accumulated dx and gain gradient.
+@pytest.mark.parametrize("rows,H", [(1, 8), (5, 1000), (300, 1032), (77, 3000), (33, 8192)])
+def test_rmsnorm_bwd_sums(rows, H):
+    from cai_b200 import ops
+    torch.manual_seed(7)
+    x = torch.randn(rows, H, device="cuda").to(torch.bfloat16)
+    g = (1 + 0.1 * torch.randn(H, device="cuda")).to(torch.bfloat16)
+    dy = torch.randn(rows, H, device="cuda").to(torch.bfloat16)
+    _, rstd = ops.rmsnorm_fwd(x, g)
+    dx0 = torch.randn(rows, H, device="cuda").to(torch.bfloat16)
+    dg0 = torch.randn(H, device="cuda")
+    dx, dg = ops.rmsnorm_bwd(x, g, rstd, dy, dx=dx0.clone(), dg=dg0.clone(), dx_accumulate=True, dg_accumulate=True)
+    xd, gd, dd, r = x.double(), g.double(), dy.double(), rstd.double()[:, None]
+    want_dg = dg0.double() + (dd * xd * r).sum(0)
+    want_dx = dx0.double() + r * dd * gd - r ** 3 * xd * (dd * gd * xd).sum(1, keepdim=True) / H
+    assert ((dg.double() - want_dg).norm() / want_dg.norm()).item() < 1e-5          # fp32 sums
+    assert ((dx.double() - want_dx).norm() / want_dx.norm()).item() < 2 ** -8       # one rounding to bf16
