@@ -605,10 +605,10 @@ gemm_pair_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
             const int r = it / W, c = it % W;
             const int row_in = row_half + r, col = col0 + c * 4;
             const uint32_t at = r * (BN * 4) + (((slice * W + c) ^ (r & 7)) << 4);
+            if (row_in >= p.M || col >= p.N) continue;   // before the loads: every one issued is consumed before the closing barrier
             float4 part[S];
 #pragma unroll
             for (int i = 0; i < S; ++i) part[i] = ld_cluster_f4(src[i] + at);
-            if (row_in >= p.M || col >= p.N) continue;
             float4 v = part[0];
 #pragma unroll
             for (int i = 1; i < S; ++i) {
@@ -633,7 +633,7 @@ gemm_pair_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
         }
     }
     __syncwarp();
-    cluster_sync();            // nobody leaves while another CTA may still read its partial
+    cluster_sync_memory();     // nobody leaves while another CTA may still read its partial (ordered behind those reads)
     if (warp == 1) {
         tc_fence_after();
         tmem_dealloc_pair(tmem_base, BN);

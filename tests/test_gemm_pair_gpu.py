@@ -50,3 +50,19 @@ def test_pair_gemm_groups_do_not_touch_each_other(M, N):
     for g in range(G):
         A, B = a[g * M:(g + 1) * M].float(), b[g * N:(g + 1) * N].float()
         assert ((out[g * M:(g + 1) * M] - A @ B.t()).abs() <= 2 * K * 2.0 ** -24 * (A.abs() @ B.abs().t()) + 1e-6).all()
+
+
+# Split along K, where a CTA of the cluster has no rows (M of at most half a tile, or half a tile past a whole one) and where the last
+# slab of columns lies partly or wholly past N. Launched back to back, so that a CTA that left early would meet its successor.
+@pytest.mark.parametrize("M,N,K", [(8, 8, 512), (128, 136, 1024), (129, 264, 4096), (264, 104, 8192), (384, 1000, 3000), (130, 1032, 264)])
+def test_split_gemm_empty_halves(M, N, K):
+    from cai_b200 import ops
+    from cai_b200.ops import _lib
+    torch.manual_seed(3)
+    a = torch.randn(M, K, device="cuda").to(torch.bfloat16)
+    b = torch.randn(N, K, device="cuda").to(torch.bfloat16)
+    bound = 2 * K * 2.0 ** -24 * (a.float().abs() @ b.float().abs().t()) + 1e-6    # two sums of K exact products in fp32
+    outs = [ops.gemm(a, b, out_dtype=torch.float32) for _ in range(50)]
+    assert ((outs[0] - a.float() @ b.float().t()).abs() <= bound).all()
+    assert all(torch.equal(outs[0], o) for o in outs[1:])
+    assert _lib.device_status(clear=True) == 0
