@@ -574,12 +574,13 @@ gemm_pair_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
             }
             if (ok && mma.leader) umma_commit_pair(tmem_full, mma.pair_mask);
         }
-    } else if (row_half < p.M) {
-        // ---------------- partial accumulator -> shared memory: row r, 16-byte chunk c at r * 512 + (c ^ (r & 7)) * 16
+    } else {
+        // ---------------- partial accumulator -> shared memory: row r, 16-byte chunk c at r * 512 + (c ^ (r & 7)) * 16.
+        // A CTA without rows waits too: the even CTA's commit arrives on its barrier as well.
         const int q = warp & 3, half = (warp - 2) >> 2;
         const uint32_t dst = smem_u32(smem) + (q * 32 + lane) * (BN * 4);
         const uint32_t tacc = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + half * HALF;
-        if (mbar_wait_warp(tmem_full, 0, abort_flag, p.status, CAI_DEV_TIMEOUT_TMEM_FULL)) {
+        if (mbar_wait_warp(tmem_full, 0, abort_flag, p.status, CAI_DEV_TIMEOUT_TMEM_FULL) && row_half < p.M) {
             tc_fence_after();
             uint32_t r[2][32];
             tmem_ld_32x32(tacc, r[0]);

@@ -66,3 +66,27 @@ def test_split_gemm_empty_halves(M, N, K):
     assert ((outs[0] - a.float() @ b.float().t()).abs() <= bound).all()
     assert all(torch.equal(outs[0], o) for o in outs[1:])
     assert _lib.device_status(clear=True) == 0
+
+
+# The even CTA's last commit arrives on both CTAs of a pair; the one without rows has to have seen it before it ends. Two streams, so that
+# the SMs of an early leaver would be handed to the other stream's clusters at once.
+def test_split_gemm_empty_halves_on_two_streams():
+    from cai_b200 import ops
+    from cai_b200.ops import _lib
+    torch.manual_seed(4)
+    cases = []
+    for M, N, K in ((8, 1024, 2048), (136, 520, 4096)):
+        a = torch.randn(M, K, device="cuda").to(torch.bfloat16)
+        b = torch.randn(N, K, device="cuda").to(torch.bfloat16)
+        bound = 2 * K * 2.0 ** -24 * (a.float().abs() @ b.float().abs().t()) + 1e-6
+        cases.append((a, b, a.float() @ b.float().t(), bound, torch.cuda.Stream()))
+    torch.cuda.synchronize()
+    outs = [[] for _ in cases]
+    for _ in range(30):
+        for o, (a, b, _, _, st) in zip(outs, cases):
+            with torch.cuda.stream(st):
+                o.append(ops.gemm(a, b, out_dtype=torch.float32))
+    torch.cuda.synchronize()
+    for o, (_, _, ref, bound, _) in zip(outs, cases):
+        assert all(((v - ref).abs() <= bound).all() for v in o)
+    assert _lib.device_status(clear=True) == 0
