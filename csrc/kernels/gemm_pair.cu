@@ -455,7 +455,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     tc_fence_before();
     __syncthreads();
     __syncwarp();
-    cluster_sync();
+    cluster_sync_memory();   // the odd CTA's last arrivals on the even one's barriers are in: nobody waits for those
     if (warp == 1) {
         tc_fence_after();
         tmem_dealloc_pair(tmem_base, 2 * BN);

@@ -90,3 +90,27 @@ def test_split_gemm_empty_halves_on_two_streams():
     for o, (_, _, ref, bound, _) in zip(outs, cases):
         assert all(((v - ref).abs() <= bound).all() for v in o)
     assert _lib.device_status(clear=True) == 0
+
+
+# A last tile's accumulator is handed back to the even CTA with nobody waiting for it: short kernels back to back on two streams, one tile
+# per pair, both widths, so that a pair that parted early would be replaced at once.
+def test_pair_gemm_short_kernels_on_two_streams():
+    from cai_b200 import ops
+    from cai_b200.ops import _lib
+    torch.manual_seed(5)
+    cases = []
+    for M, N, K in ((2000, 2000, 64), (2304, 4104, 72)):
+        a = torch.randn(M, K, device="cuda").to(torch.bfloat16)
+        b = torch.randn(N, K, device="cuda").to(torch.bfloat16)
+        bound = 2 * K * 2.0 ** -24 * (a.float().abs() @ b.float().abs().t()) + 1e-6
+        cases.append((a, b, a.float() @ b.float().t(), bound, torch.cuda.Stream()))
+    torch.cuda.synchronize()
+    outs = [[] for _ in cases]
+    for _ in range(20):
+        for o, (a, b, _, _, st) in zip(outs, cases):
+            with torch.cuda.stream(st):
+                o.append(ops.gemm(a, b, out_dtype=torch.float32))
+    torch.cuda.synchronize()
+    for o, (_, _, ref, bound, _) in zip(outs, cases):
+        assert all(((v - ref).abs() <= bound).all() for v in o)
+    assert _lib.device_status(clear=True) == 0
