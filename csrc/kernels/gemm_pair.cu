@@ -288,6 +288,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                 }
                 if (ok && mma.leader) umma_commit_pair(&tmem_full[acc], mma.pair_mask);
             }
+            // both accumulators handed back: no arrival of the odd CTA is still on its way when this one ends
+            for (int i = 0; i < 2 && ok; ++i, ++t)
+                ok = mbar_wait_warp(&tmem_empty[t & 1], ((t >> 1) & 1) ^ 1, abort_flag, p.status, CAI_DEV_TIMEOUT_TMEM_EMPTY);
         }
     } else {
         // ---------------- epilogue warps: TMEM -> registers -> shared memory -> TMA
@@ -455,7 +458,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     tc_fence_before();
     __syncthreads();
     __syncwarp();
-    cluster_sync_memory();   // the odd CTA's last arrivals on the even one's barriers are in: nobody waits for those
+    cluster_sync();
     if (warp == 1) {
         tc_fence_after();
         tmem_dealloc_pair(tmem_base, 2 * BN);
