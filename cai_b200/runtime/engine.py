@@ -148,6 +148,10 @@ class Engine:
         # The six streams come from torch's pool: tensors touched on them stay valid for torch's
         # caching allocators after the executor is gone. compute_hi and comm_tp get high priority.
         self.streams = [torch.cuda.Stream(device=self.device, priority=-1 if s in (0, 2) else 0) for s in range(6)]
+        # They start after the clearing above, which runs on the caller's stream: what is written on them from here on (rotary
+        # table, parameters, optimizer state) lands on a cleared arena.
+        for s in self.streams:
+            s.wait_stream(torch.cuda.current_stream(self.device))
         handles = (c_void_p * 6)(*[c_void_p(s.cuda_stream) for s in self.streams])
         klib.check(L.cai_exec_create(ctypes.byref(self.ex), self.plan.raw, len(self.plan.raw), c_void_p(base), handles),
                    "exec_create")

@@ -37,8 +37,9 @@ CAI_API int cai_dev_malloc(void** out, unsigned long long nbytes) {
 
 CAI_API int cai_dev_free(void* p) { return cudaFree(p) == cudaSuccess ? 0 : CAI_K_CUDA; }
 
+// Returns when the bytes are set: cudaMemset only queues the work, and the executor's streams do not wait for the default one.
 CAI_API int cai_dev_memset(void* p, int value, unsigned long long nbytes) {
-    return cudaMemset(p, value, nbytes) == cudaSuccess ? 0 : CAI_K_CUDA;
+    return cudaMemset(p, value, nbytes) == cudaSuccess && cudaStreamSynchronize(nullptr) == cudaSuccess ? 0 : CAI_K_CUDA;
 }
 
 // Blocking copies (set-up, parameter initialisation, the per-step loss): the step itself never waits on them.

@@ -680,8 +680,9 @@ CAI_API int cai_exec_create(cai_exec** out, const void* plan_bytes, size_t nbyte
     for (cudaEvent_t e : ex->events) dev_ok = dev_ok && e != nullptr;
     dev_ok = dev_ok && cudaMalloc(&ex->hyper_dev, 8 * sizeof(float)) == cudaSuccess;
     dev_ok = dev_ok && cudaMalloc(&ex->counters_dev, 256 * sizeof(unsigned int)) == cudaSuccess;
-    dev_ok = dev_ok && cudaMemset(ex->counters_dev, 0, 256 * sizeof(unsigned int)) == cudaSuccess;
-    dev_ok = dev_ok && cudaMemset(ex->hyper_dev, 0, 8 * sizeof(float)) == cudaSuccess;
+    // on the stream every step forks from: nothing orders the default stream before it
+    dev_ok = dev_ok && cudaMemsetAsync(ex->counters_dev, 0, 256 * sizeof(unsigned int), ex->streams[ST_COMPUTE_HI]) == cudaSuccess;
+    dev_ok = dev_ok && cudaMemsetAsync(ex->hyper_dev, 0, 8 * sizeof(float), ex->streams[ST_COMPUTE_HI]) == cudaSuccess;
     dev_ok = dev_ok && cudaMallocHost(&ex->hyper_host, cai_exec::kHyperSlots * 8 * sizeof(float)) == cudaSuccess;
     for (int i = 0; i < cai_exec::kHyperSlots && dev_ok; ++i)
         dev_ok = cudaEventCreateWithFlags(&ex->hyper_ev[i], cudaEventDisableTiming) == cudaSuccess;

@@ -312,3 +312,27 @@ def test_debug_mode_checks_every_operand_extent_before_launch(monkeypatch):
         assert a == a and b == b
         assert eng.check_canaries()
         eng.close()
+
+
+@pytest.mark.parametrize("side", [False, True])
+def test_engine_made_behind_work_of_the_callers_stream(side):
+    """The arena is cleared on the caller's stream and filled on the engine's: with the caller's stream busy, the parameters, the
+    optimizer state and the rotary table still land on a cleared arena, not under the clearing."""
+    from cai_b200 import ops
+    want = _engine()
+    table = want.view("@rope_table").view(-1).clone()
+    params = _torch_params(want)
+    want.close()
+    caller = torch.cuda.Stream() if side else torch.cuda.current_stream()
+    with torch.cuda.stream(caller):
+        torch.cuda._sleep(200_000_000)          # about 0.1 s in front of the clearing
+        eng = _engine()
+    got = _torch_params(eng)
+    assert all(torch.equal(got[n], params[n]) for n in params)
+    assert torch.equal(eng.view("@rope_table").view(-1), table)
+    assert float(table.abs().sum()) > 0 and all(float(p.abs().sum()) > 0 for p in params.values())
+    n = ops.rope_table(eng.model.seq_len, eng.model.head_dim, theta=eng.train.rope_theta).view(-1)
+    assert torch.equal(table[:n.numel()], n)
+    assert float(eng.view("@flat_master").abs().sum()) > 0 and float(eng.view("@flat_m").abs().sum()) == 0
+    assert eng.check_canaries()
+    eng.close()
