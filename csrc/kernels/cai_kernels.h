@@ -49,6 +49,10 @@ CAI_API int cai_gemm_bf16(const void* A, const void* B, void* C, const void* R, 
                           long long lda, long long ldb, long long ldc, long long ldr, int a_mn_major,
                           int b_mn_major, int epi, float alpha, int sm_limit, void* stream);
 
+/* The form such a product runs in: columns of its 256-row tiles, and how many slices of K are summed (1: one sum along K). It follows
+ * from the arguments alone, so the order of summation is the same on every GPU. Needs no GPU. Not for CAI_EPI_SWIGLU_BWD. */
+CAI_API int cai_gemm_bf16_form(int M, int N, int K, int groups, int epi, int segmented, int* tile_cols, int* slices);
+
 /* Same product over ragged slabs (expert buffers of a mixture-of-experts layer). The segmented
  * dimension is cut into slabs of seg_rows rows (a multiple of 128); only the first
  * seg_counts[slab] rows of a slab hold data (device array). seg_mode 1: M is segmented, output

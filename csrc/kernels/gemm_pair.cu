@@ -668,26 +668,6 @@ static bool pair_operand_maps(CUtensorMap* tmA, CUtensorMap* tmB, const void* A,
                           : pair_map(tmB, g, B, g.K, g.N, g.ldb, g.grp_b, 64, pair::kBK, 2));
 }
 
-// Split clusters of S pairs the device can hold at once (0: this form cannot run there).
-template <int S>
-static int split_clusters(int dev) {
-    static int count[64];   // value + 1, 0 = not asked yet
-    if (dev < 0 || dev >= 64) return 0;
-    if (!count[dev]) {
-        cudaLaunchConfig_t cfg = {};
-        cudaLaunchAttribute attr[1];
-        split_config<S>(cfg, attr, 2 * S, nullptr);
-        int n = 0;
-        if (cudaFuncSetAttribute(gemm_pair_split_kernel<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, pair::kSplitSmem) != cudaSuccess ||
-            cudaOccupancyMaxActiveClusters(&n, gemm_pair_split_kernel<S>, &cfg) != cudaSuccess) {
-            cudaGetLastError();
-            n = 0;
-        }
-        count[dev] = n + 1;
-    }
-    return count[dev] - 1;
-}
-
 template <int S>
 static int launch_split(const void* A, const void* B, const GemmShape& g, PairParams& p, cudaStream_t st) {
     constexpr int BN = pair::kSplitBN;
@@ -696,6 +676,15 @@ static int launch_split(const void* A, const void* B, const GemmShape& g, PairPa
     p.tiles_m = (p.M + pair::kBM - 1) / pair::kBM;
     p.tiles_n = (p.N + BN - 1) / BN;
     p.group_m = 8;
+    static bool configured[64] = {};
+    const int dev = current_device();
+    if (!configured[dev & 63]) {
+        if (cudaFuncSetAttribute(gemm_pair_split_kernel<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, pair::kSplitSmem) != cudaSuccess) {
+            set_last_error("cudaFuncSetAttribute(gemm_pair_split) failed: %s", cudaGetErrorString(cudaGetLastError()));
+            return CAI_K_CUDA;
+        }
+        configured[dev & 63] = true;
+    }
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     split_config<S>(cfg, attr, static_cast<unsigned>(2 * S * p.tiles_m * p.tiles_n * p.groups), st);
@@ -739,6 +728,34 @@ static int launch_pair(const void* A, const void* B, const GemmShape& g, PairPar
     return CAI_K_OK;
 }
 
+// Which form: the smallest estimate in SM cycles on a B200 of 74 pairs. A stage of 128 k-elements takes a CTA about 1150 cycles in the
+// 256-wide tile (1024 of MMA) and 850 in the 128-wide one (48 KB at 54 B / cycle; 512 of MMA); a wave of tiles adds the part of its
+// epilogue that nothing hides, the split form the exchange of its partials. The split form ends where its clusters no longer
+// run at once: 33 of 4 and 15 of 8 CTAs are resident where the 148 SMs sit in groups of 16 to 20 (a GPU that holds fewer takes a second
+// wave there). Nothing of the device enters the rule: the order of summation follows from the shape alone, on every GPU and under
+// every limit on the SMs.
+// Every form at 27 counts of 256 x 128 tiles from 2 to 160 and K from 256 to 8192, both operand orders (324 products): the choice is
+// within 3 % of the best form but for K = 512 in at most 8 tiles of an MN-major product (8.5 us, 4 slices 7.8). us, 256-wide /
+// 128-wide / 2 / 4 slices:
+//   14 tiles, K 2048  15.4 / 13.4 / 10.7 /  9.3       16 tiles  15.4 / 13.7 / 10.7 / 16.5      33 tiles  15.6 / 13.9 / 11.3 / 24.8
+//   36 tiles, K 2048  15.6 / 14.0 / 20.3 / 24.8       72 tiles  16.5 / 14.6 / 30.3 / 41.2      80 tiles  16.4 / 23.1
+//   16 tiles, K 512    8.8 /  7.4 /  7.9 / 13.6      135 tiles, K 2048  26.2 / 23.8            160 tiles, K 2048  26.9 / 32.7
+PairForm pair_form(int M, int N, int K, int groups, int epi, bool segmented) {
+    constexpr long long kPairs = 74, kSplitTiles2 = 33, kSplitTiles4 = 15;
+    const long long ks = (K + 127) / 128, tm = (M + pair::kBM - 1) / pair::kBM;
+    const long long t256 = tm * ((N + 255) / 256) * groups, t128 = tm * ((N + 127) / 128) * groups;
+    const double wide = static_cast<double>((t256 + kPairs - 1) / kPairs) * (ks * 1150.0 + 2500.0);
+    const double narrow = static_cast<double>((t128 + kPairs - 1) / kPairs) * (ks * 850.0 + 1500.0);
+    if (epi == CAI_EPI_SWIGLU) return {256, 1};
+    if (!segmented) {
+        const double two = ks >= 2 && t128 <= kSplitTiles2 ? (ks + 1) / 2 * 850.0 + 4500.0 : 1e30;
+        const double four = ks >= 4 && t128 <= kSplitTiles4 ? (ks + 3) / 4 * 850.0 + 4500.0 : 1e30;
+        if (four < two && four < wide && four < narrow) return {pair::kSplitBN, 4};
+        if (two < wide && two < narrow) return {pair::kSplitBN, 2};
+    }
+    return {wide <= narrow ? 256 : 128, 1};
+}
+
 int gemm_pair(const void* A, const void* B, const GemmShape& g, cudaStream_t st) {
     PairParams p;
     p.M = g.M; p.N = g.N; p.K = g.K;
@@ -753,25 +770,20 @@ int gemm_pair(const void* A, const void* B, const GemmShape& g, cudaStream_t st)
     p.status = status_words(dev);
     const int pairs = sm_count(dev) / 2;
     const int usable = g.sm_limit > 1 && g.sm_limit / 2 < pairs ? g.sm_limit / 2 : pairs;
-    // Which form: the smallest estimate in SM cycles. A stage of 128 k-elements takes a CTA about 1150 cycles in the 256-wide
-    // tile (1024 of MMA) and 850 in the 128-wide one (48 KB at 54 B / cycle; 512 of MMA); a wave of tiles adds the part of its
-    // epilogue that nothing hides, the split form the exchange of its partials. Measured, 256-wide / 128-wide / 2 / 4 slices:
-    // 3840 x 1000 x 2728 29.0 / 35.4 / 55.2 / 80.6 us, 333 x 3000 x 1024 16.6 / 12.5 / 18.8 / 27.0 us, 333 x 1024 x 3000
-    // 20.7 / 18.6 / 14.5 / 16.6 us (one-CTA kernel: 39.7, 16.2, 24.7 us). The rule looks at the shape only, so that a limit on the
-    // SMs does not change the order of summation.
-    const long long ks = (g.K + 127) / 128, tm = (g.M + pair::kBM - 1) / pair::kBM;
-    const long long t256 = tm * ((g.N + 255) / 256) * g.groups, t128 = tm * ((g.N + 127) / 128) * g.groups;
-    const double wide = static_cast<double>((t256 + pairs - 1) / pairs) * (ks * 1150.0 + 2500.0);
-    const double narrow = static_cast<double>((t128 + pairs - 1) / pairs) * (ks * 850.0 + 1500.0);
-    if (p.epi != CAI_EPI_SWIGLU && !p.seg_mode) {
-        // clusters of 4 and 8 that fit at once (33 and 15 on a GPU whose 148 SMs sit in groups of 16 to 20)
-        const bool fits2 = ks >= 2 && t128 <= split_clusters<2>(dev), fits4 = ks >= 4 && t128 <= split_clusters<4>(dev);
-        const double two = fits2 ? (ks + 1) / 2 * 850.0 + 4500.0 : 1e30, four = fits4 ? (ks + 3) / 4 * 850.0 + 4500.0 : 1e30;
-        if (four < two && four < wide && four < narrow) return launch_split<4>(A, B, g, p, st);
-        if (two < wide && two < narrow) return launch_split<2>(A, B, g, p, st);
-    }
-    if (p.epi == CAI_EPI_SWIGLU || wide <= narrow) return launch_pair<256>(A, B, g, p, usable, st);
-    return launch_pair<128>(A, B, g, p, usable, st);
+    const PairForm f = pair_form(g.M, g.N, g.K, g.groups, g.epi, g.seg_mode != 0);
+    if (f.slices == 4) return launch_split<4>(A, B, g, p, st);
+    if (f.slices == 2) return launch_split<2>(A, B, g, p, st);
+    return f.tile_cols == 256 ? launch_pair<256>(A, B, g, p, usable, st) : launch_pair<128>(A, B, g, p, usable, st);
 }
 
 }  // namespace cai
+
+using namespace cai;
+
+CAI_API int cai_gemm_bf16_form(int M, int N, int K, int groups, int epi, int segmented, int* tile_cols, int* slices) {
+    if (M <= 0 || N <= 0 || K <= 0 || groups <= 0 || epi < 0 || epi > CAI_EPI_SWIGLU) return CAI_K_BAD_ARG;
+    const PairForm f = pair_form(M, N, K, groups, epi, segmented != 0);
+    *tile_cols = f.tile_cols;
+    *slices = f.slices;
+    return CAI_K_OK;
+}
