@@ -44,14 +44,18 @@ CAI_API int cai_sm_count(void);
 /* C[M,N] = alpha * sum_k A(m,k) B(n,k).
  * a_mn_major = 0: A is stored [M,K] (pitch lda); 1: A is stored [K,M].
  * b_mn_major = 0: B is stored [N,K] (pitch ldb); 1: B is stored [K,N].
- * sm_limit > 0 caps the number of CTAs (to leave SMs to a concurrent stream). */
+ * sm_limit > 0 caps the number of CTAs that run at once (to leave SMs to a concurrent stream); the result does not depend on it. CTAs come
+ * in clusters: 2, or 2 per slice where the product is cut along K (cai_gemm_bf16_form), so that a limit below that runs one
+ * cluster, of at most 8 CTAs. */
 CAI_API int cai_gemm_bf16(const void* A, const void* B, void* C, const void* R, int M, int N, int K,
                           long long lda, long long ldb, long long ldc, long long ldr, int a_mn_major,
                           int b_mn_major, int epi, float alpha, int sm_limit, void* stream);
 
 /* The form such a product runs in: columns of its 256-row tiles, and how many slices of K are summed (1: one sum along K). It follows
- * from the arguments alone, so the order of summation is the same on every GPU. Needs no GPU. Not for CAI_EPI_SWIGLU_BWD. */
-CAI_API int cai_gemm_bf16_form(int M, int N, int K, int groups, int epi, int segmented, int* tile_cols, int* slices);
+ * from the arguments alone, so the order of summation is the same on every GPU. ctas: the most CTAs of one launch on `sms` SMs under sm_limit.
+ * Needs no GPU. Not for CAI_EPI_SWIGLU_BWD. */
+CAI_API int cai_gemm_bf16_form(int M, int N, int K, int groups, int epi, int segmented, int sms, int sm_limit, int* tile_cols, int* slices,
+                               int* ctas);
 
 /* Same product over ragged slabs (expert buffers of a mixture-of-experts layer). The segmented
  * dimension is cut into slabs of seg_rows rows (a multiple of 128); only the first

@@ -48,6 +48,7 @@ struct PairParams {
     int epi;
     float alpha;
     int tiles_m, tiles_n, group_m, groups;
+    int tile0;                    // split form: first tile of this launch
     const int* seg_counts;
     int seg_rows, seg_mode, grp_seg;
     void* C;                      // split form: results leave through registers
@@ -517,7 +518,7 @@ gemm_pair_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
     const uint32_t tmem_base = *tmem_slot;
 
     int tm, tn, grp;
-    pair_tile_coords(p, static_cast<int>(blockIdx.x) / (2 * S), tm, tn, grp);
+    pair_tile_coords(p, p.tile0 + static_cast<int>(blockIdx.x) / (2 * S), tm, tn, grp);
     const int num_kb = (p.K + kBK - 1) / kBK;
     const int num_ks = (num_kb + kPerStage - 1) / kPerStage;
     const int ks0 = num_ks * slice / S, ks1 = num_ks * (slice + 1) / S;
@@ -669,7 +670,7 @@ static bool pair_operand_maps(CUtensorMap* tmA, CUtensorMap* tmB, const void* A,
 }
 
 template <int S>
-static int launch_split(const void* A, const void* B, const GemmShape& g, PairParams& p, cudaStream_t st) {
+static int launch_split(const void* A, const void* B, const GemmShape& g, PairParams& p, int at_once, cudaStream_t st) {
     constexpr int BN = pair::kSplitBN;
     CUtensorMap tmA, tmB;
     if (!pair_operand_maps(&tmA, &tmB, A, B, g, BN)) return CAI_K_BAD_ARG;
@@ -685,13 +686,17 @@ static int launch_split(const void* A, const void* B, const GemmShape& g, PairPa
         }
         configured[dev & 63] = true;
     }
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[1];
-    split_config<S>(cfg, attr, static_cast<unsigned>(2 * S * p.tiles_m * p.tiles_n * p.groups), st);
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_pair_split_kernel<S>, tmA, tmB, p);
-    if (e != cudaSuccess) {
-        set_last_error("gemm_pair_split launch failed: %s", cudaGetErrorString(e));
-        return CAI_K_CUDA;
+    // Under a limit on the SMs the clusters go out in turns of `at_once`, one launch behind the other: the same sums in the same order.
+    const int tiles = p.tiles_m * p.tiles_n * p.groups;
+    for (p.tile0 = 0; p.tile0 < tiles; p.tile0 += at_once) {
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute attr[1];
+        split_config<S>(cfg, attr, static_cast<unsigned>(2 * S * (tiles - p.tile0 < at_once ? tiles - p.tile0 : at_once)), st);
+        const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_pair_split_kernel<S>, tmA, tmB, p);
+        if (e != cudaSuccess) {
+            set_last_error("gemm_pair_split launch failed: %s", cudaGetErrorString(e));
+            return CAI_K_CUDA;
+        }
     }
     return CAI_K_OK;
 }
@@ -756,6 +761,14 @@ PairForm pair_form(int M, int N, int K, int groups, int epi, bool segmented) {
     return {wide <= narrow ? 256 : 128, 1};
 }
 
+// Clusters (of 2 CTAs per slice) that one launch may hold: persistent pairs, or tiles of the split form.
+static int pair_clusters(const PairForm& f, int sms, int sm_limit) {
+    const int cluster = 2 * f.slices;
+    if (sm_limit <= 0 && f.slices > 1) return 1 << 20;   // every tile in one launch
+    const int n = (sm_limit > 0 && sm_limit < sms ? sm_limit : sms) / cluster;
+    return n < 1 ? 1 : n;                                // a cluster is the least that can run
+}
+
 int gemm_pair(const void* A, const void* B, const GemmShape& g, cudaStream_t st) {
     PairParams p;
     p.M = g.M; p.N = g.N; p.K = g.K;
@@ -766,24 +779,28 @@ int gemm_pair(const void* A, const void* B, const GemmShape& g, cudaStream_t st)
     p.C = g.C;
     p.R = static_cast<const __nv_bfloat16*>(g.R);
     p.ldc = g.ldc; p.ldr = g.ldr; p.grp_c = g.grp_c;
+    p.tile0 = 0;
     const int dev = current_device();
     p.status = status_words(dev);
-    const int pairs = sm_count(dev) / 2;
-    const int usable = g.sm_limit > 1 && g.sm_limit / 2 < pairs ? g.sm_limit / 2 : pairs;
     const PairForm f = pair_form(g.M, g.N, g.K, g.groups, g.epi, g.seg_mode != 0);
-    if (f.slices == 4) return launch_split<4>(A, B, g, p, st);
-    if (f.slices == 2) return launch_split<2>(A, B, g, p, st);
-    return f.tile_cols == 256 ? launch_pair<256>(A, B, g, p, usable, st) : launch_pair<128>(A, B, g, p, usable, st);
+    const int at_once = pair_clusters(f, sm_count(dev), g.sm_limit);
+    if (f.slices == 4) return launch_split<4>(A, B, g, p, at_once, st);
+    if (f.slices == 2) return launch_split<2>(A, B, g, p, at_once, st);
+    return f.tile_cols == 256 ? launch_pair<256>(A, B, g, p, at_once, st) : launch_pair<128>(A, B, g, p, at_once, st);
 }
 
 }  // namespace cai
 
 using namespace cai;
 
-CAI_API int cai_gemm_bf16_form(int M, int N, int K, int groups, int epi, int segmented, int* tile_cols, int* slices) {
+CAI_API int cai_gemm_bf16_form(int M, int N, int K, int groups, int epi, int segmented, int sms, int sm_limit, int* tile_cols, int* slices,
+                               int* ctas) {
     if (M <= 0 || N <= 0 || K <= 0 || groups <= 0 || epi < 0 || epi > CAI_EPI_SWIGLU) return CAI_K_BAD_ARG;
     const PairForm f = pair_form(M, N, K, groups, epi, segmented != 0);
     *tile_cols = f.tile_cols;
     *slices = f.slices;
+    const long long tiles = static_cast<long long>((M + pair::kBM - 1) / pair::kBM) * ((N + f.tile_cols - 1) / f.tile_cols) * groups;
+    const int at_once = pair_clusters(f, sms, sm_limit);
+    *ctas = static_cast<int>(2 * f.slices * (tiles < at_once ? tiles : at_once));
     return CAI_K_OK;
 }

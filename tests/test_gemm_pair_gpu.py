@@ -114,3 +114,22 @@ def test_pair_gemm_short_kernels_on_two_streams():
     for o, (_, _, ref, bound, _) in zip(outs, cases):
         assert all(((v - ref).abs() <= bound).all() for v in o)
     assert _lib.device_status(clear=True) == 0
+
+
+# A limit on the SMs in every form: persistent wide and narrow, two and four slices (in turns of several launches): the same bits, with
+# every epilogue, and the ragged last turn.
+@pytest.mark.parametrize("M,N,K", [(4096, 4104, 264), (1536, 1536, 520), (333, 1024, 3000), (300, 968, 2048)])
+def test_pair_gemm_under_a_limit(M, N, K):
+    from cai_b200 import ops
+    from cai_b200.ops import _lib
+    torch.manual_seed(6)
+    a = torch.randn(M, K, device="cuda").to(torch.bfloat16)
+    b = torch.randn(N, K, device="cuda").to(torch.bfloat16)
+    res = torch.randn(M, N, device="cuda").to(torch.bfloat16)
+    old = torch.randn(M, N, device="cuda")
+    want = ops.gemm(a, b, out_dtype=torch.float32), ops.gemm(a, b, residual=res), ops.gemm(a, b, out=old.clone(), accumulate=True)
+    for limit in (1, 2, 10, 60, 147):
+        got = (ops.gemm(a, b, out_dtype=torch.float32, sm_limit=limit), ops.gemm(a, b, residual=res, sm_limit=limit),
+               ops.gemm(a, b, out=old.clone(), accumulate=True, sm_limit=limit))
+        assert all(torch.equal(x, y) for x, y in zip(got, want)), limit
+    assert _lib.device_status(clear=True) == 0
