@@ -11,9 +11,9 @@
 // Warp 0 feeds a ring of shared-memory stages with TMA (no multicast: every CTA loads its own part), warp 1 of the even CTA
 // issues the MMAs, warps 2-9 drain the accumulator. Two accumulators per CTA in TMEM let the epilogue of a tile overlap the
 // main loop of the next. The epilogue goes through shared memory and leaves by TMA: full 128-byte rows instead of 16 bytes per
-// lane, edges clipped by the tensor map, the fp32 accumulation into C as a TMA reduction in L2 (one rounding, like a load and
-// an add); the residual is read into registers while the main loop still runs. (bf16 stores straight from the registers, a
-// 32-byte sector per lane, measured the same on aligned rows and up to 20 % slower on rows of 2000 bytes.)
+// lane, edges clipped by the tensor map, the fp32 accumulation into C as a TMA reduction in L2 (one rounding and subnormals kept,
+// like a load and an add); the residual is read into registers while the main loop still runs. (bf16 stores straight from the
+// registers, a 32-byte sector per lane, measured the same on aligned rows and up to 20 % slower on rows of 2000 bytes.)
 //
 // Measured against the one-CTA kernel (L2 flushed): 8192^3 812 -> 706 us (1556 TFLOP/s), 16384 x 2048 x 16384 1062 -> 712 us,
 // 16384 x 16384 x 2048 with SwiGLU 1026 -> 773 us, weight gradient 16384 x 2048 x 16384 1117 -> 794 us. One barrier round trip per

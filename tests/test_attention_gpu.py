@@ -83,3 +83,21 @@ def test_flash_attn_bwd_rings(B, S, nh, nkv):
     # P, dS and the results are rounded to bf16 (2^-9 relative each, independent): well under 1e-2 in the 2-norm
     rel = ((dqkv.float() - x.grad).norm() / x.grad.norm()).item()
     assert rel < 1e-2, rel
+
+
+def test_flash_attn_bwd_takes_an_output_on_eight_bytes():
+    """The row sums of dO * O read O in 16-byte pieces where it lies on 16 bytes and in 8-byte pieces where it does not: the same bits."""
+    from cai_b200 import ops
+    torch.manual_seed(3)
+    B, S, nh, nkv, hd = 3, 384, 3, 1, 128
+    qkv = torch.randn(B * S, (nh + 2 * nkv) * hd, device="cuda").to(torch.bfloat16)
+    dout = torch.randn(B * S, nh * hd, device="cuda").to(torch.bfloat16)
+    out, lse = ops.flash_attn_fwd(qkv, B, S, nh, nkv, hd)
+    room = torch.empty(out.numel() + 4, device="cuda", dtype=torch.bfloat16)
+    moved = room[4:].view_as(out).copy_(out)
+    assert moved.data_ptr() % 16 == 8
+    d = [torch.empty(B, nh, S, device="cuda") for _ in range(2)]
+    got = [ops.flash_attn_bwd(qkv, o, dout, lse, B, S, nh, nkv, hd, delta=x) for o, x in zip((out, moved), d)]
+    assert torch.equal(d[0], d[1]) and torch.equal(got[0], got[1])
+    want = (dout.float() * out.float()).view(B, S, nh, hd).sum(-1).transpose(1, 2)
+    assert ((d[0] - want).abs() <= 2.0 ** -23 * 128 * (dout.float() * out.float()).abs().view(B, S, nh, hd).sum(-1).transpose(1, 2)).all()

@@ -133,3 +133,53 @@ def test_pair_gemm_under_a_limit(M, N, K):
                ops.gemm(a, b, out=old.clone(), accumulate=True, sm_limit=limit))
         assert all(torch.equal(x, y) for x, y in zip(got, want)), limit
     assert _lib.device_status(clear=True) == 0
+
+
+FORMS = [(4096, 4104, 264), (1536, 1536, 520), (336, 1024, 3000), (256, 1920, 2048)]     # 256-wide, 128-wide, two and four slices
+
+
+def _padded(rows, cols, pad, value=7.0, dtype=torch.bfloat16):
+    """A random matrix as the left part of rows that are `pad` wider, and the whole."""
+    whole = torch.full((rows, cols + pad), value, device="cuda", dtype=dtype)
+    whole[:, :cols] = torch.randn(rows, cols, device="cuda").to(dtype)
+    return whole[:, :cols], whole
+
+
+# Pitches wider than the row for every operand, and the residual read in place of the result: the bits of the plain call, and nothing
+# touched beside the rows.
+@pytest.mark.parametrize("ta,tb", [(False, False), (True, True)])
+@pytest.mark.parametrize("M,N,K", FORMS)
+def test_pair_gemm_pitches_and_residual_in_place(M, N, K, ta, tb):
+    from cai_b200 import ops
+    torch.manual_seed(8)
+    a, _ = _padded(*((K, M) if ta else (M, K)), 16)
+    b, _ = _padded(*((K, N) if tb else (N, K)), 24)
+    res, res_whole = _padded(M, N, 40)
+    kw = dict(trans_a=ta, trans_b=tb)
+    want = ops.gemm(a.contiguous(), b.contiguous(), residual=res.contiguous(), **kw)
+    assert torch.equal(ops.gemm(a, b, residual=res, **kw), want)
+    ref = ((a.t() if ta else a).float() @ (b if tb else b.t()).float()) + res.float()
+    bound = 2 * K * 2.0 ** -24 * ((a.t() if ta else a).float().abs() @ (b if tb else b.t()).float().abs()) + 2.0 ** -8 * ref.abs() + 1e-6
+    assert ((want.float() - ref).abs() <= bound).all()       # two sums of K exact products, one rounding to bf16
+    out, out_whole = _padded(M, N, 8)
+    ops.gemm(a, b, residual=res, out=out, **kw)
+    assert torch.equal(out, want) and bool((out_whole[:, N:] == 7.0).all())
+    ops.gemm(a, b, residual=res, out=res, **kw)
+    assert torch.equal(res, want) and bool((res_whole[:, N:] == 7.0).all())
+    acc, acc_whole = _padded(M, N, 4, dtype=torch.float32)
+    want32 = ops.gemm(a.contiguous(), b.contiguous(), out=acc.contiguous(), accumulate=True, **kw)
+    ops.gemm(a, b, out=acc, accumulate=True, **kw)
+    assert torch.equal(acc, want32) and bool((acc_whole[:, N:] == 7.0).all())
+
+
+# Adding to gradients below 2^-126: the persistent forms add in L2, the split form in registers; neither flushes. All values exact.
+@pytest.mark.parametrize("M,N,K", [(4096, 4104, 64), (256, 128, 64), (336, 1024, 3000)])
+def test_accumulation_keeps_subnormals(M, N, K):
+    from cai_b200 import ops
+    a = torch.zeros(M, K, device="cuda", dtype=torch.bfloat16)
+    b = torch.zeros(N, K, device="cuda", dtype=torch.bfloat16)
+    a[:, 0], b[:, 0] = 2.0 ** -100, 2.0 ** -30
+    for old in (0.0, 2.0 ** -130, 2.0 ** -140, -2.0 ** -126):
+        out = torch.full((M, N), old, device="cuda")
+        ops.gemm(a, b, out=out, accumulate=True)
+        assert bool((out.double() == old + 2.0 ** -130).all()), old
