@@ -6,8 +6,8 @@
 //                          below the diagonal of every query head of the group and accumulates
 //                          dK and dV in tensor memory. Scores are computed transposed
 //                          (S^T = K Q^T, dP^T = V dO^T) so that TMEM lanes are kv rows; the bf16
-//                          P^T and dS^T are written back over S^T / dP^T and feed
-//                          dV += P^T dO and dK += dS^T Q as A operands straight from TMEM.
+//                          P^T goes through shared memory and feeds dV += P^T dO from there, dS^T is
+//                          written back over dP^T and feeds dK += dS^T Q as A operand straight from TMEM.
 //   3. attn_dq_kernel      one CTA per (q tile, head, batch): S = Q K^T, dP = dO V^T,
 //                          dS -> TMEM, dQ += dS K.
 // Q, K, V and dO tiles arrive by TMA from the packed activation; each shared-memory tile serves
@@ -71,7 +71,7 @@ __device__ unsigned int g_attn_chain[kAttnChainSlots];
 
 // Sixteen lanes per (token, head), 16 bytes a lane from each tensor, kDeltaUnroll of them in flight per thread: what bounds this is
 // bytes in flight (one pair of 8-byte loads per thread and a 64-bit division in front: 8192 tokens of
-// 32 heads 47 -> 29 us, 3 x 640 tokens of 9 heads 7.6 -> 4.5 us). The tensors are walked as one array of
+// 32 heads 47 -> 23 us, 6 x 640 tokens of 9 heads 8.5 -> 6.2 us). The tensors are walked as one array of
 // 128-element rows. (dO starts on 16 bytes, or its tensor map is refused; O may start on 8.)
 constexpr int kDeltaUnroll = 2;
 __global__ void __launch_bounds__(256)

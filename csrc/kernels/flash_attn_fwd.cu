@@ -3,8 +3,8 @@
 // One CTA owns two adjacent 128-row query tiles (A and B) of one head and sweeps the key/value
 // tiles they may attend to. Warp 0 streams Q, K and V tiles with TMA straight out of the packed
 // QKV activation; warps 1 and 2 issue the tcgen05 MMAs of tile A and tile B (one issuer for both left a tile
-// waiting behind the other's barriers: 3 x 640 tokens, 9 / 3 heads 26.0 -> 23.7 us, 8192 tokens, 32 / 8 heads
-// 615 -> 581 us); warps 4-7 and 8-11 are the softmax groups of
+// waiting behind the other's barriers: 6 x 640 tokens, 9 / 3 heads 28.5 -> 26.1 us, 8192 tokens, 32 / 8 heads
+// 658 -> 618 us); warps 4-7 and 8-11 are the softmax groups of
 // tile A and tile B, one thread per query row. Scores live in tensor memory: S = Q K^T lands in
 // TMEM, the softmax group reads it with tcgen05.ld, writes the bf16 probabilities back over the
 // same columns with tcgen05.st, and O += P V consumes P directly from TMEM as the A operand.

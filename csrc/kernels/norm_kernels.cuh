@@ -173,9 +173,8 @@ rmsnorm_bwd_dg_kernel(const __nv_bfloat16* __restrict__ x, const float* __restri
 
 // out[col] (+)= sum over parts of parts[p][col]. A block covers 32 columns. The rows form 32 chains, p modulo 32 (rows past the
 // last round of four chains that are 8 apart go to the first of them), one warp each: what bounds this is the number of
-// dependent loads in a row (eight warps with four chains each: 240 rows of 1000
-// 5.6 -> 3.4 us, 296 rows of 2048 7.7 -> 4.6 us). Chains are added in fours, the eight
-// sums in order.
+// dependent loads in a row (eight warps with four chains each: 296 rows of 1000 and of 2048 columns, cold
+// caches, 10.6 and 10.3 -> 5.5 us). Chains are added in fours, the eight sums in order.
 constexpr int kReduceWarps = 32;
 static __global__ void __launch_bounds__(kReduceWarps * 32)
 reduce_parts_kernel(const float* __restrict__ parts, float* __restrict__ out, int nparts, int H, int accumulate) {
@@ -208,7 +207,9 @@ reduce_parts_kernel(const float* __restrict__ parts, float* __restrict__ out, in
 // two-kernel form above reads them twice), the old dx together with them. Two CTAs of eight warps share an SM.
 // What bounds it is bytes in flight, and for few rows the combination of the sums: warps that took turns adding into one
 // row, eight lanes to a bank, needed 3 us more.
-// 16384 x 2048 with an accumulated dx: 88 -> 74 us (3.6 TB/s), 1920 x 1000: 14.5 -> 11.4 us.
+// With an accumulated dx and cold caches, 16384 x 2048: 74.8 -> 58.5 us (4.6 TB/s), 3840 x 1000: 15.6 -> 12.8 us.
+// Beside a product of another stream it runs on the SMs that one leaves free: none of its CTAs was seen to share an SM with a
+// persistent product's, whatever the shared memory either asks for.
 constexpr int kNormFusedThreads = 256;
 constexpr int kNormFusedCols = 1024;   // columns one warp covers: 32 lanes x 4 chunks x 8 elements
 constexpr int kNormFusedMaxH = 8192;
