@@ -7,7 +7,7 @@
 Every cost in ``csrc/plan/backend_calibrated.cc`` is linear in its constants once the op's shape is known, so each
 group is an ordinary least-squares problem over the ops of that kind in the trace:
 
-  GEMM (per operand class)   t = launch + waves * tile_us + (waves * tile FLOPs) / per-SM rate
+  GEMM (per operand class)   t = launch + waves * tile_us + (waves * tile FLOPs) / per-SM rate    (plain products, on pairs of SMs)
   attention                  t = fixed + steps * step_us            (forward; dK / dV and dQ parts of the backward)
   pointwise kernels          t = fixed + operand MB * us_per_mb
 
@@ -26,6 +26,7 @@ from . import K_GEMM, PlanFile
 from .compare import load
 
 SMS = 148
+EPI_SWIGLU_BWD = 5     # runs on the one-CTA kernel
 K_RMSNORM_FWD, K_RMSNORM_BWD, K_ROPE, K_ATTN_FWD, K_ATTN_BWD, K_SWIGLU_FWD, K_SWIGLU_BWD = 3, 4, 6, 7, 8, 9, 10
 K_CROSS_ENTROPY, K_ADAMW, K_CROSS_ENTROPY_TP, K_EMBED_FWD, K_EMBED_BWD = 11, 12, 29, 1, 2
 POINTWISE = {K_RMSNORM_FWD: "rmsnorm_fwd", K_RMSNORM_BWD: "rmsnorm_bwd", K_ROPE: "rope", K_SWIGLU_FWD: "swiglu",
@@ -34,10 +35,18 @@ POINTWISE = {K_RMSNORM_FWD: "rmsnorm_fwd", K_RMSNORM_BWD: "rmsnorm_bwd", K_ROPE:
 
 
 def gemm_features(M, N, K, sms=SMS):
-    bn = 256.0 if N % 256 == 0 else 128.0
-    tiles = math.ceil(M / 128.0) * math.ceil(N / bn)
-    waves = max(1.0, math.ceil(tiles / sms))
-    return waves, waves * 2.0 * 128.0 * bn * K
+    """Waves of tiles and the FLOPs an SM gets through in them, in the form the kernel's rule picks (csrc/kernels/gemm_pair.cu): 256 x 256
+    or 256 x 128 tiles on pairs of SMs (a narrow tile takes 0.74 of a wide one's time), or slices of K of one wave of tiles."""
+    pairs, ks, tm = sms // 2, math.ceil(K / 128), math.ceil(M / 256)
+    t256, t128 = tm * math.ceil(N / 256), tm * math.ceil(N / 128)
+    w256, w128 = math.ceil(t256 / pairs), math.ceil(t128 / pairs)
+    forms = [(w256 * (ks * 1150.0 + 2500.0), w256, 1.0), (w128 * (ks * 850.0 + 1500.0), w128, 0.74)]
+    if ks >= 2 and t128 <= 33:
+        forms.append((math.ceil(ks / 2) * 850.0 + 4500.0, 1, 0.74 / 2))
+    if ks >= 4 and t128 <= 15:
+        forms.append((math.ceil(ks / 4) * 850.0 + 4500.0, 1, 0.74 / 4))
+    _, waves, part = min(forms, key=lambda f: f[0])
+    return waves, waves * part * 256.0 * 256.0 * K
 
 
 def attention_steps(B, S, nh, nkv, sms=SMS):
@@ -75,7 +84,7 @@ def fit(pairs):
     for pf, op, us in ops:
         x = pf.exec[op.exec - 1]
         k = int(x.kernel)
-        if k == K_GEMM and not (x.flags & 0x100):
+        if k == K_GEMM and not (x.flags & 0x100) and (x.flags >> 4) & 0xF != EPI_SWIGLU_BWD:
             waves, wf = gemm_features(x.i[0], x.i[1], x.i[2])
             rows, ys = gemm[x.flags & 1]
             rows.append([1.0, waves, wf * 1e-6])          # us = launch + waves * tile_us + wf / rate   (rate in FLOP/us)

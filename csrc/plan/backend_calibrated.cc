@@ -8,8 +8,10 @@
 // each fill the GPU do not speed each other up by sitting on different streams).
 //
 // Model per kernel (constants: `Calibration`, overridable from a key = value file; sources in the comments there):
-//   GEMM            launch + waves * (tile overhead + tile FLOPs / per-SM rate), 128 x 256 (or 128 x 128) tiles on 148 SMs,
-//                   a lower rate for transposed-A products (weight gradients)
+//   GEMM            launch + waves * (tile overhead + tile FLOPs / per-SM rate): tiles of 256 x 256 or 256 x 128 on 74 pairs of SMs, or
+//                   a slice of K of one, as the kernel's own rule has it; a lower rate for transposed-A products (weight
+//                   gradients). Products fused with a collective, SwiGLU's backward epilogue and e4m3: 128 x 256 (or 128 x
+//                   128) tiles on 148 SMs with constants of their own
 //   attention       per-CTA critical path: steps = max(all steps / SMs, longest CTA) * time per 128 x 128 step
 //   pointwise       per-kernel fixed cost + operand bytes * per-kernel microseconds per MB
 //   fused TP ops    launch + max(GEMM on the SMs left beside the copy CTAs, wire bytes / measured rate under all-to-all
@@ -35,16 +37,21 @@ struct PointCost {
 
 struct Calibration {
     int sms = 148;
-    // GEMM, fitted to the per-op CUDA-event times of the headline config inside a step on one GPU (fifteen shapes,
-    // fit error <= 13 %): [0] A not transposed, [1] A transposed (weight-gradient form)
-    double gemm_launch_us = 12.0;
-    double gemm_tile_us[2] = {0.5, 4.0};
-    double gemm_sm_flops[2] = {7.9e12, 6.9e12};
-    // fp8 block-scaled GEMM: 1708 against 1361 TFLOP/s at 8192^3
+    // Plain GEMM, fitted to the per-op CUDA-event times inside steps of six models on one GPU (the headline config in launches of
+    // 16384 and of 4096 tokens, two of its layers' tensor-parallel shards as models of their own, two 8B-class layers, a
+    // small ragged model; 90 shapes, median error 4 %): [0] A not transposed, [1] A transposed (weight-gradient form)
+    double gemm_launch_us = 10.3;
+    double gemm_tile_us[2] = {1.9, 0.2};
+    double gemm_sm_flops[2] = {10.7e12, 9.4e12};
+    int gemm_pairs = 1;             // 0: plain products run one CTA per 128-row tile, as the fused ones do
+    // One-CTA GEMM (fused with a collective): the headline config's shapes on one GPU, fit error <= 13 %
+    double fused_gemm_tile_us = 0.5;
+    double fused_gemm_sm_flops = 7.9e12;
+    // fp8 block-scaled GEMM against the one-CTA bf16 one: 1708 against 1361 TFLOP/s at 8192^3
     double fp8_speedup = 1.25;
-    // attention, microseconds per 128 x 128 step of one CTA (16 / 8 heads, seq 4096, batches 1 and 4)
-    double attn_fwd_step_us = 1.64, attn_fwd_fixed_us = 20.0;
-    double attn_dkdv_step_us = 3.08, attn_dq_step_us = 2.75, attn_bwd_fixed_us = 10.0;
+    // attention, microseconds per 128 x 128 step of one CTA (the same six models)
+    double attn_fwd_step_us = 1.69, attn_fwd_fixed_us = 17.0;
+    double attn_dkdv_step_us = 2.53, attn_dq_step_us = 2.00, attn_bwd_fixed_us = 16.5;
     // fused tensor-parallel kernels: bytes a GPU moves per second while every member pulls and pushes at once
     // (steady-state chains on 2 / 4 / 8 GPUs), copy CTAs of the all-gather form, tail of the reduce-scatter form
     double link_rate[4] = {0.60e12, 0.60e12, 0.45e12, 0.35e12};  // group size 1-2, 2, 4, 8
@@ -55,10 +62,11 @@ struct Calibration {
     // NCCL collectives and p2p next to compute
     double nccl_latency_us = 20.0;
     double nccl_rate = 0.60e12;   // bytes per GPU and second of ring collectives of 17-120 MB (NCCL arms of the chains)
-    // pointwise kernels (two points each: one GPU and eight GPUs of the headline config)
+    // pointwise kernels (the same six models; worst errors 6-14 %, the embedding's backward apart, whose time goes with how
+    // often a token repeats)
     PointCost point_default = {8.0, 0.20};
-    PointCost rmsnorm_fwd = {9.3, 0.143}, rmsnorm_bwd = {30.0, 0.327}, rope = {7.9, 0.262}, swiglu = {7.6, 0.158},
-              adamw = {10.0, 0.238}, cross_entropy = {10.0, 0.20}, embed = {15.0, 0.60};
+    PointCost rmsnorm_fwd = {6.4, 0.181}, rmsnorm_bwd = {14.7, 0.305}, rope = {5.8, 0.332}, swiglu = {5.3, 0.170},
+              adamw = {4.0, 0.2456}, cross_entropy = {14.2, 0.470}, embed = {15.0, 0.60};
 };
 
 bool set_key(Calibration* c, const std::string& k, double v) {
@@ -66,6 +74,7 @@ bool set_key(Calibration* c, const std::string& k, double v) {
     Entry table[] = {
         {"gemm_launch_us", &c->gemm_launch_us}, {"gemm_tile_us", &c->gemm_tile_us[0]}, {"gemm_tile_us_ta", &c->gemm_tile_us[1]},
         {"gemm_sm_flops", &c->gemm_sm_flops[0]}, {"gemm_sm_flops_ta", &c->gemm_sm_flops[1]}, {"fp8_speedup", &c->fp8_speedup},
+        {"fused_gemm_tile_us", &c->fused_gemm_tile_us}, {"fused_gemm_sm_flops", &c->fused_gemm_sm_flops},
         {"attn_fwd_step_us", &c->attn_fwd_step_us}, {"attn_fwd_fixed_us", &c->attn_fwd_fixed_us},
         {"attn_dkdv_step_us", &c->attn_dkdv_step_us}, {"attn_dq_step_us", &c->attn_dq_step_us},
         {"attn_bwd_fixed_us", &c->attn_bwd_fixed_us}, {"link_rate_2", &c->link_rate[1]}, {"link_rate_4", &c->link_rate[2]},
@@ -87,6 +96,7 @@ bool set_key(Calibration* c, const std::string& k, double v) {
         if (k == n + "_us_per_mb") { e.dst->us_per_mb = v; return true; }
     }
     if (k == "sms") { c->sms = static_cast<int>(v); return true; }
+    if (k == "gemm_pairs") { c->gemm_pairs = v != 0.0; return true; }
     if (k == "ag_copy_ctas") { c->ag_copy_ctas = static_cast<int>(v); return true; }
     return false;
 }
@@ -98,13 +108,41 @@ struct CalibratedImpl {
     uint32_t capacity_x100 = 200;
 };
 
-double gemm_seconds(const Calibration& c, double M, double N, double K, bool ta, int sms, double* share) {
-    const int cls = ta ? 1 : 0;
+// One CTA per tile of 128 rows.
+double one_cta_gemm_seconds(const Calibration& c, double tile_us, double sm_flops, double M, double N, double K, int sms, double* share) {
     const double bn = (static_cast<long long>(N) % 256 == 0) ? 256.0 : 128.0;
     const double tiles = std::ceil(M / 128.0) * std::ceil(N / bn);
     const double waves = std::max(1.0, std::ceil(tiles / sms));
     if (share) *share = std::min(1.0, tiles / (waves * c.sms));
-    return (c.gemm_launch_us + waves * (c.gemm_tile_us[cls] + 2.0 * 128.0 * bn * K / c.gemm_sm_flops[cls] * 1e6)) * 1e-6;
+    return (c.gemm_launch_us + waves * (tile_us + 2.0 * 128.0 * bn * K / sm_flops * 1e6)) * 1e-6;
+}
+
+double fused_gemm_seconds(const Calibration& c, double M, double N, double K, int sms, double* share) {
+    return one_cta_gemm_seconds(c, c.fused_gemm_tile_us, c.fused_gemm_sm_flops, M, N, K, sms, share);
+}
+
+// A plain product: pairs of SMs, a tile of 256 rows each. The form is chosen as the kernel chooses it (cycles per 128 k-elements and per
+// tile, see csrc/kernels/gemm_pair.cu); a 128-wide tile takes 0.74 of a 256-wide one's time.
+double gemm_seconds(const Calibration& c, double M, double N, double K, bool ta, int sms, double* share, double groups = 1.0) {
+    const int cls = ta ? 1 : 0;
+    if (!c.gemm_pairs) return one_cta_gemm_seconds(c, c.gemm_tile_us[cls], c.gemm_sm_flops[cls], M, N, K, sms, share);
+    const double pairs = std::max(1.0, std::floor(sms / 2.0)), ks = std::ceil(K / 128.0), tm = std::ceil(M / 256.0);
+    const double t256 = tm * std::ceil(N / 256.0) * groups, t128 = tm * std::ceil(N / 128.0) * groups;
+    const double w256 = std::max(1.0, std::ceil(t256 / pairs)), w128 = std::max(1.0, std::ceil(t128 / pairs));
+    const double wide = w256 * (ks * 1150.0 + 2500.0), narrow = w128 * (ks * 850.0 + 1500.0);
+    const double two = ks >= 2 && t128 <= 33 ? std::ceil(ks / 2.0) * 850.0 + 4500.0 : 1e30;
+    const double four = ks >= 4 && t128 <= 15 ? std::ceil(ks / 4.0) * 850.0 + 4500.0 : 1e30;
+    const double full = 2.0 * 256.0 * 256.0 * K / (2.0 * c.gemm_sm_flops[cls]) * 1e6;   // a 256-wide tile on a pair, microseconds
+    double waves = w256, tiles = t256, work = full;
+    if (four < two && four < wide && four < narrow) {
+        waves = 1.0; tiles = 4.0 * t128; work = 0.74 / 4.0 * full;
+    } else if (two < wide && two < narrow) {
+        waves = 1.0; tiles = 2.0 * t128; work = 0.74 / 2.0 * full;
+    } else if (narrow < wide) {
+        waves = w128; tiles = t128; work = 0.74 * full;
+    }
+    if (share) *share = std::min(1.0, tiles / (waves * (c.sms / 2.0)));
+    return (c.gemm_launch_us + waves * (c.gemm_tile_us[cls] + work)) * 1e-6;
 }
 
 double operand_mb(const CalibratedImpl& im, const ExecOp& x) {
@@ -137,16 +175,19 @@ double price(const CalibratedImpl& im, const Topology& topo, const Op& op, const
             const double live = std::min(1.0, 100.0 / std::max(100u, im.capacity_x100));
             if (x.i[4] == 2050) K *= live;   // weight-gradient form: the ragged dimension is K
             else M *= live;
-            if (x.i[4] == 2050) return experts * gemm_seconds(c, M, N, K, x.flags & 1, c.sms, share);
+            if (x.i[4] == 2050)
+                return c.gemm_pairs ? gemm_seconds(c, M, N, K, x.flags & 1, c.sms, share, experts)
+                                    : experts * gemm_seconds(c, M, N, K, x.flags & 1, c.sms, share);
             M *= experts;
         }
+        if (((x.flags >> 4) & 0xF) == 5 && c.gemm_pairs) return fused_gemm_seconds(c, M, N, K, c.sms, share);   // CAI_EPI_SWIGLU_BWD
         return gemm_seconds(c, M, N, K, x.flags & 1, c.sms, share);
     }
     case K_GEMM_FP8:
-        return gemm_seconds(c, x.i[0], x.i[1], x.i[2], false, c.sms, share) / c.fp8_speedup;
+        return fused_gemm_seconds(c, x.i[0], x.i[1], x.i[2], c.sms, share) / c.fp8_speedup;
     case K_AG_GEMM: case K_GEMM_RS: {
         const bool ag = x.kernel != K_GEMM_RS;
-        const double compute = gemm_seconds(c, x.i[0], x.i[1], x.i[2], x.flags & 1, ag ? c.sms - c.ag_copy_ctas : c.sms, nullptr);
+        const double compute = fused_gemm_seconds(c, x.i[0], x.i[1], x.i[2], ag ? c.sms - c.ag_copy_ctas : c.sms, nullptr);
         const double wire = n > 1 ? (n - 1.0) / n * static_cast<double>(op.bytes) / link_rate(c, n) : 0.0;
         const double tail = (x.kernel == K_GEMM_RS && n > 1) ? c.rs_tail_us * 1e-6 : 0.0;
         const double dur = c.fused_launch_us * 1e-6 + std::max(compute, wire) + tail;
