@@ -32,7 +32,8 @@ def test_config_5_is_predicted_within_five_percent_of_the_measured_step(tmp_path
     import bench
     from cai_b200 import plan
     paths, topo, d = _stage_plans(tmp_path, bench.config_text(8, "fused", "pp2tp4"), 2)
-    r = plan.pipeline_replay(paths, topo, backend="calibrated")
+    # by the kernels that this file of constants describes
+    r = plan.pipeline_replay(paths, topo, backend="calibrated", calibration=ROOT / "configs" / "b200_calibration_one_cta.cfg")
     assert abs(r["step_time_s"] * 1e3 - 2446.0) <= 0.05 * 2446.0, r
     # the step is the longer of the longest dependency path and the SM time of the busiest stage; here the stages are
     # SM-bound (weight-gradient GEMMs on the second compute stream fill the gaps of fill and drain)
