@@ -282,10 +282,8 @@ __device__ __forceinline__ uint2 quant8(const uint4& v, float inv) {
 
 // The same by 16 lanes per 128-column block, 16 bytes a lane, four blocks in flight per thread. What bounds this is bytes in
 // flight (the kernel above has 256 per warp, behind a division of 64-bit numbers). Measured, 8192 x 14336: 144 -> 62 us (2.4
-// -> 5.6 TB/s), 2000 x 14336: 36 -> 20 us. Rows of 16-byte aligned pieces only; the kernel above takes the rest, and what is
-// too little to fill the GPU with four blocks a thread: 2048 blocks 1.9 us against 2.3 here, 5328 2.3 against 2.5, 8192 2.7 against 2.4.
+// -> 5.6 TB/s), 2000 x 14336: 36 -> 20 us. Rows of 16-byte aligned pieces only; the kernel above takes the rest.
 constexpr int kQuantUnroll = 4;
-constexpr long long kQuantWideBlocks = 6144;
 __global__ void __launch_bounds__(256)
 quant_rows_vec_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, __nv_fp8_storage_t* __restrict__ q, long long ldq,
                       float* __restrict__ scale, unsigned blocks, unsigned kb_n) {
@@ -490,7 +488,7 @@ CAI_API int cai_quant_rows_1x128(const void* x, long long ldx, void* q, long lon
     }
     const long long warps = static_cast<long long>(rows) * (cols / 128);
     if (warps == 0) return CAI_K_OK;
-    if (warps >= kQuantWideBlocks && warps < (1ll << 31) && !(ldx & 7) && !(ldq & 7) && aligned_to(x, 16) && aligned_to(q, 8)) {
+    if (warps < (1ll << 31) && !(ldx & 7) && !(ldq & 7) && aligned_to(x, 16) && aligned_to(q, 8)) {
         constexpr unsigned per_cta = 16u * kQuantUnroll;
         quant_rows_vec_kernel<<<static_cast<unsigned>((warps + per_cta - 1) / per_cta), 256, 0, static_cast<cudaStream_t>(stream)>>>(
             static_cast<const __nv_bfloat16*>(x), ldx, static_cast<__nv_fp8_storage_t*>(q), ldq, scale, static_cast<unsigned>(warps),

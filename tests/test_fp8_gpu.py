@@ -84,7 +84,7 @@ def _strided(t, pad):
 
 
 # The quantisers' wide form (16-byte pieces) against their narrow one, which takes rows at odd pitches: the same bytes.
-@pytest.mark.parametrize("rows,cols", [(1, 128), (63, 384), (65, 128), (300, 1152), (767, 1024), (768, 1024), (6145, 128), (701, 1152)])
+@pytest.mark.parametrize("rows,cols", [(1, 128), (63, 384), (65, 128), (300, 1152)])
 def test_quant_rows_forms_agree(rows, cols):
     import ctypes
     from cai_b200 import ops
