@@ -211,16 +211,13 @@ reduce_parts_kernel(const float* __restrict__ parts, float* __restrict__ out, in
 // Beside a product of another stream it runs on the SMs that one leaves free: none of its CTAs was seen to share an SM with a
 // persistent product's, whatever the shared memory either asks for.
 constexpr int kNormFusedThreads = 256;
-// A row of 32 lanes' sums and four words more: a warp that reads 32 neighbouring columns (four lanes of each of eight elements) meets no
-// bank twice, and writes 128 bytes in one piece. In the order of the lanes the columns left 32 bytes apart: 33 x 8192 8.2 -> 11.5 us.
-constexpr int kNormPitch = 36;
 constexpr int kNormFusedCols = 1024;   // columns one warp covers: 32 lanes x 4 chunks x 8 elements
 constexpr int kNormFusedMaxH = 8192;
 static __global__ void __launch_bounds__(kNormFusedThreads, 2)
 rmsnorm_bwd_fused_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ g,
                          const float* __restrict__ rstd, const __nv_bfloat16* __restrict__ dy,
                          __nv_bfloat16* __restrict__ dx, float* __restrict__ dg_partial, int rows, int H, int dx_acc, int R) {
-    extern __shared__ float sdg[];   // [warp][chunk * 8 + element][lane], rows kNormPitch apart: a warp's column sums
+    extern __shared__ float sdg[];   // [warp][chunk * 8 + element][lane]: a warp's column sums, no two lanes on one bank
     __shared__ float part[8];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int groups = 8 / R;                 // rows a CTA works on at a time
@@ -300,15 +297,17 @@ rmsnorm_bwd_fused_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat1
 #pragma unroll
     for (int c = 0; c < 4; ++c)
 #pragma unroll
-        for (int e = 0; e < 8; ++e) sdg[(warp * 32 + c * 8 + e) * kNormPitch + lane] = acc[c][e];
+        for (int e = 0; e < 8; ++e) sdg[(warp * 32 + c * 8 + e) * 32 + lane] = acc[c][e];
     __syncthreads();
-    // row groups in order, so the result does not depend on timing
-    for (int col = threadIdx.x; col < H; col += kNormFusedThreads) {
-        const int sl = col / kNormFusedCols, in = col & (kNormFusedCols - 1);   // chunk * 256 + lane * 8 + element
-        const int at = ((in >> 8) * 8 + (in & 7)) * kNormPitch + ((in >> 3) & 31);
-        float v = 0.f;
-        for (int w = 0; w < groups; ++w) v += sdg[(w * R + sl) * 32 * kNormPitch + at];
-        dg_partial[static_cast<long long>(blockIdx.x) * H + col] = v;
+    // column of slice `sl`: chunk, lane and element from its place; row groups in order, so the result does not depend on timing
+    for (int i = threadIdx.x; i < R * kNormFusedCols; i += kNormFusedThreads) {
+        const int sl = i / kNormFusedCols, in = i - sl * kNormFusedCols;    // in = (chunk * 8 + element) * 32 + lane
+        const int col = sl * kNormFusedCols + ((in >> 8) * 32 + (in & 31)) * 8 + ((in >> 5) & 7);
+        if (col < H) {
+            float v = 0.f;
+            for (int w = 0; w < groups; ++w) v += sdg[(w * R + sl) * kNormFusedCols + in];
+            dg_partial[static_cast<long long>(blockIdx.x) * H + col] = v;
+        }
     }
 }
 
@@ -326,7 +325,7 @@ static inline int launch_rmsnorm_bwd(const void* x, const void* g, const float* 
         int grid = static_cast<int>(want < 2LL * sms ? want : 2LL * sms);
         if (grid > parts_cap) grid = parts_cap;
         if (grid < 1) grid = 1;
-        constexpr size_t smem = 8 * 32 * kNormPitch * sizeof(float);
+        constexpr size_t smem = 8 * kNormFusedCols * sizeof(float);
         rmsnorm_bwd_fused_kernel<<<grid, kNormFusedThreads, smem, st>>>(static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(g),
                                                                       rstd, static_cast<const __nv_bfloat16*>(dy),
                                                                       static_cast<__nv_bfloat16*>(dx), scratch, rows, H, dx_accumulate, Rf);

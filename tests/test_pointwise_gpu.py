@@ -158,7 +158,7 @@ def test_adamw_matches_reference_rule():
 
 
 # Rows handled by 1, 2, 4 and 8 warps; fewer rows than warps, ragged last chunks, an accumulated dx and gain gradient.
-@pytest.mark.parametrize("rows,H", [(1, 8), (5, 1000), (300, 1032), (77, 3000), (33, 8192), (9, 1024), (2, 4096), (40, 5128)])
+@pytest.mark.parametrize("rows,H", [(1, 8), (5, 1000), (300, 1032), (77, 3000), (33, 8192)])
 def test_rmsnorm_bwd_sums(rows, H):
     from cai_b200 import ops
     torch.manual_seed(7)
