@@ -751,20 +751,13 @@ static int launch_pair(const void* A, const void* B, const GemmShape& g, PairPar
 // kernel unless one wave of narrow tiles holds them all. us, one-CTA / pairs, slabs half full: 32 groups of 128 x 1024 x 256 8.7 / 10.4, 64 of
 // 128 x 4096 x 1536 144 / 195, 32 of 384 x 1024 x 1024 33 / 47, 64 of 384 x 3072 x 4096 459 / 486; in one wave, 32 of 128 x 256 x 512
 // 8.3 / 8.0; 64 of 256 x 3072 x 4096 350 / 351, 16 of 640 x 2048 x 2048 (two operand orders) 67 / 77 and 75 / 68.
-//
-// SwiGLU's epilogue exists for the 256-wide tile only, and takes some 2 us where nothing hides it. Products of up to 768 k-elements that one
-// wave of the one-CTA kernel's 128 x 128 tiles holds run there: 512 x (2 x 512) x 256 10.4 us against 12.4, x 768 13.8 against 14.5, x 1024
-// 15.9 against 16.1; 512 x (2 x 2048) x 512 12.4 against 13.7; two waves, 1024 x (2 x 2048) x 256 16.1 against 13.0.
 PairForm pair_form(int M, int N, int K, int groups, int epi, int seg_mode) {
     constexpr long long kPairs = 74, kSplitTiles2 = 33, kSplitTiles4 = 15;
     const long long ks = (K + 127) / 128, tm = (M + pair::kBM - 1) / pair::kBM;
     const long long t256 = tm * ((N + 255) / 256) * groups, t128 = tm * ((N + 127) / 128) * groups;
     const double wide = static_cast<double>((t256 + kPairs - 1) / kPairs) * (ks * 1150.0 + 2500.0);
     const double narrow = static_cast<double>((t128 + kPairs - 1) / kPairs) * (ks * 850.0 + 1500.0);
-    if (epi == CAI_EPI_SWIGLU) {
-        if (K <= 768 && static_cast<long long>((M + 127) / 128) * ((N + 127) / 128) <= 2 * kPairs) return {0, 0};
-        return {256, 1};
-    }
+    if (epi == CAI_EPI_SWIGLU) return {256, 1};
     if (seg_mode == 1 && groups > 1 && epi == CAI_EPI_BF16 && (M <= 128 || (M > 256 && M <= 384)) && t128 > kPairs) return {0, 0};
     if (!seg_mode) {
         const double two = ks >= 2 && t128 <= kSplitTiles2 ? (ks + 1) / 2 * 850.0 + 4500.0 : 1e30;

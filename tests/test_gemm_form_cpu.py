@@ -60,9 +60,3 @@ def test_groups_of_few_rows_run_one_cta_per_tile():
     assert form(256, 1024, 256, groups=32, seg_mode=1)[1] == form(640, 1024, 1024, groups=32, seg_mode=1)[1] == 1
     assert form(128, 1024, 256, groups=32, seg_mode=2)[1] == form(128, 1024, 256, groups=32, epi=1, seg_mode=1)[1] == 1
     assert form(128, 1024, 256, groups=1, seg_mode=1)[1] == 1
-
-
-def test_small_swiglu_products_run_one_cta_per_tile():
-    for shape, one_cta in (((512, 1024, 256), True), ((512, 1024, 768), True), ((512, 1024, 776), False), ((1024, 2048, 512), True),
-                           ((1024, 2304, 512), True), ((1024, 2560, 512), False), ((1152, 2304, 512), False)):
-        assert (form(*shape, epi=EPI_SWIGLU) == (0, 0)) == one_cta, shape
