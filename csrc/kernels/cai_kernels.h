@@ -51,11 +51,10 @@ CAI_API int cai_gemm_bf16(const void* A, const void* B, void* C, const void* R, 
                           long long lda, long long ldb, long long ldc, long long ldr, int a_mn_major,
                           int b_mn_major, int epi, float alpha, int sm_limit, void* stream);
 
-/* The form such a product runs in: columns of its 256-row tiles, and how many slices of K are summed (1: one sum along K; 0
- * and no columns: the kernel of one CTA per 128-row tile, one sum along K). It follows
+/* The form such a product runs in: columns of its 256-row tiles, and how many slices of K are summed (1: one sum along K). It follows
  * from the arguments alone, so the order of summation is the same on every GPU. ctas: the most CTAs of one launch on `sms` SMs under sm_limit.
  * Needs no GPU. Not for CAI_EPI_SWIGLU_BWD. */
-CAI_API int cai_gemm_bf16_form(int M, int N, int K, int groups, int epi, int seg_mode, int sms, int sm_limit, int* tile_cols, int* slices,
+CAI_API int cai_gemm_bf16_form(int M, int N, int K, int groups, int epi, int segmented, int sms, int sm_limit, int* tile_cols, int* slices,
                                int* ctas);
 
 /* Same product over ragged slabs (expert buffers of a mixture-of-experts layer). The segmented

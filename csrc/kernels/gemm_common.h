@@ -20,12 +20,11 @@ struct GemmShape {
     int sm_limit;
 };
 
-// The form a plain product runs in: columns of a 256-row tile, slices of K that are summed in order (0: the one-CTA kernel, which picks
-// its own tiles). A function of the shape.
+// The form a plain product runs in: columns of a 256-row tile, slices of K that are summed in order. A function of the shape.
 struct PairForm {
     int tile_cols, slices;
 };
-PairForm pair_form(int M, int N, int K, int groups, int epi, int seg_mode);
+PairForm pair_form(int M, int N, int K, int groups, int epi, bool segmented);
 // CTA pairs, 256-row tiles (gemm_pair.cu).
 int gemm_pair(const void* A, const void* B, const GemmShape& g, cudaStream_t st);
 

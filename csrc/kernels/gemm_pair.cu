@@ -745,21 +745,14 @@ static int launch_pair(const void* A, const void* B, const GemmShape& g, PairPar
 //   14 tiles, K 2048  15.4 / 13.4 / 10.7 /  9.3       16 tiles  15.4 / 13.7 / 10.7 / 16.5      33 tiles  15.6 / 13.9 / 11.3 / 24.8
 //   36 tiles, K 2048  15.6 / 14.0 / 20.3 / 24.8       72 tiles  16.5 / 14.6 / 30.3 / 41.2      80 tiles  16.4 / 23.1
 //   16 tiles, K 512    8.8 /  7.4 /  7.9 / 13.6      135 tiles, K 2048  26.2 / 23.8            160 tiles, K 2048  26.9 / 32.7
-//
-// Row-segmented groups of up to 128 or of 257 to 384 rows (the experts of a small layer) leave a quarter to a half of a pair's 256 rows
-// empty, and with two row tiles a group of which one is dead, every other pair gets only dead ones: they run on the one-CTA
-// kernel unless one wave of narrow tiles holds them all. us, one-CTA / pairs, slabs half full: 32 groups of 128 x 1024 x 256 8.7 / 10.4, 64 of
-// 128 x 4096 x 1536 144 / 195, 32 of 384 x 1024 x 1024 33 / 47, 64 of 384 x 3072 x 4096 459 / 486; in one wave, 32 of 128 x 256 x 512
-// 8.3 / 8.0; 64 of 256 x 3072 x 4096 350 / 351, 16 of 640 x 2048 x 2048 (two operand orders) 67 / 77 and 75 / 68.
-PairForm pair_form(int M, int N, int K, int groups, int epi, int seg_mode) {
+PairForm pair_form(int M, int N, int K, int groups, int epi, bool segmented) {
     constexpr long long kPairs = 74, kSplitTiles2 = 33, kSplitTiles4 = 15;
     const long long ks = (K + 127) / 128, tm = (M + pair::kBM - 1) / pair::kBM;
     const long long t256 = tm * ((N + 255) / 256) * groups, t128 = tm * ((N + 127) / 128) * groups;
     const double wide = static_cast<double>((t256 + kPairs - 1) / kPairs) * (ks * 1150.0 + 2500.0);
     const double narrow = static_cast<double>((t128 + kPairs - 1) / kPairs) * (ks * 850.0 + 1500.0);
     if (epi == CAI_EPI_SWIGLU) return {256, 1};
-    if (seg_mode == 1 && groups > 1 && epi == CAI_EPI_BF16 && (M <= 128 || (M > 256 && M <= 384)) && t128 > kPairs) return {0, 0};
-    if (!seg_mode) {
+    if (!segmented) {
         const double two = ks >= 2 && t128 <= kSplitTiles2 ? (ks + 1) / 2 * 850.0 + 4500.0 : 1e30;
         const double four = ks >= 4 && t128 <= kSplitTiles4 ? (ks + 3) / 4 * 850.0 + 4500.0 : 1e30;
         if (four < two && four < wide && four < narrow) return {pair::kSplitBN, 4};
@@ -789,7 +782,7 @@ int gemm_pair(const void* A, const void* B, const GemmShape& g, cudaStream_t st)
     p.tile0 = 0;
     const int dev = current_device();
     p.status = status_words(dev);
-    const PairForm f = pair_form(g.M, g.N, g.K, g.groups, g.epi, g.seg_mode);
+    const PairForm f = pair_form(g.M, g.N, g.K, g.groups, g.epi, g.seg_mode != 0);
     const int at_once = pair_clusters(f, sm_count(dev), g.sm_limit);
     if (f.slices == 4) return launch_split<4>(A, B, g, p, at_once, st);
     if (f.slices == 2) return launch_split<2>(A, B, g, p, at_once, st);
@@ -800,16 +793,12 @@ int gemm_pair(const void* A, const void* B, const GemmShape& g, cudaStream_t st)
 
 using namespace cai;
 
-CAI_API int cai_gemm_bf16_form(int M, int N, int K, int groups, int epi, int seg_mode, int sms, int sm_limit, int* tile_cols, int* slices,
+CAI_API int cai_gemm_bf16_form(int M, int N, int K, int groups, int epi, int segmented, int sms, int sm_limit, int* tile_cols, int* slices,
                                int* ctas) {
     if (M <= 0 || N <= 0 || K <= 0 || groups <= 0 || epi < 0 || epi > CAI_EPI_SWIGLU) return CAI_K_BAD_ARG;
-    const PairForm f = pair_form(M, N, K, groups, epi, seg_mode);
+    const PairForm f = pair_form(M, N, K, groups, epi, segmented != 0);
     *tile_cols = f.tile_cols;
     *slices = f.slices;
-    if (!f.slices) {
-        *ctas = sm_limit > 0 && sm_limit < sms ? sm_limit : sms;
-        return CAI_K_OK;
-    }
     const long long tiles = static_cast<long long>((M + pair::kBM - 1) / pair::kBM) * ((N + f.tile_cols - 1) / f.tile_cols) * groups;
     const int at_once = pair_clusters(f, sms, sm_limit);
     *ctas = static_cast<int>(2 * f.slices * (tiles < at_once ? tiles : at_once));

@@ -1,7 +1,6 @@
 // gemm_tcgen05.cu - persistent, warp-specialised bf16 GEMM for sm_100a, one CTA per tile: the products that are fused with a
-// collective (all-gather of A, reduce-scatter of C, gather of a sharded B), the one whose epilogue is SwiGLU's backward, and
-// those plain ones that are faster here than on CTA pairs (gemm_pair.cu, which says which). The entry points of all plain products
-// are here.
+// collective (all-gather of A, reduce-scatter of C, gather of a sharded B) and the one whose epilogue is SwiGLU's backward. The
+// entry points of the plain products are here too; those run on CTA pairs (gemm_pair.cu).
 //
 //   C[M,N] = alpha * sum_k A(m,k) * B(n,k)   (+ epilogue)
 //
@@ -58,17 +57,10 @@ struct GemmParams {
     __nv_bfloat16* a_full;           // all-gather: local buffer that receives every member's rows
     long long ld_src;
     PeerTable pt;
-    // ---- ragged segments (expert slabs of a mixture-of-experts layer): the segmented dimension is
-    // cut into slabs of seg_rows rows of which only the first seg_counts[slab] hold data.
-    // M is segmented: output tiles that start past a slab's count are skipped. Null: all rows count.
+    // ---- ragged rows (expert slabs of a mixture-of-experts layer): M is cut into slabs of seg_rows rows of which only the first
+    // seg_counts[slab] hold data; output tiles that start past a slab's count are skipped. Null: all rows count.
     const int* seg_counts;
     int seg_rows;
-    // ---- groups (the local experts of a mixture-of-experts layer in one launch): `groups` independent
-    // products of the same M x N x K; group g reads A / B at row coordinate + g * grp_a / grp_b of their
-    // tensor maps, writes C (and reads R) at row + g * grp_c, and owns grp_seg entries of seg_counts.
-    int groups;
-    long long grp_a, grp_b, grp_c;
-    int grp_seg;
     // ---- kGemmGatherB: B lives in a staging buffer that the leading n_copy CTAs fill from the sharded
     // parameter space (gather.cuh); b_elem_off is the element offset of B inside the staged range.
     GatherJob gat;
@@ -125,18 +117,15 @@ __device__ __forceinline__ void stamp(const GemmParams& p, int word) {
     if (p.stamps) p.stamps[static_cast<size_t>(blockIdx.x) * 8 + word] = global_timer_ns();
 }
 
-__device__ __forceinline__ bool tile_live(const GemmParams& p, int g, int tm) {
+__device__ __forceinline__ bool tile_live(const GemmParams& p, int tm) {
     if (!p.seg_counts) return true;
     const int row0 = tm * kBM, slab = row0 / p.seg_rows;
-    return row0 - slab * p.seg_rows < p.seg_counts[g * p.grp_seg + slab];
+    return row0 - slab * p.seg_rows < p.seg_counts[slab];
 }
 
 constexpr int kGemmPlain = 0, kGemmAllGatherA = 1, kGemmReduceScatter = 2, kGemmGatherB = 3;
 
-__device__ __forceinline__ void tile_coords(const GemmParams& p, int tile_all, int& tm, int& tn, int& grp) {
-    const int tiles_per_product = p.tiles_m * p.tiles_n;
-    grp = tile_all / tiles_per_product;
-    const int tile = tile_all - grp * tiles_per_product;
+__device__ __forceinline__ void tile_coords(const GemmParams& p, int tile, int& tm, int& tn) {
     const int per_group = p.group_m * p.tiles_n;
     const int g = tile / per_group;
     const int first_m = g * p.group_m;
@@ -264,7 +253,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                     stamp(p, kStampCopyDone);
                 }
                 __syncthreads();
-                if (!*copy_ok || p.tail_start >= p.tiles_m * p.tiles_n * p.groups) return;
+                if (!*copy_ok || p.tail_start >= p.tiles_m * p.tiles_n) return;
             }
         }
         if (p.mode == kGemmGatherB && static_cast<int>(blockIdx.x) < p.n_copy) {
@@ -296,7 +285,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
-    const int num_tiles = p.tiles_m * p.tiles_n * p.groups;
+    const int num_tiles = p.tiles_m * p.tiles_n;
     const int num_kb = (p.K + kBK - 1) / kBK;
 
     if (warp == 0) {
@@ -308,11 +297,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             TileWalk walk(p, num_tiles);
             bool first_tile = true;
             for (int tile = walk.next(); tile >= 0 && ok; tile = walk.next()) {
-                int tm, tn, grp;
-                tile_coords(p, tile, tm, tn, grp);
+                int tm, tn;
+                tile_coords(p, tile, tm, tn);
                 const int m0 = tm * kBM, n0 = tn * BN;
-                if (!tile_live(p, grp, tm)) continue;
-                const int ga = static_cast<int>(grp * p.grp_a), gb = static_cast<int>(grp * p.grp_b);
+                if (!tile_live(p, tm)) continue;
                 const int own_blk0 = p.mode == kGemmAllGatherA ? p.pt.rank * (p.rows_per_rank / kBM) : 0;
                 const bool local_rows = p.mode == kGemmAllGatherA && tm >= own_blk0 && tm < own_blk0 + p.rows_per_rank / kBM;
                 if (p.mode == kGemmAllGatherA && !local_rows) {
@@ -366,23 +354,23 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                     if (local_rows) {
                         tma_load_2d(a_dst, &tmA2, &full[s], k0, m0 - own_blk0 * kBM);   // my rows, straight from their source
                     } else if (!p.a_mn) {
-                        tma_load_2d(a_dst, &tmA, &full[s], k0, m0 + ga);
+                        tma_load_2d(a_dst, &tmA, &full[s], k0, m0);
                     } else {
 #pragma unroll
                         for (int c = 0; c < kBM / 64; ++c)
-                            tma_load_2d(a_dst + c * (kBK * 128), &tmA, &full[s], m0 + c * 64, k0 + ga);
+                            tma_load_2d(a_dst + c * (kBK * 128), &tmA, &full[s], m0 + c * 64, k0);
                     }
                     if (p.epi == CAI_EPI_SWIGLU) {
                         // gate rows and the up rows of the same features, stacked in one stage
                         const int F = p.N >> 1, j0 = tn * (BN / 2);
-                        tma_load_2d(b_dst, &tmB, &full[s], k0, j0 + gb);
-                        tma_load_2d(b_dst + (BN / 2) * kBK * 2, &tmB, &full[s], k0, F + j0 + gb);
+                        tma_load_2d(b_dst, &tmB, &full[s], k0, j0);
+                        tma_load_2d(b_dst + (BN / 2) * kBK * 2, &tmB, &full[s], k0, F + j0);
                     } else if (!p.b_mn) {
-                        tma_load_2d(b_dst, &tmB, &full[s], k0, n0 + gb);
+                        tma_load_2d(b_dst, &tmB, &full[s], k0, n0);
                     } else {
 #pragma unroll
                         for (int c = 0; c < BN / 64; ++c)
-                            tma_load_2d(b_dst + c * (kBK * 128), &tmB, &full[s], n0 + c * 64, k0 + gb);
+                            tma_load_2d(b_dst + c * (kBK * 128), &tmB, &full[s], n0 + c * 64, k0);
                     }
                     if (++s == STAGES) {
                         s = 0;
@@ -405,11 +393,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             int t = 0;
             TileWalk walk(p, num_tiles);
             for (int tile = walk.next(); tile >= 0 && ok; tile = walk.next()) {
-                int grp = 0;
                 if (p.seg_counts) {
                     int tm, tn;
-                    tile_coords(p, tile, tm, tn, grp);
-                    if (!tile_live(p, grp, tm)) continue;
+                    tile_coords(p, tile, tm, tn);
+                    if (!tile_live(p, tm)) continue;
                 }
                 const int acc = t & 1;
                 const uint32_t acc_ph = (t >> 1) & 1;
@@ -460,9 +447,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         (void)rs_prev_owner; (void)rs_prev_slot; (void)rs_reduce_seen;
         TileWalk walk(p, num_tiles);
         for (int tile = walk.next(); tile >= 0 && ok; tile = walk.next()) {
-            int tm, tn, grp;
-            tile_coords(p, tile, tm, tn, grp);
-            if (!tile_live(p, grp, tm)) continue;
+            int tm, tn;
+            tile_coords(p, tile, tm, tn);
+            if (!tile_live(p, tm)) continue;
             const int acc = t & 1;
             const uint32_t acc_ph = (t >> 1) & 1;
             ++t;
@@ -628,9 +615,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                 rs_prev_owner = owner;
                 rs_prev_slot = static_cast<uint32_t>((tm - owner * blocks_per_rank) * p.tiles_n + tn);
             } else {
-            const long long row_in = (long long)tm * kBM + q * 32 + lane;   // row inside this group's product
-            const bool row_ok = row_in < p.M;
-            const long long row = row_in + grp * p.grp_c;
+            const long long row = (long long)tm * kBM + q * 32 + lane;
+            const bool row_ok = row < p.M;
             if (p.epi == CAI_EPI_SWIGLU) {
                 // accumulator columns [0, BN/2) are gate, [BN/2, BN) up, of features j0 .. j0 + BN/2
                 const int F = p.N >> 1, j0 = tn * (BN / 2);
@@ -795,7 +781,7 @@ static int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUt
     // gather mode walks every row block of an output column before the next column, so that the columns of B
     // are needed in the order the copy CTAs stage them (A stays L2 resident)
     p.group_m = p.mode == kGemmGatherB ? p.tiles_m : 8;
-    const int tiles = p.tiles_m * p.tiles_n * p.groups;
+    const int tiles = p.tiles_m * p.tiles_n;
     int grid = tiles < sms - p.n_copy ? tiles : sms - p.n_copy;
     if (grid < 1) grid = 1;
     grid += p.n_copy;
@@ -837,7 +823,7 @@ static int gemm_dispatch(const void* A, const void* B, long long lda, long long 
     // Tile width: fewer, wider tiles amortise the A operand better; narrower tiles quantise
     // into waves better when the output is small.
     auto cost = [&](int bn) {
-        const long long tiles = (long long)((M + kBM - 1) / kBM) * ((N + bn - 1) / bn) * p.groups;
+        const long long tiles = (long long)((M + kBM - 1) / kBM) * ((N + bn - 1) / bn);
         const long long waves = (tiles + usable - 1) / usable;
         // a 128-wide tile streams 128 B/clk/SM of operands for half the math of a 256-wide one and runs
         // at the L2 limit: measured 27.6 us against 30 us per wave at K = 4096, i.e. 1.84x the cost per FLOP
@@ -846,14 +832,12 @@ static int gemm_dispatch(const void* A, const void* B, long long lda, long long 
     const int BN = cost(256) <= cost(128) ? 256 : 128;
     CUtensorMap tmA, tmB;
     bool ok;
-    // the maps of a grouped launch span every group's rows
-    const long long xa = (p.groups - 1) * p.grp_a, xb = (p.groups - 1) * p.grp_b;
-    if (!p.a_mn) ok = encode_tmap_2d(&tmA, A, M + xa, K, lda, kBK, kBM, 2);
-    else ok = encode_tmap_2d(&tmA, A, K + xa, M, lda, 64, kBK, 2);
+    if (!p.a_mn) ok = encode_tmap_2d(&tmA, A, M, K, lda, kBK, kBM, 2);
+    else ok = encode_tmap_2d(&tmA, A, K, M, lda, 64, kBK, 2);
     if (!ok) return CAI_K_BAD_ARG;
-    if (p.epi == CAI_EPI_SWIGLU) ok = encode_tmap_2d(&tmB, B, N + xb, K, ldb, kBK, BN / 2, 2);
-    else if (!p.b_mn) ok = encode_tmap_2d(&tmB, B, N + xb, K, ldb, kBK, BN, 2);
-    else ok = encode_tmap_2d(&tmB, B, K + xb, N, ldb, 64, kBK, 2);
+    if (p.epi == CAI_EPI_SWIGLU) ok = encode_tmap_2d(&tmB, B, N, K, ldb, kBK, BN / 2, 2);
+    else if (!p.b_mn) ok = encode_tmap_2d(&tmB, B, N, K, ldb, kBK, BN, 2);
+    else ok = encode_tmap_2d(&tmB, B, K, N, ldb, 64, kBK, 2);
     if (!ok) return CAI_K_BAD_ARG;
     p.status = status_words(dev);
     p.stamps = p.mode != kGemmPlain ? g_stamp_buf[dev & 63] : nullptr;
@@ -875,27 +859,8 @@ static void plain_params(GemmParams& p) {
     p.epoch_base = nullptr; p.seq = 0; p.src_off = 0; p.stage_off = 0; p.a_full = nullptr; p.ld_src = 0;
     p.pt = PeerTable{};
     p.seg_counts = nullptr; p.seg_rows = 0;
-    p.groups = 1; p.grp_a = p.grp_b = p.grp_c = 0; p.grp_seg = 0;
     p.gat = GatherJob{}; p.b_elem_off = 0; p.ldb = 0; p.stamps = nullptr; p.tail_start = 0x7fffffff;
     p.R = nullptr; p.ldr = 0; p.alpha = 1.f; p.epi = CAI_EPI_BF16; p.a_mn = 0;
-}
-
-// A plain product, where its form says.
-static int gemm_plain(const void* A, const void* B, const GemmShape& g, cudaStream_t st) {
-    if (g.epi != CAI_EPI_SWIGLU_BWD && pair_form(g.M, g.N, g.K, g.groups, g.epi, g.seg_mode).slices) return gemm_pair(A, B, g, st);
-    GemmParams p;
-    plain_params(p);
-    p.M = g.M; p.N = g.N; p.K = g.K;
-    p.a_mn = g.a_mn; p.b_mn = g.b_mn;
-    p.epi = g.epi; p.alpha = g.alpha;
-    p.C = g.C; p.R = g.R;
-    p.ldc = g.ldc; p.ldr = g.ldr;
-    if (g.seg_mode == 1) {
-        p.seg_counts = g.seg_counts;
-        p.seg_rows = g.seg_rows;
-    }
-    p.groups = g.groups; p.grp_a = g.grp_a; p.grp_b = g.grp_b; p.grp_c = g.grp_c; p.grp_seg = g.grp_seg;
-    return gemm_dispatch(A, B, g.lda, g.ldb, p, g.sm_limit, st);
 }
 
 }  // namespace cai
@@ -939,9 +904,25 @@ CAI_API int cai_gemm_bf16_seg(const void* A, const void* B, void* C, const void*
         set_last_error("gemm: fused SwiGLU needs B stored [2F, K] with F a multiple of 128 (N=%d)", N);
         return CAI_K_BAD_ARG;
     }
-    const GemmShape g = {M, N, K, a_mn_major ? 1 : 0, b_mn_major ? 1 : 0, epi, alpha, C, R, lda, ldb, ldc, ldr,
-                         seg_counts, seg_rows, seg_mode, 0, 1, 0, 0, 0, sm_limit};
-    return gemm_plain(A, B, g, reinterpret_cast<cudaStream_t>(stream));
+    if (epi != CAI_EPI_SWIGLU_BWD) {
+        const GemmShape g = {M, N, K, a_mn_major ? 1 : 0, b_mn_major ? 1 : 0, epi, alpha, C, R, lda, ldb, ldc, ldr,
+                             seg_counts, seg_rows, seg_mode, 0, 1, 0, 0, 0, sm_limit};
+        return gemm_pair(A, B, g, reinterpret_cast<cudaStream_t>(stream));
+    }
+    GemmParams p;
+    plain_params(p);
+    p.M = M; p.N = N; p.K = K;
+    p.a_mn = a_mn_major ? 1 : 0;
+    p.b_mn = b_mn_major ? 1 : 0;
+    p.epi = epi;
+    p.alpha = alpha;
+    p.C = C; p.R = R;
+    p.ldc = ldc; p.ldr = ldr;
+    if (seg_mode == 1) {
+        p.seg_counts = seg_counts;
+        p.seg_rows = seg_rows;
+    }
+    return gemm_dispatch(A, B, lda, ldb, p, sm_limit, reinterpret_cast<cudaStream_t>(stream));
 }
 
 CAI_API int cai_gemm_bf16_grouped(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
@@ -957,7 +938,7 @@ CAI_API int cai_gemm_bf16_grouped(const void* A, const void* B, void* C, int M, 
     }
     const GemmShape g = {M, N, K, a_mn_major ? 1 : 0, b_mn_major ? 1 : 0, epi, 1.f, C, nullptr, lda, ldb, ldc, 0,
                          seg_counts, seg_rows, seg_mode, grp_seg, groups, grp_a, grp_b, grp_c, 0};
-    return gemm_plain(A, B, g, reinterpret_cast<cudaStream_t>(stream));
+    return gemm_pair(A, B, g, reinterpret_cast<cudaStream_t>(stream));
 }
 
 // y[T,N] = concat_rows(x_local of every member)[T,K] * op(B); also leaves the gathered rows in a_full.

@@ -10,9 +10,9 @@ pytestmark = pytest.mark.skipif(not _lib._LIB_PATH.exists(), reason="kernel libr
 EPI_BF16, EPI_SWIGLU, EPI_SWIGLU_BWD = 0, 4, 5
 
 
-def ask(M, N, K, groups=1, epi=EPI_BF16, seg_mode=0, sms=148, limit=0):
+def ask(M, N, K, groups=1, epi=EPI_BF16, segmented=0, sms=148, limit=0):
     out = [ctypes.c_int() for _ in range(3)]
-    rc = _lib.lib().cai_gemm_bf16_form(M, N, K, groups, epi, seg_mode, sms, limit, *map(ctypes.byref, out))
+    rc = _lib.lib().cai_gemm_bf16_form(M, N, K, groups, epi, segmented, sms, limit, *map(ctypes.byref, out))
     return tuple(v.value for v in out) if rc == 0 else rc
 
 
@@ -35,7 +35,7 @@ def test_form_by_shape(M, N, K, want):
 
 def test_split_only_where_sums_are_plain():
     assert form(256, 1920, 2048, epi=EPI_SWIGLU) == (256, 1)
-    assert form(256, 1920, 2048, seg_mode=1)[1] == 1
+    assert form(256, 1920, 2048, segmented=1)[1] == 1
     assert form(256, 128, 2048, groups=40)[1] == 1 and form(256, 128, 2048, groups=15)[1] == 4
     assert form(256, 128, 128, epi=EPI_SWIGLU_BWD) < 0 and form(0, 128, 128) < 0
 
@@ -50,13 +50,3 @@ def test_limit_caps_the_ctas(shape, cluster, free):
         assert f[:2] == ask(*shape)[:2] == ask(*shape, sms=132)[:2]        # the sums do not depend on the limit or the GPU
         most = max(cluster, min(limit, 148) // cluster * cluster)         # whole clusters; one at least
         assert f[2] == min(free, most), (limit, f)
-
-
-def test_groups_of_few_rows_run_one_cta_per_tile():
-    """Ragged groups that would leave a quarter to a half of a pair's 256 rows empty, unless a single wave of tiles holds them all."""
-    one_cta = (0, 0)
-    assert form(128, 1024, 256, groups=32, seg_mode=1) == form(384, 1024, 1024, groups=32, seg_mode=1) == one_cta
-    assert form(128, 256, 512, groups=32, seg_mode=1) == (128, 1)                       # 64 narrow tiles on 74 pairs
-    assert form(256, 1024, 256, groups=32, seg_mode=1)[1] == form(640, 1024, 1024, groups=32, seg_mode=1)[1] == 1
-    assert form(128, 1024, 256, groups=32, seg_mode=2)[1] == form(128, 1024, 256, groups=32, epi=1, seg_mode=1)[1] == 1
-    assert form(128, 1024, 256, groups=1, seg_mode=1)[1] == 1

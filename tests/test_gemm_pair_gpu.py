@@ -183,33 +183,3 @@ def test_accumulation_keeps_subnormals(M, N, K):
         out = torch.full((M, N), old, device="cuda")
         ops.gemm(a, b, out=out, accumulate=True)
         assert bool((out.double() == old + 2.0 ** -130).all()), old
-
-
-# Ragged groups on both sides of the line between the one-CTA kernel and the pairs: empty, partial and full slabs, both orders of B.
-@pytest.mark.parametrize("tb", [False, True])
-@pytest.mark.parametrize("G,cap,N,K,one_cta", [(40, 128, 264, 136, True), (11, 384, 520, 192, True), (10, 128, 264, 136, False),
-                                               (20, 256, 520, 192, False), (9, 640, 264, 128, False)])
-def test_ragged_groups_of_few_rows(G, cap, N, K, one_cta, tb):
-    import ctypes
-    from cai_b200 import ops
-    from cai_b200.ops import _lib
-    f = [ctypes.c_int() for _ in range(3)]
-    assert _lib.lib().cai_gemm_bf16_form(cap, N, K, G, 0, 1, 148, 0, *map(ctypes.byref, f)) == 0 and (f[1].value == 0) == one_cta
-    torch.manual_seed(9)
-    if tb:
-        K = (K + 63) // 64 * 64
-    a = torch.randn(G * cap, K, device="cuda").to(torch.bfloat16)
-    b = torch.randn(*((G * K, N) if tb else (G * N, K)), device="cuda").to(torch.bfloat16)
-    counts = torch.randint(0, cap + 1, (G,), device="cuda", dtype=torch.int32)
-    counts[0], counts[1], counts[2] = 0, cap, 1
-    out = torch.full((G * cap, N), 7.0, device="cuda", dtype=torch.bfloat16)
-    ops.gemm_grouped(a, b, out, cap, N, K, groups=G, trans_b=tb, seg_counts=counts, seg_rows=cap, seg_mode=1)
-    for g in range(G):
-        A, B = a[g * cap:(g + 1) * cap].float(), (b[g * K:(g + 1) * K] if tb else b[g * N:(g + 1) * N].t()).float()
-        ref, live = A @ B, int(counts[g])
-        got = out[g * cap:(g + 1) * cap]
-        bound = 2 * K * 2.0 ** -24 * (A.abs() @ B.abs()) + 2.0 ** -8 * ref.abs() + 1e-6
-        assert ((got.float() - ref).abs() <= bound)[:live].all(), g
-        written = (live + 127) // 128 * 128                    # whole tiles of 128 rows are written, nothing past them
-        assert bool((got[written:] == 7.0).all()), g
-    assert _lib.device_status(clear=True) == 0
