@@ -60,8 +60,8 @@ struct AttnBwdParams {
 };
 
 // chain counters of the head-split dK / dV kernel: one per (batch, kv group, kv tile).
-// ONE array serves every call on a device: each call clears the slots it uses (stream-ordered memset) before
-// its kernel, so two attention backwards that overlap on one GPU (different streams) would reset each other's
+// ONE array serves every call on a device: each call clears the slots it uses (in stream order: the row sums' kernel, or a
+// memset) before its kernel, so two attention backwards that overlap on one GPU (different streams) would reset each other's
 // counters. Calls that take the head-split path must therefore be ordered against each other; the executor
 // issues them from one stream. A CTA of turn t waits (bounded) for the CTA of turn t - 1 of the same kv tile,
 // which has a lower linear block id: with the grid no larger than the number of SMs every CTA is resident at
@@ -76,7 +76,9 @@ __device__ unsigned int g_attn_chain[kAttnChainSlots];
 constexpr int kDeltaUnroll = 2;
 __global__ void __launch_bounds__(256)
 attn_delta_kernel(const __nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ dout, float* __restrict__ delta,
-                  unsigned total, unsigned S, unsigned nh, bool out16) {
+                  unsigned total, unsigned S, unsigned nh, bool out16, unsigned int* chain, unsigned chain_slots) {
+    grid_dep_begin();
+    if (blockIdx.x * 256u + threadIdx.x < chain_slots) chain[blockIdx.x * 256u + threadIdx.x] = 0;   // for the dK / dV kernel behind this one
     const unsigned w0 = blockIdx.x * (16u * kDeltaUnroll) + (threadIdx.x >> 4);
     const int sub = threadIdx.x & 15;
     uint4 a[kDeltaUnroll], d[kDeltaUnroll];
@@ -198,9 +200,11 @@ __device__ __forceinline__ void issue_pd_ss(uint32_t d_tmem, uint64_t a_desc, ui
 __global__ void __launch_bounds__(kAttnBwdThreads, 1)
 attn_dkdv_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant__ CUtensorMap tm_do,
                  const AttnBwdParams p) {
+    grid_dep_launch();
     // no room to round the base up: tiles start on swizzle boundaries only if the shared window does (checked)
     extern __shared__ __align__(1024) uint8_t smem[];
     if (smem_u32(smem) & 1023) {
+        grid_dep_wait();
         if (threadIdx.x == 0) atomicCAS(p.status, 0, CAI_DEV_BAD_ARG);
         return;
     }
@@ -270,6 +274,7 @@ attn_dkdv_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    grid_dep_wait();
     const uint32_t tmem_base = *tmem_slot;
     const uint32_t tS = tmem_base, tdP = tmem_base + 128, tdV = tmem_base + 256, tdK = tmem_base + 384;
 
@@ -502,8 +507,10 @@ attn_dkdv_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
 __global__ void __launch_bounds__(kAttnBwdThreads, 1)
 attn_dq_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant__ CUtensorMap tm_do,
                const AttnBwdParams p) {
+    grid_dep_launch();
     extern __shared__ __align__(1024) uint8_t smem[];
     if (smem_u32(smem) & 1023) {
+        grid_dep_wait();
         if (threadIdx.x == 0) atomicCAS(p.status, 0, CAI_DEV_BAD_ARG);
         return;
     }
@@ -562,6 +569,7 @@ attn_dq_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    grid_dep_wait();
     const uint32_t tmem_base = *tmem_slot;
     const uint32_t tS = tmem_base, tdP = tmem_base + 256, tdQ = tmem_base + 384;   // two score buffers
 
@@ -741,13 +749,6 @@ CAI_API int cai_flash_attn_bwd_parts(const void* qkv, const void* out, const voi
         }
         configured[dev & 63] = true;
     }
-    const long long rows = static_cast<long long>(B) * S * nh;
-    if (parts & 1) {
-        constexpr unsigned per_cta = 16u * kDeltaUnroll;
-        attn_delta_kernel<<<static_cast<unsigned>((rows + per_cta - 1) / per_cta), 256, 0, st>>>(
-            static_cast<const __nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(dout), delta, static_cast<unsigned>(rows),
-            static_cast<unsigned>(S), static_cast<unsigned>(nh), (reinterpret_cast<uintptr_t>(out) & 15) == 0);
-    }
     AttnBwdParams p;
     p.B = B; p.S = S; p.nh = nh; p.nkv = nkv;
     p.scale = scale;
@@ -773,13 +774,22 @@ CAI_API int cai_flash_attn_bwd_parts(const void* qkv, const void* out, const voi
             set_last_error("attn_bwd: cannot resolve the chain counters");
             return CAI_K_CUDA;
         }
-        if (cudaMemsetAsync(chain_ptr[dev & 63], 0, need * sizeof(unsigned int), st) != cudaSuccess) return CAI_K_CUDA;
+        // the row sums' kernel clears the slots where it runs first (it has 8 threads for each row of a head, a slot is 128 rows)
+        if (!(parts & 1) && cudaMemsetAsync(chain_ptr[dev & 63], 0, need * sizeof(unsigned int), st) != cudaSuccess) return CAI_K_CUDA;
         p.split_heads = 1;
         p.chain = chain_ptr[dev & 63];
     }
+    const long long rows = static_cast<long long>(B) * S * nh;
+    if (parts & 1) {
+        constexpr unsigned per_cta = 16u * kDeltaUnroll;
+        launch_early(attn_delta_kernel, static_cast<unsigned>((rows + per_cta - 1) / per_cta), 256, 0, st,
+                     static_cast<const __nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(dout), delta, static_cast<unsigned>(rows),
+                     static_cast<unsigned>(S), static_cast<unsigned>(nh), (reinterpret_cast<uintptr_t>(out) & 15) == 0, p.chain,
+                     static_cast<unsigned>(p.split_heads ? need : 0));
+    }
     const dim3 grid_kv(nq, p.split_heads ? nh : nkv, B), grid_q(nq, nh, B);
-    if (parts & 2) attn_dkdv_kernel<<<grid_kv, kAttnBwdThreads, smem_bytes, st>>>(tm_qkv, tm_do, p);
-    if (parts & 4) attn_dq_kernel<<<grid_q, kAttnBwdThreads, smem_bytes, st>>>(tm_qkv, tm_do, p);
+    if (parts & 2) launch_early(attn_dkdv_kernel, grid_kv, kAttnBwdThreads, smem_bytes, st, tm_qkv, tm_do, p);
+    if (parts & 4) launch_early(attn_dq_kernel, grid_q, kAttnBwdThreads, smem_bytes, st, tm_qkv, tm_do, p);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
         set_last_error("attn_bwd launch failed: %s", cudaGetErrorString(e));

@@ -37,6 +37,7 @@ struct AttnFwdParams {
 
 __global__ void __launch_bounds__(kAttnFwdThreads, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tm, const AttnFwdParams p) {
+    grid_dep_launch();
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* sQ = smem;                            // 2 tiles
@@ -94,6 +95,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm, const AttnFwdParams p) {
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    grid_dep_wait();
     const uint32_t tmem_base = *tmem_slot;
 
     if (warp == 0) {
@@ -292,6 +294,7 @@ constexpr int kAttnFwd1Threads = 256;
 
 __global__ void __launch_bounds__(kAttnFwd1Threads, 1)
 attn_fwd1_kernel(const __grid_constant__ CUtensorMap tm, const AttnFwdParams p) {
+    grid_dep_launch();
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* sQ = smem;
@@ -342,6 +345,7 @@ attn_fwd1_kernel(const __grid_constant__ CUtensorMap tm, const AttnFwdParams p) 
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    grid_dep_wait();
     const uint32_t tmem_base = *tmem_slot;
 
     if (warp == 0) {
@@ -566,10 +570,10 @@ CAI_API int cai_flash_attn_fwd_variant(const void* qkv, void* out, float* lse, i
             }
             configured1[dev & 63] = true;
         }
-        attn_fwd1_kernel<<<dim3(S / kAttnTile, nh, B), kAttnFwd1Threads, smem1, static_cast<cudaStream_t>(stream)>>>(tm, p);
+        launch_early(attn_fwd1_kernel, dim3(S / kAttnTile, nh, B), kAttnFwd1Threads, smem1, static_cast<cudaStream_t>(stream), tm, p);
     } else {
         dim3 grid((S + 2 * kAttnTile - 1) / (2 * kAttnTile), nh, B);
-        attn_fwd_kernel<<<grid, kAttnFwdThreads, smem_bytes, static_cast<cudaStream_t>(stream)>>>(tm, p);
+        launch_early(attn_fwd_kernel, grid, kAttnFwdThreads, smem_bytes, static_cast<cudaStream_t>(stream), tm, p);
     }
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {

@@ -158,6 +158,7 @@ template <int BN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair::kThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmR, const PairParams p) {
+    grid_dep_launch();
     using namespace pair;
     constexpr int STAGES = kStages<BN>;
     constexpr int HALF = BN / 2;          // columns of the tile one epilogue warp drains; rows of B one CTA loads
@@ -197,6 +198,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     __syncthreads();
     cluster_sync();      // the other CTA's barriers are initialised before anything arrives on them
     tc_fence_after();
+    grid_dep_wait();
     const uint32_t tmem_base = *tmem_slot;
 
     const int num_tiles = p.tiles_m * p.tiles_n * p.groups;
@@ -481,6 +483,7 @@ constexpr int kSplitSmem = kStages<kSplitBN> * kPerStage * kBlock<kSplitBN> + 51
 template <int S>
 __global__ void __launch_bounds__(pair::kThreads, 1)
 gemm_pair_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const PairParams p) {
+    grid_dep_launch();
     using namespace pair;
     constexpr int BN = kSplitBN, STAGES = kStages<BN>, HALF = BN / 2;
     extern __shared__ uint8_t smem_raw[];
@@ -515,6 +518,7 @@ gemm_pair_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
     __syncthreads();
     cluster_sync();
     tc_fence_after();
+    grid_dep_wait();
     const uint32_t tmem_base = *tmem_slot;
 
     int tm, tn, grp;
@@ -654,8 +658,10 @@ static void split_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, uns
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2 * S;
     attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // see launch_early
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
 }
 
 // Tensor map of rows x cols per group, the groups `apart` rows apart.
@@ -690,7 +696,7 @@ static int launch_split(const void* A, const void* B, const GemmShape& g, PairPa
     const int tiles = p.tiles_m * p.tiles_n * p.groups;
     for (p.tile0 = 0; p.tile0 < tiles; p.tile0 += at_once) {
         cudaLaunchConfig_t cfg = {};
-        cudaLaunchAttribute attr[1];
+        cudaLaunchAttribute attr[2];
         split_config<S>(cfg, attr, static_cast<unsigned>(2 * S * (tiles - p.tile0 < at_once ? tiles - p.tile0 : at_once)), st);
         const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_pair_split_kernel<S>, tmA, tmB, p);
         if (e != cudaSuccess) {
@@ -724,7 +730,7 @@ static int launch_pair(const void* A, const void* B, const GemmShape& g, PairPar
     p.group_m = 8;
     const int tiles = p.tiles_m * p.tiles_n * p.groups;
     const int grid = 2 * (tiles < pairs ? tiles : pairs);
-    gemm_pair_kernel<BN><<<grid, pair::kThreads, pair::kSmem<BN>, st>>>(tmA, tmB, tmC, tmR, p);
+    launch_early(gemm_pair_kernel<BN>, grid, pair::kThreads, pair::kSmem<BN>, st, tmA, tmB, tmC, tmR, p);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
         set_last_error("gemm_pair launch failed: %s", cudaGetErrorString(e));

@@ -33,6 +33,7 @@ constexpr int kMoeMaxEPerLane = 8;  // experts <= 256
 __global__ void __launch_bounds__(256)
 moe_route_fwd_kernel(const float* __restrict__ logits, int* __restrict__ idx, float* __restrict__ w, int* __restrict__ pos,
                      int* __restrict__ counts, int T, int E, int k, int cap) {
+    grid_dep_begin();
     const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (t >= T) return;
@@ -97,6 +98,7 @@ moe_route_fwd_kernel(const float* __restrict__ logits, int* __restrict__ idx, fl
 // of entries that chose e, dropped ones included.
 __global__ void __launch_bounds__(256)
 moe_assign_slots_kernel(const int* __restrict__ idx, int* __restrict__ pos, int* __restrict__ counts, int n, int cap) {
+    grid_dep_begin();
     __shared__ int warp_tot[8];
     const int e = blockIdx.x, lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
     int base = 0;
@@ -139,6 +141,7 @@ moe_assign_slots_kernel(const int* __restrict__ idx, int* __restrict__ pos, int*
 __global__ void __launch_bounds__(256)
 moe_route_bwd_kernel(const float* __restrict__ logits, const int* __restrict__ idx, const float* __restrict__ dw,
                      const int* __restrict__ pos, __nv_bfloat16* __restrict__ dlogits, int T, int E, int k) {
+    grid_dep_begin();
     const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (t >= T) return;
@@ -388,15 +391,15 @@ CAI_API int cai_moe_route_fwd(const float* logits, int* idx, float* w, int* pos,
         return CAI_K_BAD_ARG;
     }
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    moe_route_fwd_kernel<<<(T * 32 + 255) / 256, 256, 0, st>>>(logits, idx, w, pos, counts, T, E, k, cap);
-    moe_assign_slots_kernel<<<E, 256, 0, st>>>(idx, pos, counts, T * k, cap);
+    launch_early(moe_route_fwd_kernel, (T * 32 + 255) / 256, 256, 0, st, logits, idx, w, pos, counts, T, E, k, cap);
+    launch_early(moe_assign_slots_kernel, E, 256, 0, st, idx, pos, counts, T * k, cap);
     return cudaGetLastError() == cudaSuccess ? 0 : CAI_K_CUDA;
 }
 
 CAI_API int cai_moe_route_bwd(const float* logits, const int* idx, const float* dw, const int* pos, void* dlogits, int T, int E,
                               int k, void* stream) {
-    moe_route_bwd_kernel<<<(T * 32 + 255) / 256, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        logits, idx, dw, pos, static_cast<__nv_bfloat16*>(dlogits), T, E, k);
+    launch_early(moe_route_bwd_kernel, (T * 32 + 255) / 256, 256, 0, static_cast<cudaStream_t>(stream), logits, idx, dw, pos,
+                 static_cast<__nv_bfloat16*>(dlogits), T, E, k);
     return cudaGetLastError() == cudaSuccess ? 0 : CAI_K_CUDA;
 }
 

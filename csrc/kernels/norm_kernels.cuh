@@ -5,6 +5,7 @@
 
 #include <math.h>
 
+#include "host_common.h"
 #include "sm100.cuh"
 
 namespace cai {
@@ -74,6 +75,7 @@ static __global__ void __launch_bounds__(kNormThreads)
 rmsnorm_bwd_dx_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ g,
                       const float* __restrict__ rstd, const __nv_bfloat16* __restrict__ dy,
                       __nv_bfloat16* __restrict__ dx, int rows, int H, int dx_acc, int R) {
+    grid_dep_begin();
     __shared__ float part[8];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int groups = 8 / R;
@@ -152,6 +154,7 @@ static __global__ void __launch_bounds__(256)
 rmsnorm_bwd_dg_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ rstd,
                       const __nv_bfloat16* __restrict__ dy, float* __restrict__ dg_partial, int rows, int H,
                       int rows_per_part) {
+    grid_dep_begin();
     const long long r0 = static_cast<long long>(blockIdx.x) * rows_per_part;
     const long long r1 = r0 + rows_per_part < rows ? r0 + rows_per_part : rows;
     for (int c = threadIdx.x; c < (H >> 3); c += 256) {
@@ -178,6 +181,7 @@ rmsnorm_bwd_dg_kernel(const __nv_bfloat16* __restrict__ x, const float* __restri
 constexpr int kReduceWarps = 32;
 static __global__ void __launch_bounds__(kReduceWarps * 32)
 reduce_parts_kernel(const float* __restrict__ parts, float* __restrict__ out, int nparts, int H, int accumulate) {
+    grid_dep_begin();
     __shared__ float acc[kReduceWarps][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int w = warp & 7, k = warp >> 3;
@@ -217,6 +221,7 @@ static __global__ void __launch_bounds__(kNormFusedThreads, 2)
 rmsnorm_bwd_fused_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ g,
                          const float* __restrict__ rstd, const __nv_bfloat16* __restrict__ dy,
                          __nv_bfloat16* __restrict__ dx, float* __restrict__ dg_partial, int rows, int H, int dx_acc, int R) {
+    grid_dep_begin();
     extern __shared__ float sdg[];   // [warp][chunk * 8 + element][lane]: a warp's column sums, no two lanes on one bank
     __shared__ float part[8];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -326,10 +331,10 @@ static inline int launch_rmsnorm_bwd(const void* x, const void* g, const float* 
         if (grid > parts_cap) grid = parts_cap;
         if (grid < 1) grid = 1;
         constexpr size_t smem = 8 * kNormFusedCols * sizeof(float);
-        rmsnorm_bwd_fused_kernel<<<grid, kNormFusedThreads, smem, st>>>(static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(g),
-                                                                      rstd, static_cast<const __nv_bfloat16*>(dy),
-                                                                      static_cast<__nv_bfloat16*>(dx), scratch, rows, H, dx_accumulate, Rf);
-        reduce_parts_kernel<<<(H + 31) / 32, kReduceWarps * 32, 0, st>>>(scratch, dg, grid, H, dg_accumulate);
+        launch_early(rmsnorm_bwd_fused_kernel, grid, kNormFusedThreads, smem, st, static_cast<const __nv_bfloat16*>(x),
+                     static_cast<const __nv_bfloat16*>(g), rstd, static_cast<const __nv_bfloat16*>(dy), static_cast<__nv_bfloat16*>(dx),
+                     scratch, rows, H, dx_accumulate, Rf);
+        launch_early(reduce_parts_kernel, (H + 31) / 32, kReduceWarps * 32, 0, st, scratch, dg, grid, H, dg_accumulate);
         return cudaGetLastError() == cudaSuccess ? 0 : 1;
     }
     const int R = (H + kNormWarpCols - 1) / kNormWarpCols;
@@ -339,13 +344,13 @@ static inline int launch_rmsnorm_bwd(const void* x, const void* g, const float* 
     int parts = rows < parts_cap ? rows : parts_cap;
     const int rows_per_part = (rows + parts - 1) / parts;
     parts = (rows + rows_per_part - 1) / rows_per_part;
-    rmsnorm_bwd_dg_kernel<<<parts, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(x), rstd, static_cast<const __nv_bfloat16*>(dy),
-                                                 scratch, rows, H, rows_per_part);
-    reduce_parts_kernel<<<(H + 31) / 32, kReduceWarps * 32, 0, st>>>(scratch, dg, parts, H, dg_accumulate);
+    launch_early(rmsnorm_bwd_dg_kernel, parts, 256, 0, st, static_cast<const __nv_bfloat16*>(x), rstd,
+                 static_cast<const __nv_bfloat16*>(dy), scratch, rows, H, rows_per_part);
+    launch_early(reduce_parts_kernel, (H + 31) / 32, kReduceWarps * 32, 0, st, scratch, dg, parts, H, dg_accumulate);
     // dx last: callers may pass dx == dy (in place), and the gain gradient needs the unmodified dy
-    rmsnorm_bwd_dx_kernel<<<grid, kNormThreads, 0, st>>>(static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(g),
-                                                        rstd, static_cast<const __nv_bfloat16*>(dy),
-                                                        static_cast<__nv_bfloat16*>(dx), rows, H, dx_accumulate, R);
+    launch_early(rmsnorm_bwd_dx_kernel, grid, kNormThreads, 0, st, static_cast<const __nv_bfloat16*>(x),
+                 static_cast<const __nv_bfloat16*>(g), rstd, static_cast<const __nv_bfloat16*>(dy), static_cast<__nv_bfloat16*>(dx), rows,
+                 H, dx_accumulate, R);
     return cudaGetLastError() == cudaSuccess ? 0 : 1;
 }
 

@@ -31,6 +31,7 @@ namespace cai {
 __global__ void __launch_bounds__(kNormThreads)
 rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ g,
                    __nv_bfloat16* __restrict__ y, float* __restrict__ rstd, int rows, int H, float eps, int R) {
+    grid_dep_begin();
     __shared__ float part[8];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int groups = 8 / R;
@@ -101,6 +102,7 @@ __global__ void rope_table_kernel(float2* table, int seq, int half, float theta)
 // One thread rotates 8 pairs (i .. i+7, i+half .. i+half+7) of one head of one token.
 __global__ void rope_apply_kernel(__nv_bfloat16* qkv, const float2* __restrict__ table, long long T, int seq,
                                   int nh, int nkv, int hd, long long ld, int inverse) {
+    grid_dep_begin();
     const int half = hd >> 1;
     const int per_head = half >> 3;
     const int heads = nh + nkv;
@@ -132,6 +134,7 @@ __global__ void rope_apply_kernel(__nv_bfloat16* qkv, const float2* __restrict__
 // ------------------------------------------------------------------ SwiGLU
 __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ act,
                                   long long T, int F) {
+    grid_dep_begin();
     const int fv = F >> 3;
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= T * fv) return;
@@ -151,6 +154,7 @@ __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfl
 
 __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gu, const __nv_bfloat16* __restrict__ dact,
                                   __nv_bfloat16* __restrict__ dgu, long long T, int F) {
+    grid_dep_begin();
     const int fv = F >> 3;
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= T * fv) return;
@@ -178,6 +182,7 @@ __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gu, const __
 // ------------------------------------------------------------------ embedding
 __global__ void embed_fwd_kernel(const int* __restrict__ tokens, const __nv_bfloat16* __restrict__ E,
                                  __nv_bfloat16* __restrict__ out, int H, int lo, int hi) {
+    grid_dep_begin();
     const long long t = blockIdx.x;
     const int tok = tokens[t];
     const int nv = H >> 3;
@@ -198,6 +203,7 @@ constexpr int kEmbRows = 32;
 __global__ void __launch_bounds__(256)
 embed_bwd_kernel(const int* __restrict__ tokens, const __nv_bfloat16* __restrict__ dout, float* __restrict__ dE, int T, int H,
                  int lo, int hi) {
+    grid_dep_begin();
     __shared__ unsigned match[8];
     __shared__ int toks[256];
     const int v0 = lo + static_cast<int>(blockIdx.x) * kEmbRows;
@@ -233,6 +239,7 @@ constexpr int kCeThreads = 512;
 __global__ void __launch_bounds__(kCeThreads)
 cross_entropy_kernel(__nv_bfloat16* logits, const int* __restrict__ targets, float* loss_sum, float* row_lse,
                      int V, long long ld, float grad_scale, float loss_scale) {
+    grid_dep_begin();
     __shared__ float red[33];
     const long long row = blockIdx.x;
     __nv_bfloat16* lr = logits + row * ld;
@@ -282,6 +289,7 @@ cross_entropy_kernel(__nv_bfloat16* logits, const int* __restrict__ targets, flo
 // exp-sums are reduced over the tensor-parallel group between the three kernels.
 __global__ void __launch_bounds__(kCeThreads)
 ce_rowmax_kernel(const __nv_bfloat16* __restrict__ logits, float* __restrict__ rowmax, int V, long long ld) {
+    grid_dep_begin();
     __shared__ float red[33];
     const long long row = blockIdx.x;
     const uint4* l4 = reinterpret_cast<const uint4*>(logits + row * ld);
@@ -298,6 +306,7 @@ ce_rowmax_kernel(const __nv_bfloat16* __restrict__ logits, float* __restrict__ r
 __global__ void __launch_bounds__(kCeThreads)
 ce_rowsum_kernel(const __nv_bfloat16* __restrict__ logits, const float* __restrict__ rowmax,
                  float* __restrict__ rowsum, int V, long long ld) {
+    grid_dep_begin();
     __shared__ float red[33];
     const long long row = blockIdx.x;
     const uint4* l4 = reinterpret_cast<const uint4*>(logits + row * ld);
@@ -316,6 +325,7 @@ __global__ void __launch_bounds__(kCeThreads)
 ce_grad_tp_kernel(__nv_bfloat16* logits, const int* __restrict__ targets, const float* __restrict__ rowmax,
                   const float* __restrict__ rowsum, float* loss_sum, int V, long long ld, int vocab_lo,
                   int add_lse, float grad_scale, float loss_scale) {
+    grid_dep_begin();
     const long long row = blockIdx.x;
     __nv_bfloat16* lr = logits + row * ld;
     uint4* l4 = reinterpret_cast<uint4*>(lr);
@@ -348,6 +358,7 @@ __global__ void adamw_kernel(float* __restrict__ master, float* __restrict__ m, 
                              const float* __restrict__ grad, __nv_bfloat16* __restrict__ param, long long n,
                              float lr, float b1, float b2, float eps, float wd, float gscale, float bc1,
                              float bc2) {
+    grid_dep_begin();
     const long long i4 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 4;
     if (i4 >= n) return;
     if (i4 + 4 <= n) {
@@ -403,6 +414,7 @@ __global__ void fill_f32_kernel(float* d, float v, long long n) {
 }
 __global__ void add_bf16_kernel(const __nv_bfloat16* __restrict__ a, const __nv_bfloat16* __restrict__ b,
                                 __nv_bfloat16* __restrict__ o, long long n8) {
+    grid_dep_begin();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n8) return;
     float x[8], y[8];
@@ -435,8 +447,8 @@ CAI_API int cai_rmsnorm_fwd(const void* x, const void* g, void* y, float* rstd, 
     const long long want = (static_cast<long long>(rows) + groups - 1) / groups;
     const int cap = cai_rmsnorm_bwd_parts(rows) * 4;
     const int grid = static_cast<int>(want < cap ? want : cap);
-    rmsnorm_fwd_kernel<<<grid, kNormThreads, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)g,
-                                                                       (__nv_bfloat16*)y, rstd, rows, H, eps, R);
+    launch_early(rmsnorm_fwd_kernel, grid, kNormThreads, 0, (cudaStream_t)stream, (const __nv_bfloat16*)x, (const __nv_bfloat16*)g,
+                 (__nv_bfloat16*)y, rstd, rows, H, eps, R);
     CAI_LAUNCH_CHECK("rmsnorm_fwd");
     return CAI_K_OK;
 }
@@ -482,8 +494,8 @@ CAI_API int cai_rope_apply(void* qkv, const float* table, int T, int seq, int nh
         return CAI_K_BAD_ARG;
     }
     const long long total = (long long)T * (nh + nkv) * (hd / 16);
-    rope_apply_kernel<<<blocks_for(total, 256), 256, 0, (cudaStream_t)stream>>>(
-        (__nv_bfloat16*)qkv, (const float2*)table, T, seq, nh, nkv, hd, ld, inverse);
+    launch_early(rope_apply_kernel, blocks_for(total, 256), 256, 0, (cudaStream_t)stream, (__nv_bfloat16*)qkv, (const float2*)table, T,
+                 seq, nh, nkv, hd, ld, inverse);
     CAI_LAUNCH_CHECK("rope_apply");
     return CAI_K_OK;
 }
@@ -494,8 +506,8 @@ CAI_API int cai_swiglu_fwd(const void* gu, void* act, int T, int F, void* stream
         set_last_error("swiglu: F must be a multiple of 8");
         return CAI_K_BAD_ARG;
     }
-    swiglu_fwd_kernel<<<blocks_for((long long)T * (F / 8), 256), 256, 0, (cudaStream_t)stream>>>(
-        (const __nv_bfloat16*)gu, (__nv_bfloat16*)act, T, F);
+    launch_early(swiglu_fwd_kernel, blocks_for((long long)T * (F / 8), 256), 256, 0, (cudaStream_t)stream, (const __nv_bfloat16*)gu,
+                 (__nv_bfloat16*)act, T, F);
     CAI_LAUNCH_CHECK("swiglu_fwd");
     return CAI_K_OK;
 }
@@ -506,8 +518,8 @@ CAI_API int cai_swiglu_bwd(const void* gu, const void* dact, void* dgu, int T, i
         set_last_error("swiglu: F must be a multiple of 8");
         return CAI_K_BAD_ARG;
     }
-    swiglu_bwd_kernel<<<blocks_for((long long)T * (F / 8), 256), 256, 0, (cudaStream_t)stream>>>(
-        (const __nv_bfloat16*)gu, (const __nv_bfloat16*)dact, (__nv_bfloat16*)dgu, T, F);
+    launch_early(swiglu_bwd_kernel, blocks_for((long long)T * (F / 8), 256), 256, 0, (cudaStream_t)stream, (const __nv_bfloat16*)gu,
+                 (const __nv_bfloat16*)dact, (__nv_bfloat16*)dgu, T, F);
     CAI_LAUNCH_CHECK("swiglu_bwd");
     return CAI_K_OK;
 }
@@ -519,8 +531,8 @@ CAI_API int cai_embed_fwd(const int* tokens, const void* E, void* out, int T, in
         set_last_error("embed: H must be a multiple of 8");
         return CAI_K_BAD_ARG;
     }
-    embed_fwd_kernel<<<T, 128, 0, (cudaStream_t)stream>>>(tokens, (const __nv_bfloat16*)E, (__nv_bfloat16*)out, H,
-                                                          vocab_lo, vocab_hi);
+    launch_early(embed_fwd_kernel, T, 128, 0, (cudaStream_t)stream, tokens, (const __nv_bfloat16*)E, (__nv_bfloat16*)out, H, vocab_lo,
+                 vocab_hi);
     CAI_LAUNCH_CHECK("embed_fwd");
     return CAI_K_OK;
 }
@@ -529,8 +541,8 @@ CAI_API int cai_embed_bwd(const int* tokens, const void* dout, float* dE, int T,
                           int vocab_hi, void* stream) {
     if (T <= 0) return CAI_K_OK;
     if (vocab_hi <= vocab_lo) return CAI_K_OK;
-    embed_bwd_kernel<<<(vocab_hi - vocab_lo + kEmbRows - 1) / kEmbRows, 256, 0, (cudaStream_t)stream>>>(
-        tokens, (const __nv_bfloat16*)dout, dE, T, H, vocab_lo, vocab_hi);
+    launch_early(embed_bwd_kernel, (vocab_hi - vocab_lo + kEmbRows - 1) / kEmbRows, 256, 0, (cudaStream_t)stream, tokens,
+                 (const __nv_bfloat16*)dout, dE, T, H, vocab_lo, vocab_hi);
     CAI_LAUNCH_CHECK("embed_bwd");
     return CAI_K_OK;
 }
@@ -542,22 +554,22 @@ CAI_API int cai_cross_entropy(void* logits, const int* targets, float* loss_sum,
         set_last_error("cross_entropy: V and ld must be multiples of 8");
         return CAI_K_BAD_ARG;
     }
-    cross_entropy_kernel<<<rows, kCeThreads, 0, (cudaStream_t)stream>>>((__nv_bfloat16*)logits, targets, loss_sum,
-                                                                        row_lse, V, ld, grad_scale, loss_scale);
+    launch_early(cross_entropy_kernel, rows, kCeThreads, 0, (cudaStream_t)stream, (__nv_bfloat16*)logits, targets, loss_sum, row_lse, V,
+                 ld, grad_scale, loss_scale);
     CAI_LAUNCH_CHECK("cross_entropy");
     return CAI_K_OK;
 }
 
 CAI_API int cai_ce_rowmax(const void* logits, float* rowmax, int rows, int V, long long ld, void* stream) {
     if (rows <= 0) return CAI_K_OK;
-    ce_rowmax_kernel<<<rows, kCeThreads, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)logits, rowmax, V, ld);
+    launch_early(ce_rowmax_kernel, rows, kCeThreads, 0, (cudaStream_t)stream, (const __nv_bfloat16*)logits, rowmax, V, ld);
     CAI_LAUNCH_CHECK("ce_rowmax");
     return CAI_K_OK;
 }
 CAI_API int cai_ce_rowsum(const void* logits, const float* rowmax, float* rowsum, int rows, int V, long long ld,
                           void* stream) {
     if (rows <= 0) return CAI_K_OK;
-    ce_rowsum_kernel<<<rows, kCeThreads, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)logits, rowmax, rowsum, V, ld);
+    launch_early(ce_rowsum_kernel, rows, kCeThreads, 0, (cudaStream_t)stream, (const __nv_bfloat16*)logits, rowmax, rowsum, V, ld);
     CAI_LAUNCH_CHECK("ce_rowsum");
     return CAI_K_OK;
 }
@@ -565,9 +577,8 @@ CAI_API int cai_ce_grad_tp(void* logits, const int* targets, const float* rowmax
                            int rows, int V, long long ld, int vocab_lo, int add_lse, float grad_scale, float loss_scale,
                            void* stream) {
     if (rows <= 0) return CAI_K_OK;
-    ce_grad_tp_kernel<<<rows, kCeThreads, 0, (cudaStream_t)stream>>>((__nv_bfloat16*)logits, targets, rowmax, rowsum,
-                                                                     loss_sum, V, ld, vocab_lo, add_lse, grad_scale,
-                                                                     loss_scale);
+    launch_early(ce_grad_tp_kernel, rows, kCeThreads, 0, (cudaStream_t)stream, (__nv_bfloat16*)logits, targets, rowmax, rowsum, loss_sum,
+                 V, ld, vocab_lo, add_lse, grad_scale, loss_scale);
     CAI_LAUNCH_CHECK("ce_grad_tp");
     return CAI_K_OK;
 }
@@ -578,8 +589,8 @@ CAI_API int cai_adamw(float* master, float* m, float* v, const float* grad, void
     if (n <= 0) return CAI_K_OK;
     const float bc1 = 1.f - powf(beta1, (float)step);
     const float bc2 = 1.f - powf(beta2, (float)step);
-    adamw_kernel<<<blocks_for((n + 3) / 4, 256), 256, 0, (cudaStream_t)stream>>>(
-        master, m, v, grad, (__nv_bfloat16*)param_bf16, n, lr, beta1, beta2, eps, wd, grad_scale, bc1, bc2);
+    launch_early(adamw_kernel, blocks_for((n + 3) / 4, 256), 256, 0, (cudaStream_t)stream, master, m, v, grad, (__nv_bfloat16*)param_bf16,
+                 n, lr, beta1, beta2, eps, wd, grad_scale, bc1, bc2);
     CAI_LAUNCH_CHECK("adamw");
     return CAI_K_OK;
 }
@@ -608,8 +619,8 @@ CAI_API int cai_add_bf16(const void* a, const void* b, void* out, long long n, v
         set_last_error("add_bf16: n must be a multiple of 8");
         return CAI_K_BAD_ARG;
     }
-    add_bf16_kernel<<<blocks_for(n / 8, 256), 256, 0, (cudaStream_t)stream>>>(
-        (const __nv_bfloat16*)a, (const __nv_bfloat16*)b, (__nv_bfloat16*)out, n / 8);
+    launch_early(add_bf16_kernel, blocks_for(n / 8, 256), 256, 0, (cudaStream_t)stream, (const __nv_bfloat16*)a, (const __nv_bfloat16*)b,
+                 (__nv_bfloat16*)out, n / 8);
     CAI_LAUNCH_CHECK("add_bf16");
     return CAI_K_OK;
 }

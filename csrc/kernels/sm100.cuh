@@ -54,6 +54,20 @@ __device__ __forceinline__ bool elect_one() {
     return pred != 0;
 }
 
+// ---------------------------------------------------------------- launches that overlap their predecessor
+// A kernel started with launch_early (host_common.h) may be on the SMs while the kernel before it in the stream still runs. It
+// reads and writes nothing in global memory before grid_dep_wait, which returns once that kernel has completed with its memory
+// operations visible; as every kernel of this form waits, everything before that one has completed too. grid_dep_launch lets
+// the next kernel of the stream start its CTAs when all CTAs of this one have got here; they take what this one leaves free. Both do
+// nothing in a kernel that was launched the ordinary way.
+__device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// For kernels without a set-up worth overlapping: what is saved is the launch itself.
+__device__ __forceinline__ void grid_dep_begin() {
+    grid_dep_launch();
+    grid_dep_wait();
+}
+
 // ---------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));

@@ -30,6 +30,7 @@
 #include "../comm/peer.cuh"
 #include "../kernels/cai_kernels.h"
 #include "../kernels/host_common.h"
+#include "../kernels/sm100.cuh"
 #include "../plan/formats.h"
 #include "cai_runtime.h"
 
@@ -94,6 +95,7 @@ static int nccl_dtype(int dt) {
 __global__ void adamw_dev_kernel(float* __restrict__ master, float* __restrict__ m, float* __restrict__ v,
                                  const float* __restrict__ grad, __nv_bfloat16* __restrict__ param, long long n,
                                  const float* __restrict__ hyper, float gscale) {
+    grid_dep_begin();
     // hyper: lr, beta1, beta2, eps, wd, 1-beta1^t, 1-beta2^t
     const float lr = hyper[0], b1 = hyper[1], b2 = hyper[2], eps = hyper[3], wd = hyper[4], bc1 = hyper[5], bc2 = hyper[6];
     const long long i4 = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) * 4;
@@ -264,8 +266,8 @@ int run_op(cai_exec* ex, const Op& op, const ExecOp& x, cudaStream_t st) {
         case K_ADAMW: {
             const long long n = (static_cast<long long>(static_cast<uint32_t>(x.i[1])) << 32) | static_cast<uint32_t>(x.i[0]);
             const unsigned blocks = static_cast<unsigned>(((n + 3) / 4 + 255) / 256);
-            adamw_dev_kernel<<<blocks, 256, 0, st>>>((float*)P(0), (float*)P(1), (float*)P(2), (const float*)P(3),
-                                                     (__nv_bfloat16*)P(4), n, ex->hyper_dev, x.f[0]);
+            launch_early(adamw_dev_kernel, blocks, 256, 0, st, (float*)P(0), (float*)P(1), (float*)P(2), (const float*)P(3),
+                         (__nv_bfloat16*)P(4), n, ex->hyper_dev, x.f[0]);
             return cudaGetLastError() == cudaSuccess ? 0 : CAI_K_CUDA;
         }
         case K_ZERO:
