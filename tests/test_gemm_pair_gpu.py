@@ -183,3 +183,68 @@ def test_accumulation_keeps_subnormals(M, N, K):
         out = torch.full((M, N), old, device="cuda")
         ops.gemm(a, b, out=out, accumulate=True)
         assert bool((out.double() == old + 2.0 ** -130).all()), old
+
+
+def _ragged_counts(kind, slabs, seg_rows, g):
+    edges = [0, 1, 63, 64, 65, 127, 128, 129, 191, 192, 255, 256, 257, seg_rows - 1, seg_rows, seg_rows + 5]
+    if kind == "edges":
+        return torch.tensor([edges[i % len(edges)] for i in range(slabs)], dtype=torch.int32)
+    if kind == "one":
+        c = torch.zeros(slabs, dtype=torch.int32)
+        c[slabs // 2] = seg_rows
+        return c
+    if kind == "none":
+        return torch.zeros(slabs, dtype=torch.int32)
+    return torch.randint(0, seg_rows + 1, (slabs,), generator=g, dtype=torch.int32)
+
+
+# Live tiles counted ahead (up to 256 slabs) and the walk over all tiles (beyond): one slab and several per group, slabs of an odd number
+# of 128-row halves (a 256-row tile must not reach into the next slab), more row tiles than a raster group of eight.
+@pytest.mark.parametrize("groups,per_group,seg_rows,N,K", [(16, 1, 128, 256, 128), (5, 3, 384, 264, 192), (4, 4, 256, 512, 64),
+                                                           (2, 2, 2432, 384, 256), (300, 1, 128, 128, 64), (100, 3, 128, 72, 64), (256, 1, 128, 136, 64)])
+@pytest.mark.parametrize("kind", ["edges", "random", "one", "none"])
+def test_grouped_ragged_rows(groups, per_group, seg_rows, N, K, kind):
+    from cai_b200 import ops
+    g = torch.Generator().manual_seed(groups * 7 + seg_rows)
+    M = per_group * seg_rows
+    counts = _ragged_counts(kind, groups * per_group, seg_rows, g)
+    a = (torch.randn(groups * M, K, generator=g) * 0.5).bfloat16().cuda()
+    b = (torch.randn(groups * N, K, generator=g) * 0.5).bfloat16().cuda()
+    out = torch.full((groups * M, N), 7.0, device="cuda", dtype=torch.bfloat16)
+    ops.gemm_grouped(a, b, out, M, N, K, groups=groups, seg_counts=counts.cuda(), seg_rows=seg_rows, seg_mode=1)
+    A, B = a.view(groups, M, K).double(), b.view(groups, N, K).double()
+    ref = torch.einsum("gmk,gnk->gmn", A, B).view(-1, seg_rows, N)
+    # one rounding to bf16, and a sum of K exact products in fp32
+    bound = 2.0 ** -8 * ref.abs() + K * 2.0 ** -24 * torch.einsum("gmk,gnk->gmn", A.abs(), B.abs()).view(-1, seg_rows, N)
+    got = out.view(-1, seg_rows, N).double()
+    for s, c in enumerate(counts.tolist()):
+        c = min(c, seg_rows)
+        whole = (c + 127) // 128 * 128           # halves of 128 rows are written whole
+        assert ((got[s, :c] - ref[s, :c]).abs() <= bound[s, :c]).all()
+        assert bool((got[s, whole:] == 7.0).all())
+
+
+@pytest.mark.parametrize("groups,per_group,seg_rows,M,N", [(8, 1, 256, 256, 128), (3, 3, 384, 264, 136), (2, 5, 128, 128, 512)])
+@pytest.mark.parametrize("kind", ["edges", "random", "one", "none"])
+@pytest.mark.parametrize("accumulate", [False, True])
+def test_grouped_ragged_depth(groups, per_group, seg_rows, M, N, kind, accumulate):
+    from cai_b200 import ops
+    g = torch.Generator().manual_seed(groups * 5 + seg_rows)
+    K = per_group * seg_rows
+    counts = _ragged_counts(kind, groups * per_group, seg_rows, g)
+    a = (torch.randn(groups * K, M, generator=g) * 0.5).bfloat16()
+    b = (torch.randn(groups * K, N, generator=g) * 0.5).bfloat16()
+    # rows past a count up to the end of its 64-row block are zero, as a dispatch leaves them; later ones are never read
+    for s, c in enumerate(counts.tolist()):
+        c = min(c, seg_rows)
+        end = (c + 63) // 64 * 64
+        for t in (a, b):
+            t[s * seg_rows + c:s * seg_rows + end] = 0
+            t[s * seg_rows + end:(s + 1) * seg_rows] = float("nan")
+    out = torch.full((groups * M, N), 3.0, device="cuda")
+    ops.gemm_grouped(a.cuda(), b.cuda(), out, M, N, K, groups=groups, trans_a=True, trans_b=True, accumulate=accumulate,
+                     seg_counts=counts.cuda(), seg_rows=seg_rows, seg_mode=2)
+    A, B = a.view(groups, K, M).nan_to_num().double(), b.view(groups, K, N).nan_to_num().double()
+    ref = torch.einsum("gkm,gkn->gmn", A, B).reshape(-1, N) + (3.0 if accumulate else 0.0)
+    bound = (K + 1) * 2.0 ** -24 * (torch.einsum("gkm,gkn->gmn", A.abs(), B.abs()).reshape(-1, N) + 3.0)
+    assert ((out.cpu().double() - ref).abs() <= bound).all()
