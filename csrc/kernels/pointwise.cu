@@ -195,36 +195,116 @@ __global__ void embed_fwd_kernel(const int* __restrict__ tokens, const __nv_bflo
     for (int i = threadIdx.x; i < nv; i += blockDim.x) o[i] = e[i];
 }
 
-// Embedding backward without atomics: a CTA owns kEmbRows consecutive vocabulary rows, scans the token list front to
-// back and adds the gradient row of every token that falls into its range, in token order. Each row of dE has one
-// writer and a fixed order of additions, so the result is the same in every run (the reference scatters with
-// atomicAdd, src/cuda/cai_kernels.cu:26-34).
+// Embedding backward without atomics: a CTA owns kEmbRows consecutive vocabulary rows and adds the gradient row of every
+// token that falls into its range, in token order. Each row of dE has one writer and a fixed order of additions, so the result is
+// the same in every run (the reference scatters with atomicAdd, src/cuda/cai_kernels.cu:26-34). The tokens are looked through
+// kEmbScan at a time, sixteen loads in flight per thread; the places of those that fall into the range are put down row by row,
+// in order. Then the warps share out the rows in pieces of 32 * V columns: a piece of dE is read once, gets all its
+// additions in registers and is written once. What bounded the earlier form was latency: 256 tokens per two barriers, and a read,
+// an addition and a write of dE behind each other for every token: 17 us for 512 tokens of 512 x 256, 67 us for 3840 of 5000 x 1000, of
+// which 10 and 60 us are saved (whole steps 443 -> 433 us and 4.78 -> 4.72 ms).
 constexpr int kEmbRows = 32;
+constexpr int kEmbScan = 4096;
+template <int V>   // columns a lane takes at a time: 8 where rows are 16-byte aligned pieces, else 1
 __global__ void __launch_bounds__(256)
 embed_bwd_kernel(const int* __restrict__ tokens, const __nv_bfloat16* __restrict__ dout, float* __restrict__ dE, int T, int H,
                  int lo, int hi) {
     grid_dep_begin();
-    __shared__ unsigned match[8];
-    __shared__ int toks[256];
+    __shared__ unsigned list[kEmbScan];            // in token order: row << 16 | place in the scan
+    __shared__ unsigned short by_row[kEmbScan];    // places, row by row
+    __shared__ int warp_tot[8], row_count[kEmbRows], row_first[kEmbRows];
     const int v0 = lo + static_cast<int>(blockIdx.x) * kEmbRows;
     const int v1 = v0 + kEmbRows < hi ? v0 + kEmbRows : hi;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int t0 = 0; t0 < T; t0 += 256) {
-        const int t = t0 + threadIdx.x;
-        const int tok = t < T ? tokens[t] : -1;
-        const unsigned m = __ballot_sync(0xffffffffu, tok >= v0 && tok < v1);
-        toks[threadIdx.x] = tok;
-        if (lane == 0) match[warp] = m;
+    const int pieces = (H + 32 * V - 1) / (32 * V);
+    for (int t0 = 0; t0 < T; t0 += kEmbScan) {
+        // a warp takes 512 tokens, 32 neighbouring ones at a time
+        const int w0 = t0 + warp * 512;
+        int row[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            const int t = w0 + i * 32 + lane, tok = t < T ? tokens[t] : -1;
+            row[i] = t < T && tok >= v0 && tok < v1 ? tok - v0 : -1;
+        }
+        int mine = 0;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) mine += __popc(__ballot_sync(0xffffffffu, row[i] >= 0));
+        if (lane == 0) warp_tot[warp] = mine;
         __syncthreads();
+        int at = 0, n = 0;
+#pragma unroll
         for (int w = 0; w < 8; ++w) {
-            unsigned bits = match[w];
-            while (bits) {
-                const int b = __ffs(bits) - 1;
-                bits &= bits - 1;
-                const int tt = t0 + w * 32 + b;
-                float* row = dE + static_cast<long long>(toks[w * 32 + b] - lo) * H;
-                const __nv_bfloat16* d = dout + static_cast<long long>(tt) * H;
-                for (int i = threadIdx.x; i < H; i += 256) row[i] += __bfloat162float(d[i]);
+            if (w < warp) at += warp_tot[w];
+            n += warp_tot[w];
+        }
+        if (n == 0) {
+            __syncthreads();   // warp_tot is written again
+            continue;
+        }
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            const unsigned m = __ballot_sync(0xffffffffu, row[i] >= 0);
+            if (row[i] >= 0) list[at + __popc(m & ((1u << lane) - 1))] = static_cast<unsigned>(row[i]) << 16 | static_cast<unsigned>(warp * 512 + i * 32 + lane);
+            at += __popc(m);
+        }
+        __syncthreads();
+        // rows warp, warp + 8, ...: how many, then where
+        int cnt[kEmbRows / 8] = {};
+        for (int e0 = 0; e0 < n; e0 += 32) {
+            const int r = e0 + lane < n ? static_cast<int>(list[e0 + lane] >> 16) : -1;
+#pragma unroll
+            for (int k = 0; k < kEmbRows / 8; ++k) cnt[k] += __popc(__ballot_sync(0xffffffffu, r == warp + 8 * k));
+        }
+        if (lane == 0)
+#pragma unroll
+            for (int k = 0; k < kEmbRows / 8; ++k) row_count[warp + 8 * k] = cnt[k];
+        __syncthreads();
+        if (warp == 0) {
+            int sum = row_count[lane];
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int up = __shfl_up_sync(0xffffffffu, sum, o);
+                if (lane >= o) sum += up;
+            }
+            row_first[lane] = sum - row_count[lane];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < kEmbRows / 8; ++k) cnt[k] = row_first[warp + 8 * k];
+        for (int e0 = 0; e0 < n; e0 += 32) {
+            const unsigned e = e0 + lane < n ? list[e0 + lane] : 0xffff0000u;
+            const int r = static_cast<int>(e >> 16);
+#pragma unroll
+            for (int k = 0; k < kEmbRows / 8; ++k) {
+                const unsigned m = __ballot_sync(0xffffffffu, r == warp + 8 * k);
+                if (r == warp + 8 * k) by_row[cnt[k] + __popc(m & ((1u << lane) - 1))] = static_cast<unsigned short>(e);
+                cnt[k] += __popc(m);
+            }
+        }
+        __syncthreads();
+        for (int item = warp; item < kEmbRows * pieces; item += 8) {
+            const int r = item / pieces, piece = item - r * pieces, c = row_count[r];
+            const int col = (piece * 32 + lane) * V;
+            if (c == 0 || col >= H) continue;
+            const unsigned short* places = by_row + row_first[r];
+            const __nv_bfloat16* d = dout + static_cast<long long>(t0) * H + col;
+            float* out = dE + static_cast<long long>(v0 - lo + r) * H + col;
+            if constexpr (V == 8) {
+                float4 a = reinterpret_cast<const float4*>(out)[0], b = reinterpret_cast<const float4*>(out)[1];
+#pragma unroll 4
+                for (int k = 0; k < c; ++k) {
+                    float f[8];
+                    unpack8(*reinterpret_cast<const uint4*>(d + static_cast<long long>(places[k]) * H), f);
+                    a.x += f[0]; a.y += f[1]; a.z += f[2]; a.w += f[3];
+                    b.x += f[4]; b.y += f[5]; b.z += f[6]; b.w += f[7];
+                }
+                reinterpret_cast<float4*>(out)[0] = a;
+                reinterpret_cast<float4*>(out)[1] = b;
+            } else {
+                float a = *out;
+#pragma unroll 4
+                for (int k = 0; k < c; ++k) a += __bfloat162float(d[static_cast<long long>(places[k]) * H]);
+                *out = a;
             }
         }
         __syncthreads();
@@ -541,7 +621,9 @@ CAI_API int cai_embed_bwd(const int* tokens, const void* dout, float* dE, int T,
                           int vocab_hi, void* stream) {
     if (T <= 0) return CAI_K_OK;
     if (vocab_hi <= vocab_lo) return CAI_K_OK;
-    launch_early(embed_bwd_kernel, (vocab_hi - vocab_lo + kEmbRows - 1) / kEmbRows, 256, 0, (cudaStream_t)stream, tokens,
+    const dim3 grid((vocab_hi - vocab_lo + kEmbRows - 1) / kEmbRows);
+    const bool pieces = !(H & 7) && !(reinterpret_cast<uintptr_t>(dout) & 15) && !(reinterpret_cast<uintptr_t>(dE) & 15);
+    launch_early(pieces ? embed_bwd_kernel<8> : embed_bwd_kernel<1>, grid, 256, 0, (cudaStream_t)stream, tokens,
                  (const __nv_bfloat16*)dout, dE, T, H, vocab_lo, vocab_hi);
     CAI_LAUNCH_CHECK("embed_bwd");
     return CAI_K_OK;

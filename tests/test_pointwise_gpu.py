@@ -174,3 +174,21 @@ def test_rmsnorm_bwd_sums(rows, H):
     want_dx = dx0.double() + r * dd * gd - r ** 3 * xd * (dd * gd * xd).sum(1, keepdim=True) / H
     assert ((dg.double() - want_dg).norm() / want_dg.norm()).item() < 1e-5          # fp32 sums
     assert ((dx.double() - want_dx).norm() / want_dx.norm()).item() < 2 ** -8       # one rounding to bf16
+
+
+# tokens of one scan and of several, one row that takes every token, rows outside the range, widths of whole pieces, of a fraction of
+# one and not a multiple of 8
+@pytest.mark.parametrize("T,V,H,lo,hi", [(1, 8, 8, 0, 8), (4096, 40, 256, 0, 40), (4097, 33, 264, 0, 33), (9000, 1000, 136, 100, 777), (700, 64, 20, 0, 64),
+                                         (5000, 1, 512, 0, 1)])
+def test_embed_bwd_adds_in_token_order(T, V, H, lo, hi):
+    from cai_b200 import ops
+    g = torch.Generator().manual_seed(T)
+    tokens = torch.randint(0, V, (T,), generator=g, dtype=torch.int32)
+    dout = torch.randn(T, H, generator=g).bfloat16()
+    start = torch.randn(hi - lo, H, generator=g)
+    got = ops.embed_bwd_(tokens.cuda(), dout.cuda(), start.cuda(), vocab_lo=lo, vocab_hi=hi).cpu()
+    want = start.clone()
+    for t, tok in enumerate(tokens.tolist()):
+        if lo <= tok < hi:
+            want[tok - lo] += dout[t].float()      # fp32, in this order: equal to the last bit
+    assert torch.equal(got, want)
