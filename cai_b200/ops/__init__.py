@@ -12,8 +12,14 @@ from ._lib import KernelError, check, device_status, lib
 EPI_BF16, EPI_F32, EPI_F32_ACCUM, EPI_BF16_RESIDUAL, EPI_SWIGLU, EPI_SWIGLU_BWD = 0, 1, 2, 3, 4, 5
 
 
+# Handle of the current stream of the current device, as torch.cuda.current_stream().cuda_stream gives it, without building a stream
+# object on the way: 0.2 instead of 3.3 us of the some 15 us an op's host path took.
+_current_device = torch._C._cuda_getDevice
+_raw_stream = torch._C._cuda_getCurrentRawStream
+
+
 def _stream():
-    return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(_current_device())
 
 
 def _p(t):
@@ -45,7 +51,7 @@ def gemm(a, b, *, trans_a=False, trans_b=False, out=None, out_dtype=torch.bfloat
     assert K == Kb, f"K mismatch {K} vs {Kb}"
     if out is None:
         assert not accumulate
-        out = torch.empty((M, N), device=a.device, dtype=out_dtype)
+        out = a.new_empty((M, N), dtype=out_dtype)
     assert out.shape == (M, N) and out.stride(1) == 1
     if out.dtype == torch.bfloat16:
         epi = EPI_BF16_RESIDUAL if residual is not None else EPI_BF16
@@ -112,10 +118,10 @@ def moe_route_fwd(logits, k, cap):
     the expert already holds ``cap`` tokens) and ``counts`` int32 ``[E]``."""
     T, E = logits.shape
     assert logits.dtype == torch.float32 and logits.is_contiguous()
-    idx = torch.empty(T, k, device=logits.device, dtype=torch.int32)
+    idx = logits.new_empty((T, k), dtype=torch.int32)
     pos = torch.empty_like(idx)
-    w = torch.empty(T, k, device=logits.device, dtype=torch.float32)
-    counts = torch.empty(E, device=logits.device, dtype=torch.int32)
+    w = logits.new_empty((T, k))
+    counts = logits.new_empty(E, dtype=torch.int32)
     check(lib().cai_moe_route_fwd(_p(logits), _p(idx), _p(w), _p(pos), _p(counts), T, E, k, int(cap), _stream()), "moe_route_fwd")
     return idx, w, pos, counts
 
@@ -123,7 +129,7 @@ def moe_route_fwd(logits, k, cap):
 def moe_route_bwd(logits, idx, dw, pos):
     """Gradient of the router logits (bf16 ``[T,E]``) from the gradient of the combine weights."""
     T, E = logits.shape
-    out = torch.empty(T, E, device=logits.device, dtype=torch.bfloat16)
+    out = logits.new_empty((T, E), dtype=torch.bfloat16)
     check(lib().cai_moe_route_bwd(_p(logits), _p(idx), _p(dw), _p(pos), _p(out), T, E, idx.shape[1], _stream()), "moe_route_bwd")
     return out
 
@@ -131,7 +137,7 @@ def moe_route_bwd(logits, idx, dw, pos):
 def rmsnorm_fwd(x, g, eps=1e-6):
     rows, H = x.shape
     y = torch.empty_like(x)
-    rstd = torch.empty(rows, device=x.device, dtype=torch.float32)
+    rstd = x.new_empty(rows, dtype=torch.float32)
     check(lib().cai_rmsnorm_fwd(_p(x), _p(g), _p(y), _p(rstd), rows, H, float(eps), _stream()), "rmsnorm_fwd")
     return y, rstd
 
@@ -143,10 +149,10 @@ def rmsnorm_bwd(x, g, rstd, dy, dx=None, dg=None, dx_accumulate=False, dg_accumu
         dx = torch.empty_like(x)
     if dg is None:
         assert not dg_accumulate
-        dg = torch.empty(H, device=x.device, dtype=torch.float32)
+        dg = x.new_empty(H, dtype=torch.float32)
     parts = lib().cai_rmsnorm_bwd_parts(rows)
     if scratch is None:
-        scratch = torch.empty(parts * H, device=x.device, dtype=torch.float32)
+        scratch = x.new_empty(parts * H, dtype=torch.float32)
     assert scratch.numel() >= parts * H
     check(lib().cai_rmsnorm_bwd(_p(x), _p(g), _p(rstd), _p(dy), _p(dx), _p(dg), _p(scratch), rows, H,
                                 int(dx_accumulate), int(dg_accumulate), _stream()), "rmsnorm_bwd")
@@ -168,7 +174,7 @@ def rope_apply_(qkv, table, seq, nh, nkv, hd, inverse=False):
 
 def swiglu_fwd(gu):
     T, F2 = gu.shape
-    act = torch.empty((T, F2 // 2), device=gu.device, dtype=gu.dtype)
+    act = gu.new_empty((T, F2 // 2))
     check(lib().cai_swiglu_fwd(_p(gu), _p(act), T, F2 // 2, _stream()), "swiglu_fwd")
     return act
 
@@ -216,8 +222,8 @@ def flash_attn_fwd(qkv, B, S, nh, nkv, hd, scale=None, variant=0):
     from the grid size, 1 = one query tile per CTA (score MMA a block ahead), 2 = two tiles per CTA in ping-pong."""
     assert qkv.dtype == torch.bfloat16 and qkv.is_contiguous()
     scale = hd ** -0.5 if scale is None else scale
-    out = torch.empty((B * S, nh * hd), device=qkv.device, dtype=torch.bfloat16)
-    lse = torch.empty((B, nh, S), device=qkv.device, dtype=torch.float32)
+    out = qkv.new_empty((B * S, nh * hd))
+    lse = qkv.new_empty((B, nh, S), dtype=torch.float32)
     check(lib().cai_flash_attn_fwd_variant(_p(qkv), _p(out), _p(lse), B, S, nh, nkv, hd, float(scale), int(variant), _stream()),
           "flash_attn_fwd")
     return out, lse
@@ -229,7 +235,7 @@ def flash_attn_bwd(qkv, out, dout, lse, B, S, nh, nkv, hd, scale=None, dqkv=None
     if dqkv is None:
         dqkv = torch.empty_like(qkv)
     if delta is None:
-        delta = torch.empty((B, nh, S), device=qkv.device, dtype=torch.float32)
+        delta = qkv.new_empty((B, nh, S), dtype=torch.float32)
     check(lib().cai_flash_attn_bwd_parts(_p(qkv), _p(out), _p(dout), _p(lse), _p(delta), _p(dqkv), B, S, nh, nkv, hd,
                                          float(scale), int(parts), _stream()), "flash_attn_bwd")
     return dqkv
@@ -244,8 +250,8 @@ def quant_rows_1x128(x):
     per row and 128 columns (``amax / 448``), the activation side of the block-scaled GEMM."""
     assert x.dtype == torch.bfloat16 and x.dim() == 2 and x.stride(1) == 1 and x.shape[1] % 128 == 0
     rows, cols = x.shape
-    q = torch.empty(rows, cols, device=x.device, dtype=torch.float8_e4m3fn)
-    s = torch.empty(rows, cols // 128, device=x.device, dtype=torch.float32)
+    q = x.new_empty((rows, cols), dtype=torch.float8_e4m3fn)
+    s = x.new_empty((rows, cols // 128), dtype=torch.float32)
     check(lib().cai_quant_rows_1x128(_p(x), x.stride(0), _p(q), cols, _p(s), rows, cols, _stream()), "quant_rows")
     return q, s
 
@@ -275,7 +281,7 @@ def gemm_fp8(aq, sa, bq, sb, *, out=None, out_dtype=torch.bfloat16, residual=Non
     assert K == Kb and K % 128 == 0 and aq.stride(1) == 1 and bq.stride(1) == 1
     assert sa.shape == (M, K // 128) and sb.shape == ((N + 127) // 128, K // 128) and sa.is_contiguous() and sb.is_contiguous()
     if out is None:
-        out = torch.empty(M, N, device=aq.device, dtype=out_dtype)
+        out = aq.new_empty((M, N), dtype=out_dtype)
     epi = EPI_F32 if out.dtype == torch.float32 else (EPI_BF16_RESIDUAL if residual is not None else EPI_BF16)
     check(lib().cai_gemm_fp8_blockscaled(_p(aq), _p(sa), _p(bq), _p(sb), _p(out), _p(residual), M, N, K, aq.stride(0), bq.stride(0),
                                          out.stride(0), residual.stride(0) if residual is not None else 0, epi, _stream()), "gemm_fp8")

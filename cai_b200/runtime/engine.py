@@ -46,6 +46,7 @@ def _declare_runtime(L):
     L.cai_exec_launches.restype = c_ulonglong
     L.cai_exec_step.argtypes = [P, I, c_float]
     L.cai_exec_sync.argtypes = [P]
+    L.cai_exec_read.argtypes = [P, P, P, c_size_t, ctypes.POINTER(I)]
     L.cai_exec_use_graph.argtypes = [P, I]
     L.cai_exec_trace_enable.argtypes = [P, I]
     L.cai_exec_nvtx_enable.argtypes = [P, I]
@@ -389,13 +390,11 @@ class Engine:
 
     def read_loss(self) -> float:
         """Device->host read of the step's mean loss (synchronises the step)."""
-        with torch.cuda.stream(self.stream):
-            self.loss_host.copy_(self.loss_dev.view(-1)[:8], non_blocking=True)
-        klib.check(self.L.cai_exec_sync(self.ex), "exec_sync")
-        st = klib.device_status(clear=True)
-        if st != 0:
+        st = c_int(0)
+        klib.check(self.L.cai_exec_read(self.ex, self.loss_dev.data_ptr(), self.loss_host.data_ptr(), 32, ctypes.byref(st)), "exec_read")
+        if st.value != 0:
             self.device_fault = True
-            raise DeviceStatusError(st)
+            raise DeviceStatusError(st.value)
         self.completed_steps = self.step_count
         return float(self.loss_host[0])
 

@@ -56,6 +56,8 @@ CAI_API void cai_exec_set_sm_limit(cai_exec* ex, int sms);
 CAI_API float* cai_exec_hyper(cai_exec* ex);
 CAI_API int cai_exec_step(cai_exec* ex, int step, float lr);
 CAI_API int cai_exec_sync(cai_exec* ex);
+/* `bytes` of device memory to pinned host memory, and the device's status word, behind everything enqueued on compute_hi. */
+CAI_API int cai_exec_read(cai_exec* ex, const void* dev, void* pinned, size_t bytes, int* status);
 CAI_API int cai_exec_use_graph(cai_exec* ex, int on);
 CAI_API int cai_exec_trace_enable(cai_exec* ex, int on);
 /* One NVTX range per op, named by its kernel, around the launches of a replay (stream replays only; a captured
