@@ -9,7 +9,7 @@
 // block into one of two TMEM buffers, eight epilogue warps read that fp32 partial back with
 // tcgen05.ld, scale it and add it to accumulators kept in registers while the tensor core works on
 // the next block in the other buffer. TMA (128-byte swizzle, one 128-byte row = 128 k-elements)
-// feeds a 4-stage shared-memory ring. Persistent, one CTA per SM, 128x256 tiles.
+// feeds a 4-stage shared-memory ring. Persistent, one CTA per SM, 128x256 tiles; most products run on pairs of CTAs (below).
 //
 // The reference only names the dtype (`param_dtype fp8e4m3`, include/cai_tensor.h:14-22) and has no
 // fp8 arithmetic anywhere.
@@ -237,6 +237,298 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     if (warp == 1) tmem_dealloc(tmem_base, 2 * f8::kBN);
 }
 
+// ---------------------------------------------------------------------------- pairs of CTAs
+// The same product on CTA pairs (a cluster of two, cta_group::2): 256 x 256 tiles, each CTA with 128 rows of A and of B per k-block. What holds the
+// one-CTA kernel at 1240 cycles per k-block (512 of MMA) is several things of that size: operands arrive at 54 B / cycle (48 KB: 900 cycles; a CTA
+// of a pair takes in 32 KB), shared memory is read and written at 128 B / cycle (768), the one issuing thread spends two waits of 200 to
+// 300 cycles per block, and eight epilogue warps read 128 columns each behind four waits. Here two warps issue, one per TMEM buffer, each
+// paying its waits under the other's MMAs; sixteen epilogue warps (112 registers each: the launch's 96 and what the other warpgroup
+// gives up) take 64 columns each; scales come in eight k-blocks at a time. 1090 cycles per k-block are left, the round trip of MMA,
+// commit, TMEM read and hand-back over two buffers. 2000 x 4096 x 14336 145 -> 129 us, 2000 x 14336 x 4096 169 -> 150, 8192^3 717 -> 612.
+namespace f8p {
+constexpr int kBM = 256, kBN = 256, kBK = 128;
+constexpr int kStages = 6;
+constexpr int kHalf = 128 * kBK;                   // bytes of A, or of B, a CTA brings in per stage
+constexpr int kEpiWarps = 16;
+constexpr int kThreads = 128 + kEpiWarps * 32;     // warp 0 TMA, warps 1-2 MMA, warp 3 scales, warps 4-19 epilogue
+constexpr int kScaleKb = 8;                        // k-blocks whose scales come in at a time
+constexpr int kScaleRow = 132;                     // 128 rows of A, padded: eight k-blocks of four rows fall on 32 banks
+constexpr int kScaleWords = kScaleKb * kScaleRow + 2 * kScaleKb;
+constexpr int kSmem = kStages * 2 * kHalf + 2 * kScaleWords * 4 + 512 + 1024;
+}  // namespace f8p
+
+__device__ __forceinline__ void umma_f8_ss_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "setp.ne.b32 p, %4, 0;\n"
+        "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n"
+        "}\n" ::"r"(tmem_d),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* m, uint32_t cluster_bar, int x, int y) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.cta_group::2"
+        " [%0], [%1, {%3, %4}], [%2];"
+        ::"r"(smem_u32(dst)), "l"(m), "r"(cluster_bar), "r"(x), "r"(y)
+        : "memory");
+}
+__device__ __forceinline__ void cp_async4(float* smem_dst, const float* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(smem_dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(f8p::kThreads, 1)
+gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmFp8Params p) {
+    grid_dep_launch();
+    using namespace f8p;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    uint8_t* sA = smem;
+    uint8_t* sB = smem + kStages * kHalf;
+    float* scales = reinterpret_cast<float*>(smem + kStages * 2 * kHalf);   // [2][kScaleWords]
+    uint64_t* bars = reinterpret_cast<uint64_t*>(scales + 2 * kScaleWords);
+    uint64_t* full = bars;                         // [kStages] used in the even CTA: both CTAs' operands have landed
+    uint64_t* empty = bars + kStages;              // [kStages] in each CTA
+    uint64_t* part_full = bars + 2 * kStages;      // [2] in each CTA: a k-block's partial product is in TMEM
+    uint64_t* sc_full = part_full + 2;             // [2] in each CTA
+    uint64_t* part_empty = sc_full + 2;            // [2] used in the even CTA: both CTAs' epilogue warps have read the partial product
+    uint64_t* sc_empty = part_empty + 2;           // [2] in each CTA
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sc_empty + 2);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t rank = cluster_ctarank();
+    if (warp == 0) {
+        constexpr int kOne = 2 * kStages + 4;
+        if (lane < kOne) mbar_init(&bars[lane], 1);
+        else if (lane < kOne + 2) mbar_init(&bars[lane], 2 * kEpiWarps);
+        else if (lane < kOne + 4) mbar_init(&bars[lane], kEpiWarps);
+        if (lane == 31) *abort_flag = 0;
+        mbar_fence_init();
+    } else if (warp == 2 && lane == 0) {
+        tma_prefetch_desc(&tmA);
+        tma_prefetch_desc(&tmB);
+    }
+    if (warp == 1) {
+        tmem_alloc_pair(tmem_slot, 2 * kBN);
+        tmem_relinquish_pair();
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync();      // the other CTA's barriers are initialised before anything arrives on them
+    tc_fence_after();
+    grid_dep_wait();
+    const uint32_t tmem_base = *tmem_slot;
+    const int num_tiles = p.tiles_m * p.tiles_n;
+    const int num_kb = p.K / kBK;
+    const int first = static_cast<int>(blockIdx.x >> 1), stride = static_cast<int>(gridDim.x >> 1);
+    // eight row tiles share a column of B before the next one
+    auto coords = [&](int tile, int& tm, int& tn) {
+        const int per_group = 8 * p.tiles_n, g = tile / per_group, in = tile - g * per_group;
+        const int gsz = min(p.tiles_m - g * 8, 8);
+        tm = g * 8 + in % gsz;
+        tn = in / gsz;
+    };
+
+    if (warp < 4) {
+        // 24 + 4 x 112 registers a thread of each of the five warpgroups: within the 5 x 96 of the launch
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 24;");
+        if (warp == 0) {
+            if (lane == 0) {
+                // ---------------- TMA producer (both CTAs)
+                int s = 0;
+                uint32_t ph = 0;
+                bool ok = true;
+                for (int tile = first; tile < num_tiles && ok; tile += stride) {
+                    int tm, tn;
+                    coords(tile, tm, tn);
+                    const int m0 = tm * kBM + static_cast<int>(rank) * 128, n0 = tn * kBN + static_cast<int>(rank) * 128;
+                    for (int kb = 0; kb < num_kb; ++kb) {
+                        if (!mbar_wait(&empty[s], ph ^ 1, abort_flag, p.status, CAI_DEV_TIMEOUT_TMA_EMPTY)) {
+                            ok = false;
+                            break;
+                        }
+                        if (rank == 0) mbar_expect_tx(&full[s], 4 * kHalf);
+                        const uint32_t bar = map_to_cta(smem_u32(&full[s]), 0);
+                        tma_load_2d_pair(sA + s * kHalf, &tmA, bar, kb * kBK, m0);
+                        tma_load_2d_pair(sB + s * kHalf, &tmB, bar, kb * kBK, n0);
+                        if (++s == kStages) {
+                            s = 0;
+                            ph ^= 1;
+                        }
+                    }
+                }
+                // every stage handed back: no arrival of the other CTA is still on its way when this CTA ends
+                for (int i = 0; i < kStages && ok; ++i) {
+                    ok = mbar_wait(&empty[s], ph ^ 1, abort_flag, p.status, CAI_DEV_TIMEOUT_TMA_EMPTY);
+                    if (++s == kStages) {
+                        s = 0;
+                        ph ^= 1;
+                    }
+                }
+                if (!ok)
+                    for (int i = 0; i < 32; ++i) __nanosleep(50000);   // let copies in flight land
+            }
+        } else if (warp < 3) {
+            if (rank == 0) {
+                // ---------------- MMA issuers (even CTA): warp 1 the even k-blocks into TMEM buffer 0, warp 2 the odd ones into buffer 1
+                const uint32_t buf = warp - 1;
+                const uint32_t idesc = umma_idesc_e4m3(kBM, kBN);
+                const uint64_t a_first = umma_smem_desc_sw128(smem_u32(sA), 0, 1024), b_first = umma_smem_desc_sw128(smem_u32(sB), 0, 1024);
+                const bool leader = elect_one();
+                const uint32_t total = static_cast<uint32_t>(num_kb) * static_cast<uint32_t>(first < num_tiles ? (num_tiles - first + stride - 1) / stride : 0);
+                uint32_t s = buf, ph = 0, n = 0;      // ring slot and its phase; k-blocks this warp has issued
+                bool ok = true;
+                for (uint32_t it = buf; it < total; it += 2, ++n) {
+                    if (!mbar_wait_warp(&full[s], ph, abort_flag, p.status, CAI_DEV_TIMEOUT_TMA_FULL) ||
+                        !mbar_wait_warp(&part_empty[buf], (n & 1) ^ 1, abort_flag, p.status, CAI_DEV_TIMEOUT_TMEM_EMPTY)) {
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after();
+                    if (leader) {
+                        const uint64_t ad = a_first + s * (kHalf >> 4), bd = b_first + s * (kHalf >> 4);
+#pragma unroll
+                        for (int k = 0; k < kBK / f8::kUmmaK; ++k)
+                            umma_f8_ss_pair(tmem_base + buf * kBN, ad + k * (f8::kUmmaK >> 4), bd + k * (f8::kUmmaK >> 4), idesc, k != 0 ? 1u : 0u);
+                        umma_commit_pair(&part_full[buf], 3);
+                        umma_commit_pair(&empty[s], 3);
+                    }
+                    s += 2;
+                    if (s >= kStages) {
+                        s -= kStages;
+                        ph ^= 1;
+                    }
+                }
+                // the buffer handed back: no arrival of the odd CTA is still on its way when this one ends
+                if (ok) mbar_wait_warp(&part_empty[buf], (n & 1) ^ 1, abort_flag, p.status, CAI_DEV_TIMEOUT_TMEM_EMPTY);
+            }
+        } else {
+            // ---------------- scales of eight k-blocks at a time: lane l takes k-block l & 7 of rows l / 8, l / 8 + 4, ...
+            uint32_t b = 0, ph = 0;
+            bool ok = true;
+            for (int tile = first; tile < num_tiles && ok; tile += stride) {
+                int tm, tn;
+                coords(tile, tm, tn);
+                const int r0 = tm * kBM + static_cast<int>(rank) * 128 + (lane >> 3);
+                for (int kb0 = 0; kb0 < num_kb; kb0 += kScaleKb) {
+                    if (!mbar_wait_warp(&sc_empty[b], ph ^ 1, abort_flag, p.status, CAI_DEV_TIMEOUT_TMEM_EMPTY)) {
+                        ok = false;
+                        break;
+                    }
+                    float* dst = scales + b * kScaleWords;
+                    const int kb = kb0 + (lane & 7);
+                    if (kb < num_kb) {
+#pragma unroll 8
+                        for (int i = 0; i < 32; ++i)
+                            cp_async4(dst + (lane & 7) * kScaleRow + (lane >> 3) + 4 * i,
+                                      p.sa + static_cast<long long>(min(r0 + 4 * i, p.M - 1)) * num_kb + kb);
+                        if (lane < 16) {
+                            const int cb = min(tn * 2 + (lane >> 3), (p.N - 1) / 128);
+                            cp_async4(dst + kScaleKb * kScaleRow + lane, p.sb + static_cast<long long>(cb) * num_kb + kb);
+                        }
+                    }
+                    cp_async_wait_all();
+                    mbar_arrive_warp(&sc_full[b]);
+                    b ^= 1;
+                    if (b == 0) ph ^= 1;
+                }
+            }
+        }
+    } else {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
+        // ---------------- epilogue warps: scale-and-add every k-block, then write the tile; 64 columns each
+        const int q = warp & 3, cg = (warp - 4) >> 2;
+        const uint32_t taddr0 = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + cg * 64;
+        const uint32_t release0 = map_to_cta(smem_u32(&part_empty[0]), 0);
+        uint32_t it = 0, sb = 0, sph = 0;
+        bool ok = true;
+        for (int tile = first; tile < num_tiles && ok; tile += stride) {
+            float acc[64];
+#pragma unroll
+            for (int e = 0; e < 64; ++e) acc[e] = 0.f;
+            for (int kb = 0; kb < num_kb; ++kb, ++it) {
+                const uint32_t buf = it & 1;
+                const int in = kb & (kScaleKb - 1);
+                if (in == 0 && !mbar_wait_warp(&sc_full[sb], sph, abort_flag, p.status, CAI_DEV_TIMEOUT_TMEM_FULL)) {
+                    ok = false;
+                    break;
+                }
+                const float* sc = scales + sb * kScaleWords;
+                const float s = sc[in * kScaleRow + q * 32 + lane] * sc[kScaleKb * kScaleRow + (cg >> 1) * kScaleKb + in];
+                if (in == kScaleKb - 1 || kb == num_kb - 1) {
+                    mbar_arrive_warp(&sc_empty[sb]);
+                    sb ^= 1;
+                    if (sb == 0) sph ^= 1;
+                }
+                if (!mbar_wait_warp(&part_full[buf], (it >> 1) & 1, abort_flag, p.status, CAI_DEV_TIMEOUT_TMEM_FULL)) {
+                    ok = false;
+                    break;
+                }
+                tc_fence_after();
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    uint32_t r[32];
+                    tmem_ld_32x32(taddr0 + buf * kBN + c * 32, r);
+                    tmem_ld_wait();
+                    if (c == 1) {
+                        // read: the buffer goes back before the last additions
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive_cluster(release0 + buf * 8);
+                    }
+#pragma unroll
+                    for (int e = 0; e < 32; ++e) acc[c * 32 + e] = fmaf(s, __uint_as_float(r[e]), acc[c * 32 + e]);
+                }
+            }
+            if (!ok) break;
+            int tm, tn;
+            coords(tile, tm, tn);
+            const long long row = static_cast<long long>(tm) * kBM + rank * 128 + q * 32 + lane;
+            const int col0 = tn * kBN + cg * 64;
+            if (row >= p.M || col0 >= p.N) {
+                // nothing of this lane's is written
+            } else if (p.epi == CAI_EPI_F32) {
+                float* crow = reinterpret_cast<float*>(p.C) + row * p.ldc + col0;
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    if (col0 + j * 4 >= p.N) break;
+                    *reinterpret_cast<float4*>(crow + j * 4) = make_float4(acc[j * 4], acc[j * 4 + 1], acc[j * 4 + 2], acc[j * 4 + 3]);
+                }
+            } else {
+                __nv_bfloat16* crow = reinterpret_cast<__nv_bfloat16*>(p.C) + row * p.ldc + col0;
+                const __nv_bfloat16* rrow =
+                    p.epi == CAI_EPI_BF16_RESIDUAL ? reinterpret_cast<const __nv_bfloat16*>(p.R) + row * p.ldr + col0 : nullptr;
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    if (col0 + j * 8 >= p.N) break;
+                    float v[8];
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) v[e] = acc[j * 8 + e];
+                    if (rrow) {
+                        float rf[8];
+                        unpack8(*reinterpret_cast<const uint4*>(rrow + j * 8), rf);
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) v[e] += rf[e];
+                    }
+                    *reinterpret_cast<uint4*>(crow + j * 8) = pack8(v);
+                }
+            }
+            __syncwarp();
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    __syncwarp();
+    cluster_sync();
+    if (warp == 1) {
+        tc_fence_after();
+        tmem_dealloc_pair(tmem_base, 2 * kBN);
+    }
+}
+
 // ------------------------------------------------------------------ quantisation
 // One warp per (row, 128-column block): amax -> scale = amax / 448, q = x / scale.
 __global__ void __launch_bounds__(256)
@@ -458,12 +750,20 @@ CAI_API int cai_gemm_fp8_blockscaled(const void* Aq, const float* sa, const void
         return CAI_K_BAD_ARG;
     }
     const int dev = current_device();
+    const int sms = sm_count(dev);
+    // Pairs of CTAs, unless the last half of their 256-row tiles stays empty and costs waves: a wave of pair tiles takes some nine tenths
+    // of one of one-CTA tiles of half the rows (us, one-CTA / pair: 2000 x 4096 x 14336 145 / 129, 128 x 14336 x 4096 27.4 / 25.3, 16 x 4096
+    // x 4096 22.9 / 19.9; two waves of pairs against one: 128 x 28672 x 4096 31.7 / 47.8). Both forms give the same bits.
+    const long long cols = (N + f8::kBN - 1) / f8::kBN, pairs = sms / 2 > 0 ? sms / 2 : 1;
+    const long long waves_one = ((M + f8::kBM - 1) / f8::kBM * cols + sms - 1) / sms, waves_pair = ((M + f8p::kBM - 1) / f8p::kBM * cols + pairs - 1) / pairs;
+    const bool pair = 9 * waves_pair <= 10 * waves_one;
     CUtensorMap tmA, tmB;
-    if (!encode_tmap_2d(&tmA, Aq, M, K, lda, f8::kBK, f8::kBM, 1) || !encode_tmap_2d(&tmB, Bq, N, K, ldb, f8::kBK, f8::kBN, 1))
+    if (!encode_tmap_2d(&tmA, Aq, M, K, lda, f8::kBK, 128, 1) || !encode_tmap_2d(&tmB, Bq, N, K, ldb, f8::kBK, pair ? 128 : f8::kBN, 1))
         return CAI_K_BAD_ARG;
     static bool configured[64] = {};
     if (!configured[dev & 63]) {
-        if (cudaFuncSetAttribute(gemm_fp8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, f8::kSmem) != cudaSuccess) {
+        if (cudaFuncSetAttribute(gemm_fp8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, f8::kSmem) != cudaSuccess ||
+            cudaFuncSetAttribute(gemm_fp8_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, f8p::kSmem) != cudaSuccess) {
             set_last_error("cudaFuncSetAttribute(gemm_fp8) failed");
             return CAI_K_CUDA;
         }
@@ -473,12 +773,17 @@ CAI_API int cai_gemm_fp8_blockscaled(const void* Aq, const float* sa, const void
     p.M = M; p.N = N; p.K = K;
     p.sa = sa; p.sb = sb;
     p.C = C; p.R = R; p.ldc = ldc; p.ldr = ldr; p.epi = epi;
-    p.tiles_m = (M + f8::kBM - 1) / f8::kBM;
-    p.tiles_n = (N + f8::kBN - 1) / f8::kBN;
+    const int rows = pair ? f8p::kBM : f8::kBM;
+    p.tiles_m = (M + rows - 1) / rows;
+    p.tiles_n = static_cast<int>(cols);
     p.status = status_words(dev);
     const int tiles = p.tiles_m * p.tiles_n;
-    const int sms = sm_count(dev);
-    launch_early(gemm_fp8_kernel, tiles < sms ? tiles : sms, f8::kThreads, f8::kSmem, static_cast<cudaStream_t>(stream), tmA, tmB, p);
+    if (pair) {
+        launch_early(gemm_fp8_pair_kernel, 2 * (tiles < pairs ? tiles : static_cast<int>(pairs)), f8p::kThreads, f8p::kSmem,
+                     static_cast<cudaStream_t>(stream), tmA, tmB, p);
+    } else {
+        launch_early(gemm_fp8_kernel, tiles < sms ? tiles : sms, f8::kThreads, f8::kSmem, static_cast<cudaStream_t>(stream), tmA, tmB, p);
+    }
     if (cudaGetLastError() != cudaSuccess) {
         set_last_error("gemm_fp8 launch failed");
         return CAI_K_CUDA;

@@ -116,3 +116,34 @@ def test_quant_blocks_forms_agree(rows, cols):
     for a, b in ((q, q2), (qt, qt2)):
         assert torch.equal(a.view(torch.uint8), b.view(torch.uint8))
     assert torch.equal(s, s2) and torch.equal(st, st2)
+
+
+# one row, halves of the 256-row pair tile, one past a tile; a fraction of a column tile; one k-block, and one past the eight whose scales
+# come in together; several tiles per pair. In float64 from the quantised operands.
+@pytest.mark.parametrize("M,N,K", [(1, 8, 128), (127, 136, 256), (129, 264, 1152), (257, 640, 1024), (300, 72, 2176), (2300, 4104, 640)])
+def test_gemm_edges(M, N, K):
+    from cai_b200 import ops
+    torch.manual_seed(M)
+    xq, sx = ops.quant_rows_1x128(torch.randn(M, K, device="cuda").to(torch.bfloat16))
+    wq, sw = ops.quant_blocks_128x128((torch.randn(N, K, device="cuda") * 0.05).to(torch.bfloat16))
+    A, B = _dequant_rows(xq, sx).double(), _dequant_blocks(wq, sw).double()
+    ref = A @ B.t()
+    bound = K * 2.0 ** -23 * (A.abs() @ B.abs().t())       # products of e4m3 are exact; sums and scalings in fp32
+    wide = torch.full((M, N + 16), 7.0, device="cuda")
+    ops.gemm_fp8(xq, sx, wq, sw, out=wide[:, :N])
+    assert ((wide[:, :N] - ref).abs() <= bound).all() and bool((wide[:, N:] == 7.0).all())
+    res = torch.randn(M, N, device="cuda").to(torch.bfloat16)
+    out = ops.gemm_fp8(xq, sx, wq, sw, residual=res)
+    want = ref + res.double()
+    assert ((out.double() - want).abs() <= bound + 2.0 ** -8 * want.abs() + 1e-6).all()
+
+
+def test_one_cta_and_pair_forms_give_the_same_bits():
+    from cai_b200 import ops
+    torch.manual_seed(0)
+    K, N = 1152, 28672                                     # 128 rows run on one CTA per tile, 256 rows on pairs
+    xq, sx = ops.quant_rows_1x128(torch.randn(256, K, device="cuda").to(torch.bfloat16))
+    wq, sw = ops.quant_blocks_128x128((torch.randn(N, K, device="cuda") * 0.05).to(torch.bfloat16))
+    both = ops.gemm_fp8(xq, sx, wq, sw, out_dtype=torch.float32)
+    half = ops.gemm_fp8(xq[:128], sx[:128].contiguous(), wq, sw, out_dtype=torch.float32)
+    assert torch.equal(both[:128], half)
