@@ -219,7 +219,8 @@ def adamw_(master, m, v, grad, param, step, lr, beta1=0.9, beta2=0.999, eps=1e-8
 
 def flash_attn_fwd(qkv, B, S, nh, nkv, hd, scale=None, variant=0):
     """Causal GQA flash attention forward over packed ``qkv`` ``[B*S, (nh + 2 nkv) * hd]``. ``variant``: 0 = chosen
-    from the grid size, 1 = one query tile per CTA (score MMA a block ahead), 2 = two tiles per CTA in ping-pong."""
+    from the grid size and the length, 1 = one query tile per CTA (score MMA a block ahead), 2 = two tiles per CTA in
+    ping-pong, 3 = one tile per CTA, two CTAs per SM."""
     assert qkv.dtype == torch.bfloat16 and qkv.is_contiguous()
     scale = hd ** -0.5 if scale is None else scale
     out = qkv.new_empty((B * S, nh * hd))

@@ -101,3 +101,15 @@ def test_flash_attn_bwd_takes_an_output_on_eight_bytes():
     assert torch.equal(d[0], d[1]) and torch.equal(got[0], got[1])
     want = (dout.float() * out.float()).view(B, S, nh, hd).sum(-1).transpose(1, 2)
     assert ((d[0] - want).abs() <= 2.0 ** -23 * 128 * (dout.float() * out.float()).abs().view(B, S, nh, hd).sum(-1).transpose(1, 2)).all()
+
+
+# one key block and several, an odd number of tiles, grouped heads; more CTAs than two per SM
+@pytest.mark.parametrize("B,S,nh,nkv", [(1, 128, 1, 1), (3, 384, 6, 2), (8, 640, 9, 3), (2, 1152, 16, 8), (1, 4224, 2, 1)])
+def test_forward_forms_give_the_same_bits(B, S, nh, nkv):
+    from cai_b200 import ops
+    torch.manual_seed(S)
+    qkv = (torch.randn(B * S, (nh + 2 * nkv) * 128, device="cuda") * 2).to(torch.bfloat16)   # the running maximum moves now and then
+    out, lse = ops.flash_attn_fwd(qkv, B, S, nh, nkv, 128, variant=2)
+    for variant in (0, 1, 3):
+        o, l = ops.flash_attn_fwd(qkv, B, S, nh, nkv, 128, variant=variant)
+        assert torch.equal(o, out) and torch.equal(l, lse)
