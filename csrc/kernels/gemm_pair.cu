@@ -52,6 +52,7 @@ struct PairParams {
     int tile0;                    // split form: first tile of this launch
     const int* seg_counts;
     int seg_rows, seg_mode, grp_seg;
+    bool overlap;                 // the next kernel of the stream may come in while this one finishes (not under a limit on the SMs)
     int slabs;                    // ragged rows, tiles counted ahead: slabs of all groups (0: the ordinary walk)
     void* C;                      // split form: results leave through registers
     const __nv_bfloat16* R;       // residual, read row by row
@@ -242,7 +243,7 @@ template <int BN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair::kThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmR, const PairParams p) {
-    grid_dep_launch();
+    if (p.overlap) grid_dep_launch();
     using namespace pair;
     constexpr int STAGES = kStages<BN>;
     constexpr int HALF = BN / 2;          // columns of the tile one epilogue warp drains; rows of B one CTA loads
@@ -563,7 +564,7 @@ constexpr int kSplitSmem = kStages<kSplitBN> * kPerStage * kBlock<kSplitBN> + 51
 template <int S>
 __global__ void __launch_bounds__(pair::kThreads, 1)
 gemm_pair_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const PairParams p) {
-    grid_dep_launch();
+    if (p.overlap) grid_dep_launch();
     using namespace pair;
     constexpr int BN = kSplitBN, STAGES = kStages<BN>, HALF = BN / 2;
     extern __shared__ uint8_t smem_raw[];
@@ -730,7 +731,7 @@ gemm_pair_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
 }
 
 template <int S>
-static void split_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, unsigned grid, cudaStream_t st) {
+static void split_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, unsigned grid, bool overlap, cudaStream_t st) {
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(pair::kThreads);
     cfg.dynamicSmemBytes = pair::kSplitSmem;
@@ -741,7 +742,7 @@ static void split_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, uns
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // see launch_early
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 2;
+    cfg.numAttrs = overlap ? 2 : 1;
 }
 
 // Tensor map of rows x cols per group, the groups `apart` rows apart.
@@ -772,12 +773,13 @@ static int launch_split(const void* A, const void* B, const GemmShape& g, PairPa
         }
         configured[dev & 63] = true;
     }
-    // Under a limit on the SMs the clusters go out in turns of `at_once`, one launch behind the other: the same sums in the same order.
+    // Under a limit on the SMs the clusters go out in turns of `at_once`, each launched when the one before has ended: the same sums in the
+    // same order.
     const int tiles = p.tiles_m * p.tiles_n * p.groups;
     for (p.tile0 = 0; p.tile0 < tiles; p.tile0 += at_once) {
         cudaLaunchConfig_t cfg = {};
         cudaLaunchAttribute attr[2];
-        split_config<S>(cfg, attr, static_cast<unsigned>(2 * S * (tiles - p.tile0 < at_once ? tiles - p.tile0 : at_once)), st);
+        split_config<S>(cfg, attr, static_cast<unsigned>(2 * S * (tiles - p.tile0 < at_once ? tiles - p.tile0 : at_once)), p.overlap, st);
         const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_pair_split_kernel<S>, tmA, tmB, p);
         if (e != cudaSuccess) {
             set_last_error("gemm_pair_split launch failed: %s", cudaGetErrorString(e));
@@ -810,7 +812,8 @@ static int launch_pair(const void* A, const void* B, const GemmShape& g, PairPar
     p.group_m = 8;
     const int tiles = p.tiles_m * p.tiles_n * p.groups;
     const int grid = 2 * (tiles < pairs ? tiles : pairs);
-    launch_early(gemm_pair_kernel<BN>, grid, pair::kThreads, pair::kSmem<BN>, st, tmA, tmB, tmC, tmR, p);
+    if (p.overlap) launch_early(gemm_pair_kernel<BN>, grid, pair::kThreads, pair::kSmem<BN>, st, tmA, tmB, tmC, tmR, p);
+    else gemm_pair_kernel<BN><<<grid, pair::kThreads, pair::kSmem<BN>, st>>>(tmA, tmB, tmC, tmR, p);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
         set_last_error("gemm_pair launch failed: %s", cudaGetErrorString(e));
@@ -866,6 +869,7 @@ int gemm_pair(const void* A, const void* B, const GemmShape& g, cudaStream_t st)
     p.R = static_cast<const __nv_bfloat16*>(g.R);
     p.ldc = g.ldc; p.ldr = g.ldr; p.grp_c = g.grp_c;
     p.tile0 = 0;
+    p.overlap = g.sm_limit <= 0;
     const long long slabs = g.seg_mode == 1 ? static_cast<long long>((g.M + g.seg_rows - 1) / g.seg_rows) * g.groups : 0;
     p.slabs = slabs <= pair::kMaxSlabs ? static_cast<int>(slabs) : 0;
     const int dev = current_device();

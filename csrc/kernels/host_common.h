@@ -38,8 +38,8 @@ bool encode_tmap_3d(CUtensorMap* out, const void* base, uint64_t cols, uint64_t 
 // it back from the data): what the chains of short kernels of a small step or layer wait for is the launch of each, the set-up of its
 // barriers and tensor memory and the end of the one before. A step of 69 launches 546 -> 443 us, one of 226 launches
 // 5.17 -> 4.76 ms, attention over 8 x 384 tokens 93 -> 85 us; long kernels gain nothing and lose nothing.
-// Only kernels that call grid_dep_wait in every CTA may be launched like this, and kernels that wait for
-// other GPUs are not: a CTA that only waits for its turn would hold an SM that the exchange on another stream may need.
+// Only kernels that call grid_dep_wait in every CTA may be launched like this. Kernels that wait for other GPUs are not, nor are products
+// under a limit on their SMs: a CTA that only waits for its turn would hold an SM that another stream may need.
 template <typename... Params, typename... Args>
 inline cudaError_t launch_early(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
     cudaLaunchConfig_t cfg = {};

@@ -1,5 +1,7 @@
 """Kernels that start before their predecessor in the stream has finished: chains in which every kernel reads what the one
 before it wrote and overwrites what the one before that read, enqueued without a pause, against the same calls one at a time."""
+import ctypes
+
 import pytest
 import torch
 
@@ -100,3 +102,71 @@ def test_attention_chain_matches_one_call_at_a_time(batch, seq, heads, kv_heads)
     for _ in range(5):
         for got, ref in zip(steps(lambda: None), want):
             assert torch.equal(got, ref)
+
+
+def _early_launches(call):
+    """How many launches of `call`, captured, may start before their predecessor has ended (programmatic edges of the graph)."""
+    call()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        call()
+    get = ctypes.CDLL("libcuda.so.1").cuGraphGetEdges_v2     # (graph, from, to, {from_port, to_port, type, ...}, count)
+    handle, n = ctypes.c_void_p(graph.raw_cuda_graph()), ctypes.c_size_t(0)
+    assert get(handle, None, None, None, ctypes.byref(n)) == 0
+    nodes, data = (ctypes.c_void_p * n.value)(), ((ctypes.c_ubyte * 8) * n.value)()
+    assert get(handle, nodes, (ctypes.c_void_p * n.value)(), data, ctypes.byref(n)) == 0
+    return sum(d[2] == 1 for d in data)
+
+
+# Under a limit no launch starts early: turns of the split form, and products behind each other in the persistent one.
+@pytest.mark.parametrize("M,N,K", [(333, 1024, 3000), (300, 968, 2048), (1536, 1536, 520), (4096, 4104, 264)])
+def test_limited_products_start_behind_each_other(M, N, K):
+    g = torch.Generator(device="cuda").manual_seed(M)
+    a = torch.randn(M, K, generator=g, device="cuda").bfloat16()
+    b = torch.randn(N, K, generator=g, device="cuda").bfloat16()
+    out = torch.empty(M, N, device="cuda", dtype=torch.bfloat16)
+
+    def twice(limit):
+        ops.gemm(a, b, out=out, sm_limit=limit)
+        ops.gemm(a, b, out=out, sm_limit=limit)
+
+    assert _early_launches(lambda: twice(0)) > 0
+    for limit in (2, 10, 60):
+        assert _early_launches(lambda: twice(limit)) == 0
+
+
+# The SMs that a limit leaves free stay free until the product ends: a product of another stream, whose
+# CTAs share an SM with no other product's, is done long before, although the next one of the first stream is already enqueued.
+@pytest.mark.parametrize("M,N,K,limit", [(4096, 4096, 4096, 32)])
+def test_sms_beside_a_product_stay_free(M, N, K, limit):
+    g = torch.Generator(device="cuda").manual_seed(0)
+    a = torch.randn(M, K, generator=g, device="cuda").bfloat16()
+    b = torch.randn(N, K, generator=g, device="cuda").bfloat16()
+    wide = torch.randn(4096, 4096, generator=g, device="cuda").bfloat16()
+    small = wide[:1024, :1024]
+    out, out_wide, out_small = (torch.empty(n, m, device="cuda", dtype=torch.bfloat16) for n, m in ((M, N), (4096, 4096), (1024, 1024)))
+    main, beside = torch.cuda.Stream(), torch.cuda.Stream()
+    start, alone, done = (torch.cuda.Event(enable_timing=True) for _ in range(3))
+    torch.cuda.synchronize()
+
+    def run(both):
+        with torch.cuda.stream(main):
+            torch.cuda._sleep(400000)          # all of it is enqueued meanwhile
+            start.record()
+            ops.gemm(a, b, out=out, sm_limit=limit)
+            if both:
+                ops.gemm(wide, wide, out=out_wide)
+            else:
+                alone.record()
+        if both:
+            with torch.cuda.stream(beside):
+                beside.wait_event(start)
+                torch.cuda._sleep(60000)       # the first product has started
+                ops.gemm(small, small, out=out_small)
+                done.record()
+        torch.cuda.synchronize()
+        return start.elapsed_time(done if both else alone)
+
+    first, beside_it = (sorted(run(both) for _ in range(7))[3] for both in (False, True))
+    assert beside_it < 0.6 * first
