@@ -200,7 +200,6 @@ __device__ __forceinline__ void issue_pd_ss(uint32_t d_tmem, uint64_t a_desc, ui
 __global__ void __launch_bounds__(kAttnBwdThreads, 1)
 attn_dkdv_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant__ CUtensorMap tm_do,
                  const AttnBwdParams p) {
-    grid_dep_launch();
     // no room to round the base up: tiles start on swizzle boundaries only if the shared window does (checked)
     extern __shared__ __align__(1024) uint8_t smem[];
     if (smem_u32(smem) & 1023) {
@@ -303,6 +302,7 @@ attn_dkdv_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
                 tma_load_2d(d, &tm_do, &do_full[slot], h * kAttnHD, q_row);
                 tma_load_2d(d + kAttnSub, &tm_do, &do_full[slot], h * kAttnHD + 64, q_row);
             }
+            grid_dep_launch();
             if (!ok)
                 for (int i = 0; i < 32; ++i) __nanosleep(50000);
         }
@@ -507,7 +507,6 @@ attn_dkdv_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_consta
 __global__ void __launch_bounds__(kAttnBwdThreads, 1)
 attn_dq_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant__ CUtensorMap tm_do,
                const AttnBwdParams p) {
-    grid_dep_launch();
     extern __shared__ __align__(1024) uint8_t smem[];
     if (smem_u32(smem) & 1023) {
         grid_dep_wait();
@@ -603,6 +602,7 @@ attn_dq_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant
                     kph ^= 1;
                 }
             }
+            grid_dep_launch();
             if (!ok)
                 for (int k = 0; k < 32; ++k) __nanosleep(50000);
         }

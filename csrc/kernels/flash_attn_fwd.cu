@@ -138,7 +138,6 @@ __device__ __forceinline__ void softmax_tile(uint32_t tS, uint32_t tO, int r, in
 
 __global__ void __launch_bounds__(kAttnFwdThreads, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tm, const AttnFwdParams p) {
-    grid_dep_launch();
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* sQ = smem;                            // 2 tiles
@@ -223,6 +222,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm, const AttnFwdParams p) {
                 tma_load_2d(sV + slot * kAttnTileBytes, &tm, &v_full[slot], col_v, kv_row);
                 tma_load_2d(sV + slot * kAttnTileBytes + kAttnSub, &tm, &v_full[slot], col_v + 64, kv_row);
             }
+            grid_dep_launch();
             if (!ok)
                 for (int i = 0; i < 32; ++i) __nanosleep(50000);
         }
@@ -301,7 +301,6 @@ constexpr int kAttnFwd1Threads = 256;
 
 __global__ void __launch_bounds__(kAttnFwd1Threads, 1)
 attn_fwd1_kernel(const __grid_constant__ CUtensorMap tm, const AttnFwdParams p) {
-    grid_dep_launch();
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* sQ = smem;
@@ -374,6 +373,7 @@ attn_fwd1_kernel(const __grid_constant__ CUtensorMap tm, const AttnFwdParams p) 
                 tma_load_2d(sV + slot * kAttnTileBytes, &tm, &v_full[slot], col_v, kv_row);
                 tma_load_2d(sV + slot * kAttnTileBytes + kAttnSub, &tm, &v_full[slot], col_v + 64, kv_row);
             }
+            grid_dep_launch();
             if (!ok)
                 for (int i = 0; i < 32; ++i) __nanosleep(50000);
         }
@@ -537,7 +537,6 @@ constexpr int kAttnHalfThreads = 192;   // warp 0 TMA, warp 1 MMA, warps 2-5 sof
 
 __global__ void __launch_bounds__(kAttnHalfThreads, 2)
 attn_fwd_half_kernel(const __grid_constant__ CUtensorMap tm, const AttnFwdParams p) {
-    grid_dep_launch();
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* sQ = smem;
@@ -600,6 +599,7 @@ attn_fwd_half_kernel(const __grid_constant__ CUtensorMap tm, const AttnFwdParams
                 tma_load_2d(sV, &tm, v_full, col_v, kv_row);
                 tma_load_2d(sV + kAttnSub, &tm, v_full, col_v + 64, kv_row);
             }
+            grid_dep_launch();
             if (!ok)
                 for (int i = 0; i < 32; ++i) __nanosleep(50000);
         }

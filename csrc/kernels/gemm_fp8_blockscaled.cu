@@ -67,7 +67,6 @@ __device__ __forceinline__ void umma_f8_ss(uint32_t tmem_d, uint64_t adesc, uint
 
 __global__ void __launch_bounds__(f8::kThreads, 1)
 gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmFp8Params p) {
-    grid_dep_launch();
     using namespace f8;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -130,6 +129,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                     }
                 }
             }
+            grid_dep_launch();
             if (!ok)
                 for (int i = 0; i < 32; ++i) __nanosleep(50000);  // let copies in flight land before the CTA's memory goes
         }
@@ -281,7 +281,6 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(f8p::kThreads, 1)
 gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmFp8Params p) {
-    grid_dep_launch();
     using namespace f8p;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -360,6 +359,7 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
                         }
                     }
                 }
+                grid_dep_launch();
                 // every stage handed back: no arrival of the other CTA is still on its way when this CTA ends
                 for (int i = 0; i < kStages && ok; ++i) {
                     ok = mbar_wait(&empty[s], ph ^ 1, abort_flag, p.status, CAI_DEV_TIMEOUT_TMA_EMPTY);

@@ -243,7 +243,6 @@ template <int BN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair::kThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmR, const PairParams p) {
-    if (p.overlap) grid_dep_launch();
     using namespace pair;
     constexpr int STAGES = kStages<BN>;
     constexpr int HALF = BN / 2;          // columns of the tile one epilogue warp drains; rows of B one CTA loads
@@ -322,6 +321,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                     }
                 }
             }
+            if (p.overlap) grid_dep_launch();
             if (ok) {
                 // every stage has been handed back: no arrival of the other CTA is still on its way when this CTA ends
                 for (int i = 0; i < STAGES && ok; ++i) {
@@ -564,7 +564,6 @@ constexpr int kSplitSmem = kStages<kSplitBN> * kPerStage * kBlock<kSplitBN> + 51
 template <int S>
 __global__ void __launch_bounds__(pair::kThreads, 1)
 gemm_pair_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const PairParams p) {
-    if (p.overlap) grid_dep_launch();
     using namespace pair;
     constexpr int BN = kSplitBN, STAGES = kStages<BN>, HALF = BN / 2;
     extern __shared__ uint8_t smem_raw[];
@@ -630,6 +629,7 @@ gemm_pair_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
                     ph ^= 1;
                 }
             }
+            if (p.overlap) grid_dep_launch();
             // every stage handed back: no arrival is still on its way when the CTA ends
             for (int i = 0; i < STAGES && ok; ++i) {
                 ok = mbar_wait(&empty[s], ph ^ 1, abort_flag, p.status, CAI_DEV_TIMEOUT_TMA_EMPTY);

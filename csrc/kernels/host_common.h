@@ -36,8 +36,10 @@ bool encode_tmap_3d(CUtensorMap* out, const void* base, uint64_t cols, uint64_t 
 
 // Launch a kernel so that it may start while the kernel before it in the stream still runs (grid_dep_wait in sm100.cuh holds
 // it back from the data): what the chains of short kernels of a small step or layer wait for is the launch of each, the set-up of its
-// barriers and tensor memory and the end of the one before. A step of 69 launches 546 -> 443 us, one of 226 launches
-// 5.17 -> 4.76 ms, attention over 8 x 384 tokens 93 -> 85 us; long kernels gain nothing and lose nothing.
+// barriers and tensor memory and the end of the one before. A step of some 60 launches 546 -> 443 us (400 since grid_dep_launch comes
+// behind the last loads), one of 220 launches 5.17 -> 4.76 ms, attention over 8 x 384 tokens 93 -> 85 us. Chains of long kernels take
+// the same time (norm, two products and SwiGLU, six times: 16384 tokens of 2048 x 8192 8.5 and 8.5 ms, 4096 of 4096 x 14336 7.0
+// and 6.9; runs differ by 3 %).
 // Only kernels that call grid_dep_wait in every CTA may be launched like this. Kernels that wait for other GPUs are not, nor are products
 // under a limit on their SMs: a CTA that only waits for its turn would hold an SM that another stream may need.
 template <typename... Params, typename... Args>

@@ -57,12 +57,18 @@ __device__ __forceinline__ bool elect_one() {
 // ---------------------------------------------------------------- launches that overlap their predecessor
 // A kernel started with launch_early (host_common.h) may be on the SMs while the kernel before it in the stream still runs. It
 // reads and writes nothing in global memory before grid_dep_wait, which returns once that kernel has completed with its memory
-// operations visible; as every kernel of this form waits, everything before that one has completed too. grid_dep_launch lets
-// the next kernel of the stream start its CTAs when all CTAs of this one have got here; they take what this one leaves free. Both do
-// nothing in a kernel that was launched the ordinary way.
+// operations visible; as every kernel of this form waits, everything before that one has completed too. In a kernel that was launched the
+// ordinary way grid_dep_wait returns at once.
+// grid_dep_launch, by one thread of every CTA, lets the next kernel of the stream start its CTAs, if that one was started with launch_early,
+// however this one was launched. They take what this kernel leaves free, shared memory and tensor memory included, and keep it
+// until it ends. So it comes behind this kernel's own tensor memory allocation (a waiting CTA on the same SM could hold the columns that
+// a CTA of this kernel has still to get, and neither would go on), and in kernels of some length behind a CTA's last loads: until then the
+// SMs that this kernel does not fill belong to other streams. A layer's backward of 16384 tokens, 2 heads / 1 kv head, with its weight gradients
+// and dQ on streams of their own: 2540 us with the call at the kernels' beginning, 2395 here, 2500 without early launches; 4096 tokens, 8 / 4 heads
+// 2352, 2240 and 2387 us.
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-// For kernels without a set-up worth overlapping: what is saved is the launch itself.
+// For short kernels without a set-up worth overlapping: what is saved is the launch itself.
 __device__ __forceinline__ void grid_dep_begin() {
     grid_dep_launch();
     grid_dep_wait();

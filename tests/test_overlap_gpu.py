@@ -136,9 +136,9 @@ def test_limited_products_start_behind_each_other(M, N, K):
         assert _early_launches(lambda: twice(limit)) == 0
 
 
-# The SMs that a limit leaves free stay free until the product ends: a product of another stream, whose
+# The SMs that a product does not fill, under a limit or for want of tiles, stay free until it ends: a product of another stream, whose
 # CTAs share an SM with no other product's, is done long before, although the next one of the first stream is already enqueued.
-@pytest.mark.parametrize("M,N,K,limit", [(4096, 4096, 4096, 32)])
+@pytest.mark.parametrize("M,N,K,limit", [(4096, 4096, 4096, 32), (256, 256, 262144, 0)])
 def test_sms_beside_a_product_stay_free(M, N, K, limit):
     g = torch.Generator(device="cuda").manual_seed(0)
     a = torch.randn(M, K, generator=g, device="cuda").bfloat16()
