@@ -68,6 +68,12 @@ CAI_API int cai_gemm_bf16_seg(const void* A, const void* B, void* C, const void*
                               int b_mn_major, int epi, float alpha, const int* seg_counts, int seg_rows, int seg_mode,
                               int sm_limit, void* stream);
 
+/* The tiles that pair `pair` of `pairs` CTA pairs takes of such a product with seg_mode 1, in order: the walk of the kernel, run on the host
+ * (seg_counts in host memory, ceil(M / seg_rows) entries per group). Six ints a tile: group, column tile, the first rows of its two 128-row
+ * halves inside the group, which of them are live. Returns the number of tiles, of which `capacity` are written. Needs no GPU. */
+CAI_API int cai_gemm_bf16_ragged_walk(int M, int N, int groups, const int* seg_counts, int seg_rows, int tile_cols, int pairs, int pair, int* tiles,
+                                      int capacity);
+
 /* `groups` independent products of one shape in ONE launch (the local experts of a mixture-of-experts layer):
  * group g reads A and B at row coordinate + g * grp_a / grp_b (rows of the [M,K] or, MN-major, [K,M] tensor),
  * writes C at row + g * grp_c and owns grp_seg entries of seg_counts. MN-major grouped operands need K % 64 == 0. */

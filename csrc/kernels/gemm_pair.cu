@@ -39,7 +39,7 @@ constexpr int kBox = 4096;            // an epilogue box: 32 rows x 128 bytes
 template <int BN> constexpr int kBBytes = BN / 2 * kBK * 2;
 template <int BN> constexpr int kBlock = kABytes + kBBytes<BN>;
 template <int BN> constexpr int kStages = BN == 256 ? 3 : 4;
-constexpr int kMaxSlabs = 256;        // ragged rows: slabs whose live tiles a launch can count ahead
+constexpr int kMaxSlabs = 256;        // ragged rows: slabs whose live halves a launch can count ahead
 template <int BN> constexpr int kSmem = kStages<BN> * kPerStage * kBlock<BN> + kEpiWarps * kBox + 512 + (kMaxSlabs + 4) * 4 + 1024;
 }  // namespace pair
 
@@ -53,19 +53,19 @@ struct PairParams {
     const int* seg_counts;
     int seg_rows, seg_mode, grp_seg;
     bool overlap;                 // the next kernel of the stream may come in while this one finishes (not under a limit on the SMs)
-    int slabs;                    // ragged rows, tiles counted ahead: slabs of all groups (0: the ordinary walk)
+    int grp_slabs;                // ragged rows, live halves counted ahead: slabs of a group (0: the ordinary walk)
     void* C;                      // split form: results leave through registers
     const __nv_bfloat16* R;       // residual, read row by row
     long long ldc, ldr, grp_c;    // grp_c: rows between the groups of C and R
     int* status;
 };
 
-__device__ __forceinline__ bool pair_seg_live(const PairParams& p, int g, int row0) {
+__host__ __device__ __forceinline__ bool pair_seg_live(const PairParams& p, int g, int row0) {
     const int slab = row0 / p.seg_rows;
     return row0 - slab * p.seg_rows < p.seg_counts[g * p.grp_seg + slab];
 }
 // Is the 128-row half that starts at row `row0` of group g computed and written?
-__device__ __forceinline__ bool pair_half_live(const PairParams& p, int g, int row0) {
+__host__ __device__ __forceinline__ bool pair_half_live(const PairParams& p, int g, int row0) {
     return row0 < p.M && (p.seg_mode != 1 || pair_seg_live(p, g, row0));
 }
 
@@ -98,7 +98,7 @@ struct PairStages {
     }
 };
 
-__device__ __forceinline__ void pair_tile_coords(const PairParams& p, int tile_all, int& tm, int& tn, int& grp) {
+__host__ __device__ __forceinline__ void pair_tile_coords(const PairParams& p, int tile_all, int& tm, int& tn, int& grp) {
     const int per_product = p.tiles_m * p.tiles_n;
     grp = tile_all / per_product;
     const int tile = tile_all - grp * per_product;
@@ -111,38 +111,45 @@ __device__ __forceinline__ void pair_tile_coords(const PairParams& p, int tile_a
     tn = in / gsz;
 }
 
-// The tiles of one pair of CTAs. Ragged rows are walked over live tiles only: first[s] is the number of live tiles before slab
-// s, so that every pair gets its share of them. (Dealt out by their place in the full slab, the live ones at the front of
-// slabs of eight row tiles fell to every other pair: an eighth more for the pairs with the even ones. 64 slabs with some 1024 of
-// 2048 rows live, 3072 x 4096: 1605 -> 1351 us, 4096 x 3072: 1707 -> 1356 us.)
+// The tiles of one pair of CTAs. Ragged rows are walked over live halves of 128 rows only, numbered group by group, with one that is
+// not live behind an odd number of them: first[s] is 2 x the number of the first half of slab s (at the end of a group + 1 where its
+// last half is not live). A tile takes two neighbouring halves of its group, of whatever slabs: each CTA of a pair loads, multiplies and
+// writes its own. So every pair gets its share of the tiles, and none is half empty but the last of a group. us, tiles by their place in
+// the full slabs / live tiles of each slab / live halves: 64 slabs of one group each, some 1024 of 2048 rows live, 3072 x 4096 1605 / 1351 /
+// 1351; 8 groups of 8 slabs, 3072 x 4096, 128 rows full 151 / 255 / 151, 384 rows full 386 / 493 / 383, 1152 rows at random 1080 / 710 / 620.
 struct PairTiles {
-    int tile = static_cast<int>(blockIdx.x >> 1), slab = 0;
-    // First row (inside the group) and column tile of the next tile, its group, and which of its 128-row halves are live.
-    __device__ __forceinline__ bool next(const PairParams& p, const int* first, int& row0, int& tn, int& grp, uint32_t& halves) {
-        const int stride = static_cast<int>(gridDim.x >> 1);
-        if (p.slabs) {
-            if (tile >= first[p.slabs]) return false;
-            while (tile >= first[slab + 1]) ++slab;
-            const int per = (p.M + p.seg_rows - 1) / p.seg_rows;
-            grp = slab / per;
-            row0 = (slab - grp * per) * p.seg_rows;
-            const int rows = min(min(p.seg_counts[grp * p.grp_seg + slab - grp * per], p.seg_rows), p.M - row0);
-            const int tiles = (rows + pair::kBM - 1) / pair::kBM, per_group = p.group_m * p.tiles_n;
-            const int g = (tile - first[slab]) / per_group, in = tile - first[slab] - g * per_group;
-            const int gsz = min(tiles - g * p.group_m, p.group_m);
-            const int at = (g * p.group_m + in % gsz) * pair::kBM;
-            row0 += at;
+    int tile, stride, group = 0;
+    __host__ __device__ __forceinline__ PairTiles(int pair, int pairs) : tile(pair), stride(pairs) {}
+    // The next tile: its column tile, its group, the first row (inside the group) of the half of CTA `rank`, and whether that half is live.
+    __host__ __device__ __forceinline__ bool next(const PairParams& p, const int* first, int rank, int& row, int& tn, int& grp, bool& live) {
+        if (p.grp_slabs) {
+            if (tile >= (first[p.grp_slabs * p.groups] >> 2) * p.tiles_n) return false;
+            while (tile >= (first[(group + 1) * p.grp_slabs] >> 2) * p.tiles_n) ++group;
+            grp = group;
+            int lo = group * p.grp_slabs, hi = lo + p.grp_slabs;
+            const int h0 = first[lo] >> 1, end = first[hi], rows = ((end >> 1) - h0) >> 1;
+            const int at = tile - (h0 >> 1) * p.tiles_n, per_raster = p.group_m * p.tiles_n;
+            const int g = at / per_raster, in = at - g * per_raster;
+            const int left = rows - g * p.group_m, gsz = left < p.group_m ? left : p.group_m;
             tn = in / gsz;
-            halves = at + 128 < rows ? 3u : 1u;
+            int h = h0 + 2 * (g * p.group_m + in - tn * gsz) + rank;
+            live = h < (end >> 1) - (end & 1);
+            if (!live) --h;                    // the other CTA's rows once more: loaded, never written
+            while (hi - lo > 1) {              // its slab: the last that starts at h or before
+                const int mid = (lo + hi) >> 1;
+                if (first[mid] >> 1 <= h) lo = mid;
+                else hi = mid;
+            }
+            row = (lo - group * p.grp_slabs) * p.seg_rows + (h - (first[lo] >> 1)) * 128;
             tile += stride;
             return true;
         }
         for (; tile < p.tiles_m * p.tiles_n * p.groups; tile += stride) {
             int tm;
             pair_tile_coords(p, tile, tm, tn, grp);
-            row0 = tm * pair::kBM;
-            halves = (pair_half_live(p, grp, row0) ? 1u : 0u) | (pair_half_live(p, grp, row0 + 128) ? 2u : 0u);
-            if (halves) {
+            row = tm * pair::kBM + rank * 128;
+            live = pair_half_live(p, grp, row);
+            if (live || pair_half_live(p, grp, row ^ 128)) {
                 tile += stride;
                 return true;
             }
@@ -150,28 +157,58 @@ struct PairTiles {
         return false;
     }
 };
-// first[s] for s = 0 .. p.slabs, by one warp.
-__device__ __forceinline__ void pair_count_tiles(const PairParams& p, int* first, int lane) {
-    const int per = (p.M + p.seg_rows - 1) / p.seg_rows;
-    int n[pair::kMaxSlabs / 32];
+__host__ __device__ __forceinline__ int pair_live_halves(const PairParams& p, int slab) {
+    const int grp = slab / p.grp_slabs, in = slab - grp * p.grp_slabs;
+    int n = p.seg_counts[grp * p.grp_seg + in];
+    if (n > p.seg_rows) n = p.seg_rows;
+    if (n > p.M - in * p.seg_rows) n = p.M - in * p.seg_rows;
+    return n > 0 ? (n + 127) / 128 : 0;
+}
+// first[s] for s = 0 .. all slabs, by one warp.
+__device__ __forceinline__ void pair_count_halves(const PairParams& p, int* first, int lane) {
+    constexpr int kChunks = pair::kMaxSlabs / 32;
+    const int slabs = p.grp_slabs * p.groups;
+    int n[kChunks];
 #pragma unroll
-    for (int i = 0; i < pair::kMaxSlabs / 32; ++i) {
-        const int s = i * 32 + lane, grp = s / per, in = s - grp * per;
-        n[i] = s < p.slabs ? min(min(p.seg_counts[grp * p.grp_seg + in], p.seg_rows), p.M - in * p.seg_rows) : 0;
-    }
+    for (int i = 0; i < kChunks; ++i) n[i] = i * 32 + lane < slabs ? pair_live_halves(p, i * 32 + lane) : 0;
     int before = 0;
     if (lane == 0) first[0] = 0;
 #pragma unroll
-    for (int i = 0; i < pair::kMaxSlabs / 32; ++i) {
-        const int s = i * 32 + lane;
-        int sum = n[i] > 0 ? (n[i] + pair::kBM - 1) / pair::kBM * p.tiles_n : 0;
+    for (int i = 0; i < kChunks; ++i) {
+        if (i * 32 >= slabs) break;
+        // one slab a group: its odd half is added here
+        const int odd = p.grp_slabs == 1 ? n[i] & 1 : 0;
+        int sum = n[i] + odd;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const int up = __shfl_up_sync(0xffffffffu, sum, o);
             if (lane >= o) sum += up;
         }
-        if (s < p.slabs) first[s + 1] = before + sum;
+        if (i * 32 + lane < slabs) first[i * 32 + lane + 1] = (before + sum) * 2 + odd;
         before += __shfl_sync(0xffffffffu, sum, 31);
+    }
+    if (p.grp_slabs == 1) return;
+    // several: which groups have an odd number (so far halves are numbered without the added ones), then every slab moves by those before it
+    __syncwarp();
+    uint32_t odd[kChunks] = {};
+#pragma unroll
+    for (int i = 0; i < kChunks; ++i) {
+        if (i * 32 >= p.groups) break;
+        const int g = i * 32 + lane;
+        odd[i] = __ballot_sync(0xffffffffu, g < p.groups && ((first[(g + 1) * p.grp_slabs] - first[g * p.grp_slabs]) >> 1 & 1));
+    }
+    __syncwarp();
+    for (int s = lane; s < slabs; s += 32) {
+        // entry s + 1 lies behind s / grp_slabs whole groups, and behind its own where it ends it
+        const int g = s / p.grp_slabs, ends = (s + 1) % p.grp_slabs == 0;
+        int moved = 0, own = 0;
+#pragma unroll
+        for (int i = 0; i < kChunks; ++i) {
+            const int k = g - i * 32;
+            moved += __popc(odd[i] & (k >= 32 ? 0xffffffffu : k > 0 ? (1u << k) - 1 : 0u));
+            if ((g >> 5) == i) own = odd[i] >> (g & 31) & ends;
+        }
+        first[s + 1] += 2 * (moved + own) + own;
     }
 }
 
@@ -258,7 +295,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     uint64_t* tmem_empty = tmem_full + 2;       // [2] used in the even CTA: both CTAs' epilogue warps have read the accumulator
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty + 2);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-    int* first = reinterpret_cast<int*>(sE + kEpiWarps * kBox + 512);   // [slabs + 1] live tiles before a slab
+    int* first = reinterpret_cast<int*>(sE + kEpiWarps * kBox + 512);   // [slabs + 1] live halves before a slab
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
@@ -286,13 +323,13 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     grid_dep_wait();
     const uint32_t tmem_base = *tmem_slot;
 
-    if (p.slabs) {
-        if (warp == 3) pair_count_tiles(p, first, lane);
+    if (p.grp_slabs) {
+        if (warp == 3) pair_count_halves(p, first, lane);
         __syncthreads();
     }
-    PairTiles tiles;
-    int row_tile, tn, grp;
-    uint32_t halves;
+    PairTiles tiles(static_cast<int>(blockIdx.x >> 1), static_cast<int>(gridDim.x >> 1));
+    int row_half, tn, grp;       // row_half: first row of this CTA's half of a tile
+    bool mine;                   // that half is live
 
     if (warp == 0) {
         if (lane == 0) {
@@ -300,8 +337,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             int s = 0;
             uint32_t ph = 0;
             bool ok = true;
-            while (ok && tiles.next(p, first, row_tile, tn, grp, halves)) {
-                const int m0 = row_tile + static_cast<int>(rank) * 128;
+            while (ok && tiles.next(p, first, static_cast<int>(rank), row_half, tn, grp, mine)) {
                 // SwiGLU: the even CTA brings the gate rows of the weight, the odd one the up rows of the same features
                 const int n0 = p.epi == CAI_EPI_SWIGLU ? tn * HALF + static_cast<int>(rank) * (p.N >> 1) : tn * BN + static_cast<int>(rank) * HALF;
                 PairStages stages(p, grp);
@@ -314,7 +350,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                     }
                     if (rank == 0) mbar_expect_tx(&full[s], 2 * kBlock<BN> * __popc(live));
                     const uint32_t bar = map_to_cta(smem_u32(&full[s]), 0);
-                    pair_load_stage<BN>(&tmA, &tmB, sA + s * kPerStage * kABytes, sB + s * kPerStage * kBBytes<BN>, bar, p, ks, live, m0, n0, grp);
+                    pair_load_stage<BN>(&tmA, &tmB, sA + s * kPerStage * kABytes, sB + s * kPerStage * kBBytes<BN>, bar, p, ks, live, row_half, n0, grp);
                     if (++s == STAGES) {
                         s = 0;
                         ph ^= 1;
@@ -345,7 +381,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             uint32_t ph = 0;
             bool ok = true;
             int t = 0;
-            while (ok && tiles.next(p, first, row_tile, tn, grp, halves)) {
+            while (ok && tiles.next(p, first, static_cast<int>(rank), row_half, tn, grp, mine)) {
                 const int acc = t & 1;
                 const uint32_t acc_ph = (t >> 1) & 1;
                 ++t;
@@ -389,9 +425,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         const uint32_t release[2] = {map_to_cta(smem_u32(&tmem_empty[0]), 0), map_to_cta(smem_u32(&tmem_empty[1]), 0)};
         int t = 0;
         bool ok = true;
-        while (ok && tiles.next(p, first, row_tile, tn, grp, halves)) {
-            const int half0 = row_tile + static_cast<int>(rank) * 128;
-            const bool mine = halves >> rank & 1;
+        while (ok && tiles.next(p, first, static_cast<int>(rank), row_half, tn, grp, mine)) {
             const int acc = t & 1;
             const uint32_t acc_ph = (t >> 1) & 1;
             ++t;
@@ -403,7 +437,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                 uint32_t any;
                 acc_valid = stages.next(p, ks, any);
             }
-            const int row0 = half0 + q * 32;
+            const int row0 = row_half + q * 32;
             const bool live = mine && row0 < p.M;
             const int col_first = tn * BN + half * HALF;
             const bool residual = p.epi == CAI_EPI_BF16_RESIDUAL;
@@ -858,6 +892,12 @@ static int pair_clusters(const PairForm& f, int sms, int sm_limit) {
     return n < 1 ? 1 : n;                                // a cluster is the least that can run
 }
 
+// Slabs of a group, where the live halves of all groups' slabs are counted ahead; 0 where they are too many.
+static int pair_counted_slabs(int M, int seg_rows, int groups) {
+    const long long slabs = (static_cast<long long>(M) + seg_rows - 1) / seg_rows;
+    return slabs * groups <= pair::kMaxSlabs ? static_cast<int>(slabs) : 0;
+}
+
 int gemm_pair(const void* A, const void* B, const GemmShape& g, cudaStream_t st) {
     PairParams p;
     p.M = g.M; p.N = g.N; p.K = g.K;
@@ -870,8 +910,7 @@ int gemm_pair(const void* A, const void* B, const GemmShape& g, cudaStream_t st)
     p.ldc = g.ldc; p.ldr = g.ldr; p.grp_c = g.grp_c;
     p.tile0 = 0;
     p.overlap = g.sm_limit <= 0;
-    const long long slabs = g.seg_mode == 1 ? static_cast<long long>((g.M + g.seg_rows - 1) / g.seg_rows) * g.groups : 0;
-    p.slabs = slabs <= pair::kMaxSlabs ? static_cast<int>(slabs) : 0;
+    p.grp_slabs = g.seg_mode == 1 ? pair_counted_slabs(g.M, g.seg_rows, g.groups) : 0;
     const int dev = current_device();
     p.status = status_words(dev);
     const PairForm f = pair_form(g.M, g.N, g.K, g.groups, g.epi, g.seg_mode != 0);
@@ -895,4 +934,38 @@ CAI_API int cai_gemm_bf16_form(int M, int N, int K, int groups, int epi, int seg
     const int at_once = pair_clusters(f, sms, sm_limit);
     *ctas = static_cast<int>(2 * f.slices * (tiles < at_once ? tiles : at_once));
     return CAI_K_OK;
+}
+
+CAI_API int cai_gemm_bf16_ragged_walk(int M, int N, int groups, const int* seg_counts, int seg_rows, int tile_cols, int pairs, int pair, int* tiles,
+                                      int capacity) {
+    if (M <= 0 || N <= 0 || groups <= 0 || !seg_counts || seg_rows <= 0 || seg_rows % 128 || tile_cols <= 0 || pair < 0 || pair >= pairs)
+        return CAI_K_BAD_ARG;
+    PairParams p = {};
+    p.M = M; p.N = N; p.groups = groups;
+    p.tiles_m = (M + pair::kBM - 1) / pair::kBM;
+    p.tiles_n = (N + tile_cols - 1) / tile_cols;
+    p.group_m = 8;
+    p.seg_counts = seg_counts; p.seg_rows = seg_rows; p.seg_mode = 1; p.grp_seg = (M + seg_rows - 1) / seg_rows;
+    p.grp_slabs = pair_counted_slabs(M, seg_rows, groups);
+    int first[pair::kMaxSlabs + 1] = {};
+    for (int s = 0, halves = 0, grp0 = 0; s < p.grp_slabs * groups; ++s) {
+        halves += pair_live_halves(p, s);
+        const bool odd = (s + 1) % p.grp_slabs == 0 && ((halves - grp0) & 1);
+        halves += odd;
+        first[s + 1] = 2 * halves + odd;
+        if ((s + 1) % p.grp_slabs == 0) grp0 = halves;
+    }
+    PairTiles walk[2] = {PairTiles(pair, pairs), PairTiles(pair, pairs)};
+    int n = 0;
+    for (;; ++n) {
+        int row[2], tn[2], grp[2];
+        bool live[2], more[2];
+        for (int r = 0; r < 2; ++r) more[r] = walk[r].next(p, first, r, row[r], tn[r], grp[r], live[r]);
+        if (more[0] != more[1] || (more[0] && (tn[0] != tn[1] || grp[0] != grp[1]))) return CAI_K_BAD_ARG;   // the CTAs of a pair would part
+        if (!more[0]) return n;
+        if (n < capacity) {
+            int* t = tiles + 6 * n;
+            t[0] = grp[0]; t[1] = tn[0]; t[2] = row[0]; t[3] = row[1]; t[4] = live[0]; t[5] = live[1];
+        }
+    }
 }

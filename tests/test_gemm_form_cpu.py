@@ -1,5 +1,6 @@
 """The form a bf16 product runs in follows from its shape alone: asked here, where there is no GPU to look at."""
 import ctypes
+import random
 
 import pytest
 
@@ -50,3 +51,44 @@ def test_limit_caps_the_ctas(shape, cluster, free):
         assert f[:2] == ask(*shape)[:2] == ask(*shape, sms=132)[:2]        # the sums do not depend on the limit or the GPU
         most = max(cluster, min(limit, 148) // cluster * cluster)         # whole clusters; one at least
         assert f[2] == min(free, most), (limit, f)
+
+
+def walk(M, N, groups, counts, seg_rows, tile_cols, pairs):
+    """Every pair's tiles: (group, column tile, row of each half, whether it is live)."""
+    c = (ctypes.c_int * len(counts))(*counts)
+    out, per_pair = [], []
+    for pair in range(pairs):
+        ask_walk = lambda buf, n: _lib.lib().cai_gemm_bf16_ragged_walk(M, N, groups, c, seg_rows, tile_cols, pairs, pair, buf, n)
+        n = ask_walk(None, 0)
+        assert n >= 0
+        buf = (ctypes.c_int * max(1, 6 * n))()
+        assert ask_walk(buf, n) == n
+        out += [tuple(buf[6 * i:6 * i + 6]) for i in range(n)]
+        per_pair.append(n)
+    return out, per_pair
+
+
+# (groups, slabs per group, rows of a slab, rows of the group if less): live halves counted ahead, up to 256 slabs, and the walk over all
+# tiles beyond. Slabs of odd numbers of halves, one slab and several, more row tiles than a raster group, a last slab cut short.
+@pytest.mark.parametrize("groups,per,seg_rows,short", [(1, 1, 128, 0), (8, 8, 128, 0), (5, 3, 384, 0), (4, 4, 256, 100), (2, 2, 2432, 0), (1, 256, 128, 0),
+                                                       (64, 1, 2048, 0), (256, 1, 128, 60), (300, 1, 128, 0), (2, 130, 384, 0)])
+@pytest.mark.parametrize("kind", ["full", "none", "one", "random", "edges"])
+def test_ragged_walk_covers_live_halves_once(groups, per, seg_rows, short, kind):
+    rng = random.Random(groups * 31 + per)
+    n = groups * per
+    edges = [0, 1, 127, 128, 129, 255, 256, 257, seg_rows - 1, seg_rows, seg_rows + 5, -1]
+    counts = {"full": [seg_rows] * n, "none": [0] * n, "one": [seg_rows if i == n // 2 else 0 for i in range(n)],
+              "random": [rng.randint(0, seg_rows) for _ in range(n)], "edges": [edges[i % len(edges)] for i in range(n)]}[kind]
+    M, N, tile_cols, pairs = per * seg_rows - short, 640, 256, 74
+    tiles, per_pair = walk(M, N, groups, counts, seg_rows, tile_cols, pairs)
+    want = set()
+    for i, c in enumerate(counts):
+        first = i % per * seg_rows
+        want |= {(i // per, tn, first + r) for r in range(0, min(c, seg_rows, M - first), 128) for tn in range(3)}
+    got = [(g, tn, row) for g, tn, r0, r1, l0, l1 in tiles for row, live in ((r0, l0), (r1, l1)) if live]
+    assert len(got) == len(set(got)) and set(got) == want
+    assert all(0 <= r < M and r % 128 == 0 for t in tiles for r in t[2:4] if n <= 256)       # a half that is not live is loaded all the same
+    if n <= 256:
+        halves = [len({h for h in want if h[0] == g and h[1] == 0}) for g in range(groups)]
+        assert len(tiles) == 3 * sum((h + 1) // 2 for h in halves)            # no half-empty tile but the last of a group
+        assert max(per_pair) - min(per_pair) <= 1

@@ -198,10 +198,11 @@ def _ragged_counts(kind, slabs, seg_rows, g):
     return torch.randint(0, seg_rows + 1, (slabs,), generator=g, dtype=torch.int32)
 
 
-# Live tiles counted ahead (up to 256 slabs) and the walk over all tiles (beyond): one slab and several per group, slabs of an odd number
-# of 128-row halves (a 256-row tile must not reach into the next slab), more row tiles than a raster group of eight.
+# Live halves counted ahead (up to 256 slabs) and the walk over all tiles (beyond): one slab and several per group, few groups and more than a
+# warp has lanes, slabs of an odd number of 128-row halves (a tile takes halves of two slabs), more row tiles than a raster group of eight.
 @pytest.mark.parametrize("groups,per_group,seg_rows,N,K", [(16, 1, 128, 256, 128), (5, 3, 384, 264, 192), (4, 4, 256, 512, 64),
-                                                           (2, 2, 2432, 384, 256), (300, 1, 128, 128, 64), (100, 3, 128, 72, 64), (256, 1, 128, 136, 64)])
+                                                           (2, 2, 2432, 384, 256), (300, 1, 128, 128, 64), (100, 3, 128, 72, 64), (256, 1, 128, 136, 64),
+                                                           (40, 3, 384, 136, 64), (85, 3, 128, 72, 64), (1, 256, 128, 72, 64)])
 @pytest.mark.parametrize("kind", ["edges", "random", "one", "none"])
 def test_grouped_ragged_rows(groups, per_group, seg_rows, N, K, kind):
     from cai_b200 import ops
@@ -248,3 +249,30 @@ def test_grouped_ragged_depth(groups, per_group, seg_rows, M, N, kind, accumulat
     ref = torch.einsum("gkm,gkn->gmn", A, B).reshape(-1, N) + (3.0 if accumulate else 0.0)
     bound = (K + 1) * 2.0 ** -24 * (torch.einsum("gkm,gkn->gmn", A.abs(), B.abs()).reshape(-1, N) + 3.0)
     assert ((out.cpu().double() - ref).abs() <= bound).all()
+
+
+# Full slabs of an odd number of 128-row halves cost what the same rows without slabs cost: two neighbouring halves share a tile, of
+# whatever slabs they are. (With tiles that end at their slab these take 1.7 and 1.4 times as long.)
+@pytest.mark.parametrize("groups,per,seg_rows", [(1, 8, 128), (8, 8, 384)])
+def test_full_slabs_cost_what_plain_rows_cost(groups, per, seg_rows):
+    from cai_b200 import ops
+    M, N, K = per * seg_rows, 3072, 4096
+    a = torch.randn(groups * M, K, device="cuda").bfloat16()
+    b = torch.randn(groups * N, K, device="cuda").bfloat16()
+    out = torch.empty(groups * M, N, device="cuda", dtype=torch.bfloat16)
+    counts = torch.full((groups * per,), seg_rows, device="cuda", dtype=torch.int32)
+
+    def us(**ragged):
+        times = []
+        for _ in range(9):
+            s, e = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            torch.cuda._sleep(100000)
+            s.record()
+            ops.gemm_grouped(a, b, out, M, N, K, groups=groups, **ragged)
+            e.record()
+            torch.cuda.synchronize()
+            times.append(s.elapsed_time(e) * 1e3)
+        return sorted(times)[4]
+
+    # both run with 256-row tiles along the whole of K; the plain one in the form that its shape asks for
+    assert us(seg_counts=counts, seg_rows=seg_rows, seg_mode=1) < 1.25 * us()
