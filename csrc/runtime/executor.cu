@@ -861,18 +861,32 @@ CAI_API int cai_exec_step(cai_exec* ex, int step, float lr) {
 }
 
 // End of a step: `bytes` of device memory (the loss) and the device's status word come to the host behind everything enqueued on
-// compute_hi, in one synchronisation. Returns 0 or an error; *status is the word, which is cleared when it is not 0. (A copy, a
-// synchronisation and a second copy on the default stream for the status took 52 us with the GPU idle.)
+// compute_hi, in one synchronisation. Returns 0 or an error; *status is the word, which is cleared when it is not 0, on compute_hi too,
+// so that a later step's word is not cleared with it. (A copy, a synchronisation and a second copy on the default stream for the
+// status took 52 us with the GPU idle.)
 CAI_API int cai_exec_read(cai_exec* ex, const void* dev, void* pinned, size_t bytes, int* status) {
+    if (!dev || !pinned || !status) {
+        set_last_error("exec_read: null pointer");
+        return CAI_K_BAD_ARG;
+    }
     cudaStream_t hi = ex->streams[ST_COMPUTE_HI];
     int* words = status_words(ex->device);
-    if (!words) return CAI_K_CUDA;
-    int* seen = reinterpret_cast<int*>(ex->hyper_host + cai_exec::kHyperSlots * 8);
-    if (cudaMemcpyAsync(pinned, dev, bytes, cudaMemcpyDeviceToHost, hi) != cudaSuccess ||
-        cudaMemcpyAsync(seen, words, sizeof(int), cudaMemcpyDeviceToHost, hi) != cudaSuccess || cudaStreamSynchronize(hi) != cudaSuccess)
+    if (!words) {
+        set_last_error("exec_read: no status words on device %d", ex->device);
         return CAI_K_CUDA;
-    *status = *seen;
-    if (*seen) cudaMemset(words, 0, sizeof(int));
+    }
+    int* seen = reinterpret_cast<int*>(ex->hyper_host + cai_exec::kHyperSlots * 8);
+    cudaError_t e = cudaMemcpyAsync(pinned, dev, bytes, cudaMemcpyDeviceToHost, hi);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(seen, words, sizeof(int), cudaMemcpyDeviceToHost, hi);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(hi);
+    if (e == cudaSuccess && (*status = *seen) != 0) {
+        e = cudaMemsetAsync(words, 0, sizeof(int), hi);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(hi);
+    }
+    if (e != cudaSuccess) {
+        set_last_error("exec_read: %s", cudaGetErrorString(e));
+        return CAI_K_CUDA;
+    }
     return 0;
 }
 

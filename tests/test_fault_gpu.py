@@ -16,25 +16,36 @@ CAI_DEV_TIMEOUT_PEER_FLAG = 105
 CAI_DEV_ABORTED_BY_HOST = 108
 
 
-def _launch_with_silent_member(torch, klib, T=256, N=256, K=128):
-    """Enqueue gemm_rs as rank 0 of 2; returns the tensors that must stay alive until the kernel is done."""
-    L = klib.lib()
-    P, I, LL, ULL = c_void_p, c_int, c_longlong, c_ulonglong
-    L.cai_fused_gemm_rs_c.argtypes = [P, I, I, ULL, I, P, P, ULL, P, P, I, I, I, LL, LL, LL, LL, I, P, c_uint32, P]
-    sig = int(L.cai_signal_block_bytes())
+def _silent_member_inputs(torch, klib, T=256, N=256, K=128):
+    sig = int(klib.lib().cai_signal_block_bytes())
     stage_off = (sig + 1023) & ~1023
     nbytes = stage_off + T * N * 2 + 4096
     members = [torch.zeros(nbytes, dtype=torch.uint8, device="cuda") for _ in range(2)]
-    bases = (c_void_p * 2)(*[c_void_p(m.data_ptr()) for m in members])
     A = torch.randn(T, K, device="cuda").to(torch.bfloat16)
     B = torch.randn(N, K, device="cuda").to(torch.bfloat16)
     out = torch.zeros(T // 2, N, device="cuda", dtype=torch.bfloat16)
     epoch = torch.zeros(1, dtype=torch.int32, device="cuda")
-    torch.cuda.synchronize()
+    return T, N, K, stage_off, members, A, B, out, epoch
+
+
+def _launch(torch, klib, inputs):
+    """Enqueue gemm_rs as rank 0 of 2 on the current stream."""
+    T, N, K, stage_off, members, A, B, out, epoch = inputs
+    L = klib.lib()
+    P, I, LL, ULL = c_void_p, c_int, c_longlong, c_ulonglong
+    L.cai_fused_gemm_rs_c.argtypes = [P, I, I, ULL, I, P, P, ULL, P, P, I, I, I, LL, LL, LL, LL, I, P, c_uint32, P]
+    bases = (c_void_p * 2)(*[c_void_p(m.data_ptr()) for m in members])
     st = torch.cuda.current_stream().cuda_stream
     klib.check(L.cai_fused_gemm_rs_c(bases, 0, 2, 0, 0, A.data_ptr(), B.data_ptr(), stage_off, out.data_ptr(), None, T, N, K,
                                      K, K, N, 0, 0, epoch.data_ptr(), 1, st), "gemm_rs")
-    return members, A, B, out, epoch
+    return bases
+
+
+def _launch_with_silent_member(torch, klib):
+    """Enqueue gemm_rs as rank 0 of 2; returns what must stay alive until the kernel is done."""
+    inputs = _silent_member_inputs(torch, klib)
+    torch.cuda.synchronize()
+    return inputs, _launch(torch, klib, inputs)
 
 
 def _ordinary_kernel_still_works(torch):
@@ -84,3 +95,54 @@ def test_host_abort_cuts_a_pending_wait_short():
     del keep
     _ordinary_kernel_still_works(torch)
     assert klib.device_status(clear=True) == 0
+
+
+def test_reading_a_step_clears_its_status_and_no_later_one():
+    """The status word is cleared on the executor's own stream: with the default stream busy, the word of a kernel enqueued after a caught
+    failure is still there when it is read."""
+    import torch
+    from pathlib import Path
+    from cai_b200.ops import _lib as klib
+    from cai_b200.runtime.engine import DeviceStatusError, Engine, synthetic_batch
+    eng = Engine(Path(__file__).resolve().parent.parent / "configs" / "tiny.cfg", rank=0, world=1, local_rank=0)
+    m = eng.model
+    batch = synthetic_batch(m.vocab_size, m.seq_len, eng.hdr.num_microbatches * m.microbatch, step=0, seed=0)
+    eng.step(*batch)
+    klib.set_wait_limit_us(20_000)
+    try:
+        with torch.cuda.stream(eng.stream):
+            inputs = _silent_member_inputs(torch, klib)
+            for busy in (False, True):
+                torch.cuda.synchronize()
+                if busy:
+                    with torch.cuda.stream(torch.cuda.default_stream()):
+                        torch.cuda._sleep(400_000_000)          # 0.2 s
+                _launch(torch, klib, inputs)
+                with pytest.raises(DeviceStatusError):
+                    eng.read_loss()
+            _launch(torch, klib, inputs)
+        torch.cuda.synchronize()
+        with pytest.raises(DeviceStatusError):
+            eng.read_loss()
+    finally:
+        klib.set_wait_limit_us(0)
+    assert klib.device_status(clear=True) == 0
+    eng.step(*batch)
+    eng.close()
+
+
+def test_a_failed_read_says_what_failed():
+    import torch
+    from pathlib import Path
+    from ctypes import byref
+    from cai_b200 import ops
+    from cai_b200.ops import _lib as klib
+    from cai_b200.runtime.engine import Engine
+    eng = Engine(Path(__file__).resolve().parent.parent / "configs" / "tiny.cfg", rank=0, world=1, local_rank=0)
+    with pytest.raises(klib.KernelError, match="swiglu"):
+        ops.swiglu_fwd(torch.zeros(4, 20, device="cuda", dtype=torch.bfloat16))     # leaves its own text behind
+    status = c_int(0)
+    with pytest.raises(klib.KernelError, match="exec_read"):
+        rc = eng.L.cai_exec_read(eng.ex, None, eng.loss_host.data_ptr(), 32, byref(status))
+        klib.check(rc, "reading")
+    eng.close()
