@@ -12,13 +12,16 @@ from ._lib import KernelError, check, device_status, lib
 EPI_BF16, EPI_F32, EPI_F32_ACCUM, EPI_BF16_RESIDUAL, EPI_SWIGLU, EPI_SWIGLU_BWD = 0, 1, 2, 3, 4, 5
 
 
-# Handle of the current stream of the current device, as torch.cuda.current_stream().cuda_stream gives it, without building a stream
-# object on the way: 0.2 instead of 3.3 us of the some 15 us an op's host path took.
-_current_device = torch._C._cuda_getDevice
-_raw_stream = torch._C._cuda_getCurrentRawStream
+_current_device = _raw_stream = None
 
 
 def _stream():
+    """Handle of the current stream of the current device, as ``torch.cuda.current_stream().cuda_stream`` gives it, without building a stream
+    object on the way: 0.2 instead of 3.3 us of the some 15 us an op's host path took. Looked up on first use: a torch without CUDA
+    does not have the two functions, and this module can be imported there all the same."""
+    global _current_device, _raw_stream
+    if _raw_stream is None:
+        _current_device, _raw_stream = torch._C._cuda_getDevice, torch._C._cuda_getCurrentRawStream
     return _raw_stream(_current_device())
 
 

@@ -19,6 +19,16 @@ def test_import_is_light_and_public_names_resolve():
     assert r.stdout.strip()
 
 
+def test_ops_import_with_a_torch_that_has_no_cuda():
+    """The two stream functions of a CUDA build are looked up when an op is called."""
+    code = ("import torch\n"
+            "for n in ('_cuda_getDevice', '_cuda_getCurrentRawStream'):\n"
+            "    if hasattr(torch._C, n): delattr(torch._C, n)\n"
+            "import cai_b200.ops\n")
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, cwd=ROOT, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+
+
 def test_unknown_attribute_is_an_attribute_error():
     import cai_b200
     with pytest.raises(AttributeError):
