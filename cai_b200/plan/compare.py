@@ -3,7 +3,9 @@
 Typical use: the measured timeline of a step (``python -m cai_b200.trainer ... --trace measured.csv``) against the one
 the calibrated backend predicts for the same plan (``bin/trainer plan topo --backend calibrated --trace predicted.csv``).
 Ops are matched by their index in the plan; the table lists, per op kind and stream, the summed durations of both files
-and their ratio, largest absolute difference first: the kernels that are off their model are where to look next.
+and their ratio, largest absolute difference first: the kernels that are off their model are where to look next. (The events
+of a traced step keep an op from starting while its predecessor finishes: a measured op is some 5 us longer than in the step that
+the backend predicts, and the measured durations of short ops add up to more than an untraced step takes.)
 
     python -m cai_b200.plan.compare measured.csv predicted.csv
 """

@@ -422,7 +422,10 @@ class Engine:
         self.L.cai_exec_nvtx_enable(self.ex, int(on))
 
     def trace_step(self, tokens, targets):
-        """Run one step with per-op CUDA events; returns a list of TraceRec with measured times."""
+        """Run one step with per-op CUDA events; returns a list of TraceRec with measured times.
+
+        The events keep kernels from starting while their predecessor in the stream finishes, so that an op takes some 5 us more than
+        untraced and a step of many short ops longer as a whole (60 launches: 593 us by their events, 331 us without)."""
         self.L.cai_exec_use_graph(self.ex, 0)
         self.L.cai_exec_trace_enable(self.ex, 1)
         self.step(tokens, targets)

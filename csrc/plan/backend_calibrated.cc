@@ -17,6 +17,9 @@
 //   fused TP ops    launch + max(GEMM on the SMs left beside the copy CTAs, wire bytes / measured rate under all-to-all
 //                   load for the group size) (+ the own-row tail of the reduce-scatter)
 //   NCCL, p2p       latency + bytes / rate
+// Fixed costs are those of an untraced step, where plain kernels are launched while their predecessor finishes. The per-op events of a
+// traced step keep an op from starting early: each takes some 5 us more there (52 ops of a tiny step 593 us by their events, 331 us
+// without; 137 of a small one 4182 and 3531).
 // Needs a version-2 plan (kernel records and shapes); version-1 plans fall back to the analytic cost.
 #include <algorithm>
 #include <cmath>
@@ -39,19 +42,21 @@ struct Calibration {
     int sms = 148;
     // Plain GEMM, fitted to the per-op CUDA-event times inside steps of six models on one GPU (the headline config in launches of
     // 16384 and of 4096 tokens, two of its layers' tensor-parallel shards as models of their own, two 8B-class layers, a
-    // small ragged model; 90 shapes, median error 4 %): [0] A not transposed, [1] A transposed (weight-gradient form)
-    double gemm_launch_us = 10.3;
+    // small ragged model; 90 shapes, median error 4 %), less what an op starts early: [0] A not transposed, [1] A transposed
+    // (weight-gradient form). Their steps (those of the headline config with 8 layers), predicted / measured on one B200, ms: 60.7 / 63.0,
+    // 66.9 / 66.8, 32.6 / 33.1, 11.9 / 11.2, 50.4 / 51.0, 4.60 / 4.62
+    double gemm_launch_us = 5.6;
     double gemm_tile_us[2] = {1.9, 0.2};
     double gemm_sm_flops[2] = {10.7e12, 9.4e12};
     int gemm_pairs = 1;             // 0: plain products run one CTA per 128-row tile, as the fused ones do
     // One-CTA GEMM (fused with a collective): the headline config's shapes on one GPU, fit error <= 13 %
     double fused_gemm_tile_us = 0.5;
     double fused_gemm_sm_flops = 7.9e12;
-    // fp8 block-scaled GEMM against the one-CTA bf16 one: 1708 against 1361 TFLOP/s at 8192^3
+    // fp8 block-scaled GEMM against the one-CTA bf16 one: 14 shapes inside steps of two models, 0.9 (short K) to 1.7 (K = 16384)
     double fp8_speedup = 1.25;
     // attention, microseconds per 128 x 128 step of one CTA (the same six models)
-    double attn_fwd_step_us = 1.69, attn_fwd_fixed_us = 17.0;
-    double attn_dkdv_step_us = 2.53, attn_dq_step_us = 2.00, attn_bwd_fixed_us = 16.5;
+    double attn_fwd_step_us = 1.59, attn_fwd_fixed_us = 8.8;
+    double attn_dkdv_step_us = 2.53, attn_dq_step_us = 2.00, attn_bwd_fixed_us = 11.8;
     // fused tensor-parallel kernels: bytes a GPU moves per second while every member pulls and pushes at once
     // (steady-state chains on 2 / 4 / 8 GPUs), copy CTAs of the all-gather form, tail of the reduce-scatter form
     double link_rate[4] = {0.60e12, 0.60e12, 0.45e12, 0.35e12};  // group size 1-2, 2, 4, 8
@@ -64,9 +69,9 @@ struct Calibration {
     double nccl_rate = 0.60e12;   // bytes per GPU and second of ring collectives of 17-120 MB (NCCL arms of the chains)
     // pointwise kernels (the same six models; worst errors 6-14 %, the embedding's backward apart, whose time goes with how
     // often a token repeats)
-    PointCost point_default = {8.0, 0.20};
-    PointCost rmsnorm_fwd = {6.4, 0.181}, rmsnorm_bwd = {14.7, 0.305}, rope = {5.8, 0.332}, swiglu = {5.3, 0.170},
-              adamw = {4.0, 0.2456}, cross_entropy = {14.2, 0.470}, embed = {15.0, 0.60};
+    PointCost point_default = {3.3, 0.20};
+    PointCost rmsnorm_fwd = {1.7, 0.181}, rmsnorm_bwd = {10.0, 0.305}, rope = {1.1, 0.332}, swiglu = {0.6, 0.170},
+              adamw = {0.0, 0.2456}, cross_entropy = {9.5, 0.470}, embed = {10.3, 0.60};
 };
 
 bool set_key(Calibration* c, const std::string& k, double v) {

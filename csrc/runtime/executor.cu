@@ -575,6 +575,7 @@ int replay(cai_exec* ex) {
             continue;
         }
         if (!op.exec) continue;
+        // events on either side of a launch: no kernel starts while its predecessor finishes, some 5 us an op
         TraceRec* tr = nullptr;
         if (ex->trace_on && !ex->use_graph) {
             TraceRec r;

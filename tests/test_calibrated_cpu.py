@@ -57,6 +57,25 @@ def test_built_in_constants_describe_the_kernels_as_they_are(tmp_path, n):
     assert abs(predicted - MEASURED_NOW_MS[n]) <= 0.10 * MEASURED_NOW_MS[n], predicted
 
 
+# Small models, whose steps are chains of short kernels that start while their predecessor finishes: ms per step measured on one B200
+SMALL_MS = {"hidden_size = 1000\nffn_hidden = 2728\nnum_layers = 6\nnum_heads = 9\nnum_kv_heads = 3\nvocab_size = 5000\nseq_len = 640\n"
+            "microbatch = 3\ngrad_accum = 2\nrecompute = 1\ntie_embeddings = 1\n": 4.62,
+            "hidden_size = 1024\nffn_hidden = 2816\nnum_layers = 6\nnum_heads = 8\nnum_kv_heads = 4\nvocab_size = 8192\nseq_len = 1024\n"
+            "microbatch = 2\ngrad_accum = 2\nrecompute = 0\ntie_embeddings = 0\n": 3.53}
+
+
+@pytest.mark.parametrize("model", SMALL_MS)
+def test_small_steps_are_within_ten_percent(tmp_path, model):
+    from cai_b200 import plan
+    text = model + ("is_moe = 0\nparam_dtype = bf16\nhead_dim = 128\ntp = 1\npp = 1\nep = 1\noptim_dtype = fp32\n"
+                    "gpus_per_rack = 1\ntrays_per_rack = 1\ngpus_per_tray = 1\nnum_racks = 1\n")
+    plan.compile_plans(text, tmp_path, ranks=(0, 1), version=2, text=True)
+    sim = plan.Simulator(tmp_path / "plan.rank000000.bin", tmp_path / "topology.bin", backend="calibrated")
+    predicted = sim.step().step_time_s * 1e3
+    sim.close()
+    assert abs(predicted - SMALL_MS[model]) <= 0.10 * SMALL_MS[model], predicted
+
+
 def test_moe_step_with_grouped_expert_gemms_is_within_ten_percent(tmp_path):
     """Config 4 (64 experts, top-8, ep = 8): 321.8 ms per step measured. The grouped expert GEMMs are priced over the live
     rows of all local experts' slabs, dispatch and combine by the bytes they move."""
