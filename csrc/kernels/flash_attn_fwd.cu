@@ -692,7 +692,9 @@ CAI_API int cai_flash_attn_fwd_variant(const void* qkv, void* out, float* lse, i
     // CTA beyond, where both take the same time and the latter reads K and V half as often. All give the same bits. us, one tile / two tiles /
     // two CTAs: 8 x 384 tokens, 12 / 4 heads 17.7 / 19.7 / 14.7; 6 x 640, 9 / 3 heads 19.6 / 19.0 / 18.6; 4 x 1024, 16 / 8 heads 40.8 / 32.4 /
     // 28.7; 2048, 32 / 32 heads 62.7 / 47.7 / 43.6; 4 x 4096, 16 / 8 heads 384 / 283 / 278; 8192, 32 / 8 heads 717 / 490-504 / 499; and, with
-    // fewer CTAs than SMs, 2 x 1024, 16 / 8 heads 21.3 / 25.0 / 22.7, 2048, 16 / 8 heads 31.9 / 42.0 / 39.0.
+    // fewer CTAs than SMs, 2 x 1024, 16 / 8 heads 21.3 / 25.0 / 22.7, 2048, 16 / 8 heads 31.9 / 42.0 / 39.0. (Short rows in grids of that size take less
+    // in another form, which the rule does not use: one behind the other, 6 x 384, 12 / 4 heads 16.4 / 11.6 / 14.1, 8 x 256, 16 / 8 14.2 / 10.0 / 11.7,
+    // 16 x 128, 16 / 8 12.8 / 12.4 / 9.5; 2 x 640, 16 / 8 13.4 / 15.3 / 14.1.)
     const long long pair_ctas = static_cast<long long>((S + 2 * kAttnTile - 1) / (2 * kAttnTile)) * nh * B;
     const int variant = force_variant ? force_variant : pair_ctas < sm_count(dev) ? 1 : S <= 4096 ? 3 : 2;
     if (variant == 3) {

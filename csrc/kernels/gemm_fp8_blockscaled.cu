@@ -801,8 +801,9 @@ CAI_API int cai_quant_rows_1x128(const void* x, long long ldx, void* q, long lon
     if (warps == 0) return CAI_K_OK;
     if (warps < (1ll << 31) && !(ldx & 7) && !(ldq & 7) && aligned_to(x, 16) && aligned_to(q, 8)) {
         constexpr unsigned per_cta = 16u * kQuantUnroll;
-        // Launched the ordinary way: started early behind a GEMM on CTA pairs, with the product above started early behind it in turn, that
-        // product took half as long again (8192 x 4096 x 28672 1161 -> 1859 us); with either of the two launched like this it does not.
+        // Launched the ordinary way: early, behind a GEMM on CTA pairs and in front of the product above, it gains nothing (the three, four times
+        // over, in ms, ordinary / early: 8192 x 4096 x 28672 9.6-10.0 / 9.9-10.3, 8192 x 28672 x 4096 5.3-5.6 / 5.6, 2048 x 4096 x 14336 1.36 /
+        // 1.36). While that product ran on one CTA a tile throughout, it took half as long again behind an early quantiser.
         quant_rows_vec_kernel<<<static_cast<unsigned>((warps + per_cta - 1) / per_cta), 256, 0, static_cast<cudaStream_t>(stream)>>>(
             static_cast<const __nv_bfloat16*>(x), ldx, static_cast<__nv_fp8_storage_t*>(q), ldq, scale, static_cast<unsigned>(warps),
             static_cast<unsigned>(cols / 128));
