@@ -113,3 +113,25 @@ def test_forward_forms_give_the_same_bits(B, S, nh, nkv):
     for variant in (0, 1, 3):
         o, l = ops.flash_attn_fwd(qkv, B, S, nh, nkv, 128, variant=variant)
         assert torch.equal(o, out) and torch.equal(l, lse)
+
+
+# dK / dV and dQ in one launch against each by itself: the same CTAs, so the same bits. Grids of one CTA each, smaller and larger than the GPU, split
+# heads (the first three with several query heads per kv head) and not.
+@pytest.mark.parametrize("B,S,nh,nkv", [(1, 128, 1, 1), (1, 128, 4, 1), (2, 384, 6, 2), (1, 512, 8, 1), (8, 384, 12, 4), (3, 640, 9, 3), (1, 2048, 16, 8)])
+def test_flash_attn_bwd_parts_together(B, S, nh, nkv):
+    from cai_b200 import ops
+    torch.manual_seed(2)
+    qkv = torch.randn(B * S, (nh + 2 * nkv) * 128, device="cuda").to(torch.bfloat16)
+    dout = torch.randn(B * S, nh * 128, device="cuda").to(torch.bfloat16)
+    out, lse = ops.flash_attn_fwd(qkv, B, S, nh, nkv, 128)
+    delta = torch.empty((B, nh, S), device="cuda")
+    whole = ops.flash_attn_bwd(qkv, out, dout, lse, B, S, nh, nkv, 128, delta=delta)
+    parts, kv_only, q_only = (torch.full_like(qkv, 7.0) for _ in range(3))
+    for p in (1, 4, 2):
+        ops.flash_attn_bwd(qkv, out, dout, lse, B, S, nh, nkv, 128, dqkv=parts, delta=torch.empty_like(delta) if p == 1 else delta, parts=p)
+    ops.flash_attn_bwd(qkv, out, dout, lse, B, S, nh, nkv, 128, dqkv=kv_only, delta=delta, parts=2)
+    ops.flash_attn_bwd(qkv, out, dout, lse, B, S, nh, nkv, 128, dqkv=q_only, delta=delta, parts=4)
+    assert torch.equal(whole, parts)
+    q = nh * 128
+    assert torch.equal(whole[:, :q], q_only[:, :q]) and bool((q_only[:, q:] == 7.0).all())
+    assert torch.equal(whole[:, q:], kv_only[:, q:]) and bool((kv_only[:, :q] == 7.0).all())
