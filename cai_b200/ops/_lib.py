@@ -14,6 +14,12 @@ _LIB_PATH = Path(__file__).resolve().parent.parent / "lib" / "libcai_kernels.so"
 _lib = None
 
 
+class GemmCall(ctypes.Structure):
+    """One product of a call of ``cai_gemm_bf16_two`` (``cai_gemm_call``)."""
+    _fields_ = [(n, c_void_p) for n in ("A", "B", "C", "R")] + [(n, c_longlong) for n in ("lda", "ldb", "ldc", "ldr")] + [
+        (n, c_int) for n in ("M", "N", "K", "a_mn_major", "b_mn_major", "epi")] + [("alpha", c_float)]
+
+
 class KernelError(RuntimeError):
     pass
 
@@ -35,6 +41,7 @@ def _declare(L):
     L.cai_status_read.argtypes = [I]
     L.cai_sm_count.argtypes = []
     L.cai_gemm_bf16.argtypes = [P, P, P, P, I, I, I, LL, LL, LL, LL, I, I, I, F, I, P]
+    L.cai_gemm_bf16_two.argtypes = [P, P, P]
     L.cai_gemm_bf16_seg.argtypes = [P, P, P, P, I, I, I, LL, LL, LL, LL, I, I, I, F, P, I, I, I, P]
     if hasattr(L, "cai_gemm_fp8_blockscaled"):
         L.cai_gemm_fp8_blockscaled.argtypes = [P, P, P, P, P, P, I, I, I, LL, LL, LL, LL, I, P]

@@ -51,6 +51,24 @@ CAI_API int cai_gemm_bf16(const void* A, const void* B, void* C, const void* R, 
                           long long lda, long long ldb, long long ldc, long long ldr, int a_mn_major,
                           int b_mn_major, int epi, float alpha, int sm_limit, void* stream);
 
+/* Two products, neither of which reads or writes what the other writes: the two gradients of a linear layer, say. They go out as one launch
+ * where both can and where that is estimated to be faster, so that the tiles of one fill the waves of the other, and as two otherwise. The
+ * results are those of two calls of cai_gemm_bf16. */
+typedef struct {
+    const void *A, *B;
+    void* C;
+    const void* R;
+    long long lda, ldb, ldc, ldr;
+    int M, N, K, a_mn_major, b_mn_major, epi;
+    float alpha;
+} cai_gemm_call;
+CAI_API int cai_gemm_bf16_two(const cai_gemm_call* first, const cai_gemm_call* second, void* stream);
+/* How many launches that takes (1 or 2); tile_cols: columns of the tiles of the one launch. Needs no GPU. */
+CAI_API int cai_gemm_bf16_two_launches(const cai_gemm_call* first, const cai_gemm_call* second, int* tile_cols);
+/* The tiles that pair `pair` of `pairs` CTA pairs takes of one launch of n0 tiles of k0 k-elements and n1 of k1 <= k0, in order: two ints a tile
+ * (product, tile). Returns their number, of which `capacity` are written. Needs no GPU. */
+CAI_API int cai_gemm_bf16_two_walk(int n0, int k0, int n1, int k1, int tile_cols, int pairs, int pair, int* tiles, int capacity);
+
 /* The form such a product runs in: columns of its 256-row tiles, and how many slices of K are summed (1: one sum along K). It follows
  * from the arguments alone, so the order of summation is the same on every GPU. ctas: the most CTAs of one launch on `sms` SMs under sm_limit.
  * Needs no GPU. Not for CAI_EPI_SWIGLU_BWD. */

@@ -60,6 +60,18 @@ struct PairParams {
     int* status;
 };
 
+// One product of a launch: maps of A, B, C and (SwiGLU) the activation, and what else the kernel has to know.
+struct PairProduct {
+    CUtensorMap map[4];
+    PairParams p;
+};
+// A launch of one product, or of two plain ones that do not touch each other's results (see gemm_pair_two).
+template <int kProducts> struct PairLaunch {
+    PairProduct product[kProducts];
+    int heavier, more_first;      // two products: how many pairs have one tile of the first product more than the others, and how
+                                  // many tiles of the second such a pair takes
+};
+
 __host__ __device__ __forceinline__ bool pair_seg_live(const PairParams& p, int g, int row0) {
     const int slab = row0 / p.seg_rows;
     return row0 - slab * p.seg_rows < p.seg_counts[g * p.grp_seg + slab];
@@ -157,6 +169,50 @@ struct PairTiles {
         return false;
     }
 };
+// Tiles of a launch of two products. The first, whose tiles take longer, goes round the pairs; the second fills up: the pairs that took a tile less
+// take more of it. A closed form of what a list ordered by length would give, and the same on every GPU.
+struct PairTwoTiles {
+    int pair, pairs, round = 0, second = 0;
+    __host__ __device__ __forceinline__ PairTwoTiles(int pair_, int pairs_) : pair(pair_), pairs(pairs_) {}
+    // The number of the next tile inside its product; which: the product.
+    __host__ __device__ __forceinline__ bool next(int tiles0, int tiles1, int heavier, int more_first, int& which, int& tile) {
+        tile = pair + round * pairs;
+        which = 0;
+        if (tile < tiles0) {
+            ++round;
+            return true;
+        }
+        which = 1;
+        if (pair < heavier) {
+            tile = second * heavier + pair;
+            return second++ < more_first && tile < tiles1;
+        }
+        tile = more_first * heavier + second * (pairs - heavier) + pair - heavier;
+        ++second;
+        return tile < tiles1;
+    }
+};
+template <int kProducts> struct PairWalk {
+    PairTiles tiles;
+    __device__ __forceinline__ PairWalk(int pair, int pairs) : tiles(pair, pairs) {}
+    __device__ __forceinline__ bool next(const PairLaunch<1>& l, const int* first, int rank, int& row, int& tn, int& grp, bool& live, int& which) {
+        which = 0;
+        return tiles.next(l.product[0].p, first, rank, row, tn, grp, live);
+    }
+};
+template <> struct PairWalk<2> {
+    PairTwoTiles tiles;
+    __device__ __forceinline__ PairWalk(int pair, int pairs) : tiles(pair, pairs) {}
+    __device__ __forceinline__ bool next(const PairLaunch<2>& l, const int*, int rank, int& row, int& tn, int& grp, bool& live, int& which) {
+        int tile, tm;
+        const PairParams &a = l.product[0].p, &b = l.product[1].p;
+        if (!tiles.next(a.tiles_m * a.tiles_n, b.tiles_m * b.tiles_n, l.heavier, l.more_first, which, tile)) return false;
+        pair_tile_coords(l.product[which].p, tile, tm, tn, grp);
+        row = tm * pair::kBM + rank * 128;
+        live = row < l.product[which].p.M;
+        return true;
+    }
+};
 __host__ __device__ __forceinline__ int pair_live_halves(const PairParams& p, int slab) {
     const int grp = slab / p.grp_slabs, in = slab - grp * p.grp_slabs;
     int n = p.seg_counts[grp * p.grp_seg + in];
@@ -248,14 +304,18 @@ struct PairMma {
     uint16_t pair_mask;
     bool leader;
     __device__ __forceinline__ PairMma(const PairParams& p, const uint8_t* sA, const uint8_t* sB, uint32_t rank) {
+        operands(p, sA, sB);
+        pair_mask = static_cast<uint16_t>(3u << rank);
+        leader = elect_one();
+    }
+    // How a product's operands lie in the ring.
+    __device__ __forceinline__ void operands(const PairParams& p, const uint8_t* sA, const uint8_t* sB) {
         using namespace pair;
         a_first = umma_smem_desc_sw128(smem_u32(sA), p.a_mn ? kBK * 128 : 0, 1024);
         b_first = umma_smem_desc_sw128(smem_u32(sB), p.b_mn ? kBK * 128 : 0, 1024);
         a_step = (p.a_mn ? kUmmaK * 128 : kUmmaK * 2) >> 4;
         b_step = (p.b_mn ? kUmmaK * 128 : kUmmaK * 2) >> 4;
         idesc = umma_idesc_bf16(kBM, BN, p.a_mn, p.b_mn);
-        pair_mask = static_cast<uint16_t>(3u << rank);
-        leader = elect_one();
     }
     // The live blocks of slot s into the accumulator; `started` is 0 before the first MMA of a tile, which overwrites it.
     __device__ __forceinline__ void stage(uint32_t d_tmem, int s, uint32_t live, uint32_t& started, uint64_t* empty) {
@@ -276,11 +336,11 @@ struct PairMma {
     }
 };
 
-template <int BN>
+template <int BN, int kProducts>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair::kThreads, 1)
-gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                 const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmR, const PairParams p) {
+gemm_pair_kernel(const __grid_constant__ PairLaunch<kProducts> launch) {
     using namespace pair;
+    const PairParams& shared = launch.product[0].p;    // status, overlap and ragged rows are the launch's
     constexpr int STAGES = kStages<BN>;
     constexpr int HALF = BN / 2;          // columns of the tile one epilogue warp drains; rows of B one CTA loads
     extern __shared__ uint8_t smem_raw[];
@@ -308,9 +368,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         if (lane == 31) *abort_flag = 0;
         mbar_fence_init();
     } else if (warp == 2 && lane == 0) {
-        tma_prefetch_desc(&tmA);
-        tma_prefetch_desc(&tmB);
-        tma_prefetch_desc(&tmC);
+#pragma unroll
+        for (int i = 0; i < 3 * kProducts; ++i) tma_prefetch_desc(&launch.product[i / 3].map[i % 3]);
     }
     if (warp == 1) {
         tmem_alloc_pair(tmem_slot, 2 * BN);
@@ -323,12 +382,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     grid_dep_wait();
     const uint32_t tmem_base = *tmem_slot;
 
-    if (p.grp_slabs) {
-        if (warp == 3) pair_count_halves(p, first, lane);
+    if (kProducts == 1 && shared.grp_slabs) {
+        if (warp == 3) pair_count_halves(shared, first, lane);
         __syncthreads();
     }
-    PairTiles tiles(static_cast<int>(blockIdx.x >> 1), static_cast<int>(gridDim.x >> 1));
-    int row_half, tn, grp;       // row_half: first row of this CTA's half of a tile
+    PairWalk<kProducts> tiles(static_cast<int>(blockIdx.x >> 1), static_cast<int>(gridDim.x >> 1));
+    int row_half, tn, grp, which; // row_half: first row of this CTA's half of a tile
     bool mine;                   // that half is live
 
     if (warp == 0) {
@@ -337,31 +396,33 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             int s = 0;
             uint32_t ph = 0;
             bool ok = true;
-            while (ok && tiles.next(p, first, static_cast<int>(rank), row_half, tn, grp, mine)) {
+            while (ok && tiles.next(launch, first, static_cast<int>(rank), row_half, tn, grp, mine, which)) {
+                const PairProduct& product = launch.product[kProducts > 1 ? which : 0];
+                const PairParams& p = product.p;
                 // SwiGLU: the even CTA brings the gate rows of the weight, the odd one the up rows of the same features
-                const int n0 = p.epi == CAI_EPI_SWIGLU ? tn * HALF + static_cast<int>(rank) * (p.N >> 1) : tn * BN + static_cast<int>(rank) * HALF;
+                const int n0 = kProducts == 1 && p.epi == CAI_EPI_SWIGLU ? tn * HALF + static_cast<int>(rank) * (p.N >> 1) : tn * BN + static_cast<int>(rank) * HALF;
                 PairStages stages(p, grp);
                 int ks;
                 uint32_t live;
                 while (stages.next(p, ks, live)) {
-                    if (!mbar_wait(&empty[s], ph ^ 1, abort_flag, p.status, CAI_DEV_TIMEOUT_TMA_EMPTY)) {
+                    if (!mbar_wait(&empty[s], ph ^ 1, abort_flag, shared.status, CAI_DEV_TIMEOUT_TMA_EMPTY)) {
                         ok = false;
                         break;
                     }
                     if (rank == 0) mbar_expect_tx(&full[s], 2 * kBlock<BN> * __popc(live));
                     const uint32_t bar = map_to_cta(smem_u32(&full[s]), 0);
-                    pair_load_stage<BN>(&tmA, &tmB, sA + s * kPerStage * kABytes, sB + s * kPerStage * kBBytes<BN>, bar, p, ks, live, row_half, n0, grp);
+                    pair_load_stage<BN>(&product.map[0], &product.map[1], sA + s * kPerStage * kABytes, sB + s * kPerStage * kBBytes<BN>, bar, p, ks, live, row_half, n0, grp);
                     if (++s == STAGES) {
                         s = 0;
                         ph ^= 1;
                     }
                 }
             }
-            if (p.overlap) grid_dep_launch();
+            if (shared.overlap) grid_dep_launch();
             if (ok) {
                 // every stage has been handed back: no arrival of the other CTA is still on its way when this CTA ends
                 for (int i = 0; i < STAGES && ok; ++i) {
-                    ok = mbar_wait(&empty[s], ph ^ 1, abort_flag, p.status, CAI_DEV_TIMEOUT_TMA_EMPTY);
+                    ok = mbar_wait(&empty[s], ph ^ 1, abort_flag, shared.status, CAI_DEV_TIMEOUT_TMA_EMPTY);
                     if (++s == STAGES) {
                         s = 0;
                         ph ^= 1;
@@ -376,16 +437,18 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     } else if (warp == 1) {
         if (rank == 0) {
             // ---------------- MMA issuer (even CTA)
-            PairMma<BN> mma(p, sA, sB, 0);
+            PairMma<BN> mma(shared, sA, sB, 0);
             int s = 0;
             uint32_t ph = 0;
             bool ok = true;
             int t = 0;
-            while (ok && tiles.next(p, first, static_cast<int>(rank), row_half, tn, grp, mine)) {
+            while (ok && tiles.next(launch, first, static_cast<int>(rank), row_half, tn, grp, mine, which)) {
+                const PairParams& p = launch.product[kProducts > 1 ? which : 0].p;
+                if (kProducts > 1) mma.operands(p, sA, sB);
                 const int acc = t & 1;
                 const uint32_t acc_ph = (t >> 1) & 1;
                 ++t;
-                if (!mbar_wait_warp(&tmem_empty[acc], acc_ph ^ 1, abort_flag, p.status, CAI_DEV_TIMEOUT_TMEM_EMPTY)) {
+                if (!mbar_wait_warp(&tmem_empty[acc], acc_ph ^ 1, abort_flag, shared.status, CAI_DEV_TIMEOUT_TMEM_EMPTY)) {
                     ok = false;
                     break;
                 }
@@ -396,7 +459,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                 int ks;
                 uint32_t live;
                 while (stages.next(p, ks, live)) {
-                    if (!mbar_wait_warp(&full[s], ph, abort_flag, p.status, CAI_DEV_TIMEOUT_TMA_FULL)) {
+                    if (!mbar_wait_warp(&full[s], ph, abort_flag, shared.status, CAI_DEV_TIMEOUT_TMA_FULL)) {
                         ok = false;
                         break;
                     }
@@ -411,7 +474,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             }
             // both accumulators handed back: no arrival of the odd CTA is still on its way when this one ends
             for (int i = 0; i < 2 && ok; ++i, ++t)
-                ok = mbar_wait_warp(&tmem_empty[t & 1], ((t >> 1) & 1) ^ 1, abort_flag, p.status, CAI_DEV_TIMEOUT_TMEM_EMPTY);
+                ok = mbar_wait_warp(&tmem_empty[t & 1], ((t >> 1) & 1) ^ 1, abort_flag, shared.status, CAI_DEV_TIMEOUT_TMEM_EMPTY);
         }
     } else {
         // ---------------- epilogue warps: TMEM -> registers -> shared memory -> TMA
@@ -425,13 +488,16 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         const uint32_t release[2] = {map_to_cta(smem_u32(&tmem_empty[0]), 0), map_to_cta(smem_u32(&tmem_empty[1]), 0)};
         int t = 0;
         bool ok = true;
-        while (ok && tiles.next(p, first, static_cast<int>(rank), row_half, tn, grp, mine)) {
+        while (ok && tiles.next(launch, first, static_cast<int>(rank), row_half, tn, grp, mine, which)) {
+            const PairProduct& product = launch.product[kProducts > 1 ? which : 0];
+            const PairParams& p = product.p;
+            const CUtensorMap &tmC = product.map[2], &tmR = product.map[3];
             const int acc = t & 1;
             const uint32_t acc_ph = (t >> 1) & 1;
             ++t;
             // a weight-gradient tile whose every k-block was skipped has an undefined accumulator: it counts as zero
             bool acc_valid = true;
-            if (p.seg_mode == 2) {
+            if (kProducts == 1 && p.seg_mode == 2) {
                 PairStages stages(p, grp);
                 int ks;
                 uint32_t any;
@@ -451,14 +517,14 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                     if (res_ok && col + j * 8 < p.N) res[j] = *reinterpret_cast<const uint4*>(rrow + col + j * 8);
             };
             if (residual) fetch(col_first);
-            if (!mbar_wait_warp(&tmem_full[acc], acc_ph, abort_flag, p.status, CAI_DEV_TIMEOUT_TMEM_FULL)) {
+            if (!mbar_wait_warp(&tmem_full[acc], acc_ph, abort_flag, shared.status, CAI_DEV_TIMEOUT_TMEM_FULL)) {
                 ok = false;
                 break;
             }
             tc_fence_after();
             const uint32_t tacc = tmem_base + lane_bits + acc * BN;
             if (live) {
-                if (p.epi == CAI_EPI_SWIGLU) {
+                if (kProducts == 1 && p.epi == CAI_EPI_SWIGLU) {
                     // columns [0, HALF) are gate, [HALF, BN) up, of features tn * HALF ...; this warp's share is HALF / 2 of each
                     const int F = p.N >> 1;
 #pragma unroll 1
@@ -595,10 +661,24 @@ constexpr int kSplitBN = 128;
 constexpr int kSplitSmem = kStages<kSplitBN> * kPerStage * kBlock<kSplitBN> + 512 + 1024;
 }  // namespace pair
 
-template <int S>
+// The operands' maps and the rest, of one product or of two. Two products in clusters of 2 S CTAs may be cut into fewer slices than S (each keeps
+// the sums of its own form): such a cluster holds S / slices tiles next to each other.
+template <int kProducts> struct SplitLaunch {
+    CUtensorMap map[kProducts][2];
+    PairParams p[kProducts];
+    int slices[kProducts];
+    int first1;                // the second product's first cluster
+};
+
+template <int S, int kProducts>
 __global__ void __launch_bounds__(pair::kThreads, 1)
-gemm_pair_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const PairParams p) {
+gemm_pair_split_kernel(const __grid_constant__ SplitLaunch<kProducts> launch) {
     using namespace pair;
+    int tile = launch.p[0].tile0 + static_cast<int>(blockIdx.x) / (2 * S);   // or, of two products, the cluster's number
+    const int which = kProducts > 1 && tile >= launch.first1;
+    const PairParams& p = launch.p[which];
+    const int slices = kProducts > 1 ? launch.slices[which] : S;
+    const CUtensorMap &tmA = launch.map[which][0], &tmB = launch.map[which][1];
     constexpr int BN = kSplitBN, STAGES = kStages<BN>, HALF = BN / 2;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -614,7 +694,16 @@ gemm_pair_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();
     const uint32_t even = rank & ~1u;          // the CTA of my pair that issues
-    const int slice = static_cast<int>(rank >> 1), side = static_cast<int>(rank & 1);
+    const int side = static_cast<int>(rank & 1);
+    int slice = static_cast<int>(rank >> 1), slice0 = 0;     // my slice of my tile; the pair of the cluster that has its first one
+    bool some = true;                                        // this pair has a tile
+    if (kProducts > 1) {
+        const int mine = slice / slices;
+        slice0 = mine * slices;
+        slice -= slice0;
+        tile = (tile - (which ? launch.first1 : 0)) * (S / slices) + mine;
+        some = tile < p.tiles_m * p.tiles_n;
+    }
 
     if (warp == 0) {
         if (lane < 2 * STAGES + 1) mbar_init(&bars[lane], 1);
@@ -636,11 +725,11 @@ gemm_pair_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
     const uint32_t tmem_base = *tmem_slot;
 
     int tm, tn, grp;
-    pair_tile_coords(p, p.tile0 + static_cast<int>(blockIdx.x) / (2 * S), tm, tn, grp);
+    pair_tile_coords(p, tile, tm, tn, grp);
     const int num_kb = (p.K + kBK - 1) / kBK;
     const int num_ks = (num_kb + kPerStage - 1) / kPerStage;
-    const int ks0 = num_ks * slice / S, ks1 = num_ks * (slice + 1) / S;
-    const int row_half = tm * kBM + side * 128;
+    const int ks0 = some ? num_ks * slice / slices : 0, ks1 = some ? num_ks * (slice + 1) / slices : 0;
+    const int row_half = some ? tm * kBM + side * 128 : p.M;
 
     if (warp == 0) {
         if (lane == 0) {
@@ -719,11 +808,11 @@ gemm_pair_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
     __syncwarp();
     cluster_sync_memory();     // every partial of the cluster is in place
     if (row_half < p.M && !*abort_flag) {
-        constexpr int W = BN / S / 4;          // 16-byte chunks of my slab per row
-        const int col0 = tn * BN + slice * (BN / S);
+        const int W = BN / 4 / slices;         // 16-byte chunks of my slab per row
+        const int col0 = tn * BN + slice * (BN / slices);
         uint32_t src[S];
 #pragma unroll
-        for (int i = 0; i < S; ++i) src[i] = map_to_cta(smem_u32(smem), 2 * i + side);
+        for (int i = 0; i < S; ++i) src[i] = map_to_cta(smem_u32(smem), 2 * (i < slices ? slice0 + i : slice0) + side);
 #pragma unroll 2
         for (int it = threadIdx.x; it < 128 * W; it += kThreads) {
             const int r = it / W, c = it % W;
@@ -732,10 +821,12 @@ gemm_pair_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
             if (row_in >= p.M || col >= p.N) continue;   // before the loads: every one issued is consumed before the closing barrier
             float4 part[S];
 #pragma unroll
-            for (int i = 0; i < S; ++i) part[i] = ld_cluster_f4(src[i] + at);
+            for (int i = 0; i < S; ++i)
+                if (i < slices) part[i] = ld_cluster_f4(src[i] + at);
             float4 v = part[0];
 #pragma unroll
             for (int i = 1; i < S; ++i) {
+                if (i >= slices) break;
                 v.x += part[i].x; v.y += part[i].y; v.z += part[i].z; v.w += part[i].w;
             }
             v.x *= p.alpha; v.y *= p.alpha; v.z *= p.alpha; v.w *= p.alpha;
@@ -790,70 +881,83 @@ static bool pair_operand_maps(CUtensorMap* tmA, CUtensorMap* tmB, const void* A,
                           : pair_map(tmB, g, B, g.K, g.N, g.ldb, g.grp_b, 64, pair::kBK, 2));
 }
 
-template <int S>
-static int launch_split(const void* A, const void* B, const GemmShape& g, PairParams& p, int at_once, cudaStream_t st) {
-    constexpr int BN = pair::kSplitBN;
-    CUtensorMap tmA, tmB;
-    if (!pair_operand_maps(&tmA, &tmB, A, B, g, BN)) return CAI_K_BAD_ARG;
+template <typename Kernel>
+static bool allow_smem(Kernel kernel, int bytes, const char* what) {
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess) return true;
+    set_last_error("cudaFuncSetAttribute(%s) failed: %s", what, cudaGetErrorString(cudaGetLastError()));
+    return false;
+}
+static int launched(cudaError_t e, const char* what) {
+    if (e == cudaSuccess) return CAI_K_OK;
+    set_last_error("%s launch failed: %s", what, cudaGetErrorString(e));
+    return CAI_K_CUDA;
+}
+static void pair_tiles(PairParams& p, int tile_cols) {
     p.tiles_m = (p.M + pair::kBM - 1) / pair::kBM;
-    p.tiles_n = (p.N + BN - 1) / BN;
+    p.tiles_n = (p.N + tile_cols - 1) / tile_cols;
     p.group_m = 8;
+}
+
+template <int S, int kProducts>
+static int launch_split(SplitLaunch<kProducts>& l, int at_once, cudaStream_t st) {
     static bool configured[64] = {};
     const int dev = current_device();
     if (!configured[dev & 63]) {
-        if (cudaFuncSetAttribute(gemm_pair_split_kernel<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, pair::kSplitSmem) != cudaSuccess) {
-            set_last_error("cudaFuncSetAttribute(gemm_pair_split) failed: %s", cudaGetErrorString(cudaGetLastError()));
-            return CAI_K_CUDA;
-        }
+        if (!allow_smem(gemm_pair_split_kernel<S, kProducts>, pair::kSplitSmem, "gemm_pair_split")) return CAI_K_CUDA;
         configured[dev & 63] = true;
+    }
+    int tiles = 0;                             // clusters, of two products
+    for (int i = 0; i < kProducts; ++i) {
+        PairParams& p = l.p[i];
+        l.first1 = tiles;
+        pair_tiles(p, pair::kSplitBN);
+        const int per_cluster = S / l.slices[i];
+        tiles += (p.tiles_m * p.tiles_n * p.groups + per_cluster - 1) / per_cluster;
     }
     // Under a limit on the SMs the clusters go out in turns of `at_once`, each launched when the one before has ended: the same sums in the
     // same order.
-    const int tiles = p.tiles_m * p.tiles_n * p.groups;
-    for (p.tile0 = 0; p.tile0 < tiles; p.tile0 += at_once) {
+    for (int& tile0 = l.p[0].tile0; tile0 < tiles; tile0 += at_once) {
         cudaLaunchConfig_t cfg = {};
         cudaLaunchAttribute attr[2];
-        split_config<S>(cfg, attr, static_cast<unsigned>(2 * S * (tiles - p.tile0 < at_once ? tiles - p.tile0 : at_once)), p.overlap, st);
-        const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_pair_split_kernel<S>, tmA, tmB, p);
-        if (e != cudaSuccess) {
-            set_last_error("gemm_pair_split launch failed: %s", cudaGetErrorString(e));
-            return CAI_K_CUDA;
-        }
+        split_config<S>(cfg, attr, static_cast<unsigned>(2 * S * (tiles - tile0 < at_once ? tiles - tile0 : at_once)), l.p[0].overlap, st);
+        const int rc = launched(cudaLaunchKernelEx(&cfg, gemm_pair_split_kernel<S, kProducts>, l), "gemm_pair_split");
+        if (rc) return rc;
     }
     return CAI_K_OK;
 }
 
+// What the kernel needs for one product in tiles of BN columns; false if its operands do not fit a tensor map.
 template <int BN>
-static int launch_pair(const void* A, const void* B, const GemmShape& g, PairParams& p, int pairs, cudaStream_t st) {
-    CUtensorMap tmA, tmB, tmC, tmR;
-    bool ok = pair_operand_maps(&tmA, &tmB, A, B, g, BN);
+static bool pair_product(PairProduct& q, const void* A, const void* B, const GemmShape& g, const PairParams& p) {
+    q.p = p;
+    pair_tiles(q.p, BN);
+    bool ok = pair_operand_maps(&q.map[0], &q.map[1], A, B, g, BN);
     const bool f32 = p.epi == CAI_EPI_F32 || p.epi == CAI_EPI_F32_ACCUM;
-    ok = ok && pair_map(&tmC, g, g.C, p.M, p.N, g.ldc, g.grp_c, f32 ? 32 : 64, 32, f32 ? 4 : 2);
-    tmR = tmC;
-    if (ok && p.epi == CAI_EPI_SWIGLU) ok = pair_map(&tmR, g, g.R, p.M, p.N / 2, g.ldr, g.grp_c, 64, 32, 2);
-    if (!ok) return CAI_K_BAD_ARG;
+    ok = ok && pair_map(&q.map[2], g, g.C, p.M, p.N, g.ldc, g.grp_c, f32 ? 32 : 64, 32, f32 ? 4 : 2);
+    q.map[3] = q.map[2];
+    if (ok && p.epi == CAI_EPI_SWIGLU) ok = pair_map(&q.map[3], g, g.R, p.M, p.N / 2, g.ldr, g.grp_c, 64, 32, 2);
+    return ok;
+}
+
+template <int BN, int kProducts>
+static int launch_pair(const PairLaunch<kProducts>& l, int pairs, cudaStream_t st) {
     static bool configured[64] = {};
     const int dev = current_device();
     if (!configured[dev & 63]) {
-        if (cudaFuncSetAttribute(gemm_pair_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, pair::kSmem<BN>) != cudaSuccess) {
-            set_last_error("cudaFuncSetAttribute(gemm_pair) failed: %s", cudaGetErrorString(cudaGetLastError()));
-            return CAI_K_CUDA;
-        }
+        if (!allow_smem(gemm_pair_kernel<BN, kProducts>, pair::kSmem<BN>, "gemm_pair")) return CAI_K_CUDA;
         configured[dev & 63] = true;
     }
-    p.tiles_m = (p.M + pair::kBM - 1) / pair::kBM;
-    p.tiles_n = (p.N + BN - 1) / BN;
-    p.group_m = 8;
-    const int tiles = p.tiles_m * p.tiles_n * p.groups;
-    const int grid = 2 * (tiles < pairs ? tiles : pairs);
-    if (p.overlap) launch_early(gemm_pair_kernel<BN>, grid, pair::kThreads, pair::kSmem<BN>, st, tmA, tmB, tmC, tmR, p);
-    else gemm_pair_kernel<BN><<<grid, pair::kThreads, pair::kSmem<BN>, st>>>(tmA, tmB, tmC, tmR, p);
-    const cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) {
-        set_last_error("gemm_pair launch failed: %s", cudaGetErrorString(e));
-        return CAI_K_CUDA;
-    }
-    return CAI_K_OK;
+    const int grid = 2 * pairs;
+    if (l.product[0].p.overlap) launch_early(gemm_pair_kernel<BN, kProducts>, grid, pair::kThreads, pair::kSmem<BN>, st, l);
+    else gemm_pair_kernel<BN, kProducts><<<grid, pair::kThreads, pair::kSmem<BN>, st>>>(l);
+    return launched(cudaGetLastError(), "gemm_pair");
+}
+template <int BN>
+static int launch_one(const void* A, const void* B, const GemmShape& g, const PairParams& p, int pairs, cudaStream_t st) {
+    PairLaunch<1> l = {};
+    if (!pair_product<BN>(l.product[0], A, B, g, p)) return CAI_K_BAD_ARG;
+    const int tiles = l.product[0].p.tiles_m * l.product[0].p.tiles_n * p.groups;
+    return launch_pair<BN, 1>(l, tiles < pairs ? tiles : pairs, st);
 }
 
 // Which form: the smallest estimate in SM cycles on a B200 of 74 pairs. A stage of 128 k-elements takes a CTA about 1150 cycles in the
@@ -868,12 +972,21 @@ static int launch_pair(const void* A, const void* B, const GemmShape& g, PairPar
 //   14 tiles, K 2048  15.4 / 13.4 / 10.7 /  9.3       16 tiles  15.4 / 13.7 / 10.7 / 16.5      33 tiles  15.6 / 13.9 / 11.3 / 24.8
 //   36 tiles, K 2048  15.6 / 14.0 / 20.3 / 24.8       72 tiles  16.5 / 14.6 / 30.3 / 41.2      80 tiles  16.4 / 23.1
 //   16 tiles, K 512    8.8 /  7.4 /  7.9 / 13.6      135 tiles, K 2048  26.2 / 23.8            160 tiles, K 2048  26.9 / 32.7
+static double pair_tile_cycles(int K, int tile_cols) {
+    const double ks = static_cast<double>((static_cast<long long>(K) + 127) / 128);
+    return tile_cols == 256 ? ks * 1150.0 + 2500.0 : ks * 850.0 + 1500.0;
+}
+static long long pair_tile_count(int M, int N, int tile_cols) {
+    return (static_cast<long long>(M) + pair::kBM - 1) / pair::kBM * ((static_cast<long long>(N) + tile_cols - 1) / tile_cols);
+}
+constexpr long long kFormPairs = 74, kSplitTiles2 = 33, kSplitTiles4 = 15;
+
 PairForm pair_form(int M, int N, int K, int groups, int epi, bool segmented) {
-    constexpr long long kPairs = 74, kSplitTiles2 = 33, kSplitTiles4 = 15;
-    const long long ks = (K + 127) / 128, tm = (M + pair::kBM - 1) / pair::kBM;
-    const long long t256 = tm * ((N + 255) / 256) * groups, t128 = tm * ((N + 127) / 128) * groups;
-    const double wide = static_cast<double>((t256 + kPairs - 1) / kPairs) * (ks * 1150.0 + 2500.0);
-    const double narrow = static_cast<double>((t128 + kPairs - 1) / kPairs) * (ks * 850.0 + 1500.0);
+    constexpr long long kPairs = kFormPairs;
+    const long long ks = (static_cast<long long>(K) + 127) / 128;
+    const long long t256 = pair_tile_count(M, N, 256) * groups, t128 = pair_tile_count(M, N, 128) * groups;
+    const double wide = static_cast<double>((t256 + kPairs - 1) / kPairs) * pair_tile_cycles(K, 256);
+    const double narrow = static_cast<double>((t128 + kPairs - 1) / kPairs) * pair_tile_cycles(K, 128);
     if (epi == CAI_EPI_SWIGLU) return {256, 1};
     if (!segmented) {
         const double two = ks >= 2 && t128 <= kSplitTiles2 ? (ks + 1) / 2 * 850.0 + 4500.0 : 1e30;
@@ -898,8 +1011,8 @@ static int pair_counted_slabs(int M, int seg_rows, int groups) {
     return slabs * groups <= pair::kMaxSlabs ? static_cast<int>(slabs) : 0;
 }
 
-int gemm_pair(const void* A, const void* B, const GemmShape& g, cudaStream_t st) {
-    PairParams p;
+static PairParams pair_params(const GemmShape& g, int dev) {
+    PairParams p = {};
     p.M = g.M; p.N = g.N; p.K = g.K;
     p.a_mn = g.a_mn; p.b_mn = g.b_mn;
     p.epi = g.epi; p.alpha = g.alpha;
@@ -908,16 +1021,133 @@ int gemm_pair(const void* A, const void* B, const GemmShape& g, cudaStream_t st)
     p.C = g.C;
     p.R = static_cast<const __nv_bfloat16*>(g.R);
     p.ldc = g.ldc; p.ldr = g.ldr; p.grp_c = g.grp_c;
-    p.tile0 = 0;
     p.overlap = g.sm_limit <= 0;
     p.grp_slabs = g.seg_mode == 1 ? pair_counted_slabs(g.M, g.seg_rows, g.groups) : 0;
-    const int dev = current_device();
     p.status = status_words(dev);
+    return p;
+}
+template <int S>
+static int split_one(const void* A, const void* B, const GemmShape& g, const PairParams& p, int at_once, cudaStream_t st) {
+    SplitLaunch<1> l = {};
+    l.p[0] = p;
+    l.slices[0] = S;
+    if (!pair_operand_maps(&l.map[0][0], &l.map[0][1], A, B, g, pair::kSplitBN)) return CAI_K_BAD_ARG;
+    return launch_split<S, 1>(l, at_once, st);
+}
+
+int gemm_pair(const void* A, const void* B, const GemmShape& g, cudaStream_t st) {
+    const int dev = current_device();
+    const PairParams p = pair_params(g, dev);
     const PairForm f = pair_form(g.M, g.N, g.K, g.groups, g.epi, g.seg_mode != 0);
     const int at_once = pair_clusters(f, sm_count(dev), g.sm_limit);
-    if (f.slices == 4) return launch_split<4>(A, B, g, p, at_once, st);
-    if (f.slices == 2) return launch_split<2>(A, B, g, p, at_once, st);
-    return f.tile_cols == 256 ? launch_pair<256>(A, B, g, p, at_once, st) : launch_pair<128>(A, B, g, p, at_once, st);
+    if (f.slices == 4) return split_one<4>(A, B, g, p, at_once, st);
+    if (f.slices == 2) return split_one<2>(A, B, g, p, at_once, st);
+    return f.tile_cols == 256 ? launch_one<256>(A, B, g, p, at_once, st) : launch_one<128>(A, B, g, p, at_once, st);
+}
+
+// The schedule of two products on `pairs` pairs, of n0 tiles of c0 cycles each and n1 of c1 <= c0 (PairTwoTiles): its length.
+static double pair_two_schedule(long long n0, double c0, long long n1, double c1, long long pairs, int* heavier, int* more_first) {
+    const long long q = n0 / pairs, r = n0 % pairs;
+    const double base = static_cast<double>(q) * c0;
+    double best = 1e30;
+    *heavier = static_cast<int>(r);
+    *more_first = 0;
+    for (long long m = 0; m == 0 || (r > 0 && base + c0 + static_cast<double>(m) * c1 < best); ++m) {
+        const long long left = n1 - m * r > 0 ? n1 - m * r : 0;
+        const double light = base + static_cast<double>((left + pairs - r - 1) / (pairs - r)) * c1;
+        const double heavy = r ? base + c0 + static_cast<double>(m) * c1 : 0.0;
+        const double t = light > heavy ? light : heavy;
+        if (t < best) {
+            best = t;
+            *more_first = static_cast<int>(m);
+        }
+    }
+    return best;
+}
+
+// Two products that do not touch each other's results (the two gradients of a linear layer) in one launch, so that the last waves of one are filled
+// by the other and the chain is a launch shorter: where both are one sum along K, in persistent tiles of one width; where one is split, in clusters,
+// while all of them run at once. Each keeps its own order of summation, so the results are those of two launches. Measured for 38 pairs of gradients
+// (tokens, in and out features; us apart / together; bursts of 3 ms with pauses):
+//   1920 1000 5456  60.0 / 44.3     1920 2728 1000  39.5 / 27.8     768 2440 5728  58.8 / 46.2      3072 2352 728  36.3 / 24.6
+//   512 256 1024    12.6 / 8.7      256 288 904     12.0 / 8.1      2816 352 512   13.7 / 10.0      768 848 848    14.9 / 8.3
+// Against it: products that fill the tensor cores to seven tenths by themselves run at the power limit, where idle SMs cost nothing and mixed
+// tiles share less in L2 (4096 2048 8192 206.8 / 210.2, 16384 2048 2048 197.8 / 201.2), and below a gain of a fifteenth by the count of waves nothing
+// is left of it (4096 2048 4096 104.1 / 107.9, 3456 1408 2944 58.0 / 59.4). Tiles of 128 columns beyond one wave are fed too slowly when every SM
+// is busy (1920 1000 5456 56.0, 3456 1408 5888 98.4 in wide tiles and 133.3). Clusters beyond those that run at once make a second
+// wave (1024 384 808, twice four slices, 13.8 / 14.6; 256 808 10040, four slices and one sum, 31.9 / 53.9).
+bool pair_two_form(const GemmShape& a, const GemmShape& b, PairTwoForm* out) {
+    const GemmShape* g[2] = {&a, &b};
+    PairForm f[2];
+    long long narrow = 0;
+    for (int i = 0; i < 2; ++i) {
+        if (g[i]->seg_mode || g[i]->groups != 1 || g[i]->sm_limit > 0 || g[i]->epi > CAI_EPI_BF16_RESIDUAL) return false;
+        f[i] = pair_form(g[i]->M, g[i]->N, g[i]->K, 1, g[i]->epi, false);
+        narrow += pair_tile_count(g[i]->M, g[i]->N, pair::kSplitBN);
+    }
+    if (narrow > (1ll << 30)) return false;
+    *out = {};
+    out->slices[0] = f[0].slices;                   // the order of each product's sums is its own form's
+    out->slices[1] = f[1].slices;
+    out->tile_cols = pair::kSplitBN;
+    const int most = f[0].slices > f[1].slices ? f[0].slices : f[1].slices;
+    if (most > 1) {
+        long long clusters = 0;
+        for (int i = 0; i < 2; ++i) {
+            const int per_cluster = most / f[i].slices;
+            clusters += (pair_tile_count(g[i]->M, g[i]->N, pair::kSplitBN) + per_cluster - 1) / per_cluster;
+        }
+        return clusters <= (most == 4 ? kSplitTiles4 : kSplitTiles2);
+    }
+    constexpr double kLaunch = 4000.0;              // cycles from the end of a launch to the main loop of the next
+    constexpr double kPairFlops = 16384.0;          // a pair's tensor cores, a cycle
+    double apart = kLaunch, flops = 0;
+    for (int i = 0; i < 2; ++i) {
+        apart += static_cast<double>((pair_tile_count(g[i]->M, g[i]->N, f[i].tile_cols) + kFormPairs - 1) / kFormPairs) * pair_tile_cycles(g[i]->K, f[i].tile_cols);
+        flops += 2.0 * g[i]->M * g[i]->N * g[i]->K;
+    }
+    if (narrow > kFormPairs) out->tile_cols = 256;
+    out->first = g[1]->K > g[0]->K;                 // the product of the longer tiles goes first
+    const GemmShape &x = *g[out->first], &y = *g[1 - out->first];
+    const long long nx = pair_tile_count(x.M, x.N, out->tile_cols), ny = pair_tile_count(y.M, y.N, out->tile_cols);
+    int heavier, more;
+    const double together = pair_two_schedule(nx, pair_tile_cycles(x.K, out->tile_cols), ny, pair_tile_cycles(y.K, out->tile_cols),
+                                              nx + ny < kFormPairs ? nx + ny : kFormPairs, &heavier, &more);
+    return together <= 14.0 / 15.0 * apart && flops <= 0.7 * apart * kFormPairs * kPairFlops;
+}
+
+template <int BN>
+static int launch_two(const void* const (&A)[2], const void* const (&B)[2], const GemmShape* const (&g)[2], int sms, int dev, cudaStream_t st) {
+    PairLaunch<2> l = {};
+    long long n[2];
+    for (int i = 0; i < 2; ++i) {
+        if (!pair_product<BN>(l.product[i], A[i], B[i], *g[i], pair_params(*g[i], dev))) return CAI_K_BAD_ARG;
+        n[i] = pair_tile_count(g[i]->M, g[i]->N, BN);
+    }
+    const long long most = sms / 2 > 0 ? sms / 2 : 1, pairs = n[0] + n[1] < most ? n[0] + n[1] : most;
+    pair_two_schedule(n[0], pair_tile_cycles(g[0]->K, BN), n[1], pair_tile_cycles(g[1]->K, BN), pairs, &l.heavier, &l.more_first);
+    return launch_pair<BN, 2>(l, static_cast<int>(pairs), st);
+}
+template <int S>
+static int split_two(const void* const (&A)[2], const void* const (&B)[2], const GemmShape* const (&g)[2], const int (&slices)[2], int dev, cudaStream_t st) {
+    SplitLaunch<2> l = {};
+    for (int i = 0; i < 2; ++i) {
+        l.p[i] = pair_params(*g[i], dev);
+        l.slices[i] = slices[i];
+        if (!pair_operand_maps(&l.map[i][0], &l.map[i][1], A[i], B[i], *g[i], pair::kSplitBN)) return CAI_K_BAD_ARG;
+    }
+    return launch_split<S, 2>(l, 1 << 30, st);
+}
+
+int gemm_pair_two(const void* A0, const void* B0, const GemmShape& g0, const void* A1, const void* B1, const GemmShape& g1, const PairTwoForm& f,
+                  cudaStream_t st) {
+    const int dev = current_device();
+    const void *const A[2] = {f.first ? A1 : A0, f.first ? A0 : A1}, *const B[2] = {f.first ? B1 : B0, f.first ? B0 : B1};
+    const GemmShape* const g[2] = {f.first ? &g1 : &g0, f.first ? &g0 : &g1};
+    const int most = f.slices[0] > f.slices[1] ? f.slices[0] : f.slices[1], slices[2] = {f.slices[f.first], f.slices[1 - f.first]};
+    if (most == 4) return split_two<4>(A, B, g, slices, dev, st);
+    if (most == 2) return split_two<2>(A, B, g, slices, dev, st);
+    return f.tile_cols == 256 ? launch_two<256>(A, B, g, sm_count(dev), dev, st) : launch_two<128>(A, B, g, sm_count(dev), dev, st);
 }
 
 }  // namespace cai
@@ -968,4 +1198,16 @@ CAI_API int cai_gemm_bf16_ragged_walk(int M, int N, int groups, const int* seg_c
             t[0] = grp[0]; t[1] = tn[0]; t[2] = row[0]; t[3] = row[1]; t[4] = live[0]; t[5] = live[1];
         }
     }
+}
+
+CAI_API int cai_gemm_bf16_two_walk(int n0, int k0, int n1, int k1, int tile_cols, int pairs, int pair, int* tiles, int capacity) {
+    if (n0 < 0 || n1 < 0 || k0 < k1 || k1 <= 0 || pairs <= 0 || pair < 0 || pair >= pairs) return CAI_K_BAD_ARG;
+    int heavier, more_first, n = 0, which, tile;
+    pair_two_schedule(n0, pair_tile_cycles(k0, tile_cols), n1, pair_tile_cycles(k1, tile_cols), pairs, &heavier, &more_first);
+    for (PairTwoTiles walk(pair, pairs); walk.next(n0, n1, heavier, more_first, which, tile); ++n)
+        if (n < capacity) {
+            tiles[2 * n] = which;
+            tiles[2 * n + 1] = tile;
+        }
+    return n;
 }

@@ -874,11 +874,9 @@ CAI_API int cai_gemm_bf16(const void* A, const void* B, void* C, const void* R, 
                              sm_limit, stream);
 }
 
-CAI_API int cai_gemm_bf16_seg(const void* A, const void* B, void* C, const void* R, int M, int N, int K,
-                              long long lda, long long ldb, long long ldc, long long ldr, int a_mn_major,
-                              int b_mn_major, int epi, float alpha, const int* seg_counts, int seg_rows, int seg_mode,
-                              int sm_limit, void* stream) {
-    if (M <= 0 || N <= 0 || K <= 0) return CAI_K_OK;
+// Arguments of a product that has something to do: CAI_K_OK or the error, with its text.
+static int check_gemm(const void* R, int N, long long lda, long long ldb, long long ldc, long long ldr, int b_mn_major, int epi,
+                      const int* seg_counts, int seg_rows, int seg_mode) {
     if (seg_mode && (!seg_counts || seg_rows <= 0 || seg_rows % 128 || seg_mode > 2)) {
         set_last_error("gemm: segmented form needs counts and a slab size that is a multiple of 128");
         return CAI_K_BAD_ARG;
@@ -904,6 +902,15 @@ CAI_API int cai_gemm_bf16_seg(const void* A, const void* B, void* C, const void*
         set_last_error("gemm: fused SwiGLU needs B stored [2F, K] with F a multiple of 128 (N=%d)", N);
         return CAI_K_BAD_ARG;
     }
+    return CAI_K_OK;
+}
+
+CAI_API int cai_gemm_bf16_seg(const void* A, const void* B, void* C, const void* R, int M, int N, int K,
+                              long long lda, long long ldb, long long ldc, long long ldr, int a_mn_major,
+                              int b_mn_major, int epi, float alpha, const int* seg_counts, int seg_rows, int seg_mode,
+                              int sm_limit, void* stream) {
+    if (M <= 0 || N <= 0 || K <= 0) return CAI_K_OK;
+    if (const int rc = check_gemm(R, N, lda, ldb, ldc, ldr, b_mn_major, epi, seg_counts, seg_rows, seg_mode)) return rc;
     if (epi != CAI_EPI_SWIGLU_BWD) {
         const GemmShape g = {M, N, K, a_mn_major ? 1 : 0, b_mn_major ? 1 : 0, epi, alpha, C, R, lda, ldb, ldc, ldr,
                              seg_counts, seg_rows, seg_mode, 0, 1, 0, 0, 0, sm_limit};
@@ -923,6 +930,38 @@ CAI_API int cai_gemm_bf16_seg(const void* A, const void* B, void* C, const void*
         p.seg_rows = seg_rows;
     }
     return gemm_dispatch(A, B, lda, ldb, p, sm_limit, reinterpret_cast<cudaStream_t>(stream));
+}
+
+static GemmShape shape_of(const cai_gemm_call& c) {
+    return {c.M, c.N, c.K, c.a_mn_major ? 1 : 0, c.b_mn_major ? 1 : 0, c.epi, c.alpha, c.C, c.R, c.lda, c.ldb, c.ldc, c.ldr,
+            nullptr, 0, 0, 0, 1, 0, 0, 0, 0};
+}
+static bool empty_call(const cai_gemm_call& c) { return c.M <= 0 || c.N <= 0 || c.K <= 0; }
+
+CAI_API int cai_gemm_bf16_two(const cai_gemm_call* first, const cai_gemm_call* second, void* stream) {
+    const cai_gemm_call* const calls[2] = {first, second};
+    PairTwoForm form;
+    bool together = !empty_call(*first) && !empty_call(*second);
+    for (int i = 0; i < 2 && together; ++i) {
+        const cai_gemm_call& c = *calls[i];
+        together = check_gemm(c.R, c.N, c.lda, c.ldb, c.ldc, c.ldr, c.b_mn_major, c.epi, nullptr, 0, 0) == CAI_K_OK;
+    }
+    if (together && pair_two_form(shape_of(*first), shape_of(*second), &form))
+        return gemm_pair_two(first->A, first->B, shape_of(*first), second->A, second->B, shape_of(*second), form,
+                             reinterpret_cast<cudaStream_t>(stream));
+    for (const cai_gemm_call* c : calls) {
+        const int rc = cai_gemm_bf16(c->A, c->B, c->C, c->R, c->M, c->N, c->K, c->lda, c->ldb, c->ldc, c->ldr, c->a_mn_major, c->b_mn_major,
+                                     c->epi, c->alpha, 0, stream);
+        if (rc) return rc;
+    }
+    return CAI_K_OK;
+}
+
+CAI_API int cai_gemm_bf16_two_launches(const cai_gemm_call* first, const cai_gemm_call* second, int* tile_cols) {
+    PairTwoForm form = {};
+    const bool together = !empty_call(*first) && !empty_call(*second) && pair_two_form(shape_of(*first), shape_of(*second), &form);
+    *tile_cols = form.tile_cols;
+    return together ? 1 : !empty_call(*first) + !empty_call(*second);
 }
 
 CAI_API int cai_gemm_bf16_grouped(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,

@@ -177,6 +177,7 @@ struct cai_exec {
     cai_fused_hook_t fused_hook = nullptr;
     void* fused_ctx = nullptr;
     int sm_limit_hi = 0;
+    std::vector<uint8_t> with_next;   // per op: a product that goes out together with the one behind it
     uint64_t launches = 0;  // kernels / collectives enqueued by the last replay
     // ZeRO-3: a parameter gather waiting to be merged into the GEMM that follows it in the op table
     GatherJob pending_gather{};
@@ -534,6 +535,47 @@ int check_operands(const cai_exec* ex, const ExecOp& x, size_t op_index) {
     return 0;
 }
 
+// The plain product of a record, as the kernel library takes it.
+cai_gemm_call gemm_call(const cai_exec* ex, const ExecOp& x) {
+    cai_gemm_call c = {};
+    c.A = ex->ptr(x.t[0]); c.B = ex->ptr(x.t[1]); c.C = ex->ptr(x.t[2]); c.R = ex->ptr(x.t[3]);
+    c.lda = ex->ld(x.t[0]); c.ldb = ex->ld(x.t[1]); c.ldc = ex->ld(x.t[2]); c.ldr = x.t[3] >= 0 ? ex->ld(x.t[3]) : 0;
+    c.M = x.i[0]; c.N = x.i[1]; c.K = x.i[2];
+    c.a_mn_major = x.flags & 1; c.b_mn_major = (x.flags >> 1) & 1;
+    c.epi = (x.flags >> 4) & 0xF;
+    c.alpha = x.f[0];
+    return c;
+}
+
+// Whether two records next to each other on one stream are plain products of which neither touches what the other writes: a layer's input gradient and
+// weight gradient, which the plan puts side by side. Ranges are those that the products address, from the records' own sizes.
+bool independent_products(const cai_exec* ex, const Op& o0, const Op& o1) {
+    if (!o0.exec || !o1.exec || o0.stream_id != o1.stream_id) return false;
+    if (o0.kind == OP_EVENT_RECORD || o0.kind == OP_EVENT_WAIT || o1.kind == OP_EVENT_RECORD || o1.kind == OP_EVENT_WAIT) return false;
+    struct Range { const uint8_t *lo, *hi; };
+    Range reads[2][3] = {}, writes[2] = {};
+    for (int k = 0; k < 2; ++k) {
+        const ExecOp& x = ex->exec[(k ? o1 : o0).exec - 1];
+        if (x.kernel != K_GEMM || (x.flags & 0x100) || x.t[4] >= 0) return false;
+        const cai_gemm_call c = gemm_call(ex, x);
+        if (c.epi > CAI_EPI_BF16_RESIDUAL) return false;
+        auto range = [](const void* at, long long rows, long long cols, long long ld, int bytes) {
+            const uint8_t* p = static_cast<const uint8_t*>(at);
+            return p && rows > 0 ? Range{p, p + ((rows - 1) * ld + cols) * bytes} : Range{nullptr, nullptr};
+        };
+        reads[k][0] = c.a_mn_major ? range(c.A, c.K, c.M, c.lda, 2) : range(c.A, c.M, c.K, c.lda, 2);
+        reads[k][1] = c.b_mn_major ? range(c.B, c.K, c.N, c.ldb, 2) : range(c.B, c.N, c.K, c.ldb, 2);
+        if (c.epi == CAI_EPI_BF16_RESIDUAL) reads[k][2] = range(c.R, c.M, c.N, c.ldr, 2);
+        writes[k] = range(c.C, c.M, c.N, c.ldc, c.epi == CAI_EPI_F32 || c.epi == CAI_EPI_F32_ACCUM ? 4 : 2);
+    }
+    auto meet = [](const Range& a, const Range& b) { return a.lo < b.hi && b.lo < a.hi; };
+    if (meet(writes[0], writes[1])) return false;
+    for (int k = 0; k < 2; ++k)
+        for (const Range& r : reads[k])
+            if (meet(writes[1 - k], r)) return false;
+    return true;
+}
+
 // How many kernels of this library one exec record launches (memsets and NCCL calls are not ours).
 int own_kernels_of(const ExecOp& x) {
     const uint16_t k = x.kernel;
@@ -591,6 +633,16 @@ int replay(cai_exec* ex) {
             if (brc != 0) return brc;
         }
         if (ex->nvtx_on) nvtxRangePushA(kernel_label(ex->exec[op.exec - 1].kernel));
+        if (ex->with_next[i] && !tr && !ex->debug_bounds && ex->sm_limit_hi <= 0 && !ex->has_pending_gather) {
+            const cai_gemm_call a = gemm_call(ex, ex->exec[op.exec - 1]), b = gemm_call(ex, ex->exec[ex->ops[i + 1].exec - 1]);
+            const int rc = cai_gemm_bf16_two(&a, &b, st);
+            if (ex->nvtx_on) nvtxRangePop();
+            if (rc != 0) return rc;
+            int cols;
+            ex->launches += cai_gemm_bf16_two_launches(&a, &b, &cols);
+            ++i;
+            continue;
+        }
         const int rc = run_op(ex, op, ex->exec[op.exec - 1], st);
         if (ex->nvtx_on) nvtxRangePop();
         if (rc != 0) return rc;
@@ -661,6 +713,9 @@ CAI_API int cai_exec_create(cai_exec** out, const void* plan_bytes, size_t nbyte
         if (o.exec || o.kind == OP_EVENT_RECORD || o.kind == OP_EVENT_WAIT) ex->used[o.stream_id] = true;
     ex->arena = static_cast<uint8_t*>(arena_base);
     ex->device = current_device();
+    ex->with_next.assign(ex->ops.size() + 1, 0);
+    for (size_t i = 0; i + 1 < ex->ops.size(); ++i)
+        ex->with_next[i] = !(i > 0 && ex->with_next[i - 1]) && independent_products(ex, ex->ops[i], ex->ops[i + 1]);
     if (const char* dbg = getenv("CAI_DEBUG_BOUNDS")) ex->debug_bounds = *dbg && *dbg != '0';
     if (ex->train.wait_limit_ms) cai_set_wait_limit_us(ex->train.wait_limit_ms * 1000u);
     int lo_prio = 0, hi_prio = 0;

@@ -336,3 +336,26 @@ def test_engine_made_behind_work_of_the_callers_stream(side):
     assert float(eng.view("@flat_master").abs().sum()) > 0 and float(eng.view("@flat_m").abs().sum()) == 0
     assert eng.check_canaries()
     eng.close()
+
+
+# Traced, every record is its own launch; untraced (and captured in a graph), a layer's input and weight gradient go out together where that is faster.
+# The gradients are the same bits. Widths that give persistent tiles and clusters, tied embeddings, microbatches that accumulate.
+@pytest.mark.parametrize("extra", ["", "hidden_size = 1000\nffn_hidden = 2728\nseq_len = 640\nmicrobatch = 3\ntie_embeddings = 1\nvocab_size = 5000\n"])
+def test_gradient_pairs_give_the_bits_of_single_launches(extra):
+    from cai_b200.runtime.engine import Engine, synthetic_batch
+    eng = Engine(config_text=(ROOT / "configs" / "tiny.cfg").read_text() + "\n" + extra, rank=0, world=1, local_rank=0)
+    m = eng.model
+    eng.lr = 0.0
+    tok, tgt = synthetic_batch(m.vocab_size, m.seq_len, eng.hdr.num_microbatches * m.microbatch, step=0, seed=0)
+    grads, launches = [], []
+    for run in ("traced", "plain", "graph"):
+        if run == "traced":
+            eng.trace_step(tok, tgt)
+        else:
+            eng.L.cai_exec_use_graph(eng.ex, int(run == "graph"))
+            eng.step(tok, tgt)
+        launches.append(eng.launches_per_step)
+        grads.append(eng.view("@flat_grad").clone())
+    eng.close()
+    assert launches[1] < launches[0]
+    assert torch.equal(grads[0], grads[1]) and torch.equal(grads[0], grads[2])

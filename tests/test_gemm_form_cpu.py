@@ -92,3 +92,53 @@ def test_ragged_walk_covers_live_halves_once(groups, per, seg_rows, short, kind)
         halves = [len({h for h in want if h[0] == g and h[1] == 0}) for g in range(groups)]
         assert len(tiles) == 3 * sum((h + 1) // 2 for h in halves)            # no half-empty tile but the last of a group
         assert max(per_pair) - min(per_pair) <= 1
+
+
+def two_walk(n0, k0, n1, k1, cols, pairs):
+    per_pair = []
+    for pair in range(pairs):
+        ask_walk = lambda buf, n: _lib.lib().cai_gemm_bf16_two_walk(n0, k0, n1, k1, cols, pairs, pair, buf, n)
+        n = ask_walk(None, 0)
+        buf = (ctypes.c_int * (2 * max(n, 1)))()
+        assert ask_walk(buf, n) == n
+        per_pair.append([(buf[2 * i], buf[2 * i + 1]) for i in range(n)])
+    return per_pair
+
+
+# Two products in one launch: every tile once, the longer tiles of a pair first, and no pair done later than a list ordered by length allows
+# (the average and one tile of either kind). Tile counts around whole rounds of the pairs, none of the second, one of each, K from equal to 64 times.
+@pytest.mark.parametrize("pairs", [1, 2, 74])
+@pytest.mark.parametrize("k0,k1", [(512, 512), (4096, 512), (1000, 136), (8192, 128)])
+def test_two_products_walk(pairs, k0, k1):
+    for n0 in (1, 2, 32, 73, 74, 75, 148, 149, 500):
+        for n1 in (0, 1, 5, 73, 74, 88, 147, 1000):
+            if n0 + n1 < pairs:
+                continue
+            walks = two_walk(n0, k0, n1, k1, 256, pairs)
+            assert sorted(t for w in walks for t in w) == [(0, i) for i in range(n0)] + [(1, i) for i in range(n1)]
+            c = [(k + 127) // 128 * 1150.0 + 2500.0 for k in (k0, k1)]
+            load = [sum(c[which] for which, _ in w) for w in walks]
+            assert all(w == sorted(w) for w in walks)
+            assert max(load) <= (n0 * c[0] + n1 * c[1]) / pairs + c[0] + c[1]
+
+
+def gemm_call(M, N, K, epi=EPI_BF16):
+    return _lib.GemmCall(M=M, N=N, K=K, epi=epi, alpha=1.0)
+
+
+def two_launches(a, b):
+    cols = ctypes.c_int()
+    return _lib.lib().cai_gemm_bf16_two_launches(ctypes.byref(a), ctypes.byref(b), ctypes.byref(cols)), cols.value
+
+
+def test_two_products_launches():
+    assert two_launches(gemm_call(1920, 1000, 5456), gemm_call(5456, 1000, 1920)) == (1, 256)     # 32 and 88 tiles: waves fill up
+    assert two_launches(gemm_call(4096, 2048, 8192), gemm_call(8192, 2048, 4096))[0] == 2         # at the power limit
+    assert two_launches(gemm_call(3456, 1408, 2944), gemm_call(2944, 1408, 3456))[0] == 2         # as many waves as apart
+    assert two_launches(gemm_call(768, 848, 848), gemm_call(848, 848, 768)) == (1, 128)           # one wave of narrow tiles
+    assert two_launches(gemm_call(512, 256, 1024), gemm_call(1024, 256, 512)) == (1, 128)         # 4 clusters of four slices, 8 tiles of one sum
+    assert two_launches(gemm_call(256, 1920, 2048), gemm_call(768, 1408, 2048))[0] == 2           # 15 clusters of four slices, 33 tiles of two
+    assert two_launches(gemm_call(256, 1792, 2048), gemm_call(256, 512, 512)) == (1, 128)         # 14 and one more with four tiles of one sum
+    assert two_launches(gemm_call(256, 1792, 2048), gemm_call(256, 640, 512))[0] == 2
+    assert two_launches(gemm_call(512, 512, 512), gemm_call(512, 512, 512, EPI_SWIGLU))[0] == 2
+    assert two_launches(gemm_call(0, 512, 512), gemm_call(512, 512, 512))[0] == 1

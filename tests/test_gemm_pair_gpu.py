@@ -274,3 +274,49 @@ def test_full_slabs_cost_what_plain_rows_cost(groups, per, seg_rows):
         times[bool(ragged)].append(s.elapsed_time(e))
     # both run with 256-row tiles along the whole of K; the plain one in the form that its shape asks for
     assert sorted(times[True])[4] < 1.25 * sorted(times[False])[4]
+
+
+def _call(x, w, dy, dw=None, accumulate=False, residual=None):
+    """A linear layer's input gradient (dw None) or weight gradient, as a call and as a function that runs it by itself."""
+    from cai_b200 import ops
+    from cai_b200.ops import _lib
+    if dw is None:
+        out = torch.full_like(x, 3.0)
+        a, b, (M, K), N, ta, tb, epi = dy, w, dy.shape, w.shape[1], 0, 1, 3 if residual is not None else 0
+    else:
+        out = dw.clone()
+        a, b, (K, M), N, ta, tb, epi = dy, x, dy.shape, x.shape[1], 1, 1, 2 if accumulate else 1
+    call = _lib.GemmCall(A=a.data_ptr(), B=b.data_ptr(), C=out.data_ptr(), R=residual.data_ptr() if residual is not None else None, lda=a.stride(0),
+                         ldb=b.stride(0), ldc=out.stride(0), ldr=residual.stride(0) if residual is not None else 0, M=M, N=N, K=K, a_mn_major=ta,
+                         b_mn_major=tb, epi=epi, alpha=1.0)
+    alone = dw.clone() if dw is not None else torch.full_like(x, 3.0)
+    ops.gemm(a, b, trans_a=bool(ta), trans_b=bool(tb), out=alone, accumulate=bool(epi == 2), residual=residual)
+    return call, out, alone
+
+
+# Both gradients of a linear layer in one launch against one launch each, and in either order: the same bits. Tokens, in and out features: persistent
+# tiles of 256 and of 128 columns; clusters of four slices and of two, of forms that differ (one sum beside a split one, two slices beside four),
+# with pairs and clusters that are left without a tile; one row, ragged edges; three that stay two launches.
+@pytest.mark.parametrize("T,I,O,launches", [
+    (1920, 1000, 5456, 1), (700, 2200, 2000, 1), (768, 848, 848, 1), (512, 256, 512, 1), (1, 8, 8, 1), (512, 256, 1024, 1), (768, 256, 248, 1),
+    (130, 264, 2048, 1), (257, 136, 1000, 1), (4096, 128, 1024, 1), (1024, 512, 1024, 1), (512, 1024, 1024, 1),
+    (4096, 1024, 1024, 2), (2048, 256, 4096, 2), (333, 1024, 3000, 2)])
+@pytest.mark.parametrize("accumulate", [False, True])
+def test_two_products_same_bits(T, I, O, launches, accumulate):
+    import ctypes
+    from cai_b200 import ops
+    from cai_b200.ops import _lib
+    torch.manual_seed(3)
+    x, dy, w = (torch.randn(*s, device="cuda").to(torch.bfloat16) for s in ((T, I), (T, O), (O, I)))
+    dw = torch.randn(O, I, device="cuda")
+    res = torch.randn(T, I, device="cuda").to(torch.bfloat16) if accumulate else None
+    stream = torch.cuda.current_stream().cuda_stream
+    for order in (1, -1):
+        calls = [_call(x, w, dy, residual=res), _call(x, w, dy, dw, accumulate)][::order]
+        cols = ctypes.c_int()
+        a, b = (ctypes.byref(c[0]) for c in calls)
+        assert ops.lib().cai_gemm_bf16_two_launches(a, b, ctypes.byref(cols)) == launches, cols.value
+        assert ops.lib().cai_gemm_bf16_two(a, b, stream) == 0
+        assert ops.device_status() == 0
+        for _, out, alone in calls:
+            assert torch.equal(out, alone)
