@@ -242,18 +242,24 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
 // one-CTA kernel at 1240 cycles per k-block (512 of MMA) is several things of that size: operands arrive at 54 B / cycle (48 KB: 900 cycles; a CTA
 // of a pair takes in 32 KB), shared memory is read and written at 128 B / cycle (768), the one issuing thread spends two waits of 200 to
 // 300 cycles per block, and eight epilogue warps read 128 columns each behind four waits. Here two warps issue, one per TMEM buffer, each
-// paying its waits under the other's MMAs; sixteen epilogue warps (112 registers each: the launch's 96 and what the other warpgroup
-// gives up) take 64 columns each; scales come in eight k-blocks at a time. 1090 cycles per k-block are left, the round trip of MMA,
-// commit, TMEM read and hand-back over two buffers. 2000 x 4096 x 14336 145 -> 129 us, 2000 x 14336 x 4096 169 -> 150, 8192^3 717 -> 612.
+// paying its waits under the other's MMAs. What is left is the chain of the epilogue warps (wait, read, add, hand back; a satisfied wait or a read of shared
+// memory takes some 200 cycles beside the operand reads) and the round trip to the issuing warps. So: the MMAs of a k-block come in two halves of
+// 128 columns with barriers of their own, each read by four warps, 128 columns a thread (eight warps of 232 registers, the launch's 168 and what the
+// other warpgroup gives up; sixteen warps of 64 columns had 112 and spilled); two reads are in flight per wait; the next part is asked
+// for before the last additions, without blocking; scales come in eight k-blocks at a time and are read and multiplied four at a time. Cycles per
+// k-block, sixteen warps and whole k-blocks / now: 965 / 820 with two pairs at work, 1100 / 983 with 72. us, bursts of 50: 2000 x 4096 x 14336
+// 131 / 118, 9472 x 4096 x 4096 176 / 158 (one CTA per tile 145 for the former). Tried on top: a half per issuing warp (911 and 1075 cycles: four
+// waits per k-block instead of three), scales two at a time (872 and 1028), halves with sixteen warps (no change), additions in pairs
+// (fma.rn.f32x2; sixteen warps, 131 -> 145 us).
 namespace f8p {
 constexpr int kBM = 256, kBN = 256, kBK = 128;
 constexpr int kStages = 6;
 constexpr int kHalf = 128 * kBK;                   // bytes of A, or of B, a CTA brings in per stage
-constexpr int kEpiWarps = 16;
-constexpr int kThreads = 128 + kEpiWarps * 32;     // warp 0 TMA, warps 1-2 MMA, warp 3 scales, warps 4-19 epilogue
+constexpr int kEpiWarps = 8;
+constexpr int kThreads = 128 + kEpiWarps * 32;     // warp 0 TMA, warps 1-2 MMA, warp 3 scales, warps 4-11 epilogue
 constexpr int kScaleKb = 8;                        // k-blocks whose scales come in at a time
-constexpr int kScaleRow = 132;                     // 128 rows of A, padded: eight k-blocks of four rows fall on 32 banks
-constexpr int kScaleWords = kScaleKb * kScaleRow + 2 * kScaleKb;
+constexpr int kScaleRow = 12;                      // a row of A's eight scales, padded: eight rows' 16 bytes fall on 32 banks
+constexpr int kScaleWords = 128 * kScaleRow + 2 * kScaleKb;
 constexpr int kSmem = kStages * 2 * kHalf + 2 * kScaleWords * 4 + 512 + 1024;
 }  // namespace f8p
 
@@ -290,20 +296,20 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     uint64_t* bars = reinterpret_cast<uint64_t*>(scales + 2 * kScaleWords);
     uint64_t* full = bars;                         // [kStages] used in the even CTA: both CTAs' operands have landed
     uint64_t* empty = bars + kStages;              // [kStages] in each CTA
-    uint64_t* part_full = bars + 2 * kStages;      // [2] in each CTA: a k-block's partial product is in TMEM
-    uint64_t* sc_full = part_full + 2;             // [2] in each CTA
-    uint64_t* part_empty = sc_full + 2;            // [2] used in the even CTA: both CTAs' epilogue warps have read the partial product
-    uint64_t* sc_empty = part_empty + 2;           // [2] in each CTA
+    uint64_t* sc_full = bars + 2 * kStages;        // [2] in each CTA
+    uint64_t* part_full = sc_full + 2;             // [buffer][half] in each CTA: that half of a k-block's partial product is in TMEM
+    uint64_t* part_empty = part_full + 4;          // [buffer][half] used in the even CTA: both CTAs' epilogue warps have read it
+    uint64_t* sc_empty = part_empty + 4;           // [2] in each CTA
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sc_empty + 2);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();
     if (warp == 0) {
-        constexpr int kOne = 2 * kStages + 4;
-        if (lane < kOne) mbar_init(&bars[lane], 1);
-        else if (lane < kOne + 2) mbar_init(&bars[lane], 2 * kEpiWarps);
-        else if (lane < kOne + 4) mbar_init(&bars[lane], kEpiWarps);
+        constexpr int kParts = 2 * kStages + 6;    // full, empty, scales and parts that arrive
+        if (lane < kParts) mbar_init(&bars[lane], 1);
+        else if (lane < kParts + 4) mbar_init(&bars[lane], kEpiWarps);         // half of the warps of either CTA
+        else if (lane < kParts + 6) mbar_init(&bars[lane], kEpiWarps);
         if (lane == 31) *abort_flag = 0;
         mbar_fence_init();
     } else if (warp == 2 && lane == 0) {
@@ -332,8 +338,8 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     };
 
     if (warp < 4) {
-        // 24 + 4 x 112 registers a thread of each of the five warpgroups: within the 5 x 96 of the launch
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 24;");
+        // 40 + 2 x 232 registers a thread of each of the three warpgroups: the 3 x 168 of the launch
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
         if (warp == 0) {
             if (lane == 0) {
                 // ---------------- TMA producer (both CTAs)
@@ -375,26 +381,33 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
             if (rank == 0) {
                 // ---------------- MMA issuers (even CTA): warp 1 the even k-blocks into TMEM buffer 0, warp 2 the odd ones into buffer 1
                 const uint32_t buf = warp - 1;
-                const uint32_t idesc = umma_idesc_e4m3(kBM, kBN);
+                const uint32_t idesc = umma_idesc_e4m3(kBM, kBN / 2);
                 const uint64_t a_first = umma_smem_desc_sw128(smem_u32(sA), 0, 1024), b_first = umma_smem_desc_sw128(smem_u32(sB), 0, 1024);
                 const bool leader = elect_one();
                 const uint32_t total = static_cast<uint32_t>(num_kb) * static_cast<uint32_t>(first < num_tiles ? (num_tiles - first + stride - 1) / stride : 0);
                 uint32_t s = buf, ph = 0, n = 0;      // ring slot and its phase; k-blocks this warp has issued
                 bool ok = true;
-                for (uint32_t it = buf; it < total; it += 2, ++n) {
-                    if (!mbar_wait_warp(&full[s], ph, abort_flag, p.status, CAI_DEV_TIMEOUT_TMA_FULL) ||
-                        !mbar_wait_warp(&part_empty[buf], (n & 1) ^ 1, abort_flag, p.status, CAI_DEV_TIMEOUT_TMEM_EMPTY)) {
+                for (uint32_t it = buf; it < total && ok; it += 2, ++n) {
+                    if (!mbar_wait_warp(&full[s], ph, abort_flag, p.status, CAI_DEV_TIMEOUT_TMA_FULL)) {
                         ok = false;
                         break;
                     }
-                    tc_fence_after();
-                    if (leader) {
-                        const uint64_t ad = a_first + s * (kHalf >> 4), bd = b_first + s * (kHalf >> 4);
 #pragma unroll
-                        for (int k = 0; k < kBK / f8::kUmmaK; ++k)
-                            umma_f8_ss_pair(tmem_base + buf * kBN, ad + k * (f8::kUmmaK >> 4), bd + k * (f8::kUmmaK >> 4), idesc, k != 0 ? 1u : 0u);
-                        umma_commit_pair(&part_full[buf], 3);
-                        umma_commit_pair(&empty[s], 3);
+                    for (int half = 0; half < 2; ++half) {
+                        const uint32_t part = buf * 2 + half;
+                        if (!mbar_wait_warp(&part_empty[part], (n & 1) ^ 1, abort_flag, p.status, CAI_DEV_TIMEOUT_TMEM_EMPTY)) {
+                            ok = false;
+                            break;
+                        }
+                        tc_fence_after();
+                        if (leader) {
+                            const uint64_t ad = a_first + s * (kHalf >> 4), bd = b_first + s * (kHalf >> 4) + half * (kHalf >> 5);
+#pragma unroll
+                            for (int k = 0; k < kBK / f8::kUmmaK; ++k)
+                                umma_f8_ss_pair(tmem_base + part * (kBN / 2), ad + k * (f8::kUmmaK >> 4), bd + k * (f8::kUmmaK >> 4), idesc, k != 0 ? 1u : 0u);
+                            umma_commit_pair(&part_full[part], 3);
+                            if (half) umma_commit_pair(&empty[s], 3);
+                        }
                     }
                     s += 2;
                     if (s >= kStages) {
@@ -402,8 +415,9 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
                         ph ^= 1;
                     }
                 }
-                // the buffer handed back: no arrival of the odd CTA is still on its way when this one ends
-                if (ok) mbar_wait_warp(&part_empty[buf], (n & 1) ^ 1, abort_flag, p.status, CAI_DEV_TIMEOUT_TMEM_EMPTY);
+                // both parts handed back: no arrival of the odd CTA is still on its way when this one ends
+                for (int half = 0; half < 2 && ok; ++half)
+                    ok = mbar_wait_warp(&part_empty[buf * 2 + half], (n & 1) ^ 1, abort_flag, p.status, CAI_DEV_TIMEOUT_TMEM_EMPTY);
             }
         } else {
             // ---------------- scales of eight k-blocks at a time: lane l takes k-block l & 7 of rows l / 8, l / 8 + 4, ...
@@ -423,11 +437,11 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
                     if (kb < num_kb) {
 #pragma unroll 8
                         for (int i = 0; i < 32; ++i)
-                            cp_async4(dst + (lane & 7) * kScaleRow + (lane >> 3) + 4 * i,
+                            cp_async4(dst + ((lane >> 3) + 4 * i) * kScaleRow + (lane & 7),
                                       p.sa + static_cast<long long>(min(r0 + 4 * i, p.M - 1)) * num_kb + kb);
                         if (lane < 16) {
                             const int cb = min(tn * 2 + (lane >> 3), (p.N - 1) / 128);
-                            cp_async4(dst + kScaleKb * kScaleRow + lane, p.sb + static_cast<long long>(cb) * num_kb + kb);
+                            cp_async4(dst + 128 * kScaleRow + lane, p.sb + static_cast<long long>(cb) * num_kb + kb);
                         }
                     }
                     cp_async_wait_all();
@@ -438,82 +452,105 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
             }
         }
     } else {
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
-        // ---------------- epilogue warps: scale-and-add every k-block, then write the tile; 64 columns each
-        const int q = warp & 3, cg = (warp - 4) >> 2;
-        const uint32_t taddr0 = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + cg * 64;
-        const uint32_t release0 = map_to_cta(smem_u32(&part_empty[0]), 0);
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 232;");
+        // ---------------- epilogue warps: scale-and-add every k-block, then write the tile; 128 columns each.
+        // The MMA of a half takes 64 rows of B from either CTA: its 128 columns are 64 of the tile's first 128 and 64 of its second.
+        const int q = warp & 3, half = (warp - 4) >> 2;
+        const uint32_t taddr0 = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + half * (kBN / 2);
+        const uint32_t release0 = map_to_cta(smem_u32(&part_empty[half]), 0);
         uint32_t it = 0, sb = 0, sph = 0;
-        bool ok = true;
+        bool ok = true, ready = false;     // ready: the next part was seen in tensor memory
         for (int tile = first; tile < num_tiles && ok; tile += stride) {
-            float acc[64];
+            float acc[128];
 #pragma unroll
-            for (int e = 0; e < 64; ++e) acc[e] = 0.f;
-            for (int kb = 0; kb < num_kb; ++kb, ++it) {
-                const uint32_t buf = it & 1;
-                const int in = kb & (kScaleKb - 1);
-                if (in == 0 && !mbar_wait_warp(&sc_full[sb], sph, abort_flag, p.status, CAI_DEV_TIMEOUT_TMEM_FULL)) {
+            for (int e = 0; e < 128; ++e) acc[e] = 0.f;
+            for (int kb0 = 0; kb0 < num_kb && ok; kb0 += 4) {
+                const int at = kb0 & (kScaleKb - 1);
+                if (at == 0 && !mbar_wait_warp(&sc_full[sb], sph, abort_flag, p.status, CAI_DEV_TIMEOUT_TMEM_FULL)) {
                     ok = false;
                     break;
                 }
-                const float* sc = scales + sb * kScaleWords;
-                const float s = sc[in * kScaleRow + q * 32 + lane] * sc[kScaleKb * kScaleRow + (cg >> 1) * kScaleKb + in];
-                if (in == kScaleKb - 1 || kb == num_kb - 1) {
+                float s0[4], s1[4];
+                {
+                    const float* sc = scales + sb * kScaleWords;
+                    const float4 a = *reinterpret_cast<const float4*>(sc + (q * 32 + lane) * kScaleRow + at);
+                    const float4 b0 = *reinterpret_cast<const float4*>(sc + 128 * kScaleRow + at);
+                    const float4 b1 = *reinterpret_cast<const float4*>(sc + 128 * kScaleRow + kScaleKb + at);
+                    s0[0] = a.x * b0.x; s0[1] = a.y * b0.y; s0[2] = a.z * b0.z; s0[3] = a.w * b0.w;
+                    s1[0] = a.x * b1.x; s1[1] = a.y * b1.y; s1[2] = a.z * b1.z; s1[3] = a.w * b1.w;
+                }
+                if (at || kb0 + 4 >= num_kb) {
                     mbar_arrive_warp(&sc_empty[sb]);
                     sb ^= 1;
                     if (sb == 0) sph ^= 1;
                 }
-                if (!mbar_wait_warp(&part_full[buf], (it >> 1) & 1, abort_flag, p.status, CAI_DEV_TIMEOUT_TMEM_FULL)) {
-                    ok = false;
-                    break;
-                }
-                tc_fence_after();
 #pragma unroll
-                for (int c = 0; c < 2; ++c) {
-                    uint32_t r[32];
-                    tmem_ld_32x32(taddr0 + buf * kBN + c * 32, r);
-                    tmem_ld_wait();
-                    if (c == 1) {
-                        // read: the buffer goes back before the last additions
-                        tc_fence_before();
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive_cluster(release0 + buf * 8);
+                for (int i = 0; i < 4; ++i, ++it) {
+                    if (kb0 + i >= num_kb) break;
+                    const uint32_t buf = it & 1;
+                    if (!ready && !mbar_wait_warp(&part_full[buf * 2 + half], (it >> 1) & 1, abort_flag, p.status, CAI_DEV_TIMEOUT_TMEM_FULL)) {
+                        ok = false;
+                        break;
                     }
+                    tc_fence_after();
+                    uint32_t r0[32], r1[32];
+                    const uint32_t ta = taddr0 + buf * kBN;
+                    tmem_ld_32x32(ta, r0);
+                    tmem_ld_32x32(ta + 32, r1);
+                    tmem_ld_wait();
 #pragma unroll
-                    for (int e = 0; e < 32; ++e) acc[c * 32 + e] = fmaf(s, __uint_as_float(r[e]), acc[c * 32 + e]);
+                    for (int e = 0; e < 32; ++e) acc[e] = fmaf(s0[i], __uint_as_float(r0[e]), acc[e]);
+                    tmem_ld_32x32(ta + 64, r0);
+#pragma unroll
+                    for (int e = 0; e < 32; ++e) acc[32 + e] = fmaf(s0[i], __uint_as_float(r1[e]), acc[32 + e]);
+                    tmem_ld_32x32(ta + 96, r1);
+                    tmem_ld_wait();
+                    // read: the buffer goes back before the last additions, and the next part is asked for under them
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_cluster(release0 + buf * 16);
+                    const bool next = mbar_test_wait(&part_full[(buf ^ 1) * 2 + half], ((it + 1) >> 1) & 1);
+#pragma unroll
+                    for (int e = 0; e < 32; ++e) acc[64 + e] = fmaf(s1[i], __uint_as_float(r0[e]), acc[64 + e]);
+#pragma unroll
+                    for (int e = 0; e < 32; ++e) acc[96 + e] = fmaf(s1[i], __uint_as_float(r1[e]), acc[96 + e]);
+                    ready = __all_sync(0xffffffffu, next);
                 }
             }
             if (!ok) break;
             int tm, tn;
             coords(tile, tm, tn);
             const long long row = static_cast<long long>(tm) * kBM + rank * 128 + q * 32 + lane;
-            const int col0 = tn * kBN + cg * 64;
-            if (row >= p.M || col0 >= p.N) {
-                // nothing of this lane's is written
-            } else if (p.epi == CAI_EPI_F32) {
-                float* crow = reinterpret_cast<float*>(p.C) + row * p.ldc + col0;
 #pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    if (col0 + j * 4 >= p.N) break;
-                    *reinterpret_cast<float4*>(crow + j * 4) = make_float4(acc[j * 4], acc[j * 4 + 1], acc[j * 4 + 2], acc[j * 4 + 3]);
-                }
-            } else {
-                __nv_bfloat16* crow = reinterpret_cast<__nv_bfloat16*>(p.C) + row * p.ldc + col0;
-                const __nv_bfloat16* rrow =
-                    p.epi == CAI_EPI_BF16_RESIDUAL ? reinterpret_cast<const __nv_bfloat16*>(p.R) + row * p.ldr + col0 : nullptr;
+            for (int side = 0; side < 2; ++side) {
+                const int col0 = tn * kBN + side * 128 + half * 64;
+                if (row >= p.M || col0 >= p.N) continue;   // nothing of this lane's is written
+                if (p.epi == CAI_EPI_F32) {
+                    float* crow = reinterpret_cast<float*>(p.C) + row * p.ldc + col0;
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    if (col0 + j * 8 >= p.N) break;
-                    float v[8];
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) v[e] = acc[j * 8 + e];
-                    if (rrow) {
-                        float rf[8];
-                        unpack8(*reinterpret_cast<const uint4*>(rrow + j * 8), rf);
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) v[e] += rf[e];
+                    for (int j = 0; j < 16; ++j) {
+                        if (col0 + j * 4 >= p.N) break;
+                        const float* v = acc + side * 64 + j * 4;
+                        *reinterpret_cast<float4*>(crow + j * 4) = make_float4(v[0], v[1], v[2], v[3]);
                     }
-                    *reinterpret_cast<uint4*>(crow + j * 8) = pack8(v);
+                } else {
+                    __nv_bfloat16* crow = reinterpret_cast<__nv_bfloat16*>(p.C) + row * p.ldc + col0;
+                    const __nv_bfloat16* rrow =
+                        p.epi == CAI_EPI_BF16_RESIDUAL ? reinterpret_cast<const __nv_bfloat16*>(p.R) + row * p.ldr + col0 : nullptr;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        if (col0 + j * 8 >= p.N) break;
+                        float v[8];
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) v[e] = acc[side * 64 + j * 8 + e];
+                        if (rrow) {
+                            float rf[8];
+                            unpack8(*reinterpret_cast<const uint4*>(rrow + j * 8), rf);
+#pragma unroll
+                            for (int e = 0; e < 8; ++e) v[e] += rf[e];
+                        }
+                        *reinterpret_cast<uint4*>(crow + j * 8) = pack8(v);
+                    }
                 }
             }
             __syncwarp();

@@ -147,3 +147,21 @@ def test_one_cta_and_pair_forms_give_the_same_bits():
     both = ops.gemm_fp8(xq, sx, wq, sw, out_dtype=torch.float32)
     half = ops.gemm_fp8(xq[:128], sx[:128].contiguous(), wq, sw, out_dtype=torch.float32)
     assert torch.equal(both[:128], half)
+
+
+# k-blocks around the scales' groups of four and eight, odd and even (the TMEM buffer a tile starts in), more tiles than CTA pairs, ragged edges.
+@pytest.mark.parametrize("kb", [1, 2, 3, 4, 5, 7, 8, 9, 13, 17])
+@pytest.mark.parametrize("M,N", [(2304, 2304), (300, 1000)])
+def test_pair_form_k_blocks(M, N, kb):
+    from cai_b200 import ops
+    torch.manual_seed(kb)
+    x = torch.randn(M, kb * 128, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(N, kb * 128, device="cuda") * 0.05).to(torch.bfloat16)
+    (xq, sx), (wq, sw) = ops.quant_rows_1x128(x), ops.quant_blocks_128x128(w)
+    a, b = _dequant_rows(xq, sx).double(), _dequant_blocks(wq, sw).double()
+    out = ops.gemm_fp8(xq, sx, wq, sw, out_dtype=torch.float32)
+    # products of e4m3 are exact in fp32; K sums and a scaling per k-block, each off by at most 2^-24 of what it adds up to (the tensor
+    # core's sums within a k-block may be truncated to 2^-13 of their largest term, as they are in every product of this format)
+    bound = (2.0 ** -13 + (128 + 3 * kb) * 2.0 ** -24) * (a.abs() @ b.abs().t()) + 1e-9
+    assert ((out.double() - a @ b.t()).abs() <= bound).all()
+    assert ops.device_status() == 0
