@@ -85,11 +85,12 @@ __host__ __device__ __forceinline__ bool pair_half_live(const PairParams& p, int
 // (a stage lies in one slab). A step costs no division, and a count is read once per slab; asking for both blocks of every
 // stage whether they are live (two divisions and two reads) kept the issuing thread some 350 cycles per stage, dead ones included.
 // 64 products of 4096 x 1536, and of 3072 x 4096, over some 1024 of 2048 rows each: 1246 -> 881 and 2477 -> 1773 us.
+template <bool kRagged>
 struct PairStages {
     const int* counts;
     int slab_rows, slabs, slab = -1, base = 0, rows = 0, at = 0;   // at: element of the next stage inside the slab
     __device__ __forceinline__ PairStages(const PairParams& p, int g) {
-        const bool ragged = p.seg_mode == 2;
+        const bool ragged = kRagged && p.seg_mode == 2;
         counts = ragged ? p.seg_counts + g * p.grp_seg : nullptr;
         slab_rows = ragged ? p.seg_rows : p.K;
         slabs = ragged ? (p.K + p.seg_rows - 1) / p.seg_rows : 1;
@@ -100,7 +101,7 @@ struct PairStages {
             if (++slab >= slabs) return false;
             base = slab * slab_rows;
             rows = min(slab_rows, p.K - base);
-            if (counts) rows = min(rows, counts[slab]);
+            if (kRagged && counts) rows = min(rows, counts[slab]);
             at = 0;
         }
         ks = (base + at) / (pair::kPerStage * pair::kBK);
@@ -192,15 +193,23 @@ struct PairTwoTiles {
         return tile < tiles1;
     }
 };
-template <int kProducts> struct PairWalk {
+template <int kProducts, bool kRagged> struct PairWalk {
     PairTiles tiles;
     __device__ __forceinline__ PairWalk(int pair, int pairs) : tiles(pair, pairs) {}
     __device__ __forceinline__ bool next(const PairLaunch<1>& l, const int* first, int rank, int& row, int& tn, int& grp, bool& live, int& which) {
         which = 0;
-        return tiles.next(l.product[0].p, first, rank, row, tn, grp, live);
+        const PairParams& p = l.product[0].p;
+        if (kRagged) return tiles.next(p, first, rank, row, tn, grp, live);
+        if (tiles.tile >= p.tiles_m * p.tiles_n * p.groups) return false;
+        int tm;
+        pair_tile_coords(p, tiles.tile, tm, tn, grp);
+        tiles.tile += tiles.stride;
+        row = tm * pair::kBM + rank * 128;
+        live = row < p.M;
+        return true;
     }
 };
-template <> struct PairWalk<2> {
+template <> struct PairWalk<2, false> {
     PairTwoTiles tiles;
     __device__ __forceinline__ PairWalk(int pair, int pairs) : tiles(pair, pairs) {}
     __device__ __forceinline__ bool next(const PairLaunch<2>& l, const int*, int rank, int& row, int& tn, int& grp, bool& live, int& which) {
@@ -336,7 +345,12 @@ struct PairMma {
     }
 };
 
-template <int BN, int kProducts>
+// What a kernel's epilogue can do. One kernel with every epilogue and both walks spilled registers and is so long that short products wait for
+// its instructions. us, one kernel / one for each kind, plain and ragged: a step of 49 launches 325 / 308, one of 189 launches 4150 / 4000, the expert half of
+// a layer on 4068 tokens, 32 experts, 256 x 1152, 148 / 139.
+enum PairKind { kPairBf16, kPairF32, kPairSwiglu, kPairAny };   // kPairAny: bf16 and fp32, of two products
+
+template <int BN, int kProducts, PairKind kKind, bool kRagged>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair::kThreads, 1)
 gemm_pair_kernel(const __grid_constant__ PairLaunch<kProducts> launch) {
     using namespace pair;
@@ -382,11 +396,11 @@ gemm_pair_kernel(const __grid_constant__ PairLaunch<kProducts> launch) {
     grid_dep_wait();
     const uint32_t tmem_base = *tmem_slot;
 
-    if (kProducts == 1 && shared.grp_slabs) {
+    if (kRagged && shared.grp_slabs) {
         if (warp == 3) pair_count_halves(shared, first, lane);
         __syncthreads();
     }
-    PairWalk<kProducts> tiles(static_cast<int>(blockIdx.x >> 1), static_cast<int>(gridDim.x >> 1));
+    PairWalk<kProducts, kRagged> tiles(static_cast<int>(blockIdx.x >> 1), static_cast<int>(gridDim.x >> 1));
     int row_half, tn, grp, which; // row_half: first row of this CTA's half of a tile
     bool mine;                   // that half is live
 
@@ -400,8 +414,8 @@ gemm_pair_kernel(const __grid_constant__ PairLaunch<kProducts> launch) {
                 const PairProduct& product = launch.product[kProducts > 1 ? which : 0];
                 const PairParams& p = product.p;
                 // SwiGLU: the even CTA brings the gate rows of the weight, the odd one the up rows of the same features
-                const int n0 = kProducts == 1 && p.epi == CAI_EPI_SWIGLU ? tn * HALF + static_cast<int>(rank) * (p.N >> 1) : tn * BN + static_cast<int>(rank) * HALF;
-                PairStages stages(p, grp);
+                const int n0 = kKind == kPairSwiglu ? tn * HALF + static_cast<int>(rank) * (p.N >> 1) : tn * BN + static_cast<int>(rank) * HALF;
+                PairStages<kRagged> stages(p, grp);
                 int ks;
                 uint32_t live;
                 while (stages.next(p, ks, live)) {
@@ -455,7 +469,7 @@ gemm_pair_kernel(const __grid_constant__ PairLaunch<kProducts> launch) {
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + acc * BN;
                 uint32_t started = 0;   // 0 for the first MMA of a tile, which overwrites the accumulator
-                PairStages stages(p, grp);
+                PairStages<kRagged> stages(p, grp);
                 int ks;
                 uint32_t live;
                 while (stages.next(p, ks, live)) {
@@ -497,8 +511,8 @@ gemm_pair_kernel(const __grid_constant__ PairLaunch<kProducts> launch) {
             ++t;
             // a weight-gradient tile whose every k-block was skipped has an undefined accumulator: it counts as zero
             bool acc_valid = true;
-            if (kProducts == 1 && p.seg_mode == 2) {
-                PairStages stages(p, grp);
+            if (kRagged && p.seg_mode == 2) {
+                PairStages<kRagged> stages(p, grp);
                 int ks;
                 uint32_t any;
                 acc_valid = stages.next(p, ks, any);
@@ -506,7 +520,7 @@ gemm_pair_kernel(const __grid_constant__ PairLaunch<kProducts> launch) {
             const int row0 = row_half + q * 32;
             const bool live = mine && row0 < p.M;
             const int col_first = tn * BN + half * HALF;
-            const bool residual = p.epi == CAI_EPI_BF16_RESIDUAL;
+            const bool residual = (kKind == kPairBf16 || kKind == kPairAny) && p.epi == CAI_EPI_BF16_RESIDUAL;
             // this lane's row of the residual: the first 64 columns come in while the main loop runs
             const bool res_ok = residual && mine && row0 + lane < p.M;
             const __nv_bfloat16* rrow = p.R + (static_cast<long long>(grp) * p.grp_c + row0 + lane) * p.ldr;
@@ -524,7 +538,7 @@ gemm_pair_kernel(const __grid_constant__ PairLaunch<kProducts> launch) {
             tc_fence_after();
             const uint32_t tacc = tmem_base + lane_bits + acc * BN;
             if (live) {
-                if (kProducts == 1 && p.epi == CAI_EPI_SWIGLU) {
+                if constexpr (kKind == kPairSwiglu) {
                     // columns [0, HALF) are gate, [HALF, BN) up, of features tn * HALF ...; this warp's share is HALF / 2 of each
                     const int F = p.N >> 1;
 #pragma unroll 1
@@ -566,7 +580,7 @@ gemm_pair_kernel(const __grid_constant__ PairLaunch<kProducts> launch) {
                             }
                         }
                     }
-                } else if (p.epi == CAI_EPI_BF16 || residual) {
+                } else if (kKind == kPairBf16 || (kKind == kPairAny && (p.epi == CAI_EPI_BF16 || residual))) {
 #pragma unroll 1
                     for (int c = 0; c < HALF; c += 64) {
                         const int col = col_first + c;
@@ -575,7 +589,7 @@ gemm_pair_kernel(const __grid_constant__ PairLaunch<kProducts> launch) {
                         tmem_ld_32x32(tacc + half * HALF + c, r[0]);
                         tmem_ld_32x32(tacc + half * HALF + c + 32, r[1]);
                         tmem_ld_wait();
-                        if (!acc_valid) {
+                        if (kRagged && !acc_valid) {
 #pragma unroll
                             for (int e = 0; e < 32; ++e) r[0][e] = r[1][e] = 0u;
                         }
@@ -619,7 +633,7 @@ gemm_pair_kernel(const __grid_constant__ PairLaunch<kProducts> launch) {
                         for (int k = 0; k < 8; ++k) {
                             uint32_t v[4];
 #pragma unroll
-                            for (int e = 0; e < 4; ++e) v[e] = acc_valid ? __float_as_uint(__uint_as_float(r[4 * k + e]) * p.alpha) : 0u;
+                            for (int e = 0; e < 4; ++e) v[e] = !kRagged || acc_valid ? __float_as_uint(__uint_as_float(r[4 * k + e]) * p.alpha) : 0u;
                             st_shared_v4(box_row + ((k ^ sw) << 4), v[0], v[1], v[2], v[3]);
                         }
                         fence_proxy_async_smem();
@@ -939,17 +953,17 @@ static bool pair_product(PairProduct& q, const void* A, const void* B, const Gem
     return ok;
 }
 
-template <int BN, int kProducts>
+template <int BN, int kProducts, PairKind kKind, bool kRagged>
 static int launch_pair(const PairLaunch<kProducts>& l, int pairs, cudaStream_t st) {
     static bool configured[64] = {};
     const int dev = current_device();
     if (!configured[dev & 63]) {
-        if (!allow_smem(gemm_pair_kernel<BN, kProducts>, pair::kSmem<BN>, "gemm_pair")) return CAI_K_CUDA;
+        if (!allow_smem(gemm_pair_kernel<BN, kProducts, kKind, kRagged>, pair::kSmem<BN>, "gemm_pair")) return CAI_K_CUDA;
         configured[dev & 63] = true;
     }
     const int grid = 2 * pairs;
-    if (l.product[0].p.overlap) launch_early(gemm_pair_kernel<BN, kProducts>, grid, pair::kThreads, pair::kSmem<BN>, st, l);
-    else gemm_pair_kernel<BN, kProducts><<<grid, pair::kThreads, pair::kSmem<BN>, st>>>(l);
+    if (l.product[0].p.overlap) launch_early(gemm_pair_kernel<BN, kProducts, kKind, kRagged>, grid, pair::kThreads, pair::kSmem<BN>, st, l);
+    else gemm_pair_kernel<BN, kProducts, kKind, kRagged><<<grid, pair::kThreads, pair::kSmem<BN>, st>>>(l);
     return launched(cudaGetLastError(), "gemm_pair");
 }
 template <int BN>
@@ -957,7 +971,13 @@ static int launch_one(const void* A, const void* B, const GemmShape& g, const Pa
     PairLaunch<1> l = {};
     if (!pair_product<BN>(l.product[0], A, B, g, p)) return CAI_K_BAD_ARG;
     const int tiles = l.product[0].p.tiles_m * l.product[0].p.tiles_n * p.groups;
-    return launch_pair<BN, 1>(l, tiles < pairs ? tiles : pairs, st);
+    const int at_once = tiles < pairs ? tiles : pairs;
+    if constexpr (BN == 256)                        // the only form that has it
+        if (p.epi == CAI_EPI_SWIGLU)
+            return p.seg_mode ? launch_pair<BN, 1, kPairSwiglu, true>(l, at_once, st) : launch_pair<BN, 1, kPairSwiglu, false>(l, at_once, st);
+    if (p.epi == CAI_EPI_F32 || p.epi == CAI_EPI_F32_ACCUM)
+        return p.seg_mode ? launch_pair<BN, 1, kPairF32, true>(l, at_once, st) : launch_pair<BN, 1, kPairF32, false>(l, at_once, st);
+    return p.seg_mode ? launch_pair<BN, 1, kPairBf16, true>(l, at_once, st) : launch_pair<BN, 1, kPairBf16, false>(l, at_once, st);
 }
 
 // Which form: the smallest estimate in SM cycles on a B200 of 74 pairs. A stage of 128 k-elements takes a CTA about 1150 cycles in the
@@ -1126,7 +1146,7 @@ static int launch_two(const void* const (&A)[2], const void* const (&B)[2], cons
     }
     const long long most = sms / 2 > 0 ? sms / 2 : 1, pairs = n[0] + n[1] < most ? n[0] + n[1] : most;
     pair_two_schedule(n[0], pair_tile_cycles(g[0]->K, BN), n[1], pair_tile_cycles(g[1]->K, BN), pairs, &l.heavier, &l.more_first);
-    return launch_pair<BN, 2>(l, static_cast<int>(pairs), st);
+    return launch_pair<BN, 2, kPairAny, false>(l, static_cast<int>(pairs), st);
 }
 template <int S>
 static int split_two(const void* const (&A)[2], const void* const (&B)[2], const GemmShape* const (&g)[2], const int (&slices)[2], int dev, cudaStream_t st) {
