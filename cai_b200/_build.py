@@ -13,6 +13,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -86,6 +87,7 @@ def build_kernels(verbose=False, ptxas_info=False) -> Path:
     lib = LIBDIR / "libcai_kernels.so"
     if jobs or _newer(lib, objs):
         _run([NVCC, "-shared", "-o", lib] + objs + ["-cudart", "static", "-ldl", "-lpthread"], verbose)
+    build_calls(verbose)
     # stand-alone CUDA tools (measurement programs that need no Python): bin/<name>
     BINDIR.mkdir(parents=True, exist_ok=True)
     for t in sorted((CSRC / "tools").glob("*.cu")):
@@ -93,6 +95,20 @@ def build_kernels(verbose=False, ptxas_info=False) -> Path:
         if _newer(exe, [t] + headers):
             _run([NVCC] + NVCC_FLAGS + [t, "-o", exe, "-cudart", "static", "-lcuda"], verbose)
     return lib
+
+
+def build_calls(verbose=False):
+    """The launchers as a Python extension (lib/_calls.<abi>.so), for the ops' host path. Without Python's headers there is none, and the ops go
+    through ctypes to the same launchers."""
+    include = Path(sysconfig.get_paths()["include"])
+    src, out = CSRC / "python" / "calls.cc", LIBDIR / ("_calls" + sysconfig.get_config_var("EXT_SUFFIX"))
+    if not (include / "Python.h").exists():
+        return None
+    if _newer(out, [src, CSRC / "kernels" / "cai_kernels.h", CSRC / "comm" / "moe.h"]):
+        cuda = Path(NVCC).resolve().parent.parent / "include"
+        _run([CXX] + CXX_FLAGS + ["-fvisibility=hidden", "-shared", "-I", include, "-I", cuda, src, "-o", out, "-L", LIBDIR, "-lcai_kernels",
+              "-Wl,-rpath,$ORIGIN"], verbose)
+    return out
 
 
 def build_host(verbose=False) -> Path:

@@ -7,11 +7,15 @@ to PyTorch ops: on a GPU box the CUDA path is the only path.
 from __future__ import annotations
 
 import ctypes
+import importlib.machinery
+import importlib.util
+import sysconfig
 from ctypes import c_char_p, c_float, c_int, c_longlong, c_void_p
 from pathlib import Path
 
 _LIB_PATH = Path(__file__).resolve().parent.parent / "lib" / "libcai_kernels.so"
 _lib = None
+_calls = None
 
 
 class GemmCall(ctypes.Structure):
@@ -33,6 +37,24 @@ def lib() -> ctypes.CDLL:
         _lib = ctypes.CDLL(str(_LIB_PATH), mode=ctypes.RTLD_GLOBAL)
         _declare(_lib)
     return _lib
+
+
+def calls():
+    """The launchers the ops use: the extension built next to the library, or, where there was no Python header to build it with (or another
+    Python runs), the ctypes functions of the same names."""
+    global _calls
+    if _calls is None:
+        _calls = lib()
+        path = _LIB_PATH.with_name("_calls" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
+        if path.exists():
+            loader = importlib.machinery.ExtensionFileLoader("_calls", str(path))
+            try:
+                module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_calls", loader))
+                loader.exec_module(module)
+                _calls = module
+            except ImportError:
+                pass
+    return _calls
 
 
 def _declare(L):

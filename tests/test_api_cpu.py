@@ -57,3 +57,26 @@ def test_log_level_from_the_environment_and_the_api(tmp_path):
     assert "[cai INFO]" not in run(env_level="0")
     assert "[cai INFO] plan loaded" in run(env_level="warn", arg="info")
     assert "[cai INFO]" not in run(arg="error")
+
+
+def test_launchers_of_the_extension_are_those_of_the_library():
+    """The extension the ops call through against ctypes: same results and errors for calls that need no GPU, arguments taken alike."""
+    import pytest
+    from cai_b200.ops import _lib
+    if not _lib._LIB_PATH.exists():
+        pytest.skip("kernel library not built")
+    fast, slow = _lib.calls(), _lib.lib()
+    for rows in (1, 100, 5000, True):
+        assert fast.cai_rmsnorm_bwd_parts(rows) == slow.cai_rmsnorm_bwd_parts(rows)
+    bad = (None, 0, 16, None, 16, 12, 16, 16, 16, 16, 0, 0, False, 0, 1, 0, None)     # N not a multiple of 8; null pointers, an integer for a float
+    assert fast.cai_gemm_bf16(*bad) == slow.cai_gemm_bf16(*bad) < 0
+    assert b"multiples of 8" in slow.cai_last_error()
+    empty = (0, 0, 0, 0, -1, 16, 16, 1 << 40, 16, 16, 0, 0, 0, 0, 1.0, 0, 0)          # nothing to do
+    assert fast.cai_gemm_bf16(*empty) == slow.cai_gemm_bf16(*empty) == 0
+    with pytest.raises(TypeError):
+        fast.cai_gemm_bf16(*bad[:-1])
+    if fast is not slow:
+        with pytest.raises(TypeError):
+            fast.cai_gemm_bf16("x", *bad[1:])
+        with pytest.raises(TypeError):
+            fast.cai_gemm_bf16(*bad[:4], 1.5, *bad[5:])
