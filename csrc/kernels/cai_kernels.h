@@ -69,6 +69,13 @@ CAI_API int cai_gemm_bf16_two_launches(const cai_gemm_call* first, const cai_gem
  * (product, tile). Returns their number, of which `capacity` are written. Needs no GPU. */
 CAI_API int cai_gemm_bf16_two_walk(int n0, int k0, int n1, int k1, int tile_cols, int pairs, int pair, int* tiles, int capacity);
 
+/* The gate / up projection with SwiGLU (CAI_EPI_SWIGLU, B stored [2F, K]) for any F that is a multiple of 8: gu[M, 2F] (pitch ldc) and
+ * act[M, F] (pitch ldr). The results are those of the product and cai_swiglu_fwd where the product is one sum along K; cai_gemm_bf16_swiglu_pays:
+ * whether it is, and the one launch is estimated to be faster (needs no GPU). */
+CAI_API int cai_gemm_bf16_swiglu(const void* A, const void* B, void* gu, void* act, int M, int F, int K, long long lda, long long ldb,
+                                 long long ldc, long long ldr, void* stream);
+CAI_API int cai_gemm_bf16_swiglu_pays(int M, int F, int K);
+
 /* The form such a product runs in: columns of its 256-row tiles, and how many slices of K are summed (1: one sum along K). It follows
  * from the arguments alone, so the order of summation is the same on every GPU. ctas: the most CTAs of one launch on `sms` SMs under sm_limit.
  * Needs no GPU. Not for CAI_EPI_SWIGLU_BWD. */

@@ -575,7 +575,7 @@ gemm_pair_kernel(const __grid_constant__ PairLaunch<kProducts> launch) {
                             __syncwarp();
                             if (lane == 0) {
                                 if (o == 2) tma_store_3d(&tmR, box, j, row0, grp);
-                                else tma_store_3d(&tmC, box, o == 0 ? j : F + j, row0, grp);
+                                else tma_store_3d(&tmC, box, j, o, row0);   // gate, up: the halves of a row
                                 tma_store_commit();
                             }
                         }
@@ -947,9 +947,12 @@ static bool pair_product(PairProduct& q, const void* A, const void* B, const Gem
     pair_tiles(q.p, BN);
     bool ok = pair_operand_maps(&q.map[0], &q.map[1], A, B, g, BN);
     const bool f32 = p.epi == CAI_EPI_F32 || p.epi == CAI_EPI_F32_ACCUM;
+    if (p.epi == CAI_EPI_SWIGLU)
+        // a row of C as its gate half and its up half, so that a box of either ends with it: F need not be a multiple of a tile
+        return ok && encode_tmap_3d(&q.map[2], g.C, p.N / 2, 2, p.M, p.N / 2, g.ldc, 64, 1, 2, 32) &&
+               pair_map(&q.map[3], g, g.R, p.M, p.N / 2, g.ldr, g.grp_c, 64, 32, 2);
     ok = ok && pair_map(&q.map[2], g, g.C, p.M, p.N, g.ldc, g.grp_c, f32 ? 32 : 64, 32, f32 ? 4 : 2);
     q.map[3] = q.map[2];
-    if (ok && p.epi == CAI_EPI_SWIGLU) ok = pair_map(&q.map[3], g, g.R, p.M, p.N / 2, g.ldr, g.grp_c, 64, 32, 2);
     return ok;
 }
 
@@ -1218,6 +1221,16 @@ CAI_API int cai_gemm_bf16_ragged_walk(int M, int N, int groups, const int* seg_c
             t[0] = grp[0]; t[1] = tn[0]; t[2] = row[0]; t[3] = row[1]; t[4] = live[0]; t[5] = live[1];
         }
     }
+}
+
+CAI_API int cai_gemm_bf16_swiglu_pays(int M, int F, int K) {
+    if (M <= 0 || F <= 0 || K <= 0 || (F & 7) || F > (1 << 29)) return 0;
+    const PairForm f = pair_form(M, 2 * F, K, 1, CAI_EPI_BF16, false);
+    if (f.slices > 1) return 0;                     // the sums would be others
+    auto cycles = [&](int cols) { return static_cast<double>((pair_tile_count(M, 2 * F, cols) + kFormPairs - 1) / kFormPairs) * pair_tile_cycles(K, cols); };
+    // against the plain product: the exponentials of the last tile; a launch less, and gu and act not carried once more (three words of a feature at
+    // 3.4 KB a cycle)
+    return cycles(256) + 2000.0 <= cycles(f.tile_cols) + 4000.0 + 6.0 / 3400.0 * M * F;
 }
 
 CAI_API int cai_gemm_bf16_two_walk(int n0, int k0, int n1, int k1, int tile_cols, int pairs, int pair, int* tiles, int capacity) {

@@ -932,6 +932,17 @@ CAI_API int cai_gemm_bf16_seg(const void* A, const void* B, void* C, const void*
     return gemm_dispatch(A, B, lda, ldb, p, sm_limit, reinterpret_cast<cudaStream_t>(stream));
 }
 
+CAI_API int cai_gemm_bf16_swiglu(const void* A, const void* B, void* gu, void* act, int M, int F, int K, long long lda, long long ldb,
+                                 long long ldc, long long ldr, void* stream) {
+    if (M <= 0 || F <= 0 || K <= 0) return CAI_K_OK;
+    if ((F & 7) || F > (1 << 29) || (lda & 7) || (ldb & 7) || (ldc & 7) || (ldr & 7) || !act) {
+        set_last_error("gemm_swiglu: F, lda, ldb, ldc and ldr must be multiples of 8 (F=%d lda=%lld ldb=%lld ldc=%lld ldr=%lld)", F, lda, ldb, ldc, ldr);
+        return CAI_K_BAD_ARG;
+    }
+    const GemmShape g = {M, 2 * F, K, 0, 0, CAI_EPI_SWIGLU, 1.f, gu, act, lda, ldb, ldc, ldr, nullptr, 0, 0, 0, 1, 0, 0, 0, 0};
+    return gemm_pair(A, B, g, reinterpret_cast<cudaStream_t>(stream));
+}
+
 static GemmShape shape_of(const cai_gemm_call& c) {
     return {c.M, c.N, c.K, c.a_mn_major ? 1 : 0, c.b_mn_major ? 1 : 0, c.epi, c.alpha, c.C, c.R, c.lda, c.ldb, c.ldc, c.ldr,
             nullptr, 0, 0, 0, 1, 0, 0, 0, 0};

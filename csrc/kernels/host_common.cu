@@ -101,7 +101,7 @@ bool encode_tmap_2d(CUtensorMap* out, const void* base, uint64_t rows, uint64_t 
 
 bool encode_tmap_3d(CUtensorMap* out, const void* base, uint64_t cols, uint64_t rows, uint64_t batch,
                     uint64_t ld_row, uint64_t ld_batch, uint32_t box_cols, uint32_t box_rows,
-                    int elem_bytes) {
+                    int elem_bytes, uint32_t box_batch) {
     auto fn = encode_fn();
     if (!fn) {
         set_last_error("cuTensorMapEncodeTiled entry point unavailable");
@@ -110,7 +110,7 @@ bool encode_tmap_3d(CUtensorMap* out, const void* base, uint64_t cols, uint64_t 
     cuuint64_t gdim[3] = {cols, rows, batch};
     cuuint64_t gstr[2] = {ld_row * static_cast<uint64_t>(elem_bytes),
                           ld_batch * static_cast<uint64_t>(elem_bytes)};
-    cuuint32_t box[3] = {box_cols, box_rows, 1};
+    cuuint32_t box[3] = {box_cols, box_rows, box_batch};
     cuuint32_t estr[3] = {1, 1, 1};
     CUresult r = fn(out, dtype_of(elem_bytes), 3, const_cast<void*>(base), gdim, gstr, box, estr,
                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,

@@ -32,7 +32,7 @@ bool encode_tmap_2d(CUtensorMap* out, const void* base, uint64_t rows, uint64_t 
 // 3-D variant: dims (cols, rows, batch) with pitches in elements.
 bool encode_tmap_3d(CUtensorMap* out, const void* base, uint64_t cols, uint64_t rows, uint64_t batch,
                     uint64_t ld_row, uint64_t ld_batch, uint32_t box_cols, uint32_t box_rows,
-                    int elem_bytes);
+                    int elem_bytes, uint32_t box_batch = 1);
 
 // Launch a kernel so that it may start while the kernel before it in the stream still runs (grid_dep_wait in sm100.cuh holds
 // it back from the data): what the chains of short kernels of a small step or layer wait for is the launch of each, the set-up of its

@@ -19,6 +19,7 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <algorithm>
 #include <string>
 #include <vector>
 
@@ -177,7 +178,9 @@ struct cai_exec {
     cai_fused_hook_t fused_hook = nullptr;
     void* fused_ctx = nullptr;
     int sm_limit_hi = 0;
-    std::vector<uint8_t> with_next;   // per op: a product that goes out together with the one behind it
+    enum : uint8_t { kAlone, kPairOfProducts, kWithSwiglu };
+    std::vector<uint8_t> with_next;   // per op: whether, and how, it goes out together with the one behind it
+    std::vector<uint8_t> unread;      // per op: a product whose result nothing reads; a traced or checked replay runs it all the same
     uint64_t launches = 0;  // kernels / collectives enqueued by the last replay
     // ZeRO-3: a parameter gather waiting to be merged into the GEMM that follows it in the op table
     GatherJob pending_gather{};
@@ -576,6 +579,48 @@ bool independent_products(const cai_exec* ex, const Op& o0, const Op& o1) {
     return true;
 }
 
+// Whether two records next to each other on one stream are a gate / up projection and the SwiGLU of its result, of a width that the plan compiler leaves
+// apart (F no multiple of 128), and one product with SwiGLU in its epilogue is the faster way.
+bool projection_with_swiglu(const cai_exec* ex, const Op& o0, const Op& o1) {
+    if (!ex->train.fuse_swiglu || !o0.exec || !o1.exec || o0.stream_id != o1.stream_id) return false;
+    if (o0.kind == OP_EVENT_RECORD || o0.kind == OP_EVENT_WAIT || o1.kind == OP_EVENT_RECORD || o1.kind == OP_EVENT_WAIT) return false;
+    const ExecOp &x = ex->exec[o0.exec - 1], &y = ex->exec[o1.exec - 1];
+    if (x.kernel != K_GEMM || y.kernel != K_SWIGLU_FWD || (x.flags & 0x100) || x.t[4] >= 0) return false;
+    const cai_gemm_call c = gemm_call(ex, x);
+    if (c.epi != CAI_EPI_BF16 || c.a_mn_major || c.b_mn_major || c.alpha != 1.f) return false;
+    return ex->ptr(y.t[0]) == c.C && y.i[0] == c.M && 2 * y.i[1] == c.N && c.ldc == c.N && ex->ld(y.t[1]) == y.i[1] && y.i[1] % 128 != 0 &&
+           cai_gemm_bf16_swiglu_pays(c.M, y.i[1], c.K);
+}
+
+// Products whose results no record of the plan reads: with activation recompute, the down projection of a layer that is run again for its
+// backward. Of everything that any record names, only outputs of such products may lie in the bytes of a result for it to count as unread, and no
+// tensor that the plan gives a name to.
+void find_unread(const cai_exec* ex, std::vector<uint8_t>* unread) {
+    unread->assign(ex->ops.size() + 1, 0);
+    auto product = [](const ExecOp& x) {
+        const int epi = (x.flags >> 4) & 0xF;
+        return x.kernel == K_GEMM && !(x.flags & 0x100) && x.t[4] < 0 && (epi == CAI_EPI_BF16 || epi == CAI_EPI_BF16_RESIDUAL);
+    };
+    struct Range { uint64_t lo, hi; };
+    std::vector<Range> used, results;
+    auto range = [&](int t) { return Range{ex->tensors[t].offset, ex->tensors[t].offset + ex->tensors[t].nbytes}; };
+    for (const NamedTensor& n : ex->named)
+        for (const int t : {n.tensor, n.grad})
+            if (t >= 0 && static_cast<size_t>(t) < ex->tensors.size()) used.push_back(range(t));
+    for (const ExecOp& x : ex->exec)
+        for (int k = 0; k < static_cast<int>(sizeof x.t / sizeof x.t[0]); ++k)
+            if (x.t[k] >= 0 && static_cast<size_t>(x.t[k]) < ex->tensors.size() && !(k == 2 && product(x))) used.push_back(range(x.t[k]));
+    std::sort(used.begin(), used.end(), [](const Range& a, const Range& b) { return a.lo < b.lo; });
+    std::vector<uint64_t> reach(used.size());      // the furthest end of the ranges up to this one
+    for (size_t i = 0; i < used.size(); ++i) reach[i] = i && reach[i - 1] > used[i].hi ? reach[i - 1] : used[i].hi;
+    for (size_t i = 0; i < ex->ops.size(); ++i) {
+        if (!ex->ops[i].exec || !product(ex->exec[ex->ops[i].exec - 1])) continue;
+        const Range r = range(ex->exec[ex->ops[i].exec - 1].t[2]);
+        const size_t n = std::lower_bound(used.begin(), used.end(), r.hi, [](const Range& a, uint64_t hi) { return a.lo < hi; }) - used.begin();
+        (*unread)[i] = n == 0 || reach[n - 1] <= r.lo;
+    }
+}
+
 // How many kernels of this library one exec record launches (memsets and NCCL calls are not ours).
 int own_kernels_of(const ExecOp& x) {
     const uint16_t k = x.kernel;
@@ -617,6 +662,7 @@ int replay(cai_exec* ex) {
             continue;
         }
         if (!op.exec) continue;
+        if (ex->unread[i] && !ex->has_pending_gather && !ex->debug_bounds && !(ex->trace_on && !ex->use_graph)) continue;
         // events on either side of a launch: no kernel starts while its predecessor finishes, some 5 us an op
         TraceRec* tr = nullptr;
         if (ex->trace_on && !ex->use_graph) {
@@ -634,12 +680,19 @@ int replay(cai_exec* ex) {
         }
         if (ex->nvtx_on) nvtxRangePushA(kernel_label(ex->exec[op.exec - 1].kernel));
         if (ex->with_next[i] && !tr && !ex->debug_bounds && ex->sm_limit_hi <= 0 && !ex->has_pending_gather) {
-            const cai_gemm_call a = gemm_call(ex, ex->exec[op.exec - 1]), b = gemm_call(ex, ex->exec[ex->ops[i + 1].exec - 1]);
-            const int rc = cai_gemm_bf16_two(&a, &b, st);
+            const ExecOp& next = ex->exec[ex->ops[i + 1].exec - 1];
+            const cai_gemm_call a = gemm_call(ex, ex->exec[op.exec - 1]);
+            int rc, launches = 1, cols;
+            if (ex->with_next[i] == cai_exec::kWithSwiglu) {
+                rc = cai_gemm_bf16_swiglu(a.A, a.B, a.C, ex->ptr(next.t[1]), a.M, next.i[1], a.K, a.lda, a.ldb, a.ldc, next.i[1], st);
+            } else {
+                const cai_gemm_call b = gemm_call(ex, next);
+                rc = cai_gemm_bf16_two(&a, &b, st);
+                launches = cai_gemm_bf16_two_launches(&a, &b, &cols);
+            }
             if (ex->nvtx_on) nvtxRangePop();
             if (rc != 0) return rc;
-            int cols;
-            ex->launches += cai_gemm_bf16_two_launches(&a, &b, &cols);
+            ex->launches += launches;
             ++i;
             continue;
         }
@@ -713,9 +766,13 @@ CAI_API int cai_exec_create(cai_exec** out, const void* plan_bytes, size_t nbyte
         if (o.exec || o.kind == OP_EVENT_RECORD || o.kind == OP_EVENT_WAIT) ex->used[o.stream_id] = true;
     ex->arena = static_cast<uint8_t*>(arena_base);
     ex->device = current_device();
+    find_unread(ex, &ex->unread);
     ex->with_next.assign(ex->ops.size() + 1, 0);
     for (size_t i = 0; i + 1 < ex->ops.size(); ++i)
-        ex->with_next[i] = !(i > 0 && ex->with_next[i - 1]) && independent_products(ex, ex->ops[i], ex->ops[i + 1]);
+        if (!ex->unread[i] && !ex->unread[i + 1] && !(i > 0 && ex->with_next[i - 1]))
+            ex->with_next[i] = independent_products(ex, ex->ops[i], ex->ops[i + 1])     ? cai_exec::kPairOfProducts
+                               : projection_with_swiglu(ex, ex->ops[i], ex->ops[i + 1]) ? cai_exec::kWithSwiglu
+                                                                                        : cai_exec::kAlone;
     if (const char* dbg = getenv("CAI_DEBUG_BOUNDS")) ex->debug_bounds = *dbg && *dbg != '0';
     if (ex->train.wait_limit_ms) cai_set_wait_limit_us(ex->train.wait_limit_ms * 1000u);
     int lo_prio = 0, hi_prio = 0;

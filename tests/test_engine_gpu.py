@@ -338,10 +338,14 @@ def test_engine_made_behind_work_of_the_callers_stream(side):
     eng.close()
 
 
-# Traced, every record is its own launch; untraced (and captured in a graph), a layer's input and weight gradient go out together where that is faster.
-# The gradients are the same bits. Widths that give persistent tiles and clusters, tied embeddings, microbatches that accumulate.
-@pytest.mark.parametrize("extra", ["", "hidden_size = 1000\nffn_hidden = 2728\nseq_len = 640\nmicrobatch = 3\ntie_embeddings = 1\nvocab_size = 5000\n"])
-def test_gradient_pairs_give_the_bits_of_single_launches(extra):
+# Traced, every record is its own launch; untraced (and captured in a graph), a layer's input and weight gradient go out together where that is faster, a
+# gate / up projection of odd width with its SwiGLU, and the last product of a layer that is run again, which nothing reads, not at all. The
+# gradients are the same bits. Widths that give persistent tiles and clusters, tied embeddings, microbatches that accumulate, recompute.
+ODD = "hidden_size = 1000\nffn_hidden = 2728\nseq_len = 640\nmicrobatch = 3\ntie_embeddings = 1\nvocab_size = 5000\n"
+
+
+@pytest.mark.parametrize("extra", ["", ODD, ODD + "recompute = 1\n", "ffn_hidden = 328\n", "param_dtype = fp8e4m3\nrecompute = 1\n"])
+def test_records_that_go_out_together_give_the_bits_of_single_launches(extra):
     from cai_b200.runtime.engine import Engine, synthetic_batch
     eng = Engine(config_text=(ROOT / "configs" / "tiny.cfg").read_text() + "\n" + extra, rank=0, world=1, local_rank=0)
     m = eng.model

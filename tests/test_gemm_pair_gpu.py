@@ -320,3 +320,27 @@ def test_two_products_same_bits(T, I, O, launches, accumulate):
         assert ops.device_status() == 0
         for _, out, alone in calls:
             assert torch.equal(out, alone)
+
+
+# The gate / up projection with SwiGLU in its epilogue at widths that are no multiple of a tile: the bits of the product and the stand-alone
+# kernel, and nothing beside the results. One feature group, edges of 64 and 128 features, several waves, one row.
+@pytest.mark.parametrize("F", [8, 56, 64, 72, 120, 136, 200, 1000, 2728])
+@pytest.mark.parametrize("M,K", [(1, 64), (300, 264), (1920, 1000)])
+def test_swiglu_of_any_width(M, K, F):
+    import ctypes
+    from cai_b200 import ops
+    out = [ctypes.c_int() for _ in range(3)]
+    ops.lib().cai_gemm_bf16_form(M, 2 * F, K, 1, 0, 0, 148, 0, *map(ctypes.byref, out))
+    torch.manual_seed(4)
+    x, w = (torch.randn(*s, device="cuda").to(torch.bfloat16) for s in ((M, K), (2 * F, K)))
+    gu, act = torch.full((M + 1, 2 * F), 5.0, device="cuda").to(torch.bfloat16), torch.full((M + 1, F), 5.0, device="cuda").to(torch.bfloat16)
+    p = [ctypes.c_void_p(t.data_ptr()) for t in (x, w, gu, act)]
+    q = ctypes.c_longlong
+    assert ops.lib().cai_gemm_bf16_swiglu(*p, M, F, K, q(K), q(K), q(2 * F), q(F), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+    want = ops.gemm(x, w)
+    if out[1].value == 1:
+        assert torch.equal(gu[:M], want)
+    assert torch.equal(act[:M], ops.swiglu_fwd(gu[:M].contiguous()))
+    assert torch.allclose(gu[:M].float(), want.float(), rtol=2.0 ** -7, atol=1e-2)
+    assert bool((gu[M] == 5.0).all()) and bool((act[M] == 5.0).all())
+    assert ops.device_status() == 0
