@@ -35,10 +35,35 @@ struct AttnFwdParams {
     int* status;
 };
 
+// A warp's 32 finished rows of O, each lane with one: times `inv` to bf16, through 8 KB of the query tile, which nobody reads any more, so that the warp
+// writes two whole rows at a time; from the registers every store met 32 lines. us, two CTAs to an SM,
+// before / now: 8 x 384 tokens, 12 / 4 heads 14.8 / 11.9; 8 x 256, 32 / 8 17.2 / 15.6; 16 x 384, 16 / 4 27.7 / 25.2; 4 x 1024, 16 / 8 28.2 / 26.7.
+__device__ __forceinline__ void put_out_rows(uint32_t stage, uint32_t tO, float inv, __nv_bfloat16* out, long long ld, int lane) {
+#pragma unroll 1
+    for (int c = 0; c < 4; ++c) {
+        uint32_t v[32];
+        tmem_ld_32x32(tO + c * 32, v);
+        tmem_ld_wait();
+#pragma unroll
+        for (int j4 = 0; j4 < 4; ++j4) {
+            uint32_t o[4];
+#pragma unroll
+            for (int t = 0; t < 4; ++t) o[t] = pack_bf16(__uint_as_float(v[j4 * 8 + 2 * t]) * inv, __uint_as_float(v[j4 * 8 + 2 * t + 1]) * inv);
+            st_shared_v4(stage + lane * 256 + (((c * 4 + j4) ^ (lane & 7)) << 4), o[0], o[1], o[2], o[3]);
+        }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        const int row = i * 2 + (lane >> 4), chunk = lane & 15;
+        *reinterpret_cast<uint4*>(out + row * ld + chunk * 8) = ld_shared_v4(stage + row * 256 + ((chunk ^ (row & 7)) << 4));
+    }
+}
+
 // Softmax of one query tile, whose scores arrive block by block in one buffer of tensor memory: one thread per query row (row r of
 // the tile, lane bits in tS and tO), 128 threads. Ends by writing the tile's rows of the output.
 __device__ __forceinline__ void softmax_tile(uint32_t tS, uint32_t tO, int r, int nx, uint64_t* s_full, uint64_t* p_full, uint64_t* o_final,
-                                             volatile int* abort_flag, const AttnFwdParams& p, int b, int h, int row_base, int q0) {
+                                             volatile int* abort_flag, const AttnFwdParams& p, int b, int h, int row_base, int q0, const uint8_t* q_tile) {
     float m_used = -INFINITY, l = 0.f;
     bool ok = true;
     for (int j = 0; j < nx; ++j) {
@@ -113,23 +138,8 @@ __device__ __forceinline__ void softmax_tile(uint32_t tS, uint32_t tO, int r, in
     if (ok && mbar_wait_warp(o_final, 0, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN)) {
         tc_fence_after();
         const float inv = 1.f / l;
-        const long long grow = static_cast<long long>(row_base) + q0 + r;
-        __nv_bfloat16* orow = p.out + grow * (static_cast<long long>(p.nh) * kAttnHD) + h * kAttnHD;
-#pragma unroll 1
-        for (int c = 0; c < 4; ++c) {
-            uint32_t v[32];
-            tmem_ld_32x32(tO + c * 32, v);
-            tmem_ld_wait();
-#pragma unroll
-            for (int j4 = 0; j4 < 4; ++j4) {
-                uint4 o;
-                o.x = pack_bf16(__uint_as_float(v[j4 * 8 + 0]) * inv, __uint_as_float(v[j4 * 8 + 1]) * inv);
-                o.y = pack_bf16(__uint_as_float(v[j4 * 8 + 2]) * inv, __uint_as_float(v[j4 * 8 + 3]) * inv);
-                o.z = pack_bf16(__uint_as_float(v[j4 * 8 + 4]) * inv, __uint_as_float(v[j4 * 8 + 5]) * inv);
-                o.w = pack_bf16(__uint_as_float(v[j4 * 8 + 6]) * inv, __uint_as_float(v[j4 * 8 + 7]) * inv);
-                *reinterpret_cast<uint4*>(orow + c * 32 + j4 * 8) = o;
-            }
-        }
+        const long long ldo = static_cast<long long>(p.nh) * kAttnHD;
+        put_out_rows(smem_u32(q_tile) + (r >> 5) * 8192, tO, inv, p.out + (static_cast<long long>(row_base) + q0 + (r & ~31)) * ldo + h * kAttnHD, ldo, r & 31);
         if (p.lse)
             p.lse[(static_cast<long long>(b) * p.nh + h) * p.S + q0 + r] =
                 (m_used + log2f(l)) * 0.6931471805599453f;
@@ -275,7 +285,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm, const AttnFwdParams p) {
             const uint32_t lane_bits = static_cast<uint32_t>((warp & 3) * 32) << 16;
             const uint32_t tS = tmem_base + X * 128 + lane_bits;
             const uint32_t tO = tmem_base + 256 + X * 128 + lane_bits;
-            softmax_tile(tS, tO, r, nx, &s_full[X], &p_full[X], &o_final[X], abort_flag, p, b, h, row_base, q0);
+            softmax_tile(tS, tO, r, nx, &s_full[X], &p_full[X], &o_final[X], abort_flag, p, b, h, row_base, q0, sQ + X * kAttnTileBytes);
         }
     }
 
@@ -497,23 +507,8 @@ attn_fwd1_kernel(const __grid_constant__ CUtensorMap tm, const AttnFwdParams p) 
         if (ok && mbar_wait_warp(pv_done, (n - 1) & 1, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN)) {
             tc_fence_after();
             const float inv = 1.f / l;
-            const long long grow = static_cast<long long>(row_base) + q0 + r;
-            __nv_bfloat16* orow = p.out + grow * (static_cast<long long>(p.nh) * kAttnHD) + h * kAttnHD;
-#pragma unroll 1
-            for (int c = 0; c < 4; ++c) {
-                uint32_t v[32];
-                tmem_ld_32x32(tO + c * 32, v);
-                tmem_ld_wait();
-#pragma unroll
-                for (int j4 = 0; j4 < 4; ++j4) {
-                    uint4 o;
-                    o.x = pack_bf16(__uint_as_float(v[j4 * 8 + 0]) * inv, __uint_as_float(v[j4 * 8 + 1]) * inv);
-                    o.y = pack_bf16(__uint_as_float(v[j4 * 8 + 2]) * inv, __uint_as_float(v[j4 * 8 + 3]) * inv);
-                    o.z = pack_bf16(__uint_as_float(v[j4 * 8 + 4]) * inv, __uint_as_float(v[j4 * 8 + 5]) * inv);
-                    o.w = pack_bf16(__uint_as_float(v[j4 * 8 + 6]) * inv, __uint_as_float(v[j4 * 8 + 7]) * inv);
-                    *reinterpret_cast<uint4*>(orow + c * 32 + j4 * 8) = o;
-                }
-            }
+            const long long ldo = static_cast<long long>(p.nh) * kAttnHD;
+            put_out_rows(smem_u32(sQ) + (r >> 5) * 8192, tO, inv, p.out + (static_cast<long long>(row_base) + q0 + (r & ~31)) * ldo + h * kAttnHD, ldo, r & 31);
             if (p.lse)
                 p.lse[(static_cast<long long>(b) * p.nh + h) * p.S + q0 + r] = (m_used + log2f(l)) * 0.6931471805599453f;
         }
@@ -640,7 +635,7 @@ attn_fwd_half_kernel(const __grid_constant__ CUtensorMap tm, const AttnFwdParams
     } else {
         const uint32_t lane_bits = static_cast<uint32_t>((warp & 3) * 32) << 16;
         softmax_tile(tmem_base + lane_bits, tmem_base + 128 + lane_bits, (warp & 3) * 32 + lane, n, s_full, p_full, o_final, abort_flag, p, b, h,
-                     row_base, q0);
+                     row_base, q0, sQ);
     }
 
     tc_fence_before();
@@ -690,13 +685,16 @@ CAI_API int cai_flash_attn_fwd_variant(const void* qkv, void* out, float* lse, i
     // Grids that leave SMs idle (few heads per GPU) are bound by their heaviest CTA: one tile per CTA with the score MMA running a block
     // ahead halves that path. Larger ones put two CTAs of one tile on each SM up to 4096 tokens, and two tiles in ping-pong into one
     // CTA beyond, where both take the same time and the latter reads K and V half as often. All give the same bits. us, one tile / two tiles /
-    // two CTAs: 8 x 384 tokens, 12 / 4 heads 17.7 / 19.7 / 14.7; 6 x 640, 9 / 3 heads 19.6 / 19.0 / 18.6; 4 x 1024, 16 / 8 heads 40.8 / 32.4 /
-    // 28.7; 2048, 32 / 32 heads 62.7 / 47.7 / 43.6; 4 x 4096, 16 / 8 heads 384 / 283 / 278; 8192, 32 / 8 heads 717 / 490-504 / 499; and, with
-    // fewer CTAs than SMs, 2 x 1024, 16 / 8 heads 21.3 / 25.0 / 22.7, 2048, 16 / 8 heads 31.9 / 42.0 / 39.0. (Short rows in grids of that size take less
-    // in another form, which the rule does not use: one behind the other, 6 x 384, 12 / 4 heads 16.4 / 11.6 / 14.1, 8 x 256, 16 / 8 14.2 / 10.0 / 11.7,
-    // 16 x 128, 16 / 8 12.8 / 12.4 / 9.5; 2 x 640, 16 / 8 13.4 / 15.3 / 14.1.)
+    // two CTAs: 8 x 384 tokens, 12 / 4 heads 15.7 / 17.2 / 11.9; 6 x 640, 9 / 3 heads 17.7 / 17.1 / 15.0; 4 x 1024, 16 / 8 heads 40.7 / 31.9 /
+    // 26.7; 2048, 32 / 32 heads 61.0 / 46.7 / 45.7; 4 x 4096, 16 / 8 heads 388 / 309 / 306; 8192, 32 / 8 heads 721 / 490 / 544.
+    // In between, a wave of two-tile CTAs fills the SMs that one of one-tile CTAs overflows: 8 x 256, 16 / 8 13.6 / 9.3 / 10.2, 6 x 384, 12 / 4
+    // 14.0 / 9.7 / 11.3, 4 x 512, 16 / 8 16.1 / 14.5 / 13.3, 2 x 1024, 16 / 8 21.3 / 24.4 / 20.1; the second tile's steps cost more than the second
+    // wave from 2048 tokens (2048, 16 / 8 31.6 / 39.2 / 33.3). In one wave of one-tile CTAs: 2 x 256, 16 / 8 7.2 / 8.3 / 7.4, 2048, 4 / 2
+    // 25.6 / 35.9 / 30.0.
     const long long pair_ctas = static_cast<long long>((S + 2 * kAttnTile - 1) / (2 * kAttnTile)) * nh * B;
-    const int variant = force_variant ? force_variant : pair_ctas < sm_count(dev) ? 1 : S <= 4096 ? 3 : 2;
+    const long long ctas = static_cast<long long>(S / kAttnTile) * nh * B;
+    const int small = ctas <= sm_count(dev) || S >= 2048 ? 1 : S <= 384 ? 2 : 3;
+    const int variant = force_variant ? force_variant : pair_ctas < sm_count(dev) ? small : S <= 4096 ? 3 : 2;
     if (variant == 3) {
         constexpr int smem_half = 3 * kAttnTileBytes + 1024 + 256;
         static bool configured_half[64] = {};
