@@ -248,19 +248,21 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
 // other warpgroup gives up; sixteen warps of 64 columns had 112 and spilled); two reads are in flight per wait; the next part is asked
 // for before the last additions, without blocking; scales come in eight k-blocks at a time and are read and multiplied four at a time. Cycles per
 // k-block, sixteen warps and whole k-blocks / now: 965 / 820 with two pairs at work, 1100 / 983 with 72. us, bursts of 50: 2000 x 4096 x 14336
-// 131 / 118, 9472 x 4096 x 4096 176 / 158 (one CTA per tile 145 for the former). Tried on top: a half per issuing warp (911 and 1075 cycles: four
+// 131 / 118, 9472 x 4096 x 4096 176 / 158 (one CTA per tile 145 for the former); with results that leave by TMA through boxes of shared memory,
+// for which the ring gave up its sixth stage, instead of 32 lines a store 116 / 150 (a tile's end 8.8 -> 6.5 us). Tried on top: a half per issuing warp (911 and 1075 cycles: four
 // waits per k-block instead of three), scales two at a time (872 and 1028), halves with sixteen warps (no change), additions in pairs
 // (fma.rn.f32x2; sixteen warps, 131 -> 145 us).
 namespace f8p {
 constexpr int kBM = 256, kBN = 256, kBK = 128;
-constexpr int kStages = 6;
+constexpr int kStages = 5;
 constexpr int kHalf = 128 * kBK;                   // bytes of A, or of B, a CTA brings in per stage
 constexpr int kEpiWarps = 8;
 constexpr int kThreads = 128 + kEpiWarps * 32;     // warp 0 TMA, warps 1-2 MMA, warp 3 scales, warps 4-11 epilogue
 constexpr int kScaleKb = 8;                        // k-blocks whose scales come in at a time
 constexpr int kScaleRow = 12;                      // a row of A's eight scales, padded: eight rows' 16 bytes fall on 32 banks
 constexpr int kScaleWords = 128 * kScaleRow + 2 * kScaleKb;
-constexpr int kSmem = kStages * 2 * kHalf + 2 * kScaleWords * 4 + 512 + 1024;
+constexpr int kBox = 4096;                         // a warp's box of results: 32 rows x 128 bytes
+constexpr int kSmem = kStages * 2 * kHalf + kEpiWarps * kBox + 2 * kScaleWords * 4 + 512 + 1024;
 }  // namespace f8p
 
 __device__ __forceinline__ void umma_f8_ss_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
@@ -286,13 +288,15 @@ __device__ __forceinline__ void cp_async4(float* smem_dst, const float* src) {
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(f8p::kThreads, 1)
-gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmFp8Params p) {
+gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmC,
+                     const GemmFp8Params p) {
     using namespace f8p;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* sA = smem;
     uint8_t* sB = smem + kStages * kHalf;
-    float* scales = reinterpret_cast<float*>(smem + kStages * 2 * kHalf);   // [2][kScaleWords]
+    uint8_t* sE = smem + kStages * 2 * kHalf;
+    float* scales = reinterpret_cast<float*>(sE + kEpiWarps * kBox);        // [2][kScaleWords]
     uint64_t* bars = reinterpret_cast<uint64_t*>(scales + 2 * kScaleWords);
     uint64_t* full = bars;                         // [kStages] used in the even CTA: both CTAs' operands have landed
     uint64_t* empty = bars + kStages;              // [kStages] in each CTA
@@ -315,6 +319,7 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     } else if (warp == 2 && lane == 0) {
         tma_prefetch_desc(&tmA);
         tma_prefetch_desc(&tmB);
+        tma_prefetch_desc(&tmC);
     }
     if (warp == 1) {
         tmem_alloc_pair(tmem_slot, 2 * kBN);
@@ -458,6 +463,8 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         const int q = warp & 3, half = (warp - 4) >> 2;
         const uint32_t taddr0 = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + half * (kBN / 2);
         const uint32_t release0 = map_to_cta(smem_u32(&part_empty[half]), 0);
+        uint8_t* box = sE + (warp - 4) * kBox;
+        const uint32_t box_row = smem_u32(box) + lane * 128, sw = lane & 7;
         uint32_t it = 0, sb = 0, sph = 0;
         bool ok = true, ready = false;     // ready: the next part was seen in tensor memory
         for (int tile = first; tile < num_tiles && ok; tile += stride) {
@@ -520,41 +527,62 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
             if (!ok) break;
             int tm, tn;
             coords(tile, tm, tn);
-            const long long row = static_cast<long long>(tm) * kBM + rank * 128 + q * 32 + lane;
+            // through a box of shared memory by TMA, edges clipped by the tensor map: whole lines, and the registers are free for the next tile
+            // as soon as the last box is written
+            const int row0 = tm * kBM + static_cast<int>(rank) * 128 + q * 32;
+            if (row0 >= p.M) continue;
 #pragma unroll
             for (int side = 0; side < 2; ++side) {
                 const int col0 = tn * kBN + side * 128 + half * 64;
-                if (row >= p.M || col0 >= p.N) continue;   // nothing of this lane's is written
+                if (col0 >= p.N) break;
                 if (p.epi == CAI_EPI_F32) {
-                    float* crow = reinterpret_cast<float*>(p.C) + row * p.ldc + col0;
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) {
-                        if (col0 + j * 4 >= p.N) break;
-                        const float* v = acc + side * 64 + j * 4;
-                        *reinterpret_cast<float4*>(crow + j * 4) = make_float4(v[0], v[1], v[2], v[3]);
+                    for (int h = 0; h < 2; ++h) {
+                        if (col0 + h * 32 >= p.N) break;
+                        if (lane == 0) tma_store_wait_read0();
+                        __syncwarp();
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) {
+                            const float* v = acc + side * 64 + h * 32 + j * 4;
+                            st_shared_v4(box_row + ((j ^ sw) << 4), __float_as_uint(v[0]), __float_as_uint(v[1]), __float_as_uint(v[2]), __float_as_uint(v[3]));
+                        }
+                        fence_proxy_async_smem();
+                        __syncwarp();
+                        if (lane == 0) {
+                            tma_store_2d(&tmC, box, col0 + h * 32, row0);
+                            tma_store_commit();
+                        }
                     }
                 } else {
-                    __nv_bfloat16* crow = reinterpret_cast<__nv_bfloat16*>(p.C) + row * p.ldc + col0;
-                    const __nv_bfloat16* rrow =
-                        p.epi == CAI_EPI_BF16_RESIDUAL ? reinterpret_cast<const __nv_bfloat16*>(p.R) + row * p.ldr + col0 : nullptr;
+                    const __nv_bfloat16* rrow = p.epi == CAI_EPI_BF16_RESIDUAL && row0 + lane < p.M
+                                                    ? reinterpret_cast<const __nv_bfloat16*>(p.R) + static_cast<long long>(row0 + lane) * p.ldr + col0
+                                                    : nullptr;
+                    if (lane == 0) tma_store_wait_read0();
+                    __syncwarp();
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
-                        if (col0 + j * 8 >= p.N) break;
                         float v[8];
 #pragma unroll
                         for (int e = 0; e < 8; ++e) v[e] = acc[side * 64 + j * 8 + e];
-                        if (rrow) {
+                        if (rrow && col0 + j * 8 < p.N) {
                             float rf[8];
                             unpack8(*reinterpret_cast<const uint4*>(rrow + j * 8), rf);
 #pragma unroll
                             for (int e = 0; e < 8; ++e) v[e] += rf[e];
                         }
-                        *reinterpret_cast<uint4*>(crow + j * 8) = pack8(v);
+                        const uint4 o = pack8(v);
+                        st_shared_v4(box_row + ((j ^ sw) << 4), o.x, o.y, o.z, o.w);
+                    }
+                    fence_proxy_async_smem();
+                    __syncwarp();
+                    if (lane == 0) {
+                        tma_store_2d(&tmC, box, col0, row0);
+                        tma_store_commit();
                     }
                 }
             }
-            __syncwarp();
         }
+        if (lane == 0) tma_store_wait0();
     }
     tc_fence_before();
     __syncthreads();
@@ -788,14 +816,15 @@ CAI_API int cai_gemm_fp8_blockscaled(const void* Aq, const float* sa, const void
     }
     const int dev = current_device();
     const int sms = sm_count(dev);
-    // Pairs of CTAs, unless the last half of their 256-row tiles stays empty and costs waves: a wave of pair tiles takes some nine tenths
-    // of one of one-CTA tiles of half the rows (us, one-CTA / pair: 2000 x 4096 x 14336 145 / 129, 128 x 14336 x 4096 27.4 / 25.3, 16 x 4096
+    // Pairs of CTAs, unless the last half of their 256-row tiles stays empty and costs waves: a wave of pair tiles takes some eight tenths
+    // of one of one-CTA tiles of half the rows (us, one-CTA / pair: 2000 x 4096 x 14336 145 / 116, 128 x 14336 x 4096 27.4 / 25.3, 16 x 4096
     // x 4096 22.9 / 19.9; two waves of pairs against one: 128 x 28672 x 4096 31.7 / 47.8). Both forms give the same bits.
     const long long cols = (N + f8::kBN - 1) / f8::kBN, pairs = sms / 2 > 0 ? sms / 2 : 1;
     const long long waves_one = ((M + f8::kBM - 1) / f8::kBM * cols + sms - 1) / sms, waves_pair = ((M + f8p::kBM - 1) / f8p::kBM * cols + pairs - 1) / pairs;
-    const bool pair = 9 * waves_pair <= 10 * waves_one;
-    CUtensorMap tmA, tmB;
-    if (!encode_tmap_2d(&tmA, Aq, M, K, lda, f8::kBK, 128, 1) || !encode_tmap_2d(&tmB, Bq, N, K, ldb, f8::kBK, pair ? 128 : f8::kBN, 1))
+    const bool pair = 8 * waves_pair <= 10 * waves_one;
+    CUtensorMap tmA, tmB, tmC;
+    const int c_bytes = epi == CAI_EPI_F32 ? 4 : 2;
+    if ((pair && !encode_tmap_2d(&tmC, C, M, N, ldc, 128 / c_bytes, 32, c_bytes)) || !encode_tmap_2d(&tmA, Aq, M, K, lda, f8::kBK, 128, 1) || !encode_tmap_2d(&tmB, Bq, N, K, ldb, f8::kBK, pair ? 128 : f8::kBN, 1))
         return CAI_K_BAD_ARG;
     static bool configured[64] = {};
     if (!configured[dev & 63]) {
@@ -817,7 +846,7 @@ CAI_API int cai_gemm_fp8_blockscaled(const void* Aq, const float* sa, const void
     const int tiles = p.tiles_m * p.tiles_n;
     if (pair) {
         launch_early(gemm_fp8_pair_kernel, 2 * (tiles < pairs ? tiles : static_cast<int>(pairs)), f8p::kThreads, f8p::kSmem,
-                     static_cast<cudaStream_t>(stream), tmA, tmB, p);
+                     static_cast<cudaStream_t>(stream), tmA, tmB, tmC, p);
     } else {
         launch_early(gemm_fp8_kernel, tiles < sms ? tiles : sms, f8::kThreads, f8::kSmem, static_cast<cudaStream_t>(stream), tmA, tmB, p);
     }
