@@ -58,6 +58,7 @@ struct AttnBwdParams {
     // contribution to the group's dK / dV rows; chain[b][g][kv tile] counts the heads that are done.
     int split_heads;
     unsigned int* chain;
+    const float2* rope;          // (cos, sin) [S][64]: dQ and dK leave rotated back (null: as they are)
 };
 
 // chain counters of the head-split dK / dV kernel: one per (batch, kv group, kv tile).
@@ -139,40 +140,60 @@ __device__ __forceinline__ void stage_acc_chunk(uint32_t tacc, uint32_t stage, i
     for (int k = 0; k < 8; ++k)
         st_shared_v4(stage + r * 512 + (((c * 8 + k) ^ (r & 7)) << 4), v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
 }
-// kPieces pieces of eight columns of a thread, 512 threads: piece `first` of them, then every 512th; sixteen pieces a row, 128 rows a tile of 64 KB.
-// Tile t leaves at dst[t], times mul[t].
+// A thread of 512 takes kPieces times eight columns and the eight that are 64 further on: item `first` of eight a row, 128 rows a tile of 64 KB, then
+// every 512th. Tile t leaves at dst[t], times mul[t]; where `rope` is given (the row of its table that belongs to row 0), tile 0 is rounded, as it
+// would be in memory, and rotated back.
 template <bool kAdd, int kPieces>
-__device__ __forceinline__ void write_staged(uint32_t stage, __nv_bfloat16* const (&dst)[2], const float (&mul)[2], long long ld, int first) {
-    uint4 old[kPieces];
+__device__ __forceinline__ void write_staged(uint32_t stage, __nv_bfloat16* const (&dst)[2], const float (&mul)[2], long long ld, int first, const float2* rope) {
+    uint4 old[kPieces][2];
     if constexpr (kAdd) {
 #pragma unroll
-        for (int i = 0; i < kPieces; ++i) {
-            const int piece = first + i * 512;
-            old[i] = *reinterpret_cast<const uint4*>(dst[i >> 2] + ((piece >> 4) & 127) * ld + (piece & 15) * 8);
-        }
+        for (int i = 0; i < kPieces; ++i)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int item = first + i * 512;
+                old[i][h] = *reinterpret_cast<const uint4*>(dst[i >> 1] + ((item >> 3) & 127) * ld + h * 64 + (item & 7) * 8);
+            }
     }
 #pragma unroll
     for (int i = 0; i < kPieces; ++i) {
-        const int piece = first + i * 512, r = (piece >> 4) & 127, c = (piece & 15) * 2;
-        const uint32_t row = stage + (i >> 2) * 65536 + r * 512;
-        float v[8];
+        const int item = first + i * 512, r = (item >> 3) & 127, c = (item & 7) * 2;
+        const uint32_t row = stage + (i >> 1) * 65536 + r * 512;
+        uint32_t o[2][4];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            const float4 f = ld_shared_f4(row + (((c + h) ^ (r & 7)) << 4));
-            v[4 * h] = f.x; v[4 * h + 1] = f.y; v[4 * h + 2] = f.z; v[4 * h + 3] = f.w;
-        }
-        const uint32_t ov[4] = {kAdd ? old[i].x : 0u, kAdd ? old[i].y : 0u, kAdd ? old[i].z : 0u, kAdd ? old[i].w : 0u};
-        uint32_t o[4];
+            float v[8];
 #pragma unroll
-        for (int t = 0; t < 4; ++t) {
-            float lo = v[2 * t] * mul[i >> 2], hi = v[2 * t + 1] * mul[i >> 2];
-            if constexpr (kAdd) {
-                lo += bf16_lo(ov[t]);
-                hi += bf16_hi(ov[t]);
+            for (int k = 0; k < 2; ++k) {
+                const float4 f = ld_shared_f4(row + ((((h * 16) + c + k) ^ (r & 7)) << 4));
+                v[4 * k] = f.x; v[4 * k + 1] = f.y; v[4 * k + 2] = f.z; v[4 * k + 3] = f.w;
             }
-            o[t] = pack_bf16(lo, hi);
+            const uint32_t ov[4] = {kAdd ? old[i][h].x : 0u, kAdd ? old[i][h].y : 0u, kAdd ? old[i][h].z : 0u, kAdd ? old[i][h].w : 0u};
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                float lo = v[2 * t] * mul[i >> 1], hi = v[2 * t + 1] * mul[i >> 1];
+                if constexpr (kAdd) {
+                    lo += bf16_lo(ov[t]);
+                    hi += bf16_hi(ov[t]);
+                }
+                o[h][t] = pack_bf16(lo, hi);
+            }
         }
-        *reinterpret_cast<uint4*>(dst[i >> 2] + r * ld + (piece & 15) * 8) = make_uint4(o[0], o[1], o[2], o[3]);
+        if (rope && (i >> 1) == 0) {
+            const float4* cs = reinterpret_cast<const float4*>(rope + r * 64 + (item & 7) * 8);
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                const float4 q = cs[t];      // of two columns
+                float a0 = bf16_lo(o[0][t]), a1 = bf16_hi(o[0][t]), b0 = bf16_lo(o[1][t]), b1 = bf16_hi(o[1][t]);
+                rope_rotate(a0, b0, q.x, -q.y);
+                rope_rotate(a1, b1, q.z, -q.w);
+                o[0][t] = pack_bf16(a0, a1);
+                o[1][t] = pack_bf16(b0, b1);
+            }
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+            *reinterpret_cast<uint4*>(dst[i >> 1] + r * ld + h * 64 + (item & 7) * 8) = make_uint4(o[h][0], o[h][1], o[h][2], o[h][3]);
     }
 }
 
@@ -495,8 +516,10 @@ __device__ __forceinline__ void attn_dkdv(const CUtensorMap& tm_qkv, const CUten
             if (!ok) atomicCAS(p.status, 0, CAI_DEV_TIMEOUT_ATTN);
         }
         if (ok) {
-            if (turn == 0) write_staged<false, 8>(stage, dst, mul, ld, first);
-            else write_staged<true, 8>(stage, dst, mul, ld, first);
+            // the last of the heads turns the finished sum
+            const float2* rope = p.rope && (!p.split_heads || turn + 1 == rep) ? p.rope + static_cast<long long>(j) * kAttnTile * 64 : nullptr;
+            if (turn == 0) write_staged<false, 4>(stage, dst, mul, ld, first, rope);
+            else write_staged<true, 4>(stage, dst, mul, ld, first, rope);
         }
         if (p.split_heads) {
             __threadfence();
@@ -715,7 +738,7 @@ __device__ __forceinline__ void attn_dq(const CUtensorMap& tm_qkv, const CUtenso
             __nv_bfloat16* dst0 = p.dqkv + (static_cast<long long>(row_base) + i * kAttnTile) * ld + col_q;
             __nv_bfloat16* const dst[2] = {dst0, nullptr};
             const float mul[2] = {p.scale, 0.f};
-            write_staged<false, 4>(stage, dst, mul, ld, threadIdx.x - 128);
+            write_staged<false, 2>(stage, dst, mul, ld, threadIdx.x - 128, p.rope ? p.rope + static_cast<long long>(i) * kAttnTile * 64 : nullptr);
         }
     }
 
@@ -760,6 +783,11 @@ CAI_API int cai_flash_attn_bwd(const void* qkv, const void* out, const void* dou
 
 CAI_API int cai_flash_attn_bwd_parts(const void* qkv, const void* out, const void* dout, const float* lse, float* delta,
                                      void* dqkv, int B, int S, int nh, int nkv, int hd, float scale, int parts, void* stream) {
+    return cai_flash_attn_bwd_rope(qkv, out, dout, lse, delta, dqkv, nullptr, B, S, nh, nkv, hd, scale, parts, stream);
+}
+
+CAI_API int cai_flash_attn_bwd_rope(const void* qkv, const void* out, const void* dout, const float* lse, float* delta, void* dqkv,
+                                    const float* table, int B, int S, int nh, int nkv, int hd, float scale, int parts, void* stream) {
     if (hd != kAttnHD || S % kAttnTile || nkv <= 0 || nh % nkv) {
         set_last_error("flash_attn_bwd: needs head_dim 128, seq %% 128 == 0, heads %% kv_heads == 0");
         return CAI_K_BAD_ARG;
@@ -794,6 +822,7 @@ CAI_API int cai_flash_attn_bwd_parts(const void* qkv, const void* out, const voi
     // longest CTA by the group size; the heads of a group then add into dK / dV in turn (chain counters).
     p.split_heads = 0;
     p.chain = nullptr;
+    p.rope = reinterpret_cast<const float2*>(table);
     const size_t need = static_cast<size_t>(B) * nkv * nq;
     if ((parts & 2) && nh > nkv && static_cast<long long>(nq) * nkv * B < sm_count(dev) &&
         static_cast<long long>(nq) * nh * B <= sm_count(dev) && need <= kAttnChainSlots) {

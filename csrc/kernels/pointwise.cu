@@ -121,11 +121,7 @@ __global__ void rope_apply_kernel(__nv_bfloat16* qkv, const float2* __restrict__
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
         const float2 cs = tb[e];
-        const float sn = inverse ? -cs.y : cs.y;
-        const float x1 = a[e] * cs.x - b[e] * sn;
-        const float x2 = b[e] * cs.x + a[e] * sn;
-        a[e] = x1;
-        b[e] = x2;
+        rope_rotate(a[e], b[e], cs.x, inverse ? -cs.y : cs.y);
     }
     *reinterpret_cast<uint4*>(base) = pack8(a);
     *reinterpret_cast<uint4*>(base + half) = pack8(b);

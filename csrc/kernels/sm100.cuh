@@ -489,6 +489,13 @@ __device__ __forceinline__ bool wait_flag_ge(const uint32_t* p, uint32_t target,
 
 __device__ __forceinline__ float bf16_lo(uint32_t v) { return __uint_as_float(v << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t v) { return __uint_as_float(v & 0xFFFF0000u); }
+// A pair of rotary embedding: (a, b) turned by the angle of cosine c and sine s. Which product is rounded is written out: left to the compiler it
+// differed from one kernel to the next, and two kernels have to give the same bits.
+__device__ __forceinline__ void rope_rotate(float& a, float& b, float c, float s) {
+    const float x = __fmaf_rn(a, c, -__fmul_rn(b, s)), y = __fmaf_rn(b, c, __fmul_rn(a, s));
+    a = x;
+    b = y;
+}
 __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
     __nv_bfloat162 t = __floats2bfloat162_rn(a, b);
     return *reinterpret_cast<uint32_t*>(&t);

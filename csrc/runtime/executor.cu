@@ -178,7 +178,7 @@ struct cai_exec {
     cai_fused_hook_t fused_hook = nullptr;
     void* fused_ctx = nullptr;
     int sm_limit_hi = 0;
-    enum : uint8_t { kAlone, kPairOfProducts, kWithSwiglu };
+    enum : uint8_t { kAlone, kPairOfProducts, kWithSwiglu, kWithRotation };
     std::vector<uint8_t> with_next;   // per op: whether, and how, it goes out together with the one behind it
     std::vector<uint8_t> unread;      // per op: a product whose result nothing reads; a traced or checked replay runs it all the same
     uint64_t launches = 0;  // kernels / collectives enqueued by the last replay
@@ -592,6 +592,17 @@ bool projection_with_swiglu(const cai_exec* ex, const Op& o0, const Op& o1) {
            cai_gemm_bf16_swiglu_pays(c.M, y.i[1], c.K);
 }
 
+// Whether two records next to each other on one stream are an attention backward and the inverse rotary embedding of its result.
+bool backward_with_rotation(const cai_exec* ex, const Op& o0, const Op& o1) {
+    if (!o0.exec || !o1.exec || o0.stream_id != o1.stream_id) return false;
+    if (o0.kind == OP_EVENT_RECORD || o0.kind == OP_EVENT_WAIT || o1.kind == OP_EVENT_RECORD || o1.kind == OP_EVENT_WAIT) return false;
+    const ExecOp &x = ex->exec[o0.exec - 1], &y = ex->exec[o1.exec - 1];
+    if (x.kernel != K_ATTN_BWD || y.kernel != K_ROPE || (x.flags && x.flags != 7) || !(y.flags & 1)) return false;
+    // B, S, heads of the one; rows, S, heads of the other, over rows of the same pitch
+    return ex->ptr(x.t[5]) == ex->ptr(y.t[0]) && y.i[0] == x.i[0] * x.i[1] && y.i[1] == x.i[1] && y.i[2] == x.i[2] && y.i[3] == x.i[3] &&
+           y.i[4] == x.i[4] && ex->ld(y.t[0]) == static_cast<long long>(x.i[2] + 2 * x.i[3]) * x.i[4];
+}
+
 // Products whose results no record of the plan reads: with activation recompute, the down projection of a layer that is run again for its
 // backward. Of everything that any record names, only outputs of such products may lie in the bytes of a result for it to count as unread, and no
 // tensor that the plan gives a name to.
@@ -680,13 +691,18 @@ int replay(cai_exec* ex) {
         }
         if (ex->nvtx_on) nvtxRangePushA(kernel_label(ex->exec[op.exec - 1].kernel));
         if (ex->with_next[i] && !tr && !ex->debug_bounds && ex->sm_limit_hi <= 0 && !ex->has_pending_gather) {
-            const ExecOp& next = ex->exec[ex->ops[i + 1].exec - 1];
-            const cai_gemm_call a = gemm_call(ex, ex->exec[op.exec - 1]);
+            const ExecOp &x = ex->exec[op.exec - 1], &next = ex->exec[ex->ops[i + 1].exec - 1];
             int rc, launches = 1, cols;
-            if (ex->with_next[i] == cai_exec::kWithSwiglu) {
+            if (ex->with_next[i] == cai_exec::kWithRotation) {
+                auto P = [&](int t) { return ex->ptr(x.t[t]); };
+                rc = cai_flash_attn_bwd_rope(P(0), P(1), P(2), (const float*)P(3), (float*)P(4), P(5), (const float*)ex->ptr(next.t[1]), x.i[0], x.i[1],
+                                             x.i[2], x.i[3], x.i[4], x.f[0], 7, st);
+                launches = own_kernels_of(x);
+            } else if (ex->with_next[i] == cai_exec::kWithSwiglu) {
+                const cai_gemm_call a = gemm_call(ex, x);
                 rc = cai_gemm_bf16_swiglu(a.A, a.B, a.C, ex->ptr(next.t[1]), a.M, next.i[1], a.K, a.lda, a.ldb, a.ldc, next.i[1], st);
             } else {
-                const cai_gemm_call b = gemm_call(ex, next);
+                const cai_gemm_call a = gemm_call(ex, x), b = gemm_call(ex, next);
                 rc = cai_gemm_bf16_two(&a, &b, st);
                 launches = cai_gemm_bf16_two_launches(&a, &b, &cols);
             }
@@ -772,6 +788,7 @@ CAI_API int cai_exec_create(cai_exec** out, const void* plan_bytes, size_t nbyte
         if (!ex->unread[i] && !ex->unread[i + 1] && !(i > 0 && ex->with_next[i - 1]))
             ex->with_next[i] = independent_products(ex, ex->ops[i], ex->ops[i + 1])     ? cai_exec::kPairOfProducts
                                : projection_with_swiglu(ex, ex->ops[i], ex->ops[i + 1]) ? cai_exec::kWithSwiglu
+                               : backward_with_rotation(ex, ex->ops[i], ex->ops[i + 1]) ? cai_exec::kWithRotation
                                                                                         : cai_exec::kAlone;
     if (const char* dbg = getenv("CAI_DEBUG_BOUNDS")) ex->debug_bounds = *dbg && *dbg != '0';
     if (ex->train.wait_limit_ms) cai_set_wait_limit_us(ex->train.wait_limit_ms * 1000u);

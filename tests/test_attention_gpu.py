@@ -135,3 +135,30 @@ def test_flash_attn_bwd_parts_together(B, S, nh, nkv):
     q = nh * 128
     assert torch.equal(whole[:, :q], q_only[:, :q]) and bool((q_only[:, q:] == 7.0).all())
     assert torch.equal(whole[:, q:], kv_only[:, q:]) and bool((kv_only[:, :q] == 7.0).all())
+
+
+# The backward with the inverse rotary embedding of dQ and dK in it against the two passes: the same bits. Chained heads and not.
+@pytest.mark.parametrize("B,S,nh,nkv", [(1, 128, 1, 1), (4, 128, 2, 1), (1, 512, 8, 1), (3, 640, 9, 3), (2, 1024, 16, 8)])
+@pytest.mark.parametrize("parts", [7, 4, 2])
+def test_flash_attn_bwd_rotated_back(B, S, nh, nkv, parts):
+    import ctypes
+    from cai_b200 import ops
+    torch.manual_seed(3)
+    qkv = torch.randn(B * S, (nh + 2 * nkv) * 128, device="cuda").to(torch.bfloat16)
+    dout = torch.randn(B * S, nh * 128, device="cuda").to(torch.bfloat16)
+    table = ops.rope_table(S, 128)
+    out, lse = ops.flash_attn_fwd(qkv, B, S, nh, nkv, 128)
+    delta = torch.empty((B, nh, S), device="cuda")
+    want = torch.zeros_like(qkv)
+    ops.flash_attn_bwd(qkv, out, dout, lse, B, S, nh, nkv, 128, dqkv=want, delta=delta)
+    ops.rope_apply_(want, table, S, nh, nkv, 128, inverse=True)
+    got = torch.zeros_like(qkv)
+    p = [ctypes.c_void_p(t.data_ptr()) for t in (qkv, out, dout, lse, delta, got, table)]
+    rc = ops.lib().cai_flash_attn_bwd_rope(*p, B, S, nh, nkv, 128, ctypes.c_float(128 ** -0.5), parts, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert rc == 0 and ops.device_status() == 0
+    q = nh * 128
+    if parts & 4:
+        assert torch.equal(got[:, :q], want[:, :q])
+    if parts & 2:
+        assert torch.equal(got[:, q:], want[:, q:])
+    assert bool((got[:, :q] == 0).all()) == (not parts & 4) and bool((got[:, q:] == 0).all()) == (not parts & 2)
