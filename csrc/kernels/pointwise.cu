@@ -199,9 +199,9 @@ __global__ void embed_fwd_kernel(const int* __restrict__ tokens, const __nv_bflo
 // additions in registers and is written once. What bounded the earlier form was latency: 256 tokens per two barriers, and a read,
 // an addition and a write of dE behind each other for every token: 17 us for 512 tokens of 512 x 256, 67 us for 3840 of 5000 x 1000, of
 // which 10 and 60 us are saved (whole steps 443 -> 433 us and 4.78 -> 4.72 ms).
-constexpr int kEmbRows = 32;
 constexpr int kEmbScan = 4096;
-template <int V>   // columns a lane takes at a time: 8 where rows are 16-byte aligned pieces, else 1
+// V: columns a lane takes at a time, 8 where rows are 16-byte aligned pieces, else 1
+template <int V, int kEmbRows>
 __global__ void __launch_bounds__(256)
 embed_bwd_kernel(const int* __restrict__ tokens, const __nv_bfloat16* __restrict__ dout, float* __restrict__ dE, int T, int H,
                  int lo, int hi) {
@@ -256,13 +256,14 @@ embed_bwd_kernel(const int* __restrict__ tokens, const __nv_bfloat16* __restrict
             for (int k = 0; k < kEmbRows / 8; ++k) row_count[warp + 8 * k] = cnt[k];
         __syncthreads();
         if (warp == 0) {
-            int sum = row_count[lane];
+            const int own = lane < kEmbRows ? row_count[lane] : 0;
+            int sum = own;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
                 const int up = __shfl_up_sync(0xffffffffu, sum, o);
                 if (lane >= o) sum += up;
             }
-            row_first[lane] = sum - row_count[lane];
+            if (lane < kEmbRows) row_first[lane] = sum - own;
         }
         __syncthreads();
 #pragma unroll
@@ -617,9 +618,14 @@ CAI_API int cai_embed_bwd(const int* tokens, const void* dout, float* dE, int T,
                           int vocab_hi, void* stream) {
     if (T <= 0) return CAI_K_OK;
     if (vocab_hi <= vocab_lo) return CAI_K_OK;
-    const dim3 grid((vocab_hi - vocab_lo + kEmbRows - 1) / kEmbRows);
+    // Every CTA looks through all tokens, which 8 rows a CTA do four times as often as 32: few rows of the vocabulary leave the
+    // SMs idle otherwise, and one behind the other what a warp adds up. us, 32 / 8: 512 tokens of 512 x 256 6.0 / 4.1, 3840 of 5000 x 1000 14.7 / 9.8,
+    // 16384 of 1000 x 256 33.4 / 16.6 and of 9480 x 1024 52.9 / 44.8; 512 of 16000 x 256 7.3 / 10.3, 4096 of 16000 x 2048 23.2 / 21.4 and of
+    // 32000 x 1024 16.9 / 25.4.
+    const int few = vocab_hi - vocab_lo <= 32 * 2 * sm_count(current_device()), rows = few ? 8 : 32;
+    const dim3 grid((vocab_hi - vocab_lo + rows - 1) / rows);
     const bool pieces = !(H & 7) && !(reinterpret_cast<uintptr_t>(dout) & 15) && !(reinterpret_cast<uintptr_t>(dE) & 15);
-    launch_early(pieces ? embed_bwd_kernel<8> : embed_bwd_kernel<1>, grid, 256, 0, (cudaStream_t)stream, tokens,
+    launch_early(pieces ? (few ? embed_bwd_kernel<8, 8> : embed_bwd_kernel<8, 32>) : few ? embed_bwd_kernel<1, 8> : embed_bwd_kernel<1, 32>, grid, 256, 0, (cudaStream_t)stream, tokens,
                  (const __nv_bfloat16*)dout, dE, T, H, vocab_lo, vocab_hi);
     CAI_LAUNCH_CHECK("embed_bwd");
     return CAI_K_OK;
