@@ -211,19 +211,36 @@ reduce_parts_kernel(const float* __restrict__ parts, float* __restrict__ out, in
 // two-kernel form above reads them twice), the old dx together with them. Two CTAs of eight warps share an SM.
 // What bounds it is bytes in flight, and for few rows the combination of the sums: warps that took turns adding into one
 // row, eight lanes to a bank, needed 3 us more.
-// With an accumulated dx and cold caches, 16384 x 2048: 74.8 -> 58.5 us (4.6 TB/s), 3840 x 1000: 15.6 -> 12.8 us.
+// With an accumulated dx and cold caches, 16384 x 2048: 74.8 -> 58.5 us (4.6 TB/s), 3840 x 1000: 15.6 -> 12.8 us (before rows came ahead).
 // Beside a product of another stream it runs on the SMs that one leaves free: none of its CTAs was seen to share an SM with a
 // persistent product's, whatever the shared memory either asks for.
 constexpr int kNormFusedThreads = 256;
 constexpr int kNormFusedCols = 1024;   // columns one warp covers: 32 lanes x 4 chunks x 8 elements
 constexpr int kNormFusedMaxH = 8192;
+constexpr int kNormStageBytes = 8 * kNormFusedCols * 2;   // a tensor's rows of one round: neighbours in memory, at most 8 x 1024 elements
+// kStaged: a CTA's rows of the next round are on their way to shared memory, one bulk copy for each tensor, while this round's are worked on from
+// registers. A warp that loads its own has nothing in flight while it computes and writes. us with the reduction, before /
+// now, dx accumulated and written: 16384 x 2048 61.3 / 55.6 and 56.2 / 48.7 (4.8 and 4.1 TB/s), 5000 x 8192 77.6 / 72.5 and 69.9 / 62.4, 20000 x 256
+// 19.6 / 16.6 and 18.1 / 15.8. Up to two rounds nothing is gained (3840 x 1000 12.8 / 12.9), and a warp loads its own rows.
+template <bool kStaged>
 static __global__ void __launch_bounds__(kNormFusedThreads, 2)
 rmsnorm_bwd_fused_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ g,
                          const float* __restrict__ rstd, const __nv_bfloat16* __restrict__ dy,
-                         __nv_bfloat16* __restrict__ dx, float* __restrict__ dg_partial, int rows, int H, int dx_acc, int R) {
-    grid_dep_begin();
-    extern __shared__ float sdg[];   // [warp][chunk * 8 + element][lane]: a warp's column sums, no two lanes on one bank
+                         __nv_bfloat16* dx, float* __restrict__ dg_partial, int rows, int H, int dx_acc, int R, int* status) {
+    extern __shared__ __align__(16) float sdg[];   // [warp][chunk * 8 + element][lane]: a warp's column sums, no two lanes on one bank
     __shared__ float part[8];
+    __shared__ uint64_t landed;
+    __shared__ volatile int abort_flag;
+    uint8_t* const stage = reinterpret_cast<uint8_t*>(sdg + 8 * kNormFusedCols);   // x, dy, dx
+    if constexpr (kStaged) {
+        if (threadIdx.x == 0) {
+            mbar_init(&landed, 1);
+            abort_flag = 0;
+            mbar_fence_init();
+        }
+        __syncthreads();
+    }
+    grid_dep_begin();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int groups = 8 / R;                 // rows a CTA works on at a time
     const int grp = warp / R, sub = warp - grp * R;
@@ -235,23 +252,46 @@ rmsnorm_bwd_fused_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat1
     for (int c = 0; c < 4; ++c)
 #pragma unroll
         for (int e = 0; e < 8; ++e) acc[c][e] = 0.f;
-    for (long long base = static_cast<long long>(blockIdx.x) * groups; base < rows; base += static_cast<long long>(gridDim.x) * groups) {
+    // one thread fetches the rows from `first` on
+    auto fetch = [&](long long first) {
+        const uint32_t bytes = static_cast<uint32_t>(rows - first < groups ? rows - first : groups) * static_cast<uint32_t>(H) * 2u;
+        mbar_expect_tx(&landed, dx_acc ? 3 * bytes : 2 * bytes);
+        bulk_load(stage, x + first * H, bytes, &landed);
+        bulk_load(stage + kNormStageBytes, dy + first * H, bytes, &landed);
+        if (dx_acc) bulk_load(stage + 2 * kNormStageBytes, dx + first * H, bytes, &landed);
+    };
+    const long long step = static_cast<long long>(gridDim.x) * groups;
+    uint32_t round = 0;
+    if (kStaged && threadIdx.x == 0 && static_cast<long long>(blockIdx.x) * groups < rows) fetch(static_cast<long long>(blockIdx.x) * groups);
+    for (long long base = static_cast<long long>(blockIdx.x) * groups; base < rows; base += step, ++round) {
         const long long row = base + grp;
         const bool live = active && row < rows;
         uint4 xv[4], dv[4], old[4];
         float S = 0.f;
+        const float rr = live ? rstd[row] : 0.f;      // asked for here: behind the sum it would be waited for
+        if (kStaged && !mbar_wait(&landed, round & 1, &abort_flag, status, CAI_DEV_TIMEOUT_TMA_FULL)) {
+            // a copy that does not come: the status word says so; it is given time to land before the CTA's memory goes
+            for (int i = 0; i < 32; ++i) __nanosleep(50000);
+        }
         if (live) {
-            const uint4* xr = reinterpret_cast<const uint4*>(x + row * H);
-            const uint4* dyr = reinterpret_cast<const uint4*>(dy + row * H);
+            const uint4* xr = reinterpret_cast<const uint4*>(kStaged ? reinterpret_cast<const __nv_bfloat16*>(stage) + grp * H : x + row * H);
+            const uint4* dyr = reinterpret_cast<const uint4*>(kStaged ? reinterpret_cast<const __nv_bfloat16*>(stage + kNormStageBytes) + grp * H : dy + row * H);
+            const uint4* oldr = reinterpret_cast<const uint4*>(kStaged ? reinterpret_cast<const __nv_bfloat16*>(stage + 2 * kNormStageBytes) + grp * H : dx + row * H);
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
                 const int col = col0 + (c * 32 + lane) * 8;
                 if (col < H) {
                     xv[c] = xr[col >> 3];
                     dv[c] = dyr[col >> 3];
-                    if (dx_acc) old[c] = reinterpret_cast<const uint4*>(dx + row * H)[col >> 3];
+                    if (dx_acc) old[c] = oldr[col >> 3];
                 }
             }
+        }
+        if (kStaged) {
+            __syncthreads();      // everybody has this round's rows in registers
+            if (threadIdx.x == 0 && base + step < rows) fetch(base + step);
+        }
+        if (live) {
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
                 const int col = col0 + (c * 32 + lane) * 8;
@@ -276,7 +316,6 @@ rmsnorm_bwd_fused_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat1
             __syncthreads();
         }
         if (live) {
-            const float rr = rstd[row];
             const float k3 = rr * rr * rr * S / H;
             uint4* dxr = reinterpret_cast<uint4*>(dx + row * H);
 #pragma unroll
@@ -330,10 +369,19 @@ static inline int launch_rmsnorm_bwd(const void* x, const void* g, const float* 
         int grid = static_cast<int>(want < 2LL * sms ? want : 2LL * sms);
         if (grid > parts_cap) grid = parts_cap;
         if (grid < 1) grid = 1;
-        constexpr size_t smem = 8 * kNormFusedCols * sizeof(float);
-        launch_early(rmsnorm_bwd_fused_kernel, grid, kNormFusedThreads, smem, st, static_cast<const __nv_bfloat16*>(x),
-                     static_cast<const __nv_bfloat16*>(g), rstd, static_cast<const __nv_bfloat16*>(dy), static_cast<__nv_bfloat16*>(dx),
-                     scratch, rows, H, dx_accumulate, Rf);
+        constexpr size_t smem = 8 * kNormFusedCols * sizeof(float), smem_staged = smem + 3 * kNormStageBytes;
+        const bool staged = want > 2LL * grid;             // three rounds and more
+        if (staged) {
+            static bool configured[64] = {};
+            const int dev = current_device();
+            if (!configured[dev & 63]) {
+                if (cudaFuncSetAttribute(rmsnorm_bwd_fused_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem_staged)) != cudaSuccess) return 1;
+                configured[dev & 63] = true;
+            }
+        }
+        launch_early(staged ? rmsnorm_bwd_fused_kernel<true> : rmsnorm_bwd_fused_kernel<false>, grid, kNormFusedThreads, staged ? smem_staged : smem, st,
+                     static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(g), rstd, static_cast<const __nv_bfloat16*>(dy),
+                     static_cast<__nv_bfloat16*>(dx), scratch, rows, H, dx_accumulate, Rf, status_words(current_device()));
         launch_early(reduce_parts_kernel, (H + 31) / 32, kReduceWarps * 32, 0, st, scratch, dg, grid, H, dg_accumulate);
         return cudaGetLastError() == cudaSuccess ? 0 : 1;
     }

@@ -157,8 +157,9 @@ def test_adamw_matches_reference_rule():
     assert torch.equal(pb, p.to(torch.bfloat16))
 
 
-# Rows handled by 1, 2, 4 and 8 warps; fewer rows than warps, ragged last chunks, an accumulated dx and gain gradient.
-@pytest.mark.parametrize("rows,H", [(1, 8), (5, 1000), (300, 1032), (77, 3000), (33, 8192)])
+# Rows handled by 1, 2, 4 and 8 warps; fewer rows than warps, ragged last chunks, an accumulated dx and gain gradient; and rows enough for three rounds of
+# every CTA, where they come ahead by bulk copies, the last round not full.
+@pytest.mark.parametrize("rows,H", [(1, 8), (5, 1000), (300, 1032), (77, 3000), (33, 8192), (4737, 8), (7500, 1000), (2500, 1032), (1201, 3000), (650, 8192)])
 def test_rmsnorm_bwd_sums(rows, H):
     from cai_b200 import ops
     torch.manual_seed(7)
