@@ -303,8 +303,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm, const AttnFwdParams p) {
 // the critical path of the heaviest CTA. One CTA owns ONE query tile, the scores are double buffered in tensor
 // memory and the MMA warp runs one key block ahead: S(j+1) = Q K(j+1)^T is issued before the softmax of block
 // j has finished, so a step of the chain costs a softmax, not a softmax plus two MMAs plus two barrier round
-// trips. O is rescaled only after the P V of the previous block has completed (own barrier, waited for in
-// the rare rescale path, otherwise at the end of the step when it has long completed).
+// trips. O is rescaled only after the P V of the previous block has completed (barriers of its own, waited for in
+// the rare rescale path and at the end).
 //
 // TMEM map: S0/P0 0-127, S1/P1 128-255, O 256-383.
 constexpr int kAttnFwd1Threads = 256;
@@ -324,8 +324,12 @@ attn_fwd1_kernel(const __grid_constant__ CUtensorMap tm, const AttnFwdParams p) 
     uint64_t* v_empty = bars + 7;
     uint64_t* s_full = bars + 9;    // [2] scores of a block are in S[b]
     uint64_t* p_full = bars + 11;   // [2] probabilities of a block are in S[b]
-    uint64_t* pv_done = bars + 13;  // P V of a block has completed (O may be touched)
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 14);
+    // [2] P V of a block has completed (O may be touched), for even and for odd blocks. A warp that waits for block j - 1 has seen S(j), issued behind the
+    // P V of block j - 2, and has not arrived for block j + 1: its barrier is in that phase or has just left it. (With a single barrier, waited for
+    // behind the arrival for block j, the P V of block j could complete first; the parity of j - 1 was then that of a phase that
+    // needed this warp's next arrival, and the CTA waited until its bound ran out.)
+    uint64_t* pv_done = bars + 13;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -350,7 +354,8 @@ attn_fwd1_kernel(const __grid_constant__ CUtensorMap tm, const AttnFwdParams p) 
             mbar_init(&s_full[i], 1);
             mbar_init(&p_full[i], 4);
         }
-        mbar_init(pv_done, 1);
+        mbar_init(&pv_done[0], 1);
+        mbar_init(&pv_done[1], 1);
         *abort_flag = 0;
         mbar_fence_init();
     }
@@ -419,7 +424,7 @@ attn_fwd1_kernel(const __grid_constant__ CUtensorMap tm, const AttnFwdParams p) 
                 tc_fence_after();
                 issue_pv(tO, tS[slot], sV0 + slot * kAttnTileBytes, idesc_pv, j > 0);
                 umma_commit(&v_empty[slot]);
-                umma_commit(pv_done);
+                umma_commit(&pv_done[slot]);
             }
         }
     } else if (warp >= 4) {
@@ -456,14 +461,12 @@ attn_fwd1_kernel(const __grid_constant__ CUtensorMap tm, const AttnFwdParams p) 
                         if (c * 32 + e <= r) mx = fmaxf(mx, __uint_as_float(sc[c][e]));
             }
             const float m_new = fmaxf(m_used, mx * p.scale_log2);
-            bool waited_pv = false;
             if (__any_sync(0xffffffffu, m_new > m_used + 8.f)) {
                 const float alpha = fast_exp2(m_used - m_new);  // 0 on the first block
                 l *= alpha;
                 if (j > 0) {
                     // O is complete up to block j-1 only when that block's P V has finished
-                    if (!mbar_wait_warp(pv_done, (j - 1) & 1, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN)) { ok = false; break; }
-                    waited_pv = true;
+                    if (!mbar_wait_warp(&pv_done[(j - 1) & 1], ((j - 1) >> 1) & 1, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN)) { ok = false; break; }
                     tc_fence_after();
 #pragma unroll 1
                     for (int c = 0; c < 4; ++c) {
@@ -500,11 +503,8 @@ attn_fwd1_kernel(const __grid_constant__ CUtensorMap tm, const AttnFwdParams p) 
             tmem_st_wait();
             tc_fence_before();
             mbar_arrive_warp(&p_full[j & 1]);
-            // every phase of pv_done is consumed exactly once per step, so its parity never runs ahead
-            if (j > 0 && !waited_pv &&
-                !mbar_wait_warp(pv_done, (j - 1) & 1, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN)) { ok = false; break; }
         }
-        if (ok && mbar_wait_warp(pv_done, (n - 1) & 1, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN)) {
+        if (ok && mbar_wait_warp(&pv_done[(n - 1) & 1], ((n - 1) >> 1) & 1, abort_flag, p.status, CAI_DEV_TIMEOUT_ATTN)) {
             tc_fence_after();
             const float inv = 1.f / l;
             const long long ldo = static_cast<long long>(p.nh) * kAttnHD;
