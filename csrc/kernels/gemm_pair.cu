@@ -12,7 +12,7 @@
 // issues the MMAs, warps 2-9 drain the accumulator. Two accumulators per CTA in TMEM let the epilogue of a tile overlap the
 // main loop of the next. The epilogue goes through shared memory and leaves by TMA: full 128-byte rows instead of 16 bytes per
 // lane, edges clipped by the tensor map, the fp32 accumulation into C as a TMA reduction in L2 (one rounding and subnormals kept,
-// like a load and an add); the residual is read into registers while the main loop still runs. (bf16 stores straight from the
+// like a load and an add); the residual is read into registers while the main loop still runs, whole rows at a time. (bf16 stores straight from the
 // registers, a 32-byte sector per lane, measured the same on aligned rows and up to 20 % slower on rows of 2000 bytes.)
 //
 // Measured against the one-CTA kernel (L2 flushed): 8192^3 812 -> 706 us (1556 TFLOP/s), 16384 x 2048 x 16384 1062 -> 712 us,
@@ -521,14 +521,16 @@ gemm_pair_kernel(const __grid_constant__ PairLaunch<kProducts> launch) {
             const bool live = mine && row0 < p.M;
             const int col_first = tn * BN + half * HALF;
             const bool residual = (kKind == kPairBf16 || kKind == kPairAny) && p.epi == CAI_EPI_BF16_RESIDUAL;
-            // this lane's row of the residual: the first 64 columns come in while the main loop runs
-            const bool res_ok = residual && mine && row0 + lane < p.M;
-            const __nv_bfloat16* rrow = p.R + (static_cast<long long>(grp) * p.grp_c + row0 + lane) * p.ldr;
+            // the residual of 64 columns, eight lanes to a row of 128 bytes; the first 64 come in while the main loop runs. They reach the lanes that
+            // own the rows through the box. (A row per lane met 32 lines a load. us, before / now, without a residual:
+            // 3840 x 5456 x 1000 50.6 / 47.9, 43.6; 4096 x 4096 x 1024 32.4 / 31.2, 28.8; 3840 x 1000 x 2728 25.3 / 24.2, 23.3.)
+            const __nv_bfloat16* rfirst = p.R + (static_cast<long long>(grp) * p.grp_c + row0 + (lane >> 3)) * p.ldr + (lane & 7) * 8;
             uint4 res[8];
             auto fetch = [&](int col) {
 #pragma unroll
-                for (int j = 0; j < 8; ++j)
-                    if (res_ok && col + j * 8 < p.N) res[j] = *reinterpret_cast<const uint4*>(rrow + col + j * 8);
+                for (int i = 0; i < 8; ++i)
+                    if (mine && row0 + i * 4 + (lane >> 3) < p.M && col + (lane & 7) * 8 < p.N)
+                        res[i] = *reinterpret_cast<const uint4*>(rfirst + static_cast<long long>(i * 4) * p.ldr + col);
             };
             if (residual) fetch(col_first);
             if (!mbar_wait_warp(&tmem_full[acc], acc_ph, abort_flag, shared.status, CAI_DEV_TIMEOUT_TMEM_FULL)) {
@@ -595,6 +597,15 @@ gemm_pair_kernel(const __grid_constant__ PairLaunch<kProducts> launch) {
                         }
                         if (lane == 0) tma_store_wait_read0();
                         __syncwarp();
+                        if (residual) {
+#pragma unroll
+                            for (int i = 0; i < 8; ++i) {
+                                const int r4 = i * 4 + (lane >> 3);
+                                st_shared_v4(smem_u32(box) + r4 * 128 + (((lane ^ r4) & 7) << 4), res[i].x, res[i].y, res[i].z, res[i].w);
+                            }
+                            __syncwarp();
+                            if (c + 64 < HALF) fetch(col + 64);
+                        }
 #pragma unroll
                         for (int k = 0; k < 8; ++k) {
                             float v[8];
@@ -602,7 +613,7 @@ gemm_pair_kernel(const __grid_constant__ PairLaunch<kProducts> launch) {
                             for (int e = 0; e < 8; ++e) v[e] = __uint_as_float(r[k >> 2][(k & 3) * 8 + e]) * p.alpha;
                             const uint32_t at = box_row + ((k ^ sw) << 4);
                             if (residual) {
-                                const uint4 rv = res[k];
+                                const uint4 rv = ld_shared_v4(at);
                                 v[0] += bf16_lo(rv.x); v[1] += bf16_hi(rv.x);
                                 v[2] += bf16_lo(rv.y); v[3] += bf16_hi(rv.y);
                                 v[4] += bf16_lo(rv.z); v[5] += bf16_hi(rv.z);
@@ -610,7 +621,6 @@ gemm_pair_kernel(const __grid_constant__ PairLaunch<kProducts> launch) {
                             }
                             st_shared_v4(at, pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
                         }
-                        if (residual && c + 64 < HALF) fetch(col + 64);
                         fence_proxy_async_smem();
                         __syncwarp();
                         if (lane == 0) {
