@@ -219,7 +219,8 @@ CAI_API int cai_flash_attn_bwd(const void* qkv, const void* out, const void* dou
  * capture. */
 CAI_API int cai_flash_attn_bwd_parts(const void* qkv, const void* out, const void* dout, const float* lse, float* delta,
                                      void* dqkv, int B, int S, int nh, int nkv, int hd, float scale, int parts, void* stream);
-/* The same, and dQ and dK rotated back (cai_rope_apply with inverse = 1) where a table is given: its results, bit for bit, without the pass. */
+/* The same, and dQ and dK rotated back (cai_rope_apply with inverse = 1) where a table is given (it starts on 16 bytes): its results, bit for
+ * bit, without the pass. */
 CAI_API int cai_flash_attn_bwd_rope(const void* qkv, const void* out, const void* dout, const float* lse, float* delta, void* dqkv,
                                     const float* table, int B, int S, int nh, int nkv, int hd, float scale, int parts, void* stream);
 #endif /* CAI_KERNELS_H */

@@ -793,6 +793,10 @@ CAI_API int cai_flash_attn_bwd_rope(const void* qkv, const void* out, const void
         return CAI_K_BAD_ARG;
     }
     if (B <= 0 || S <= 0) return CAI_K_OK;
+    if (reinterpret_cast<uintptr_t>(table) & 15) {
+        set_last_error("flash_attn_bwd: the rotary table must start on 16 bytes");
+        return CAI_K_BAD_ARG;
+    }
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const long long ld = static_cast<long long>(nh + 2 * nkv) * hd;
     const long long ldo = static_cast<long long>(nh) * hd;
