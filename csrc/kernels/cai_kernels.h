@@ -148,6 +148,20 @@ CAI_API int cai_rmsnorm_bwd(const void* x, const void* g, const float* rstd, con
                             float* dg, float* dg_partial, int rows, int H, int dx_accumulate,
                             int dg_accumulate, void* stream);
 
+/* The same in two steps, for callers with several of them in a chain: dx and the partial sums of dg (`parts` rows of H floats, as many as
+ * cai_rmsnorm_bwd_partial_rows says; 0 where H has no such form), then up to CAI_DG_SUMS sums of one width in one launch. The results are
+ * those of cai_rmsnorm_bwd. Sums of one launch must not name one dg twice. */
+#define CAI_DG_SUMS 8
+typedef struct {
+    const float* partial;
+    float* dg;
+    int parts, accumulate;
+} cai_dg_sum;
+CAI_API int cai_rmsnorm_bwd_partial_rows(int rows, int H);
+CAI_API int cai_rmsnorm_bwd_partial(const void* x, const void* g, const float* rstd, const void* dy, void* dx, float* dg_partial, int rows,
+                                    int H, int dx_accumulate, void* stream);
+CAI_API int cai_rmsnorm_dg_sums(const cai_dg_sum* sums, int n, int H, void* stream);
+
 /* ---- rotary embedding, in place on the q and k heads of a packed [T, (nh+2*nkv)*hd] buffer.
  * table is float2 [seq, hd/2] (cos, sin); position of row t is t % seq. inverse=1 applies the
  * transpose rotation (backward). */

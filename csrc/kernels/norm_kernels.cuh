@@ -179,9 +179,17 @@ rmsnorm_bwd_dg_kernel(const __nv_bfloat16* __restrict__ x, const float* __restri
 // dependent loads in a row (eight warps with four chains each: 296 rows of 1000 and of 2048 columns, cold
 // caches, 10.6 and 10.3 -> 5.5 us). Chains are added in fours, the eight sums in order.
 constexpr int kReduceWarps = 32;
+// Several sums of one width go out together, one to a row of blocks: in a chain of short kernels each launch costs what it takes.
+struct ReduceJobs {
+    cai_dg_sum job[CAI_DG_SUMS];
+};
 static __global__ void __launch_bounds__(kReduceWarps * 32)
-reduce_parts_kernel(const float* __restrict__ parts, float* __restrict__ out, int nparts, int H, int accumulate) {
+reduce_parts_kernel(const __grid_constant__ ReduceJobs jobs, int H) {
     grid_dep_begin();
+    const cai_dg_sum& job = jobs.job[blockIdx.y];
+    const float* __restrict__ parts = job.partial;
+    float* __restrict__ out = job.dg;
+    const int nparts = job.parts, accumulate = job.accumulate;
     __shared__ float acc[kReduceWarps][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int w = warp & 7, k = warp >> 3;
@@ -355,6 +363,46 @@ rmsnorm_bwd_fused_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat1
     }
 }
 
+static inline int launch_reduce_parts(const cai_dg_sum* sums, int n, int H, cudaStream_t st) {
+    ReduceJobs jobs = {};
+    for (int i = 0; i < n; ++i) jobs.job[i] = sums[i];
+    launch_early(reduce_parts_kernel, dim3((H + 31) / 32, n), kReduceWarps * 32, 0, st, jobs, H);
+    return cudaGetLastError() == cudaSuccess ? 0 : 1;
+}
+
+// Rows of partial sums that the one-sweep form writes.
+static inline int rmsnorm_fused_row_warps(int H) {
+    const int R = (H + kNormFusedCols - 1) / kNormFusedCols;
+    return R <= 1 ? 1 : R <= 2 ? 2 : R <= 4 ? 4 : 8;         // a divisor of the CTA's eight warps
+}
+static inline int rmsnorm_fused_parts(int rows, int H, int parts_cap, int sms) {
+    const int groups = 8 / rmsnorm_fused_row_warps(H);
+    const long long want = (static_cast<long long>(rows) + groups - 1) / groups;
+    int grid = static_cast<int>(want < 2LL * sms ? want : 2LL * sms);
+    if (grid > parts_cap) grid = parts_cap;
+    return grid < 1 ? 1 : grid;
+}
+// The one-sweep form without the reduction of its `grid` partial rows.
+static inline int launch_rmsnorm_sweep(const void* x, const void* g, const float* rstd, const void* dy, void* dx, float* partial, int grid, int rows, int H,
+                                       int dx_accumulate, cudaStream_t st) {
+    const int Rf = rmsnorm_fused_row_warps(H), groups = 8 / Rf;
+    const long long want = (static_cast<long long>(rows) + groups - 1) / groups;
+    constexpr size_t smem = 8 * kNormFusedCols * sizeof(float), smem_staged = smem + 3 * kNormStageBytes;
+    const bool staged = want > 2LL * grid;                 // three rounds and more
+    if (staged) {
+        static bool configured[64] = {};
+        const int dev = current_device();
+        if (!configured[dev & 63]) {
+            if (cudaFuncSetAttribute(rmsnorm_bwd_fused_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem_staged)) != cudaSuccess) return 1;
+            configured[dev & 63] = true;
+        }
+    }
+    launch_early(staged ? rmsnorm_bwd_fused_kernel<true> : rmsnorm_bwd_fused_kernel<false>, grid, kNormFusedThreads, staged ? smem_staged : smem, st,
+                 static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(g), rstd, static_cast<const __nv_bfloat16*>(dy),
+                 static_cast<__nv_bfloat16*>(dx), partial, rows, H, dx_accumulate, Rf, status_words(current_device()));
+    return cudaGetLastError() == cudaSuccess ? 0 : 1;
+}
+
 // Host side of RMSNorm backward, shared by the entry points: `scratch` holds at most `parts_cap`
 // rows of H floats. Returns a cudaError_t-style 0 / non-zero.
 static inline int launch_rmsnorm_bwd(const void* x, const void* g, const float* rstd, const void* dy, void* dx, float* dg,
@@ -362,28 +410,10 @@ static inline int launch_rmsnorm_bwd(const void* x, const void* g, const float* 
                                      int dg_accumulate, cudaStream_t st) {
     if (H <= kNormFusedMaxH && (H & 7) == 0 && parts_cap >= 1) {
         // one sweep: dx and the partial gain gradients from the same read of x and dy
-        int Rf = (H + kNormFusedCols - 1) / kNormFusedCols;
-        Rf = Rf <= 1 ? 1 : Rf <= 2 ? 2 : Rf <= 4 ? 4 : 8;        // a divisor of the CTA's eight warps
-        const int gpc = 8 / Rf;
-        long long want = (static_cast<long long>(rows) + gpc - 1) / gpc;
-        int grid = static_cast<int>(want < 2LL * sms ? want : 2LL * sms);
-        if (grid > parts_cap) grid = parts_cap;
-        if (grid < 1) grid = 1;
-        constexpr size_t smem = 8 * kNormFusedCols * sizeof(float), smem_staged = smem + 3 * kNormStageBytes;
-        const bool staged = want > 2LL * grid;             // three rounds and more
-        if (staged) {
-            static bool configured[64] = {};
-            const int dev = current_device();
-            if (!configured[dev & 63]) {
-                if (cudaFuncSetAttribute(rmsnorm_bwd_fused_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem_staged)) != cudaSuccess) return 1;
-                configured[dev & 63] = true;
-            }
-        }
-        launch_early(staged ? rmsnorm_bwd_fused_kernel<true> : rmsnorm_bwd_fused_kernel<false>, grid, kNormFusedThreads, staged ? smem_staged : smem, st,
-                     static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(g), rstd, static_cast<const __nv_bfloat16*>(dy),
-                     static_cast<__nv_bfloat16*>(dx), scratch, rows, H, dx_accumulate, Rf, status_words(current_device()));
-        launch_early(reduce_parts_kernel, (H + 31) / 32, kReduceWarps * 32, 0, st, scratch, dg, grid, H, dg_accumulate);
-        return cudaGetLastError() == cudaSuccess ? 0 : 1;
+        const int grid = rmsnorm_fused_parts(rows, H, parts_cap, sms);
+        if (launch_rmsnorm_sweep(x, g, rstd, dy, dx, scratch, grid, rows, H, dx_accumulate, st)) return 1;
+        const cai_dg_sum sum = {scratch, dg, grid, dg_accumulate};
+        return launch_reduce_parts(&sum, 1, H, st);
     }
     const int R = (H + kNormWarpCols - 1) / kNormWarpCols;
     const int groups = 8 / R;
@@ -394,7 +424,8 @@ static inline int launch_rmsnorm_bwd(const void* x, const void* g, const float* 
     parts = (rows + rows_per_part - 1) / rows_per_part;
     launch_early(rmsnorm_bwd_dg_kernel, parts, 256, 0, st, static_cast<const __nv_bfloat16*>(x), rstd,
                  static_cast<const __nv_bfloat16*>(dy), scratch, rows, H, rows_per_part);
-    launch_early(reduce_parts_kernel, (H + 31) / 32, kReduceWarps * 32, 0, st, scratch, dg, parts, H, dg_accumulate);
+    const cai_dg_sum sum = {scratch, dg, parts, dg_accumulate};
+    if (launch_reduce_parts(&sum, 1, H, st)) return 1;
     // dx last: callers may pass dx == dy (in place), and the gain gradient needs the unmodified dy
     launch_early(rmsnorm_bwd_dx_kernel, grid, kNormThreads, 0, st, static_cast<const __nv_bfloat16*>(x),
                  static_cast<const __nv_bfloat16*>(g), rstd, static_cast<const __nv_bfloat16*>(dy), static_cast<__nv_bfloat16*>(dx), rows,

@@ -555,6 +555,38 @@ CAI_API int cai_rmsnorm_bwd(const void* x, const void* g, const float* rstd, con
     return CAI_K_OK;
 }
 
+CAI_API int cai_rmsnorm_bwd_partial_rows(int rows, int H) {
+    if (rows <= 0 || H <= 0 || (H & 7) || H > kNormFusedMaxH) return 0;
+    return rmsnorm_fused_parts(rows, H, cai_rmsnorm_bwd_parts(rows), sm_count(current_device()));
+}
+
+CAI_API int cai_rmsnorm_bwd_partial(const void* x, const void* g, const float* rstd, const void* dy, void* dx, float* dg_partial, int rows,
+                                    int H, int dx_accumulate, void* stream) {
+    const int parts = cai_rmsnorm_bwd_partial_rows(rows, H);
+    if (parts <= 0) {
+        set_last_error("rmsnorm_bwd_partial: H must be a multiple of 8 and <= %d", kNormFusedMaxH);
+        return CAI_K_BAD_ARG;
+    }
+    if (launch_rmsnorm_sweep(x, g, rstd, dy, dx, dg_partial, parts, rows, H, dx_accumulate, (cudaStream_t)stream) != 0) {
+        set_last_error("rmsnorm_bwd_partial launch failed");
+        return CAI_K_CUDA;
+    }
+    return CAI_K_OK;
+}
+
+CAI_API int cai_rmsnorm_dg_sums(const cai_dg_sum* sums, int n, int H, void* stream) {
+    if (n <= 0) return CAI_K_OK;
+    if (n > CAI_DG_SUMS || H <= 0) {
+        set_last_error("rmsnorm_dg_sums: at most %d sums", CAI_DG_SUMS);
+        return CAI_K_BAD_ARG;
+    }
+    if (launch_reduce_parts(sums, n, H, (cudaStream_t)stream) != 0) {
+        set_last_error("rmsnorm_dg_sums launch failed");
+        return CAI_K_CUDA;
+    }
+    return CAI_K_OK;
+}
+
 CAI_API int cai_rope_table(float* table, int seq, int hd, float theta, void* stream) {
     const int half = hd / 2;
     rope_table_kernel<<<blocks_for((long long)seq * half, 256), 256, 0, (cudaStream_t)stream>>>(

@@ -654,6 +654,71 @@ const char* kernel_label(uint16_t k) {
     return k < K_COUNT ? n[k] : "?";
 }
 
+// Sums of gain gradients that are still to go out (RMSNorm backward without its last step): they wait for each other in the rows of the plan's scratch
+// that one norm leaves free, and go out before anything that could name what they read or write. A chain of short kernels is some 5 us shorter for each
+// launch less: a step of 45 launches 298 -> 288 us, 8 layers of 896 tokens, three times over, 3632 -> 3519; 3840 tokens, where two norms fit, no change.
+struct WaitingSums {
+    cai_dg_sum sum[CAI_DG_SUMS];
+    int n = 0, H = 0, stream = 0;
+    const uint8_t *scratch = nullptr, *scratch_end = nullptr;   // the whole scratch
+    float* next = nullptr;                                      // its first free row
+
+    int flush(cai_exec* ex) {
+        if (!n) return 0;
+        const int count = n;
+        n = 0;
+        ex->launches += 1;
+        return cai_rmsnorm_dg_sums(sum, count, H, ex->streams[stream]);
+    }
+    // Must they go out before this operation? Those that only name tensors of their own record are looked at by range; others (whole
+    // buffers, other ranks, other streams) and events count as naming everything.
+    bool before(const cai_exec* ex, const Op& op) const {
+        if (!n) return false;
+        if (op.kind == OP_EVENT_RECORD || op.kind == OP_EVENT_WAIT) return true;
+        if (!op.exec) return false;
+        if (op.stream_id != stream) return true;
+        const ExecOp& x = ex->exec[op.exec - 1];
+        switch (x.kernel) {
+            case K_GEMM: case K_GEMM_FP8: case K_QUANT_FP8: case K_SWIGLU_FWD: case K_SWIGLU_BWD: case K_ATTN_FWD: case K_ATTN_BWD: case K_ROPE:
+            case K_RMSNORM_FWD: case K_RMSNORM_BWD: case K_EMBED_FWD: case K_EMBED_BWD: case K_CROSS_ENTROPY: case K_ADD: break;
+            default: return true;
+        }
+        for (int k = 0; k < static_cast<int>(sizeof x.t / sizeof x.t[0]); ++k) {
+            if (x.t[k] < 0 || (x.kernel == K_RMSNORM_BWD && k == 6)) continue;       // (the scratch itself: add() looks after its rows)
+            const uint8_t *lo = static_cast<const uint8_t*>(ex->ptr(x.t[k])), *hi = lo + ex->tensors[x.t[k]].nbytes;
+            if (lo < scratch_end && scratch < hi) return true;
+            for (int i = 0; i < n; ++i) {
+                const uint8_t *d0 = reinterpret_cast<const uint8_t*>(sum[i].dg), *d1 = d0 + static_cast<size_t>(H) * sizeof(float);
+                if (lo < d1 && d0 < hi) return true;
+            }
+        }
+        return false;
+    }
+    // RMSNorm backward of a record: its sweep now, its sum later. False if the record has no such form.
+    bool add(cai_exec* ex, const Op& op, const ExecOp& x, cudaStream_t st, int* rc) {
+        const int rows = x.i[0], width = x.i[1], parts = cai_rmsnorm_bwd_partial_rows(rows, width);
+        const size_t need = static_cast<size_t>(parts) * width;
+        if (parts <= 0 || need * sizeof(float) > ex->tensors[x.t[6]].nbytes) return false;
+        const uint8_t* at = static_cast<const uint8_t*>(ex->ptr(x.t[6]));
+        const bool fits = n && n < CAI_DG_SUMS && width == H && op.stream_id == stream && at == scratch &&
+                          reinterpret_cast<const uint8_t*>(next + need) <= scratch_end;
+        if (!fits) {
+            if ((*rc = flush(ex)) != 0) return true;
+            H = width;
+            stream = op.stream_id;
+            scratch = at;
+            scratch_end = at + ex->tensors[x.t[6]].nbytes;
+            next = static_cast<float*>(ex->ptr(x.t[6]));
+        }
+        sum[n++] = {next, static_cast<float*>(ex->ptr(x.t[5])), parts, x.i[3]};
+        *rc = cai_rmsnorm_bwd_partial(ex->ptr(x.t[0]), ex->ptr(x.t[1]), static_cast<const float*>(ex->ptr(x.t[2])), ex->ptr(x.t[3]), ex->ptr(x.t[4]), next,
+                                      rows, width, x.i[2], st);
+        next += need;
+        ex->launches += 1;
+        return true;
+    }
+};
+
 int replay(cai_exec* ex) {
     cudaStream_t hi = ex->streams[ST_COMPUTE_HI];
     // fork: every stream the plan uses starts after everything already queued on compute_hi
@@ -661,9 +726,12 @@ int replay(cai_exec* ex) {
     for (int s = 1; s < ST_COUNT; ++s)
         if (ex->used[s]) cudaStreamWaitEvent(ex->streams[s], ex->fork_ev, 0);
     ex->launches = 0;
+    WaitingSums sums;
     for (size_t i = 0; i < ex->ops.size(); ++i) {
         const Op& op = ex->ops[i];
         cudaStream_t st = ex->streams[op.stream_id];
+        if (sums.before(ex, op) || (ex->with_next[i] && sums.before(ex, ex->ops[i + 1])))
+            if (const int rc = sums.flush(ex)) return rc;
         if (op.kind == OP_EVENT_RECORD) {
             if (cudaEventRecord(ex->events[op.aux0], st) != cudaSuccess) return CAI_K_CUDA;
             continue;
@@ -690,6 +758,14 @@ int replay(cai_exec* ex) {
             if (brc != 0) return brc;
         }
         if (ex->nvtx_on) nvtxRangePushA(kernel_label(ex->exec[op.exec - 1].kernel));
+        if (ex->exec[op.exec - 1].kernel == K_RMSNORM_BWD && !tr && !ex->debug_bounds) {
+            int rc = 0;
+            if (sums.add(ex, op, ex->exec[op.exec - 1], st, &rc)) {
+                if (ex->nvtx_on) nvtxRangePop();
+                if (rc != 0) return rc;
+                continue;
+            }
+        }
         if (ex->with_next[i] && !tr && !ex->debug_bounds && ex->sm_limit_hi <= 0 && !ex->has_pending_gather) {
             const ExecOp &x = ex->exec[op.exec - 1], &next = ex->exec[ex->ops[i + 1].exec - 1];
             int rc, launches = 1, cols;
@@ -720,6 +796,7 @@ int replay(cai_exec* ex) {
         }
         if (tr) cudaEventRecord(tr->stop, st);
     }
+    if (const int rc = sums.flush(ex)) return rc;
     // join: compute_hi waits for every other one of them
     for (int s = 1; s < ST_COUNT; ++s) {
         if (!ex->used[s]) continue;

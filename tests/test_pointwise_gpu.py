@@ -193,3 +193,33 @@ def test_embed_bwd_adds_in_token_order(T, V, H, lo, hi):
         if lo <= tok < hi:
             want[tok - lo] += dout[t].float()      # fp32, in this order: equal to the last bit
     assert torch.equal(got, want)
+
+
+# RMSNorm backward in two steps, the sums of several norms in one launch, against one call each: the same bits. Few rows and many (rows that come ahead),
+# written and accumulated gains, as many sums as a launch takes.
+@pytest.mark.parametrize("rows,H,n", [(1, 8, 1), (300, 1000, 3), (512, 256, 8), (5000, 1032, 2), (40, 8192, 2)])
+def test_rmsnorm_gain_sums_together(rows, H, n):
+    import ctypes
+    from cai_b200 import ops
+
+    class Sum(ctypes.Structure):
+        _fields_ = [("partial", ctypes.c_void_p), ("dg", ctypes.c_void_p), ("parts", ctypes.c_int), ("accumulate", ctypes.c_int)]
+
+    L, st = ops.lib(), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    parts = L.cai_rmsnorm_bwd_partial_rows(rows, H)
+    assert 0 < parts <= L.cai_rmsnorm_bwd_parts(rows) and L.cai_rmsnorm_bwd_partial_rows(rows, 8200) == 0
+    scratch, sums, want, got, keep = torch.full((n * parts, H), 9.0, device="cuda"), (Sum * n)(), [], [], []
+    for i in range(n):
+        torch.manual_seed(i)
+        x, dy, dx0 = (torch.randn(rows, H, device="cuda").to(torch.bfloat16) for _ in range(3))
+        g, rstd, dg0 = torch.randn(H, device="cuda").to(torch.bfloat16), torch.rand(rows, device="cuda") + 0.5, torch.randn(H, device="cuda")
+        want.append(ops.rmsnorm_bwd(x, g, rstd, dy, dx=dx0.clone(), dg=dg0.clone(), dx_accumulate=i % 2 == 0, dg_accumulate=i % 3 == 0))
+        got.append((dx0.clone(), dg0.clone()))
+        at = scratch[i * parts:]
+        assert L.cai_rmsnorm_bwd_partial(*(ctypes.c_void_p(t.data_ptr()) for t in (x, g, rstd, dy, got[i][0], at)), rows, H, int(i % 2 == 0), st) == 0
+        sums[i] = Sum(at.data_ptr(), got[i][1].data_ptr(), parts, int(i % 3 == 0))
+        keep.append((x, g, rstd, dy))
+    assert L.cai_rmsnorm_dg_sums(sums, n, H, st) == 0 and L.cai_rmsnorm_dg_sums(sums, 9, H, st) < 0
+    for (wx, wg), (gx, gg) in zip(want, got):
+        assert torch.equal(wx, gx) and torch.equal(wg, gg)
+    assert ops.device_status() == 0
