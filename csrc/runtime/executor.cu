@@ -656,7 +656,7 @@ const char* kernel_label(uint16_t k) {
 
 // Sums of gain gradients that are still to go out (RMSNorm backward without its last step): they wait for each other in the rows of the plan's scratch
 // that one norm leaves free, and go out before anything that could name what they read or write. A chain of short kernels is some 5 us shorter for each
-// launch less: a step of 45 launches 298 -> 288 us, 8 layers of 896 tokens, three times over, 3632 -> 3519; 3840 tokens, where two norms fit, no change.
+// launch less: a step of 47 launches 298 -> 288 us, 8 layers of 896 tokens, three times over, 3632 -> 3519; 3840 tokens, where two norms fit, no change.
 struct WaitingSums {
     cai_dg_sum sum[CAI_DG_SUMS];
     int n = 0, H = 0, stream = 0;
@@ -694,11 +694,14 @@ struct WaitingSums {
         }
         return false;
     }
-    // RMSNorm backward of a record: its sweep now, its sum later. False if the record has no such form.
+    // RMSNorm backward of a record: its sweep now, its sum later. False if the record has no such form (and no sum waits any more).
     bool add(cai_exec* ex, const Op& op, const ExecOp& x, cudaStream_t st, int* rc) {
         const int rows = x.i[0], width = x.i[1], parts = cai_rmsnorm_bwd_partial_rows(rows, width);
         const size_t need = static_cast<size_t>(parts) * width;
-        if (parts <= 0 || need * sizeof(float) > ex->tensors[x.t[6]].nbytes) return false;
+        if (parts <= 0 || need * sizeof(float) > ex->tensors[x.t[6]].nbytes) {
+            *rc = flush(ex);          // the whole form uses the scratch from its beginning
+            return *rc != 0;
+        }
         const uint8_t* at = static_cast<const uint8_t*>(ex->ptr(x.t[6]));
         const bool fits = n && n < CAI_DG_SUMS && width == H && op.stream_id == stream && at == scratch &&
                           reinterpret_cast<const uint8_t*>(next + need) <= scratch_end;
