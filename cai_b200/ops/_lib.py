@@ -2,7 +2,7 @@
 
 The library is built in-tree by :mod:`cai_b200._build`. Loading it never needs a GPU; launching
 does. If the library is missing the import of this module fails loudly rather than falling back
-to PyTorch ops: on a GPU box the CUDA path is the only path.
+to PyTorch ops: where there is a GPU the CUDA path is the only path.
 """
 from __future__ import annotations
 
