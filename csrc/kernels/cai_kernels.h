@@ -161,6 +161,10 @@ CAI_API int cai_rmsnorm_bwd_partial_rows(int rows, int H);
 CAI_API int cai_rmsnorm_bwd_partial(const void* x, const void* g, const float* rstd, const void* dy, void* dx, float* dg_partial, int rows,
                                     int H, int dx_accumulate, void* stream);
 CAI_API int cai_rmsnorm_dg_sums(const cai_dg_sum* sums, int n, int H, void* stream);
+/* What CTA `cta` of `ctas` does in the form whose rows come ahead, in order: two ints an event, 0 and the first row it fetches or 1 and the first row
+ * it works on. The wait for the rows of round `lost_round` (-1: none) runs out. Returns the number of events, of which `capacity` are
+ * written. Needs no GPU. */
+CAI_API int cai_rmsnorm_bwd_rounds(int rows, int H, int ctas, int cta, int lost_round, int* events, int capacity);
 
 /* ---- rotary embedding, in place on the q and k heads of a packed [T, (nh+2*nkv)*hd] buffer.
  * table is float2 [seq, hd/2] (cos, sin); position of row t is t % seq. inverse=1 applies the

@@ -226,6 +226,17 @@ constexpr int kNormFusedThreads = 256;
 constexpr int kNormFusedCols = 1024;   // columns one warp covers: 32 lanes x 4 chunks x 8 elements
 constexpr int kNormFusedMaxH = 8192;
 constexpr int kNormStageBytes = 8 * kNormFusedCols * 2;   // a tensor's rows of one round: neighbours in memory, at most 8 x 1024 elements
+// A CTA's rounds. Rows that did not come (a wait that ran out) are neither used nor followed by more: the phase of the barrier that they belong to is still
+// open. The barrier behind the wait tells all threads alike (a word of shared memory read behind it cost 0.1 us a round).
+struct NormRounds {
+    struct Next { bool use, fetch; };
+    long long first, step;         // first row of the round; rows that all CTAs take in one
+    int rows;
+    __host__ __device__ __forceinline__ NormRounds(int cta, int ctas, int groups, int rows_)
+        : first(static_cast<long long>(cta) * groups), step(static_cast<long long>(ctas) * groups), rows(rows_) {}
+    __host__ __device__ __forceinline__ bool more() const { return first < rows; }
+    __host__ __device__ __forceinline__ Next behind_wait(bool came) const { return {came, came && first + step < rows}; }
+};
 // kStaged: a CTA's rows of the next round are on their way to shared memory, one bulk copy for each tensor, while this round's are worked on from
 // registers. A warp that loads its own has nothing in flight while it computes and writes. us with the reduction, before /
 // now, dx accumulated and written: 16384 x 2048 61.3 / 55.6 and 56.2 / 48.7 (4.8 and 4.1 TB/s), 5000 x 8192 77.6 / 72.5 and 69.9 / 62.4, 20000 x 256
@@ -268,19 +279,16 @@ rmsnorm_bwd_fused_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat1
         bulk_load(stage + kNormStageBytes, dy + first * H, bytes, &landed);
         if (dx_acc) bulk_load(stage + 2 * kNormStageBytes, dx + first * H, bytes, &landed);
     };
-    const long long step = static_cast<long long>(gridDim.x) * groups;
+    NormRounds r(static_cast<int>(blockIdx.x), static_cast<int>(gridDim.x), groups, rows);
     uint32_t round = 0;
-    if (kStaged && threadIdx.x == 0 && static_cast<long long>(blockIdx.x) * groups < rows) fetch(static_cast<long long>(blockIdx.x) * groups);
-    for (long long base = static_cast<long long>(blockIdx.x) * groups; base < rows; base += step, ++round) {
-        const long long row = base + grp;
+    if (kStaged && threadIdx.x == 0 && r.more()) fetch(r.first);
+    for (; r.more(); r.first += r.step, ++round) {
+        const long long row = r.first + grp;
         const bool live = active && row < rows;
         uint4 xv[4], dv[4], old[4];
         float S = 0.f;
         const float rr = live ? rstd[row] : 0.f;      // asked for here: behind the sum it would be waited for
-        if (kStaged && !mbar_wait(&landed, round & 1, &abort_flag, status, CAI_DEV_TIMEOUT_TMA_FULL)) {
-            // a copy that does not come: the status word says so; it is given time to land before the CTA's memory goes
-            for (int i = 0; i < 32; ++i) __nanosleep(50000);
-        }
+        const bool came = !kStaged || mbar_wait(&landed, round & 1, &abort_flag, status, CAI_DEV_TIMEOUT_TMA_FULL);
         if (live) {
             const uint4* xr = reinterpret_cast<const uint4*>(kStaged ? reinterpret_cast<const __nv_bfloat16*>(stage) + grp * H : x + row * H);
             const uint4* dyr = reinterpret_cast<const uint4*>(kStaged ? reinterpret_cast<const __nv_bfloat16*>(stage + kNormStageBytes) + grp * H : dy + row * H);
@@ -296,8 +304,13 @@ rmsnorm_bwd_fused_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat1
             }
         }
         if (kStaged) {
-            __syncthreads();      // everybody has this round's rows in registers
-            if (threadIdx.x == 0 && base + step < rows) fetch(base + step);
+            const NormRounds::Next next = r.behind_wait(__syncthreads_and(came));      // everybody has this round's rows in registers
+            if (!next.use) {
+                // the status word says so; copies under way are given time to land before the CTA's memory goes
+                for (int i = 0; i < 32; ++i) __nanosleep(50000);
+                break;
+            }
+            if (threadIdx.x == 0 && next.fetch) fetch(r.first + r.step);
         }
         if (live) {
 #pragma unroll

@@ -574,6 +574,27 @@ CAI_API int cai_rmsnorm_bwd_partial(const void* x, const void* g, const float* r
     return CAI_K_OK;
 }
 
+CAI_API int cai_rmsnorm_bwd_rounds(int rows, int H, int ctas, int cta, int lost_round, int* events, int capacity) {
+    if (rows <= 0 || H <= 0 || (H & 7) || H > kNormFusedMaxH || ctas <= 0 || cta < 0 || cta >= ctas) return CAI_K_BAD_ARG;
+    int n = 0;
+    auto event = [&](int what, long long row) {
+        if (n < capacity) {
+            events[2 * n] = what;
+            events[2 * n + 1] = static_cast<int>(row);
+        }
+        ++n;
+    };
+    NormRounds r(cta, ctas, 8 / rmsnorm_fused_row_warps(H), rows);
+    if (r.more()) event(0, r.first);
+    for (int round = 0; r.more(); r.first += r.step, ++round) {
+        const NormRounds::Next next = r.behind_wait(round != lost_round);
+        if (next.fetch) event(0, r.first + r.step);
+        if (!next.use) break;
+        event(1, r.first);
+    }
+    return n;
+}
+
 CAI_API int cai_rmsnorm_dg_sums(const cai_dg_sum* sums, int n, int H, void* stream) {
     if (n <= 0) return CAI_K_OK;
     if (n > CAI_DG_SUMS || H <= 0) {

@@ -80,3 +80,31 @@ def test_launchers_of_the_extension_are_those_of_the_library():
             fast.cai_gemm_bf16("x", *bad[1:])
         with pytest.raises(TypeError):
             fast.cai_gemm_bf16(*bad[:4], 1.5, *bad[5:])
+
+
+# RMSNorm backward whose rows come ahead: which rows a CTA fetches and works on. Row groups of 8, 4 and 1, CTAs without rows, a last round that is not full.
+@pytest.mark.parametrize("rows,H,ctas", [(4737, 8, 296), (100, 1000, 3), (2500, 1032, 7), (650, 8192, 296), (5, 1000, 2)])
+def test_norm_rows_that_do_not_come_end_the_ctas_work(rows, H, ctas):
+    import ctypes
+    from cai_b200.ops import _lib
+    if not _lib._LIB_PATH.exists():
+        pytest.skip("kernel library not built")
+    groups = 8 if H <= 1024 else 4 if H <= 2048 else 1
+
+    def events(cta, lost):
+        n = _lib.lib().cai_rmsnorm_bwd_rounds(rows, H, ctas, cta, lost, None, 0)
+        buf = (ctypes.c_int * (2 * max(n, 1)))()
+        assert _lib.lib().cai_rmsnorm_bwd_rounds(rows, H, ctas, cta, lost, buf, n) == n
+        return [(buf[2 * i], buf[2 * i + 1]) for i in range(n)]
+
+    worked = []
+    for cta in range(ctas):
+        whole = events(cta, -1)
+        mine = list(range(cta * groups, rows, ctas * groups))
+        assert [r for what, r in whole if what == 0] == mine and [r for what, r in whole if what == 1] == mine
+        worked += mine
+        for lost in range(len(mine)):
+            # this round's rows were fetched; nothing is done with them, and nothing is fetched over them
+            want = [(0, mine[0])] + [e for k in range(lost) for e in ((0, mine[k + 1]), (1, mine[k]))]
+            assert events(cta, lost) == want
+    assert sorted(worked) == list(range(0, rows, groups))
