@@ -69,7 +69,8 @@ def build_kernels(verbose=False, ptxas_info=False) -> Path:
     objdir.mkdir(parents=True, exist_ok=True)
     LIBDIR.mkdir(parents=True, exist_ok=True)
     headers = list((CSRC / "kernels").glob("*.h")) + list((CSRC / "kernels").glob("*.cuh")) + list(
-        (CSRC / "comm").glob("*.h")) + list((CSRC / "comm").glob("*.cuh")) + list((CSRC / "runtime").glob("*.h"))
+        (CSRC / "comm").glob("*.h")) + list((CSRC / "comm").glob("*.cuh")) + list((CSRC / "runtime").glob("*.h")) + list(
+        (CSRC / "plan").glob("*.h"))
     srcs = kernel_sources()
     jobs = []
     objs = []

@@ -557,7 +557,8 @@ CAI_API int cai_rmsnorm_bwd(const void* x, const void* g, const float* rstd, con
 
 CAI_API int cai_rmsnorm_bwd_partial_rows(int rows, int H) {
     if (rows <= 0 || H <= 0 || (H & 7) || H > kNormFusedMaxH) return 0;
-    return rmsnorm_fused_parts(rows, H, cai_rmsnorm_bwd_parts(rows), sm_count(current_device()));
+    const int sms = sm_count(current_device());
+    return rmsnorm_fused_parts(rows, H, cai_rmsnorm_bwd_parts(rows), sms > 0 ? sms : 148);
 }
 
 CAI_API int cai_rmsnorm_bwd_partial(const void* x, const void* g, const float* rstd, const void* dy, void* dx, float* dg_partial, int rows,

@@ -36,6 +36,12 @@ typedef struct {
 CAI_API int cai_exec_create(cai_exec** out, const void* plan_bytes, size_t nbytes, void* arena_base,
                             void* const* caller_streams);
 CAI_API void cai_exec_destroy(cai_exec* ex);
+/* What a replay of the plan launches, in order: four ints a launch. What: 0 an event, 1 a record by itself, 2 two products, 3 a projection and its SwiGLU, 4 an
+ * attention backward and the rotation of its result, 5 the sweep of an RMSNorm backward, whose sum waits, 6 the sums that wait. The first operation it covers (of 6:
+ * the one before which they go out, or the number of operations). How many sums go out. How many kernels of this library that is. An operation that no
+ * launch covers is left out: nothing reads its result. join = 0: as traced replays and those that check extents go, every record by itself. Returns the number of
+ * launches, of which `capacity` are written, or an error. Needs no GPU. */
+CAI_API int cai_plan_launches(const void* plan_bytes, size_t nbytes, int join, int* launches, int capacity);
 CAI_API int cai_nccl_unique_id(const char* libpath, void* id128);
 CAI_API int cai_exec_init_comm(cai_exec* ex, const char* libpath, int group_kind, const void* id128,
                                const void* id128_second, int nranks, int rank);

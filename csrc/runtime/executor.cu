@@ -19,7 +19,6 @@
 #include <stdlib.h>
 #include <string.h>
 
-#include <algorithm>
 #include <string>
 #include <vector>
 
@@ -32,8 +31,8 @@
 #include "../kernels/cai_kernels.h"
 #include "../kernels/host_common.h"
 #include "../kernels/sm100.cuh"
-#include "../plan/formats.h"
 #include "cai_runtime.h"
+#include "launches.h"
 
 namespace cai {
 
@@ -135,17 +134,7 @@ struct TraceRec { uint32_t op; cudaEvent_t start, stop; };
 
 using namespace cai;
 
-struct cai_exec {
-    PlanHeader hdr{};
-    ExecHeader xhdr{};
-    TrainSpec train{};
-    ModelSpec model{};
-    std::vector<TensorDesc> tensors;
-    std::vector<CommGroup> groups;
-    std::vector<Op> ops;
-    std::vector<ExecOp> exec;
-    std::vector<NamedTensor> named;
-    std::vector<uint32_t> shapes;
+struct cai_exec : Plan {
     uint8_t* arena = nullptr;
     int device = 0;
     cudaStream_t streams[ST_COUNT] = {};
@@ -178,9 +167,7 @@ struct cai_exec {
     cai_fused_hook_t fused_hook = nullptr;
     void* fused_ctx = nullptr;
     int sm_limit_hi = 0;
-    enum : uint8_t { kAlone, kPairOfProducts, kWithSwiglu, kWithRotation };
-    std::vector<uint8_t> with_next;   // per op: whether, and how, it goes out together with the one behind it
-    std::vector<uint8_t> unread;      // per op: a product whose result nothing reads; a traced or checked replay runs it all the same
+    std::vector<uint8_t> joins;   // per op: how it goes out (launches.h)
     uint64_t launches = 0;  // kernels / collectives enqueued by the last replay
     // ZeRO-3: a parameter gather waiting to be merged into the GEMM that follows it in the op table
     GatherJob pending_gather{};
@@ -550,88 +537,6 @@ cai_gemm_call gemm_call(const cai_exec* ex, const ExecOp& x) {
     return c;
 }
 
-// Whether two records next to each other on one stream are plain products of which neither touches what the other writes: a layer's input gradient and
-// weight gradient, which the plan puts side by side. Ranges are those that the products address, from the records' own sizes.
-bool independent_products(const cai_exec* ex, const Op& o0, const Op& o1) {
-    if (!o0.exec || !o1.exec || o0.stream_id != o1.stream_id) return false;
-    if (o0.kind == OP_EVENT_RECORD || o0.kind == OP_EVENT_WAIT || o1.kind == OP_EVENT_RECORD || o1.kind == OP_EVENT_WAIT) return false;
-    struct Range { const uint8_t *lo, *hi; };
-    Range reads[2][3] = {}, writes[2] = {};
-    for (int k = 0; k < 2; ++k) {
-        const ExecOp& x = ex->exec[(k ? o1 : o0).exec - 1];
-        if (x.kernel != K_GEMM || (x.flags & 0x100) || x.t[4] >= 0) return false;
-        const cai_gemm_call c = gemm_call(ex, x);
-        if (c.epi > CAI_EPI_BF16_RESIDUAL) return false;
-        auto range = [](const void* at, long long rows, long long cols, long long ld, int bytes) {
-            const uint8_t* p = static_cast<const uint8_t*>(at);
-            return p && rows > 0 ? Range{p, p + ((rows - 1) * ld + cols) * bytes} : Range{nullptr, nullptr};
-        };
-        reads[k][0] = c.a_mn_major ? range(c.A, c.K, c.M, c.lda, 2) : range(c.A, c.M, c.K, c.lda, 2);
-        reads[k][1] = c.b_mn_major ? range(c.B, c.K, c.N, c.ldb, 2) : range(c.B, c.N, c.K, c.ldb, 2);
-        if (c.epi == CAI_EPI_BF16_RESIDUAL) reads[k][2] = range(c.R, c.M, c.N, c.ldr, 2);
-        writes[k] = range(c.C, c.M, c.N, c.ldc, c.epi == CAI_EPI_F32 || c.epi == CAI_EPI_F32_ACCUM ? 4 : 2);
-    }
-    auto meet = [](const Range& a, const Range& b) { return a.lo < b.hi && b.lo < a.hi; };
-    if (meet(writes[0], writes[1])) return false;
-    for (int k = 0; k < 2; ++k)
-        for (const Range& r : reads[k])
-            if (meet(writes[1 - k], r)) return false;
-    return true;
-}
-
-// Whether two records next to each other on one stream are a gate / up projection and the SwiGLU of its result, of a width that the plan compiler leaves
-// apart (F no multiple of 128), and one product with SwiGLU in its epilogue is the faster way.
-bool projection_with_swiglu(const cai_exec* ex, const Op& o0, const Op& o1) {
-    if (!ex->train.fuse_swiglu || !o0.exec || !o1.exec || o0.stream_id != o1.stream_id) return false;
-    if (o0.kind == OP_EVENT_RECORD || o0.kind == OP_EVENT_WAIT || o1.kind == OP_EVENT_RECORD || o1.kind == OP_EVENT_WAIT) return false;
-    const ExecOp &x = ex->exec[o0.exec - 1], &y = ex->exec[o1.exec - 1];
-    if (x.kernel != K_GEMM || y.kernel != K_SWIGLU_FWD || (x.flags & 0x100) || x.t[4] >= 0) return false;
-    const cai_gemm_call c = gemm_call(ex, x);
-    if (c.epi != CAI_EPI_BF16 || c.a_mn_major || c.b_mn_major || c.alpha != 1.f) return false;
-    return ex->ptr(y.t[0]) == c.C && y.i[0] == c.M && 2 * y.i[1] == c.N && c.ldc == c.N && ex->ld(y.t[1]) == y.i[1] && y.i[1] % 128 != 0 &&
-           cai_gemm_bf16_swiglu_pays(c.M, y.i[1], c.K);
-}
-
-// Whether two records next to each other on one stream are an attention backward and the inverse rotary embedding of its result.
-bool backward_with_rotation(const cai_exec* ex, const Op& o0, const Op& o1) {
-    if (!o0.exec || !o1.exec || o0.stream_id != o1.stream_id) return false;
-    if (o0.kind == OP_EVENT_RECORD || o0.kind == OP_EVENT_WAIT || o1.kind == OP_EVENT_RECORD || o1.kind == OP_EVENT_WAIT) return false;
-    const ExecOp &x = ex->exec[o0.exec - 1], &y = ex->exec[o1.exec - 1];
-    if (x.kernel != K_ATTN_BWD || y.kernel != K_ROPE || (x.flags && x.flags != 7) || !(y.flags & 1)) return false;
-    // B, S, heads of the one; rows, S, heads of the other, over rows of the same pitch
-    return ex->ptr(x.t[5]) == ex->ptr(y.t[0]) && y.i[0] == x.i[0] * x.i[1] && y.i[1] == x.i[1] && y.i[2] == x.i[2] && y.i[3] == x.i[3] &&
-           y.i[4] == x.i[4] && ex->ld(y.t[0]) == static_cast<long long>(x.i[2] + 2 * x.i[3]) * x.i[4];
-}
-
-// Products whose results no record of the plan reads: with activation recompute, the down projection of a layer that is run again for its
-// backward. Of everything that any record names, only outputs of such products may lie in the bytes of a result for it to count as unread, and no
-// tensor that the plan gives a name to.
-void find_unread(const cai_exec* ex, std::vector<uint8_t>* unread) {
-    unread->assign(ex->ops.size() + 1, 0);
-    auto product = [](const ExecOp& x) {
-        const int epi = (x.flags >> 4) & 0xF;
-        return x.kernel == K_GEMM && !(x.flags & 0x100) && x.t[4] < 0 && (epi == CAI_EPI_BF16 || epi == CAI_EPI_BF16_RESIDUAL);
-    };
-    struct Range { uint64_t lo, hi; };
-    std::vector<Range> used, results;
-    auto range = [&](int t) { return Range{ex->tensors[t].offset, ex->tensors[t].offset + ex->tensors[t].nbytes}; };
-    for (const NamedTensor& n : ex->named)
-        for (const int t : {n.tensor, n.grad})
-            if (t >= 0 && static_cast<size_t>(t) < ex->tensors.size()) used.push_back(range(t));
-    for (const ExecOp& x : ex->exec)
-        for (int k = 0; k < static_cast<int>(sizeof x.t / sizeof x.t[0]); ++k)
-            if (x.t[k] >= 0 && static_cast<size_t>(x.t[k]) < ex->tensors.size() && !(k == 2 && product(x))) used.push_back(range(x.t[k]));
-    std::sort(used.begin(), used.end(), [](const Range& a, const Range& b) { return a.lo < b.lo; });
-    std::vector<uint64_t> reach(used.size());      // the furthest end of the ranges up to this one
-    for (size_t i = 0; i < used.size(); ++i) reach[i] = i && reach[i - 1] > used[i].hi ? reach[i - 1] : used[i].hi;
-    for (size_t i = 0; i < ex->ops.size(); ++i) {
-        if (!ex->ops[i].exec || !product(ex->exec[ex->ops[i].exec - 1])) continue;
-        const Range r = range(ex->exec[ex->ops[i].exec - 1].t[2]);
-        const size_t n = std::lower_bound(used.begin(), used.end(), r.hi, [](const Range& a, uint64_t hi) { return a.lo < hi; }) - used.begin();
-        (*unread)[i] = n == 0 || reach[n - 1] <= r.lo;
-    }
-}
-
 // How many kernels of this library one exec record launches (memsets and NCCL calls are not ours).
 int own_kernels_of(const ExecOp& x) {
     const uint16_t k = x.kernel;
@@ -654,73 +559,46 @@ const char* kernel_label(uint16_t k) {
     return k < K_COUNT ? n[k] : "?";
 }
 
-// Sums of gain gradients that are still to go out (RMSNorm backward without its last step): they wait for each other in the rows of the plan's scratch
-// that one norm leaves free, and go out before anything that could name what they read or write. A chain of short kernels is some 5 us shorter for each
-// launch less: a step of 47 launches 298 -> 288 us, 8 layers of 896 tokens, three times over, 3632 -> 3519; 3840 tokens, where two norms fit, no change.
-struct WaitingSums {
-    cai_dg_sum sum[CAI_DG_SUMS];
-    int n = 0, H = 0, stream = 0;
-    const uint8_t *scratch = nullptr, *scratch_end = nullptr;   // the whole scratch
-    float* next = nullptr;                                      // its first free row
+// How many kernels of this library a launch is.
+int own_kernels_of(const cai_exec* ex, const Launch& l) {
+    if (l.what == Launch::kEvent) return 0;
+    const Op& op = ex->ops[l.op < ex->ops.size() ? l.op : 0];
+    switch (l.what) {
+        case Launch::kRecord: case Launch::kRotated: return own_kernels_of(ex->exec[op.exec - 1]);
+        case Launch::kTwoProducts: {
+            const cai_gemm_call a = gemm_call(ex, ex->exec[op.exec - 1]), b = gemm_call(ex, ex->exec[ex->ops[l.op + 1].exec - 1]);
+            int cols;
+            return cai_gemm_bf16_two_launches(&a, &b, &cols);
+        }
+        default: return 1;
+    }
+}
 
-    int flush(cai_exec* ex) {
-        if (!n) return 0;
-        const int count = n;
-        n = 0;
-        ex->launches += 1;
-        return cai_rmsnorm_dg_sums(sum, count, H, ex->streams[stream]);
-    }
-    // Must they go out before this operation? Those that only name tensors of their own record are looked at by range; others (whole
-    // buffers, other ranks, other streams) and events count as naming everything.
-    bool before(const cai_exec* ex, const Op& op) const {
-        if (!n) return false;
-        if (op.kind == OP_EVENT_RECORD || op.kind == OP_EVENT_WAIT) return true;
-        if (!op.exec) return false;
-        if (op.stream_id != stream) return true;
-        const ExecOp& x = ex->exec[op.exec - 1];
-        switch (x.kernel) {
-            case K_GEMM: case K_GEMM_FP8: case K_QUANT_FP8: case K_SWIGLU_FWD: case K_SWIGLU_BWD: case K_ATTN_FWD: case K_ATTN_BWD: case K_ROPE:
-            case K_RMSNORM_FWD: case K_RMSNORM_BWD: case K_EMBED_FWD: case K_EMBED_BWD: case K_CROSS_ENTROPY: case K_ADD: break;
-            default: return true;
-        }
-        for (int k = 0; k < static_cast<int>(sizeof x.t / sizeof x.t[0]); ++k) {
-            if (x.t[k] < 0 || (x.kernel == K_RMSNORM_BWD && k == 6)) continue;       // (the scratch itself: add() looks after its rows)
-            const uint8_t *lo = static_cast<const uint8_t*>(ex->ptr(x.t[k])), *hi = lo + ex->tensors[x.t[k]].nbytes;
-            if (lo < scratch_end && scratch < hi) return true;
-            for (int i = 0; i < n; ++i) {
-                const uint8_t *d0 = reinterpret_cast<const uint8_t*>(sum[i].dg), *d1 = d0 + static_cast<size_t>(H) * sizeof(float);
-                if (lo < d1 && d0 < hi) return true;
-            }
-        }
-        return false;
-    }
-    // RMSNorm backward of a record: its sweep now, its sum later. False if the record has no such form (and no sum waits any more).
-    bool add(cai_exec* ex, const Op& op, const ExecOp& x, cudaStream_t st, int* rc) {
-        const int rows = x.i[0], width = x.i[1], parts = cai_rmsnorm_bwd_partial_rows(rows, width);
-        const size_t need = static_cast<size_t>(parts) * width;
-        if (parts <= 0 || need * sizeof(float) > ex->tensors[x.t[6]].nbytes) {
-            *rc = flush(ex);          // the whole form uses the scratch from its beginning
-            return *rc != 0;
-        }
-        const uint8_t* at = static_cast<const uint8_t*>(ex->ptr(x.t[6]));
-        const bool fits = n && n < CAI_DG_SUMS && width == H && op.stream_id == stream && at == scratch &&
-                          reinterpret_cast<const uint8_t*>(next + need) <= scratch_end;
-        if (!fits) {
-            if ((*rc = flush(ex)) != 0) return true;
-            H = width;
-            stream = op.stream_id;
-            scratch = at;
-            scratch_end = at + ex->tensors[x.t[6]].nbytes;
-            next = static_cast<float*>(ex->ptr(x.t[6]));
-        }
-        sum[n++] = {next, static_cast<float*>(ex->ptr(x.t[5])), parts, x.i[3]};
-        *rc = cai_rmsnorm_bwd_partial(ex->ptr(x.t[0]), ex->ptr(x.t[1]), static_cast<const float*>(ex->ptr(x.t[2])), ex->ptr(x.t[3]), ex->ptr(x.t[4]), next,
-                                      rows, width, x.i[2], st);
-        next += need;
-        ex->launches += 1;
-        return true;
-    }
-};
+int launch_sums(cai_exec* ex, const WaitingSums& w) {
+    cai_dg_sum sums[CAI_DG_SUMS];
+    for (int i = 0; i < w.n; ++i)
+        sums[i] = {reinterpret_cast<const float*>(ex->arena + w.sum[i].partial), static_cast<float*>(ex->ptr(w.sum[i].dg)), w.sum[i].parts,
+                   w.sum[i].accumulate};
+    return cai_rmsnorm_dg_sums(sums, w.n, w.H, ex->streams[w.stream]);
+}
+
+// A launch that is more, or less, than a record by itself.
+int run_joined(cai_exec* ex, const Launch& l, cudaStream_t st) {
+    const ExecOp& x = ex->exec[ex->ops[l.op].exec - 1];
+    auto P = [&](int i) { return ex->ptr(x.t[i]); };
+    if (l.what == Launch::kNormSweep)
+        return cai_rmsnorm_bwd_partial(P(0), P(1), static_cast<const float*>(P(2)), P(3), P(4),
+                                       reinterpret_cast<float*>(ex->arena + l.sums->sum[l.sums->n - 1].partial), x.i[0], x.i[1], x.i[2], st);
+    const ExecOp& next = ex->exec[ex->ops[l.op + 1].exec - 1];
+    if (l.what == Launch::kRotated)
+        return cai_flash_attn_bwd_rope(P(0), P(1), P(2), (const float*)P(3), (float*)P(4), P(5), (const float*)ex->ptr(next.t[1]), x.i[0], x.i[1], x.i[2],
+                                       x.i[3], x.i[4], x.f[0], 7, st);
+    const cai_gemm_call a = gemm_call(ex, x);
+    if (l.what == Launch::kSwiglu)
+        return cai_gemm_bf16_swiglu(a.A, a.B, a.C, ex->ptr(next.t[1]), a.M, next.i[1], a.K, a.lda, a.ldb, a.ldc, next.i[1], st);
+    const cai_gemm_call b = gemm_call(ex, next);
+    return cai_gemm_bf16_two(&a, &b, st);
+}
 
 int replay(cai_exec* ex) {
     cudaStream_t hi = ex->streams[ST_COMPUTE_HI];
@@ -729,12 +607,17 @@ int replay(cai_exec* ex) {
     for (int s = 1; s < ST_COUNT; ++s)
         if (ex->used[s]) cudaStreamWaitEvent(ex->streams[s], ex->fork_ev, 0);
     ex->launches = 0;
-    WaitingSums sums;
-    for (size_t i = 0; i < ex->ops.size(); ++i) {
-        const Op& op = ex->ops[i];
+    const bool traced = ex->trace_on && !ex->use_graph;
+    LaunchWalk walk(*ex, ex->joins, !traced && !ex->debug_bounds, ex->sm_limit_hi <= 0);
+    for (Launch l; walk.next(&l);) {
+        if (l.what == Launch::kNormSums) {
+            const int rc = launch_sums(ex, *l.sums);
+            if (rc != 0) return rc;
+            ex->launches += 1;
+            continue;
+        }
+        const Op& op = ex->ops[l.op];
         cudaStream_t st = ex->streams[op.stream_id];
-        if (sums.before(ex, op) || (ex->with_next[i] && sums.before(ex, ex->ops[i + 1])))
-            if (const int rc = sums.flush(ex)) return rc;
         if (op.kind == OP_EVENT_RECORD) {
             if (cudaEventRecord(ex->events[op.aux0], st) != cudaSuccess) return CAI_K_CUDA;
             continue;
@@ -743,13 +626,11 @@ int replay(cai_exec* ex) {
             if (cudaStreamWaitEvent(st, ex->events[op.aux0], 0) != cudaSuccess) return CAI_K_CUDA;
             continue;
         }
-        if (!op.exec) continue;
-        if (ex->unread[i] && !ex->has_pending_gather && !ex->debug_bounds && !(ex->trace_on && !ex->use_graph)) continue;
         // events on either side of a launch: no kernel starts while its predecessor finishes, some 5 us an op
         TraceRec* tr = nullptr;
-        if (ex->trace_on && !ex->use_graph) {
+        if (traced) {
             TraceRec r;
-            r.op = static_cast<uint32_t>(i);
+            r.op = l.op;
             cudaEventCreate(&r.start);
             cudaEventCreate(&r.stop);
             ex->trace.push_back(r);
@@ -757,49 +638,16 @@ int replay(cai_exec* ex) {
             cudaEventRecord(tr->start, st);
         }
         if (ex->debug_bounds) {
-            const int brc = check_operands(ex, ex->exec[op.exec - 1], i);
+            const int brc = check_operands(ex, ex->exec[op.exec - 1], l.op);
             if (brc != 0) return brc;
         }
         if (ex->nvtx_on) nvtxRangePushA(kernel_label(ex->exec[op.exec - 1].kernel));
-        if (ex->exec[op.exec - 1].kernel == K_RMSNORM_BWD && !tr && !ex->debug_bounds) {
-            int rc = 0;
-            if (sums.add(ex, op, ex->exec[op.exec - 1], st, &rc)) {
-                if (ex->nvtx_on) nvtxRangePop();
-                if (rc != 0) return rc;
-                continue;
-            }
-        }
-        if (ex->with_next[i] && !tr && !ex->debug_bounds && ex->sm_limit_hi <= 0 && !ex->has_pending_gather) {
-            const ExecOp &x = ex->exec[op.exec - 1], &next = ex->exec[ex->ops[i + 1].exec - 1];
-            int rc, launches = 1, cols;
-            if (ex->with_next[i] == cai_exec::kWithRotation) {
-                auto P = [&](int t) { return ex->ptr(x.t[t]); };
-                rc = cai_flash_attn_bwd_rope(P(0), P(1), P(2), (const float*)P(3), (float*)P(4), P(5), (const float*)ex->ptr(next.t[1]), x.i[0], x.i[1],
-                                             x.i[2], x.i[3], x.i[4], x.f[0], 7, st);
-                launches = own_kernels_of(x);
-            } else if (ex->with_next[i] == cai_exec::kWithSwiglu) {
-                const cai_gemm_call a = gemm_call(ex, x);
-                rc = cai_gemm_bf16_swiglu(a.A, a.B, a.C, ex->ptr(next.t[1]), a.M, next.i[1], a.K, a.lda, a.ldb, a.ldc, next.i[1], st);
-            } else {
-                const cai_gemm_call a = gemm_call(ex, x), b = gemm_call(ex, next);
-                rc = cai_gemm_bf16_two(&a, &b, st);
-                launches = cai_gemm_bf16_two_launches(&a, &b, &cols);
-            }
-            if (ex->nvtx_on) nvtxRangePop();
-            if (rc != 0) return rc;
-            ex->launches += launches;
-            ++i;
-            continue;
-        }
-        const int rc = run_op(ex, op, ex->exec[op.exec - 1], st);
+        const int rc = l.what == Launch::kRecord ? run_op(ex, op, ex->exec[op.exec - 1], st) : run_joined(ex, l, st);
         if (ex->nvtx_on) nvtxRangePop();
         if (rc != 0) return rc;
-        {
-            ex->launches += own_kernels_of(ex->exec[op.exec - 1]);
-        }
+        ex->launches += own_kernels_of(ex, l);
         if (tr) cudaEventRecord(tr->stop, st);
     }
-    if (const int rc = sums.flush(ex)) return rc;
     // join: compute_hi waits for every other one of them
     for (int s = 1; s < ST_COUNT; ++s) {
         if (!ex->used[s]) continue;
@@ -809,11 +657,8 @@ int replay(cai_exec* ex) {
     return cudaGetLastError() == cudaSuccess ? 0 : CAI_K_CUDA;
 }
 
-}  // namespace
-
-CAI_API int cai_exec_create(cai_exec** out, const void* plan_bytes, size_t nbytes, void* arena_base,
-                            void* const* caller_streams) {
-    auto ex = new cai_exec();
+// The tables of a version-2 plan; false, with the reason as the last error, if these bytes are none.
+bool read_tables(Plan* plan, const void* plan_bytes, size_t nbytes) {
     const uint8_t* p = static_cast<const uint8_t*>(plan_bytes);
     const uint8_t* end = p + nbytes;
     auto take = [&](void* dst, size_t n) {
@@ -822,54 +667,56 @@ CAI_API int cai_exec_create(cai_exec** out, const void* plan_bytes, size_t nbyte
         p += n;
         return true;
     };
-    bool ok = take(&ex->hdr, sizeof ex->hdr) && ex->hdr.magic == kPlanMagic && ex->hdr.version == 2;
+    bool ok = take(&plan->hdr, sizeof plan->hdr) && plan->hdr.magic == kPlanMagic && plan->hdr.version == 2;
     if (ok) {
-        ex->tensors.resize(ex->hdr.num_tensors);
-        ex->groups.resize(ex->hdr.num_groups);
-        ex->ops.resize(ex->hdr.num_ops);
-        ok = take(ex->tensors.data(), ex->tensors.size() * sizeof(TensorDesc)) &&
-             take(ex->groups.data(), ex->groups.size() * sizeof(CommGroup)) &&
-             take(ex->ops.data(), ex->ops.size() * sizeof(Op)) && take(&ex->xhdr, sizeof ex->xhdr) &&
-             ex->xhdr.magic == kExecMagic && take(&ex->train, sizeof ex->train) && take(&ex->model, sizeof ex->model);
+        plan->tensors.resize(plan->hdr.num_tensors);
+        plan->groups.resize(plan->hdr.num_groups);
+        plan->ops.resize(plan->hdr.num_ops);
+        ok = take(plan->tensors.data(), plan->tensors.size() * sizeof(TensorDesc)) &&
+             take(plan->groups.data(), plan->groups.size() * sizeof(CommGroup)) &&
+             take(plan->ops.data(), plan->ops.size() * sizeof(Op)) && take(&plan->xhdr, sizeof plan->xhdr) &&
+             plan->xhdr.magic == kExecMagic && take(&plan->train, sizeof plan->train) && take(&plan->model, sizeof plan->model);
     }
     if (ok) {
-        ex->exec.resize(ex->xhdr.num_exec);
-        ex->named.resize(ex->xhdr.num_named);
-        ex->shapes.resize(static_cast<size_t>(ex->hdr.num_tensors) * 4);
-        ok = take(ex->exec.data(), ex->exec.size() * sizeof(ExecOp)) &&
-             take(ex->named.data(), ex->named.size() * sizeof(NamedTensor)) &&
-             take(ex->shapes.data(), ex->shapes.size() * sizeof(uint32_t));
+        plan->exec.resize(plan->xhdr.num_exec);
+        plan->named.resize(plan->xhdr.num_named);
+        plan->shapes.resize(static_cast<size_t>(plan->hdr.num_tensors) * 4);
+        ok = take(plan->exec.data(), plan->exec.size() * sizeof(ExecOp)) &&
+             take(plan->named.data(), plan->named.size() * sizeof(NamedTensor)) &&
+             take(plan->shapes.data(), plan->shapes.size() * sizeof(uint32_t));
     }
     if (!ok) {
         set_last_error("not a version-2 plan (or truncated)");
+        return false;
+    }
+    for (const TensorDesc& t : plan->tensors)
+        if (t.offset + t.nbytes > plan->hdr.arena_bytes) {
+            set_last_error("tensor outside the arena");
+            return false;
+        }
+    for (const Op& o : plan->ops)
+        if (o.stream_id >= ST_COUNT || ((o.kind == OP_EVENT_RECORD || o.kind == OP_EVENT_WAIT) && o.aux0 >= plan->hdr.num_events) ||
+            o.exec > plan->exec.size()) {
+            set_last_error("malformed op table");
+            return false;
+        }
+    return true;
+}
+
+}  // namespace
+
+CAI_API int cai_exec_create(cai_exec** out, const void* plan_bytes, size_t nbytes, void* arena_base,
+                            void* const* caller_streams) {
+    auto ex = new cai_exec();
+    if (!read_tables(ex, plan_bytes, nbytes)) {
         delete ex;
         return CAI_K_BAD_ARG;
     }
-    for (const TensorDesc& t : ex->tensors)
-        if (t.offset + t.nbytes > ex->hdr.arena_bytes) {
-            set_last_error("tensor outside the arena");
-            delete ex;
-            return CAI_K_BAD_ARG;
-        }
-    for (const Op& o : ex->ops)
-        if (o.stream_id >= ST_COUNT || ((o.kind == OP_EVENT_RECORD || o.kind == OP_EVENT_WAIT) && o.aux0 >= ex->hdr.num_events) ||
-            o.exec > ex->exec.size()) {
-            set_last_error("malformed op table");
-            delete ex;
-            return CAI_K_BAD_ARG;
-        }
     for (const Op& o : ex->ops)
         if (o.exec || o.kind == OP_EVENT_RECORD || o.kind == OP_EVENT_WAIT) ex->used[o.stream_id] = true;
     ex->arena = static_cast<uint8_t*>(arena_base);
     ex->device = current_device();
-    find_unread(ex, &ex->unread);
-    ex->with_next.assign(ex->ops.size() + 1, 0);
-    for (size_t i = 0; i + 1 < ex->ops.size(); ++i)
-        if (!ex->unread[i] && !ex->unread[i + 1] && !(i > 0 && ex->with_next[i - 1]))
-            ex->with_next[i] = independent_products(ex, ex->ops[i], ex->ops[i + 1])     ? cai_exec::kPairOfProducts
-                               : projection_with_swiglu(ex, ex->ops[i], ex->ops[i + 1]) ? cai_exec::kWithSwiglu
-                               : backward_with_rotation(ex, ex->ops[i], ex->ops[i + 1]) ? cai_exec::kWithRotation
-                                                                                        : cai_exec::kAlone;
+    ex->joins = find_joins(*ex);
     if (const char* dbg = getenv("CAI_DEBUG_BOUNDS")) ex->debug_bounds = *dbg && *dbg != '0';
     if (ex->train.wait_limit_ms) cai_set_wait_limit_us(ex->train.wait_limit_ms * 1000u);
     int lo_prio = 0, hi_prio = 0;
@@ -927,6 +774,22 @@ CAI_API int cai_exec_create(cai_exec** out, const void* plan_bytes, size_t nbyte
     }
     *out = ex;
     return 0;
+}
+
+CAI_API int cai_plan_launches(const void* plan_bytes, size_t nbytes, int join, int* launches, int capacity) {
+    cai_exec ex;
+    if (!read_tables(&ex, plan_bytes, nbytes)) return CAI_K_BAD_ARG;
+    ex.joins = find_joins(ex);
+    LaunchWalk walk(ex, ex.joins, join != 0, join != 0);
+    int n = 0;
+    for (Launch l; walk.next(&l); ++n)
+        if (n < capacity) {
+            launches[4 * n] = l.what;
+            launches[4 * n + 1] = static_cast<int>(l.op);
+            launches[4 * n + 2] = l.what == Launch::kNormSums ? l.sums->n : 0;
+            launches[4 * n + 3] = own_kernels_of(&ex, l);
+        }
+    return n;
 }
 
 CAI_API void cai_exec_destroy(cai_exec* ex) {

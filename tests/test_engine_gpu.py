@@ -344,8 +344,12 @@ def test_engine_made_behind_work_of_the_callers_stream(side):
 ODD = "hidden_size = 1000\nffn_hidden = 2728\nseq_len = 640\nmicrobatch = 3\ntie_embeddings = 1\nvocab_size = 5000\n"
 
 
-@pytest.mark.parametrize("extra", ["", ODD, ODD + "recompute = 1\n", "ffn_hidden = 328\n", "param_dtype = fp8e4m3\nrecompute = 1\n"])
-def test_records_that_go_out_together_give_the_bits_of_single_launches(extra):
+@pytest.mark.parametrize("extra,kinds", [("", {"pair", "rotated", "sums"}), (ODD, {"pair", "swiglu", "rotated", "sums"}),
+                                         (ODD + "recompute = 1\n", {"pair", "swiglu", "rotated", "sums", "unread"}),
+                                         ("ffn_hidden = 328\n", {"pair", "swiglu", "rotated", "sums"}),
+                                         ("param_dtype = fp8e4m3\nrecompute = 1\n", {"pair", "rotated", "sums"})])
+def test_records_that_go_out_together_give_the_bits_of_single_launches(extra, kinds):
+    from test_launches_cpu import EVENT, NORM_SUMS, NORM_SWEEP, ROTATED, SWIGLU, TWO_PRODUCTS, launches as launched
     from cai_b200.runtime.engine import Engine, synthetic_batch
     eng = Engine(config_text=(ROOT / "configs" / "tiny.cfg").read_text() + "\n" + extra, rank=0, world=1, local_rank=0)
     m = eng.model
@@ -361,5 +365,15 @@ def test_records_that_go_out_together_give_the_bits_of_single_launches(extra):
         launches.append(eng.launches_per_step)
         grads.append(eng.view("@flat_grad").clone())
     eng.close()
+    # what the untraced steps launched is what the plan says, and each form that is compared is among it
+    steps = launched(eng.plan.raw)
+    assert launches[1] == sum(kernels for _, _, _, kernels in steps) and launches[0] == sum(kernels for _, _, _, kernels in launched(eng.plan.raw, 0))
+    records = sum(1 for op in eng.plan.ops if op.exec)
+    found = {name for name, seen in (("pair", any(s[0] == TWO_PRODUCTS and s[3] == 1 for s in steps)), ("swiglu", any(s[0] == SWIGLU for s in steps)),
+                                     ("rotated", any(s[0] == ROTATED for s in steps)),
+                                     ("sums", any(s[0] == NORM_SUMS and s[2] > 1 for s in steps) and any(s[0] == NORM_SWEEP for s in steps)),
+                                     ("unread", sum({EVENT: 0, NORM_SUMS: 0, TWO_PRODUCTS: 2, SWIGLU: 2, ROTATED: 2}.get(s[0], 1) for s in steps) < records))
+             if seen}
+    assert found == kinds
     assert launches[1] < launches[0]
     assert torch.equal(grads[0], grads[1]) and torch.equal(grads[0], grads[2])
