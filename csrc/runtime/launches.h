@@ -71,12 +71,15 @@ inline bool independent_products(const Plan& p, const ExecOp& x, const ExecOp& y
 }
 
 // Whether two records next to each other are a gate / up projection and the SwiGLU of its result, of a width that the plan compiler leaves
-// apart (F no multiple of 128), and one product with SwiGLU in its epilogue is the faster way.
+// apart (F no multiple of 128), and one product with SwiGLU in its epilogue is the faster way. Tiles of the activation are written while others still read the
+// operands: it must not lie over them, as it may where the two go out one behind the other.
 inline bool projection_with_swiglu(const Plan& p, const ExecOp& x, const ExecOp& y) {
     if (!p.train.fuse_swiglu || !plain_product(x) || y.kernel != K_SWIGLU_FWD) return false;
     if (!has_tensor(p, x.t[0]) || !has_tensor(p, x.t[1]) || !has_tensor(p, x.t[2]) || !has_tensor(p, y.t[0]) || !has_tensor(p, y.t[1])) return false;
     if (epilogue(x) != CAI_EPI_BF16 || (x.flags & 3) || x.f[0] != 1.f) return false;
     const int M = x.i[0], F = y.i[1];
+    const Bytes act = rows_of(p, y.t[1], M, F, 2);
+    if (act.meets(operand_a(p, x)) || act.meets(operand_b(p, x)) || act.meets(result_c(p, x))) return false;
     return p.tensors[y.t[0]].offset == p.tensors[x.t[2]].offset && y.i[0] == M && 2 * F == x.i[1] && pitch(p, x.t[2]) == x.i[1] && pitch(p, y.t[1]) == F &&
            F % 128 != 0 && cai_gemm_bf16_swiglu_pays(M, F, x.i[2]);
 }

@@ -199,3 +199,31 @@ def test_what_is_launched_trains_to_the_bits_of_the_plan(name):
     for k in a:
         for key in ("master", "m", "v"):
             assert (a[k][key] == b[k][key]).all(), (name, k, key)
+
+
+def moved(pf, t, **fields):
+    """The plan's bytes with fields of tensor t's entry replaced."""
+    raw = bytearray(pf.raw)
+    at = ctypes.sizeof(planlib.PlanHeader) + t * ctypes.sizeof(planlib.TensorDesc)
+    entry = planlib.TensorDesc.from_buffer_copy(raw, at)
+    for k, v in fields.items():
+        setattr(entry, k, v)
+    raw[at:at + ctypes.sizeof(entry)] = bytes(entry)
+    return bytes(raw)
+
+
+def first(raw, what):
+    return next((i for w, i, _, _ in launches(raw) if w == what), None)
+
+
+# An activation that lies over what the product reads or writes is right where the records go out one behind the other.
+@pytest.mark.parametrize("over", [0, 1, 2])
+def test_swiglu_over_its_products_operands_goes_out_by_itself(tmp_path, over):
+    pf, = plans(tmp_path, "tiny.cfg", 1, ODD)
+    i = first(pf.raw, SWIGLU)
+    x, y = (pf.exec[pf.ops[j].exec - 1] for j in (i, i + 1))
+    lo, hi = tensor_bytes(pf, x.t[over])
+    act = pf.tensors[y.t[1]].nbytes
+    for at in (lo, hi - 512, max(lo - act + 512, 0)):      # over its beginning, its end, and with its own end
+        if at + act <= pf.hdr.arena_bytes:
+            assert (RECORD, i) in [(w, j) for w, j, _, _ in launches(moved(pf, y.t[1], offset=at))]
