@@ -84,10 +84,13 @@ inline bool projection_with_swiglu(const Plan& p, const ExecOp& x, const ExecOp&
            F % 128 != 0 && cai_gemm_bf16_swiglu_pays(M, F, x.i[2]);
 }
 
-// Whether two records next to each other are an attention backward and the inverse rotary embedding of its result.
+// Whether two records next to each other are an attention backward and the inverse rotary embedding of its result. The table is read while other rows of
+// the result are written, by pieces of 16 bytes (cai_rope_apply by 8).
 inline bool backward_with_rotation(const Plan& p, const ExecOp& x, const ExecOp& y) {
     if (x.kernel != K_ATTN_BWD || y.kernel != K_ROPE || (x.flags && x.flags != 7) || !(y.flags & 1)) return false;
     if (!has_tensor(p, x.t[5]) || !has_tensor(p, y.t[0]) || !has_tensor(p, y.t[1])) return false;
+    const Bytes table = tensor_bytes(p, y.t[1]), result = tensor_bytes(p, x.t[5]);
+    if ((table.lo & 15) || table.meets(result)) return false;
     // B, S, heads of the one; rows, S, heads of the other, over rows of the same pitch
     return p.tensors[x.t[5]].offset == p.tensors[y.t[0]].offset && y.i[0] == x.i[0] * x.i[1] && y.i[1] == x.i[1] && y.i[2] == x.i[2] && y.i[3] == x.i[3] &&
            y.i[4] == x.i[4] && pitch(p, y.t[0]) == static_cast<long long>(x.i[2] + 2 * x.i[3]) * x.i[4];

@@ -227,3 +227,14 @@ def test_swiglu_over_its_products_operands_goes_out_by_itself(tmp_path, over):
     for at in (lo, hi - 512, max(lo - act + 512, 0)):      # over its beginning, its end, and with its own end
         if at + act <= pf.hdr.arena_bytes:
             assert (RECORD, i) in [(w, j) for w, j, _, _ in launches(moved(pf, y.t[1], offset=at))]
+
+
+def test_rotation_whose_table_the_backward_cannot_take_goes_out_by_itself(tmp_path):
+    pf, = plans(tmp_path, "tiny.cfg", 1)
+    i = first(pf.raw, ROTATED)
+    x, y = (pf.exec[pf.ops[j].exec - 1] for j in (i, i + 1))
+    alone = lambda raw: {(RECORD, i), (RECORD, i + 1)} <= {(w, j) for w, j, _, _ in launches(raw)}
+    table, (lo, hi) = pf.tensors[y.t[1]], tensor_bytes(pf, x.t[5])
+    assert table.offset % 16 == 0 and not alone(pf.raw) and not alone(moved(pf, y.t[1], offset=table.offset + 16, nbytes=table.nbytes - 16))
+    assert alone(moved(pf, y.t[1], offset=table.offset + 8, nbytes=table.nbytes - 8))      # 8 bytes are enough for the rotation by itself
+    assert alone(moved(pf, y.t[1], offset=lo)) and alone(moved(pf, y.t[1], offset=hi - 512))
