@@ -214,6 +214,9 @@ class Engine:
 
     # ------------------------------------------------------------------ arena views
     def tensor_view(self, tid: int) -> torch.Tensor:
+        """Tensor ``tid`` of the plan, in the arena. A step leaves out products whose result no record of the plan reads (with
+        recompute, the output of a layer that is run again): such a tensor without a name of its own holds what a step with ``trace_step`` or
+        ``debug_bounds``, which run every record, left there."""
         t = self.plan.tensors[tid]
         rows, cols, ld = self.plan.shape(tid)
         dt = _TORCH_DTYPE[t.dtype]

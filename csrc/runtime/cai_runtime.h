@@ -51,6 +51,8 @@ CAI_API int cai_ipc_export(void* ptr, void* handle64, unsigned long long* offset
 CAI_API int cai_ipc_open(const void* handle64, unsigned long long offset, void** out);
 CAI_API int cai_ipc_close(void* mapped, unsigned long long offset);
 CAI_API void* cai_exec_stream(cai_exec* ex, int stream_id);
+/* Where a tensor lies. A replay leaves out products whose result no record of the plan reads (cai_plan_launches); traced replays and those that check
+ * extents run them. */
 CAI_API void* cai_exec_tensor_ptr(cai_exec* ex, int tensor);
 CAI_API long long cai_exec_tensor_ld(cai_exec* ex, int tensor);
 CAI_API unsigned long long cai_exec_tensor_bytes(cai_exec* ex, int tensor);

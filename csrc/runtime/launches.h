@@ -97,11 +97,11 @@ inline bool backward_with_rotation(const Plan& p, const ExecOp& x, const ExecOp&
 }
 
 // Products whose results no record of the plan reads: with activation recompute, the down projection of a layer that is run again for its
-// backward. Of everything that any record names, only outputs of such products may lie in the bytes of a result for it to count as unread, and no
-// tensor that the plan gives a name to.
+// backward. Nothing that any record names may lie in the bytes of a result for it to count as unread, outputs of plain bf16 products apart, and no
+// tensor that the plan gives a name to. Only activations: other ranks read some of the rest, by records of their own.
 inline void find_unread(const Plan& p, std::vector<uint8_t>* join) {
     auto product = [](const ExecOp& x) { return plain_product(x) && (epilogue(x) == CAI_EPI_BF16 || epilogue(x) == CAI_EPI_BF16_RESIDUAL); };
-    std::vector<Bytes> used, results;
+    std::vector<Bytes> used;
     for (const NamedTensor& n : p.named)
         for (const int t : {n.tensor, n.grad})
             if (has_tensor(p, t)) used.push_back(tensor_bytes(p, t));
@@ -112,8 +112,10 @@ inline void find_unread(const Plan& p, std::vector<uint8_t>* join) {
     std::vector<uint64_t> reach(used.size());      // the furthest end of the ranges up to this one
     for (size_t i = 0; i < used.size(); ++i) reach[i] = i && reach[i - 1] > used[i].hi ? reach[i - 1] : used[i].hi;
     for (size_t i = 0; i < p.ops.size(); ++i) {
-        if (!p.ops[i].exec || !product(p.exec[p.ops[i].exec - 1]) || !has_tensor(p, p.exec[p.ops[i].exec - 1].t[2])) continue;
-        const Bytes r = tensor_bytes(p, p.exec[p.ops[i].exec - 1].t[2]);
+        if (!p.ops[i].exec || !product(p.exec[p.ops[i].exec - 1])) continue;
+        const int result = p.exec[p.ops[i].exec - 1].t[2];
+        if (!has_tensor(p, result) || p.tensors[result].tclass != TC_ACTIVATION) continue;
+        const Bytes r = tensor_bytes(p, result);
         const size_t n = std::lower_bound(used.begin(), used.end(), r.hi, [](const Bytes& a, uint64_t hi) { return a.lo < hi; }) - used.begin();
         if (n == 0 || reach[n - 1] <= r.lo) (*join)[i] = kUnread;
     }

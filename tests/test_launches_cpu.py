@@ -238,3 +238,20 @@ def test_rotation_whose_table_the_backward_cannot_take_goes_out_by_itself(tmp_pa
     assert table.offset % 16 == 0 and not alone(pf.raw) and not alone(moved(pf, y.t[1], offset=table.offset + 16, nbytes=table.nbytes - 16))
     assert alone(moved(pf, y.t[1], offset=table.offset + 8, nbytes=table.nbytes - 8))      # 8 bytes are enough for the rotation by itself
     assert alone(moved(pf, y.t[1], offset=lo)) and alone(moved(pf, y.t[1], offset=hi - 512))
+
+
+def test_only_activations_are_left_out(tmp_path):
+    pf, = plans(tmp_path, "tiny.cfg", 1, ODD + "recompute = 1")
+
+    def left_out(raw):
+        covered = set()
+        for what, i, _, _ in launches(raw):
+            if what != NORM_SUMS:
+                covered |= {i, i + 1} if what in (TWO_PRODUCTS, SWIGLU, ROTATED) else {i}
+        return [i for i, op in enumerate(pf.ops) if op.exec and i not in covered]
+
+    result = {pf.exec[pf.ops[i].exec - 1].t[2] for i in left_out(pf.raw)}
+    assert len(result) == 1
+    t, = result
+    for tclass, name in enumerate(planlib.TCLASSES):
+        assert bool(left_out(moved(pf, t, tclass=tclass))) == (name == "activation"), name
