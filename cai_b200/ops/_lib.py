@@ -41,19 +41,16 @@ def lib() -> ctypes.CDLL:
 
 def calls():
     """The launchers the ops use: the extension built next to the library, or, where there was no Python header to build it with (or another
-    Python runs), the ctypes functions of the same names."""
+    Python runs), the ctypes functions of the same names. An extension that is there but cannot be loaded is an error."""
     global _calls
     if _calls is None:
-        _calls = lib()
         path = _LIB_PATH.with_name("_calls" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
+        module = lib()
         if path.exists():
             loader = importlib.machinery.ExtensionFileLoader("_calls", str(path))
-            try:
-                module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_calls", loader))
-                loader.exec_module(module)
-                _calls = module
-            except ImportError:
-                pass
+            module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_calls", loader))
+            loader.exec_module(module)
+        _calls = module
     return _calls
 
 

@@ -1,6 +1,7 @@
 """The package's front door: public names resolve lazily, and importing the package needs no GPU and no torch."""
 import subprocess
 import sys
+import sysconfig
 from pathlib import Path
 
 import pytest
@@ -61,11 +62,13 @@ def test_log_level_from_the_environment_and_the_api(tmp_path):
 
 def test_launchers_of_the_extension_are_those_of_the_library():
     """The extension the ops call through against ctypes: same results and errors for calls that need no GPU, arguments taken alike."""
-    import pytest
     from cai_b200.ops import _lib
     if not _lib._LIB_PATH.exists():
         pytest.skip("kernel library not built")
     fast, slow = _lib.calls(), _lib.lib()
+    if not (Path(sysconfig.get_paths()["include"]) / "Python.h").exists():
+        pytest.skip("no Python header to build the extension with")
+    assert fast is not slow
     for rows in (1, 100, 5000, True):
         assert fast.cai_rmsnorm_bwd_parts(rows) == slow.cai_rmsnorm_bwd_parts(rows)
     bad = (None, 0, 16, None, 16, 12, 16, 16, 16, 16, 0, 0, False, 0, 1, 0, None)     # N not a multiple of 8; null pointers, an integer for a float
@@ -75,11 +78,26 @@ def test_launchers_of_the_extension_are_those_of_the_library():
     assert fast.cai_gemm_bf16(*empty) == slow.cai_gemm_bf16(*empty) == 0
     with pytest.raises(TypeError):
         fast.cai_gemm_bf16(*bad[:-1])
-    if fast is not slow:
-        with pytest.raises(TypeError):
-            fast.cai_gemm_bf16("x", *bad[1:])
-        with pytest.raises(TypeError):
-            fast.cai_gemm_bf16(*bad[:4], 1.5, *bad[5:])
+    with pytest.raises(TypeError):
+        fast.cai_gemm_bf16("x", *bad[1:])
+    with pytest.raises(TypeError):
+        fast.cai_gemm_bf16(*bad[:4], 1.5, *bad[5:])
+
+
+def test_an_extension_that_cannot_be_loaded_is_an_error(tmp_path, monkeypatch):
+    """Not a silent way to ctypes, which is for where none was built."""
+    from cai_b200.ops import _lib
+    if not _lib._LIB_PATH.exists():
+        pytest.skip("kernel library not built")
+    slow = _lib.lib()
+    monkeypatch.setattr(_lib, "_LIB_PATH", tmp_path / "libcai_kernels.so")
+    monkeypatch.setattr(_lib, "_calls", None)
+    assert _lib.calls() is slow
+    (tmp_path / ("_calls" + sysconfig.get_config_var("EXT_SUFFIX"))).write_bytes(b"no shared object")
+    for _ in range(2):
+        monkeypatch.setattr(_lib, "_calls", None)
+        with pytest.raises(ImportError):
+            _lib.calls()
 
 
 # RMSNorm backward whose rows come ahead: which rows a CTA fetches and works on. Row groups of 8, 4 and 1, CTAs without rows, a last round that is not full.
