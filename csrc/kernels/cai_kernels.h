@@ -225,6 +225,9 @@ CAI_API int cai_flash_attn_fwd(const void* qkv, void* out, float* lse, int B, in
  * 2 = two query tiles per CTA in ping-pong, 3 = one query tile per CTA, two CTAs per SM. All give the same bits. */
 CAI_API int cai_flash_attn_fwd_variant(const void* qkv, void* out, float* lse, int B, int S, int nh, int nkv, int hd,
                                        float scale, int force_variant, void* stream);
+/* The form that is chosen for a grid on `sms` SMs: 1, one query tile per CTA, the scores a block ahead; 2, two tiles per CTA; 3, one tile per CTA, two CTAs an
+ * SM. Needs no GPU. */
+CAI_API int cai_flash_attn_fwd_form(int B, int S, int nh, int sms);
 /* dqkv packed like qkv. delta is scratch f32 [B, nh, S]. */
 CAI_API int cai_flash_attn_bwd(const void* qkv, const void* out, const void* dout, const float* lse, float* delta,
                                void* dqkv, int B, int S, int nh, int nkv, int hd, float scale, void* stream);

@@ -655,6 +655,25 @@ CAI_API int cai_flash_attn_fwd(const void* qkv, void* out, float* lse, int B, in
     return cai_flash_attn_fwd_variant(qkv, out, lse, B, S, nh, nkv, hd, scale, 0, stream);
 }
 
+// Grids that leave SMs idle (few heads per GPU) are bound by their heaviest CTA: one tile per CTA with the score MMA running a block
+// ahead halves that path. Larger ones put two CTAs of one tile on each SM up to 4096 tokens, and two tiles in ping-pong into one
+// CTA beyond, where both take the same time and the latter reads K and V half as often. All give the same bits. us, one tile / two tiles /
+// two CTAs: 8 x 384 tokens, 12 / 4 heads 15.7 / 17.2 / 11.9; 6 x 640, 9 / 3 heads 17.7 / 17.1 / 15.0; 4 x 1024, 16 / 8 heads 40.7 / 31.9 /
+// 26.7; 2048, 32 / 32 heads 61.0 / 46.7 / 45.7; 4 x 4096, 16 / 8 heads 388 / 309 / 306; 8192, 32 / 8 heads 721 / 490 / 544. In one wave of
+// one-tile CTAs: 2 x 256, 16 / 8 7.2 / 8.3 / 7.4, 2048, 4 / 2 25.6 / 35.9 / 30.0.
+// In between, one-tile CTAs overflow a wave. Up to three key tiles a wave of two-tile CTAs fills the SMs (256 tokens, 75 heads 11.6 / 9.2 / 8.9, 125 heads 14.0 /
+// 10.1 / 10.8; 384, 50 heads 11.5 / 10.0 / 10.2, 70 heads 14.2 / 10.1 / 11.9). With more, the second wave of one-tile CTAs, the light ones, fits beside the
+// heavy ones of the first until the sum of all steps holds it up, the later the more tiles a row has: from 1.25 CTAs an SM at 5 tiles, 1.6 at 8, 1.75 at 10 (one tile /
+// two CTAs: 640 tokens, 33 heads 13.3 / 13.8, 42 heads 16.0 / 15.1; 1024, 25 heads 18.0 / 19.5, 34 heads 22.0 / 20.7; 1280, 20 heads 19.4 / 22.8, 29
+// heads 25.5 / 24.4), and from 14 tiles on never within two waves (1792, 18 heads 27.5 / 31.1, 21 heads 31.4 / 31.6).
+CAI_API int cai_flash_attn_fwd_form(int B, int S, int nh, int sms) {
+    const long long tiles = S / kAttnTile, ctas = tiles * nh * B;
+    if ((tiles + 1) / 2 * nh * B >= sms) return S <= 4096 ? 3 : 2;
+    if (ctas <= sms) return 1;
+    if (tiles <= 3) return 2;
+    return tiles < 14 && 4 * tiles * ctas > sms * (9 * tiles - 20) ? 3 : 1;      // 2.25 - 5 / tiles CTAs an SM
+}
+
 CAI_API int cai_flash_attn_fwd_variant(const void* qkv, void* out, float* lse, int B, int S, int nh, int nkv, int hd,
                                        float scale, int force_variant, void* stream) {
     if (hd != kAttnHD || S % kAttnTile || nkv <= 0 || nh % nkv) {
@@ -682,19 +701,7 @@ CAI_API int cai_flash_attn_fwd_variant(const void* qkv, void* out, float* lse, i
     p.out = static_cast<__nv_bfloat16*>(out);
     p.lse = lse;
     p.status = status_words(dev);
-    // Grids that leave SMs idle (few heads per GPU) are bound by their heaviest CTA: one tile per CTA with the score MMA running a block
-    // ahead halves that path. Larger ones put two CTAs of one tile on each SM up to 4096 tokens, and two tiles in ping-pong into one
-    // CTA beyond, where both take the same time and the latter reads K and V half as often. All give the same bits. us, one tile / two tiles /
-    // two CTAs: 8 x 384 tokens, 12 / 4 heads 15.7 / 17.2 / 11.9; 6 x 640, 9 / 3 heads 17.7 / 17.1 / 15.0; 4 x 1024, 16 / 8 heads 40.7 / 31.9 /
-    // 26.7; 2048, 32 / 32 heads 61.0 / 46.7 / 45.7; 4 x 4096, 16 / 8 heads 388 / 309 / 306; 8192, 32 / 8 heads 721 / 490 / 544.
-    // In between, a wave of two-tile CTAs fills the SMs that one of one-tile CTAs overflows: 8 x 256, 16 / 8 13.6 / 9.3 / 10.2, 6 x 384, 12 / 4
-    // 14.0 / 9.7 / 11.3, 4 x 512, 16 / 8 16.1 / 14.5 / 13.3, 2 x 1024, 16 / 8 21.3 / 24.4 / 20.1; the second tile's steps cost more than the second
-    // wave from 2048 tokens (2048, 16 / 8 31.6 / 39.2 / 33.3). In one wave of one-tile CTAs: 2 x 256, 16 / 8 7.2 / 8.3 / 7.4, 2048, 4 / 2
-    // 25.6 / 35.9 / 30.0.
-    const long long pair_ctas = static_cast<long long>((S + 2 * kAttnTile - 1) / (2 * kAttnTile)) * nh * B;
-    const long long ctas = static_cast<long long>(S / kAttnTile) * nh * B;
-    const int small = ctas <= sm_count(dev) || S >= 2048 ? 1 : S <= 384 ? 2 : 3;
-    const int variant = force_variant ? force_variant : pair_ctas < sm_count(dev) ? small : S <= 4096 ? 3 : 2;
+    const int variant = force_variant ? force_variant : cai_flash_attn_fwd_form(B, S, nh, sm_count(dev));
     if (variant == 3) {
         constexpr int smem_half = 3 * kAttnTileBytes + 1024 + 256;
         static bool configured_half[64] = {};
