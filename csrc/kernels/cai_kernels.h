@@ -183,6 +183,8 @@ CAI_API int cai_embed_fwd(const int* tokens, const void* E, void* out, int T, in
                           void* stream);
 CAI_API int cai_embed_bwd(const int* tokens, const void* dout, float* dE, int T, int H, int vocab_lo,
                           int vocab_hi, void* stream);
+/* Rows of the vocabulary a CTA of it takes (8 or 32); pieces_of_8: H a multiple of 8, dout and dE on 16 bytes. Needs no GPU. */
+CAI_API int cai_embed_bwd_rows(int T, int vocab_rows, int H, int pieces_of_8, int sms);
 
 /* ---- fused softmax cross-entropy over bf16 logits [rows, V] (pitch ld).
  * In place: logits are overwritten by dlogits = (softmax - onehot) * grad_scale.

@@ -668,17 +668,26 @@ CAI_API int cai_embed_fwd(const int* tokens, const void* E, void* out, int T, in
     return CAI_K_OK;
 }
 
+// Every CTA looks through all tokens, which 8 rows a CTA do four times as often as 32. It pays while few rows of the vocabulary leave SMs idle, and where
+// what a warp adds up one behind the other, its rows times the pieces of a row (256 columns, or 32 single ones), is more than the looking: with four pieces
+// up to 64 rows an SM; with fewer up to 8 rows an SM and piece, 12 from 1024 tokens and 16 from 2048 on, whose additions pile up. us, 32 rows / 8, by the
+// number of tokens: 512 x 256, 512 tokens 6.0 / 4.1; 2368 x 128, 256 tokens 4.3 / 4.7, 3000 6.9 / 5.6; 3600 x 264, 256 5.1 / 5.8, 8192 16.7 / 13.5; 4736 x 640,
+// 1024 7.2 / 7.6, 8192 18.7 / 15.0; 5000 x 1000, 3840 14.7 / 9.8; 9472 x 256, 512 6.1 / 8.1, 8192 12.9 / 17.3; 9472 x 1000, 512 to 8192 the same; 9472 x 2048, 1024 14.6 /
+// 12.3; 16000 x 256, 512 7.3 / 10.3; 16000 x 2048, 4096 23.2 / 21.4; 32000 x 1024, 4096 16.9 / 25.4.
+CAI_API int cai_embed_bwd_rows(int T, int vocab_rows, int H, int pieces_of_8, int sms) {
+    const long long pieces = (static_cast<long long>(H) + (pieces_of_8 ? 255 : 31)) / (pieces_of_8 ? 256 : 32);
+    const long long rows_an_sm = pieces >= 4 ? 64 : pieces * (T < 1024 ? 8 : T < 2048 ? 12 : 16);
+    return vocab_rows <= rows_an_sm * sms ? 8 : 32;
+}
+
 CAI_API int cai_embed_bwd(const int* tokens, const void* dout, float* dE, int T, int H, int vocab_lo,
                           int vocab_hi, void* stream) {
     if (T <= 0) return CAI_K_OK;
     if (vocab_hi <= vocab_lo) return CAI_K_OK;
-    // Every CTA looks through all tokens, which 8 rows a CTA do four times as often as 32: few rows of the vocabulary leave the
-    // SMs idle otherwise, and one behind the other what a warp adds up. us, 32 / 8: 512 tokens of 512 x 256 6.0 / 4.1, 3840 of 5000 x 1000 14.7 / 9.8,
-    // 16384 of 1000 x 256 33.4 / 16.6 and of 9480 x 1024 52.9 / 44.8; 512 of 16000 x 256 7.3 / 10.3, 4096 of 16000 x 2048 23.2 / 21.4 and of
-    // 32000 x 1024 16.9 / 25.4.
-    const int few = vocab_hi - vocab_lo <= 32 * 2 * sm_count(current_device()), rows = few ? 8 : 32;
-    const dim3 grid((vocab_hi - vocab_lo + rows - 1) / rows);
     const bool pieces = !(H & 7) && !(reinterpret_cast<uintptr_t>(dout) & 15) && !(reinterpret_cast<uintptr_t>(dE) & 15);
+    const int rows = cai_embed_bwd_rows(T, vocab_hi - vocab_lo, H, pieces, sm_count(current_device()));
+    const bool few = rows == 8;
+    const dim3 grid((vocab_hi - vocab_lo + rows - 1) / rows);
     launch_early(pieces ? (few ? embed_bwd_kernel<8, 8> : embed_bwd_kernel<8, 32>) : few ? embed_bwd_kernel<1, 8> : embed_bwd_kernel<1, 32>, grid, 256, 0, (cudaStream_t)stream, tokens,
                  (const __nv_bfloat16*)dout, dE, T, H, vocab_lo, vocab_hi);
     CAI_LAUNCH_CHECK("embed_bwd");

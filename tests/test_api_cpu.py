@@ -126,3 +126,26 @@ def test_norm_rows_that_do_not_come_end_the_ctas_work(rows, H, ctas):
             want = [(0, mine[0])] + [e for k in range(lost) for e in ((0, mine[k + 1]), (1, mine[k]))]
             assert events(cta, lost) == want
     assert sorted(worked) == list(range(0, rows, groups))
+
+
+# Rows of the vocabulary a CTA of the embedding backward takes: the faster of the two where they were measured apart, on both sides of each line the rule draws
+@pytest.mark.parametrize("T,rows,H,best", [
+    (512, 512, 256, 8), (256, 1184, 128, 8), (256, 3000, 128, 32), (512, 9472, 256, 32), (1024, 5000, 128, 32), (3000, 2368, 128, 8), (8192, 7000, 256, 32),
+    (256, 2368, 384, 8), (256, 4736, 264, 32), (1024, 4736, 512, 32), (8192, 4736, 512, 8), (16384, 7000, 512, 32),
+    (256, 3000, 640, 8), (256, 4736, 768, 32), (3000, 6000, 768, 8), (8192, 9472, 768, 32),
+    (3840, 5000, 1000, 8), (64, 9472, 1400, 8), (16384, 9472, 4096, 8), (4096, 32000, 1024, 32), (512, 16000, 256, 32)])
+def test_rows_of_an_embedding_cta(T, rows, H, best):
+    from cai_b200.ops import _lib
+    if not _lib._LIB_PATH.exists():
+        pytest.skip("kernel library not built")
+    assert _lib.lib().cai_embed_bwd_rows(T, rows, H, 1, 148) == best
+
+
+@pytest.mark.parametrize("T,pieces,rows_an_sm", [(1, 1, 8), (1023, 1, 8), (1024, 1, 12), (2047, 1, 12), (2048, 1, 16), (1023, 2, 16), (2048, 2, 32), (2048, 3, 48), (1, 4, 64)])
+def test_lines_of_the_embedding_rule(T, pieces, rows_an_sm):
+    from cai_b200.ops import _lib
+    if not _lib._LIB_PATH.exists():
+        pytest.skip("kernel library not built")
+    rows = _lib.lib().cai_embed_bwd_rows
+    for H, wide in ((256 * pieces, 1), (256 * pieces - 248, 1), (32 * pieces, 0), (32 * pieces - 31, 0)):
+        assert rows(T, rows_an_sm * 148, H, wide, 148) == 8 and rows(T, rows_an_sm * 148 + 1, H, wide, 148) == 32

@@ -180,7 +180,8 @@ def test_rmsnorm_bwd_sums(rows, H):
 # tokens of one scan and of several, one row that takes every token, rows outside the range, widths of whole pieces, of a fraction of
 # one and not a multiple of 8; vocabularies on both sides of the line between 8 and 32 rows a CTA
 @pytest.mark.parametrize("T,V,H,lo,hi", [(1, 8, 8, 0, 8), (4096, 40, 256, 0, 40), (4097, 33, 264, 0, 33), (9000, 1000, 136, 100, 777), (700, 64, 20, 0, 64),
-                                         (5000, 1, 512, 0, 1), (900, 9472, 24, 0, 9472), (900, 9600, 24, 0, 9600)])
+                                         (5000, 1, 512, 0, 1), (900, 9472, 24, 0, 9472), (900, 9600, 24, 0, 9600),
+                                         (900, 1184, 24, 0, 1184), (900, 1185, 24, 0, 1185), (900, 9472, 1000, 0, 9472), (900, 9473, 1000, 0, 9473), (700, 8000, 100, 0, 8000)])
 def test_embed_bwd_adds_in_token_order(T, V, H, lo, hi):
     from cai_b200 import ops
     g = torch.Generator().manual_seed(T)
