@@ -118,7 +118,8 @@ def build_host(verbose=False) -> Path:
     objdir.mkdir(parents=True, exist_ok=True)
     LIBDIR.mkdir(parents=True, exist_ok=True)
     BINDIR.mkdir(parents=True, exist_ok=True)
-    headers = list((CSRC / "plan").glob("*.h")) + list((CSRC / "ref").glob("*.h"))
+    headers = list((CSRC / "plan").glob("*.h")) + list((CSRC / "ref").glob("*.h")) + [CSRC / "runtime" / "launches.h"] + [
+        CSRC / "kernels" / h for h in ("cai_kernels.h", "norm_form.h", "pair_form.h")]
     srcs = host_lib_sources()
     jobs, objs = [], []
     for s in srcs:
@@ -148,7 +149,8 @@ def build_sanitized_selftest(verbose=False) -> Path:
     out = BUILD / "asan" / "cai_selftest_asan"
     out.parent.mkdir(parents=True, exist_ok=True)
     srcs = host_lib_sources() + [CSRC / "tools" / "cai_selftest.cc"]
-    headers = list((CSRC / "plan").glob("*.h")) + list((CSRC / "ref").glob("*.h"))
+    headers = list((CSRC / "plan").glob("*.h")) + list((CSRC / "ref").glob("*.h")) + [CSRC / "runtime" / "launches.h"] + [
+        CSRC / "kernels" / h for h in ("cai_kernels.h", "norm_form.h", "pair_form.h")]
     if _newer(out, srcs + headers):
         _run([CXX, "-std=c++17", "-O1", "-g", "-fsanitize=address,undefined", "-fno-omit-frame-pointer", "-fno-sanitize-recover=undefined",
               "-I", CSRC, "-I", CSRC / "plan"] + srcs + ["-o", out, "-lm", "-lpthread", "-ldl"], verbose)

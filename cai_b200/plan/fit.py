@@ -57,8 +57,10 @@ def attention_steps(B, S, nh, nkv, sms=SMS):
     tri = nq * (nq + 1.0) / 2.0
     rep = nh / max(1, nkv)
     split = rep > 1 and B * nkv * nq < sms and B * nh * nq <= sms
-    return {"fwd": max(B * nh * tri / sms, nq), "dkdv": max(B * nh * tri / sms, (1.0 if split else rep) * nq),
-            "dq": max(B * nh * tri / sms, nq)}
+    steps, longest = B * nh * tri / sms, (1.0 if split else rep) * nq
+    # both parts in one launch: the longest dK / dV CTA, or all steps of both
+    both = (longest, 0.0) if longest > 1.8 * steps else (steps, steps)
+    return {"fwd": max(steps, nq), "dkdv": max(steps, longest), "dq": max(steps, nq), "both": both}
 
 
 def _lstsq(rows, y, names, min_rows):
@@ -103,7 +105,7 @@ def fit(pairs):
                 elif parts == 4:
                     attn["dq"][0].append([1.0, st["dq"]]); attn["dq"][1].append(us)
                 elif parts == 7:
-                    attn["bwd_all"][0].append([1.0, st["dkdv"], st["dq"]]); attn["bwd_all"][1].append(us)
+                    attn["bwd_all"][0].append([1.0, *st["both"]]); attn["bwd_all"][1].append(us)
         elif k in POINTWISE:
             mb = sum(pf.tensors[t].nbytes for t in x.t if 0 <= t < len(pf.tensors)) / 1e6
             rows, ys = point.setdefault(POINTWISE[k], ([], []))

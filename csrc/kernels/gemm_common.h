@@ -3,6 +3,8 @@
 
 #include <cuda_runtime.h>
 
+#include "pair_form.h"
+
 namespace cai {
 
 struct GemmShape {
@@ -20,19 +22,10 @@ struct GemmShape {
     int sm_limit;
 };
 
-// The form a plain product runs in: columns of a 256-row tile, slices of K that are summed in order. A function of the shape.
-struct PairForm {
-    int tile_cols, slices;
-};
-PairForm pair_form(int M, int N, int K, int groups, int epi, bool segmented);
 // CTA pairs, 256-row tiles (gemm_pair.cu).
 int gemm_pair(const void* A, const void* B, const GemmShape& g, cudaStream_t st);
 
-// Two products in one launch: columns of their tiles, slices of each one's K, which of them goes first. pair_two_form says whether they can go
-// together and whether that is the faster way; neither may read or write what the other writes.
-struct PairTwoForm {
-    int tile_cols, slices[2], first;
-};
+// Two products in one launch (pair_form.h).
 bool pair_two_form(const GemmShape& a, const GemmShape& b, PairTwoForm* form);
 int gemm_pair_two(const void* A0, const void* B0, const GemmShape& g0, const void* A1, const void* B1, const GemmShape& g1, const PairTwoForm& form,
                   cudaStream_t st);

@@ -6,6 +6,7 @@
 #include <math.h>
 
 #include "host_common.h"
+#include "norm_form.h"
 #include "sm100.cuh"
 
 namespace cai {
@@ -223,8 +224,6 @@ reduce_parts_kernel(const __grid_constant__ ReduceJobs jobs, int H) {
 // Beside a product of another stream it runs on the SMs that one leaves free: none of its CTAs was seen to share an SM with a
 // persistent product's, whatever the shared memory either asks for.
 constexpr int kNormFusedThreads = 256;
-constexpr int kNormFusedCols = 1024;   // columns one warp covers: 32 lanes x 4 chunks x 8 elements
-constexpr int kNormFusedMaxH = 8192;
 constexpr int kNormStageBytes = 8 * kNormFusedCols * 2;   // a tensor's rows of one round: neighbours in memory, at most 8 x 1024 elements
 // A CTA's rounds. Rows that did not come (a wait that ran out) are neither used nor followed by more: the phase of the barrier that they belong to is still
 // open. The barrier behind the wait tells all threads alike (a word of shared memory read behind it cost 0.1 us a round).
@@ -383,18 +382,6 @@ static inline int launch_reduce_parts(const cai_dg_sum* sums, int n, int H, cuda
     return cudaGetLastError() == cudaSuccess ? 0 : 1;
 }
 
-// Rows of partial sums that the one-sweep form writes.
-static inline int rmsnorm_fused_row_warps(int H) {
-    const int R = (H + kNormFusedCols - 1) / kNormFusedCols;
-    return R <= 1 ? 1 : R <= 2 ? 2 : R <= 4 ? 4 : 8;         // a divisor of the CTA's eight warps
-}
-static inline int rmsnorm_fused_parts(int rows, int H, int parts_cap, int sms) {
-    const int groups = 8 / rmsnorm_fused_row_warps(H);
-    const long long want = (static_cast<long long>(rows) + groups - 1) / groups;
-    int grid = static_cast<int>(want < 2LL * sms ? want : 2LL * sms);
-    if (grid > parts_cap) grid = parts_cap;
-    return grid < 1 ? 1 : grid;
-}
 // The one-sweep form without the reduction of its `grid` partial rows.
 static inline int launch_rmsnorm_sweep(const void* x, const void* g, const float* rstd, const void* dy, void* dx, float* partial, int grid, int rows, int H,
                                        int dx_accumulate, cudaStream_t st) {

@@ -530,13 +530,14 @@ CAI_API int cai_rmsnorm_fwd(const void* x, const void* g, void* y, float* rstd, 
     return CAI_K_OK;
 }
 
-// Number of [H]-float partial rows cai_rmsnorm_bwd writes into its scratch buffer.
-CAI_API int cai_rmsnorm_bwd_parts(int rows) {
-    int sms = sm_count(current_device());
-    if (sms <= 0) sms = 148;
-    const int cap = sms * 2;
-    return rows < cap ? rows : cap;
+// The SMs of the current device, or those of a B200 where there is none to ask.
+static int sms_or_default() {
+    const int sms = sm_count(current_device());
+    return sms > 0 ? sms : 148;
 }
+
+// Number of [H]-float partial rows cai_rmsnorm_bwd writes into its scratch buffer.
+CAI_API int cai_rmsnorm_bwd_parts(int rows) { return rmsnorm_most_parts(rows, sms_or_default()); }
 
 CAI_API int cai_rmsnorm_bwd(const void* x, const void* g, const float* rstd, const void* dy, void* dx, float* dg,
                             float* dg_partial, int rows, int H, int dx_accumulate, int dg_accumulate,
@@ -555,11 +556,7 @@ CAI_API int cai_rmsnorm_bwd(const void* x, const void* g, const float* rstd, con
     return CAI_K_OK;
 }
 
-CAI_API int cai_rmsnorm_bwd_partial_rows(int rows, int H) {
-    if (rows <= 0 || H <= 0 || (H & 7) || H > kNormFusedMaxH) return 0;
-    const int sms = sm_count(current_device());
-    return rmsnorm_fused_parts(rows, H, cai_rmsnorm_bwd_parts(rows), sms > 0 ? sms : 148);
-}
+CAI_API int cai_rmsnorm_bwd_partial_rows(int rows, int H) { return rmsnorm_partial_rows(rows, H, sms_or_default()); }
 
 CAI_API int cai_rmsnorm_bwd_partial(const void* x, const void* g, const float* rstd, const void* dy, void* dx, float* dg_partial, int rows,
                                     int H, int dx_accumulate, void* stream) {

@@ -37,6 +37,9 @@ struct Backend {
     // Optional for pricing backends: the share of the GPU's SMs the op keeps busy while it runs (0..1). When given,
     // the replayer does not let a step be shorter than the sum of duration x share over all streams.
     double (*op_sm_share)(Backend* be, const Topology& topo, const Op& op, const CommGroup* g) = nullptr;
+    // Optional for pricing backends: price what an untraced step launches (records that go out together, results left out, sums that wait) instead of every
+    // record by itself, as traced steps run them.
+    void (*price_launches)(Backend* be, bool on) = nullptr;
     // Executing backends: bind a plan (file bytes; the plan is parsed again by the executor) ...
     int (*load_plan)(Backend* be, const Plan& plan, const std::string& path, uint32_t rank, uint32_t world);
     // ... and run one optimizer step of it on a synthetic batch drawn from `seed`.

@@ -17,9 +17,12 @@
 //   fused TP ops    launch + max(GEMM on the SMs left beside the copy CTAs, wire bytes / measured rate under all-to-all
 //                   load for the group size) (+ the own-row tail of the reduce-scatter)
 //   NCCL, p2p       latency + bytes / rate
+//   joined records  what an untraced step launches instead (csrc/runtime/launches.h): two products as one schedule of both one's tiles, a projection with its
+//                   SwiGLU as one product, a rotation behind an attention backward and results that nobody reads as nothing, the last sums of
+//                   RMSNorm backward once for all that wait. Timelines are of single records, as traced steps run them
 // Fixed costs are those of an untraced step, where plain kernels are launched while their predecessor finishes. The per-op events of a
-// traced step keep an op from starting early: each takes some 5 us more there (52 ops of a tiny step 593 us by their events, 331 us
-// without; 137 of a small one 4182 and 3531).
+// traced step keep an op from starting early: each takes some 5 us more there (before records went out together, 52 ops of a tiny step 593 us by their
+// events, 331 us without; 137 of a small one 4182 and 3531).
 // Needs a version-2 plan (kernel records and shapes); version-1 plans fall back to the analytic cost.
 #include <algorithm>
 #include <cmath>
@@ -28,6 +31,7 @@
 #include <fstream>
 #include <sstream>
 
+#include "../runtime/launches.h"
 #include "backend.h"
 
 namespace cai {
@@ -43,20 +47,23 @@ struct Calibration {
     // Plain GEMM, fitted to the per-op CUDA-event times inside steps of six models on one GPU (the headline config in launches of
     // 16384 and of 4096 tokens, two of its layers' tensor-parallel shards as models of their own, two 8B-class layers, a
     // small ragged model; 90 shapes, median error 4 %), less what an op starts early: [0] A not transposed, [1] A transposed
-    // (weight-gradient form). Their steps (those of the headline config with 8 layers), predicted / measured on one B200, ms: 60.7 / 63.0,
-    // 66.9 / 66.8, 32.6 / 33.1, 11.9 / 11.2, 50.4 / 51.0, 4.60 / 4.62
-    double gemm_launch_us = 5.6;
+    // (weight-gradient form). The fixed costs here and below are since set by twelve models, less what a traced op takes more; their untraced steps,
+    // predicted / measured on one B200, ms: 59.8 / 61.5, 18.2 / 18.2, 27.5 / 28.6, 47.3 / 48.0, 17.1 / 17.4, 5.19 / 4.93, 4.94 / 5.06, 3.52 / 3.71,
+    // 3.25 / 3.16, 3.06 / 3.08, 1.83 / 1.92, 0.248 / 0.251
+    double gemm_launch_us = 4.0;
     double gemm_tile_us[2] = {1.9, 0.2};
     double gemm_sm_flops[2] = {10.7e12, 9.4e12};
+    int joins = 1;                  // 0: every record by itself, as kernels before there were joined forms ran them
     int gemm_pairs = 1;             // 0: plain products run one CTA per 128-row tile, as the fused ones do
     // One-CTA GEMM (fused with a collective): the headline config's shapes on one GPU, fit error <= 13 %
     double fused_gemm_tile_us = 0.5;
     double fused_gemm_sm_flops = 7.9e12;
-    // fp8 block-scaled GEMM against the one-CTA bf16 one: 14 shapes inside steps of two models, 0.9 (short K) to 1.7 (K = 16384)
-    double fp8_speedup = 1.25;
+    // fp8 block-scaled GEMM against the one-CTA bf16 one: inside steps of two models, 1.5 (hidden 1024) and 2.2 (hidden 4096)
+    double fp8_speedup = 1.9;
     // attention, microseconds per 128 x 128 step of one CTA (the same six models)
-    double attn_fwd_step_us = 1.59, attn_fwd_fixed_us = 8.8;
+    double attn_fwd_step_us = 1.59, attn_fwd_fixed_us = 7.0;
     double attn_dkdv_step_us = 2.53, attn_dq_step_us = 2.00, attn_bwd_fixed_us = 11.8;
+    double dg_sums_us = 3.0;        // the last sums of RMSNorm backward, which a norm by itself launches too
     // fused tensor-parallel kernels: bytes a GPU moves per second while every member pulls and pushes at once
     // (steady-state chains on 2 / 4 / 8 GPUs), copy CTAs of the all-gather form, tail of the reduce-scatter form
     double link_rate[4] = {0.60e12, 0.60e12, 0.45e12, 0.35e12};  // group size 1-2, 2, 4, 8
@@ -70,8 +77,8 @@ struct Calibration {
     // pointwise kernels (the same six models; worst errors 6-14 %, the embedding's backward apart, whose time goes with how
     // often a token repeats)
     PointCost point_default = {3.3, 0.20};
-    PointCost rmsnorm_fwd = {1.7, 0.181}, rmsnorm_bwd = {10.0, 0.305}, rope = {1.1, 0.332}, swiglu = {0.6, 0.170},
-              adamw = {0.0, 0.2456}, cross_entropy = {9.5, 0.470}, embed = {10.3, 0.60};
+    PointCost rmsnorm_fwd = {1.7, 0.181}, rmsnorm_bwd = {6.0, 0.305}, rope = {1.1, 0.332}, swiglu = {0.6, 0.170},
+              adamw = {0.0, 0.2456}, cross_entropy = {9.5, 0.470}, embed = {6.0, 0.25};
 };
 
 bool set_key(Calibration* c, const std::string& k, double v) {
@@ -84,7 +91,7 @@ bool set_key(Calibration* c, const std::string& k, double v) {
         {"attn_dkdv_step_us", &c->attn_dkdv_step_us}, {"attn_dq_step_us", &c->attn_dq_step_us},
         {"attn_bwd_fixed_us", &c->attn_bwd_fixed_us}, {"link_rate_2", &c->link_rate[1]}, {"link_rate_4", &c->link_rate[2]},
         {"link_rate_8", &c->link_rate[3]}, {"rs_tail_us", &c->rs_tail_us}, {"fused_launch_us", &c->fused_launch_us},
-        {"nccl_latency_us", &c->nccl_latency_us}, {"nccl_rate", &c->nccl_rate}, {"fused_min_share", &c->fused_min_share},
+        {"dg_sums_us", &c->dg_sums_us}, {"nccl_latency_us", &c->nccl_latency_us}, {"nccl_rate", &c->nccl_rate}, {"fused_min_share", &c->fused_min_share},
     };
     for (const Entry& e : table)
         if (k == e.name) {
@@ -101,6 +108,7 @@ bool set_key(Calibration* c, const std::string& k, double v) {
         if (k == n + "_us_per_mb") { e.dst->us_per_mb = v; return true; }
     }
     if (k == "sms") { c->sms = static_cast<int>(v); return true; }
+    if (k == "joins") { c->joins = v != 0.0; return true; }
     if (k == "gemm_pairs") { c->gemm_pairs = v != 0.0; return true; }
     if (k == "ag_copy_ctas") { c->ag_copy_ctas = static_cast<int>(v); return true; }
     return false;
@@ -111,6 +119,15 @@ struct CalibratedImpl {
     std::vector<ExecOp> exec;
     std::vector<TensorDesc> tensors;
     uint32_t capacity_x100 = 200;
+    // How a record goes out in an untraced step: the (first) record of a launch with the one behind it, or none (it goes out with the one before, or not at all);
+    // sums that go out behind a sweep.
+    struct Joined {
+        enum How : uint8_t { kRecord, kTwoProducts, kSwiglu, kRotated, kNormSweep, kNothing } how = kRecord;
+        uint32_t next = 0;
+        int sums = 0;
+    };
+    std::vector<Joined> joined;
+    bool join = false;
 };
 
 // One CTA per tile of 128 rows.
@@ -150,6 +167,32 @@ double gemm_seconds(const Calibration& c, double M, double N, double K, bool ta,
     return (c.gemm_launch_us + waves * (c.gemm_tile_us[cls] + work)) * 1e-6;
 }
 
+// Two plain products that can go out together: one launch of both one's tiles, or slices of tiles that all run at once.
+double two_products_seconds(const Calibration& c, const ExecOp& x, const ExecOp& y, int sms, double* share) {
+    const ExecOp* o[2] = {&x, &y};
+    PairTwoForm f;
+    double s[2], w[2], t[2];
+    if (!c.gemm_pairs || !pair_two_form({x.i[0], x.i[1], x.i[2], epilogue(x)}, {y.i[0], y.i[1], y.i[2], epilogue(y)}, &f)) {
+        for (int k = 0; k < 2; ++k) s[k] = gemm_seconds(c, o[k]->i[0], o[k]->i[1], o[k]->i[2], o[k]->flags & 1, sms, &w[k]);
+        if (share) *share = (s[0] * w[0] + s[1] * w[1]) / (s[0] + s[1]);
+        return s[0] + s[1];
+    }
+    long long n[2];
+    for (int k = 0; k < 2; ++k) {
+        const int cls = o[k]->flags & 1;
+        n[k] = pair_tile_count(o[k]->i[0], o[k]->i[1], f.tile_cols);
+        t[k] = c.gemm_tile_us[cls] + (f.tile_cols == 256 ? 1.0 : 0.74) / f.slices[k] * 2.0 * 256.0 * 256.0 * o[k]->i[2] / (2.0 * c.gemm_sm_flops[cls]) * 1e6;
+    }
+    const long long pairs = std::max(1, sms / 2);
+    double us = std::max(t[0], t[1]);                       // split: every slice runs at once
+    if (f.slices[0] == 1 && f.slices[1] == 1) {
+        int heavier, more;
+        us = pair_two_schedule(n[f.first], t[f.first], n[1 - f.first], t[1 - f.first], std::min(pairs, n[0] + n[1]), &heavier, &more);
+    }
+    if (share) *share = std::min(1.0, (n[0] * t[0] * f.slices[0] + n[1] * t[1] * f.slices[1]) / (us * (c.sms / 2.0)));
+    return (c.gemm_launch_us + us) * 1e-6;
+}
+
 double operand_mb(const CalibratedImpl& im, const ExecOp& x) {
     double b = 0.0;
     for (int t : x.t)
@@ -158,6 +201,8 @@ double operand_mb(const CalibratedImpl& im, const ExecOp& x) {
 }
 
 double link_rate(const Calibration& c, uint32_t n) { return c.link_rate[n <= 2 ? 1 : n <= 4 ? 2 : 3]; }
+
+constexpr double kBothParts = 1.8;       // steps of dK / dV that both parts' steps on an SM come to, one of each (the steps' times above)
 
 // Seconds and the share of the GPU's SMs the op keeps busy while it runs.
 double price(const CalibratedImpl& im, const Topology& topo, const Op& op, const CommGroup* g, double* share) {
@@ -169,6 +214,12 @@ double price(const CalibratedImpl& im, const Topology& topo, const Op& op, const
     }
     const ExecOp& x = im.exec[op.exec - 1];
     const uint32_t n = g ? g->size : 1;
+    const CalibratedImpl::Joined joined = im.join ? im.joined[op.exec - 1] : CalibratedImpl::Joined{};
+    if (joined.how == CalibratedImpl::Joined::kNothing) {
+        *share = 0.0;
+        return 0.0;
+    }
+    if (joined.how == CalibratedImpl::Joined::kTwoProducts) return two_products_seconds(c, x, im.exec[joined.next], c.sms, share);
     auto point = [&](const PointCost& pc) { return (pc.fixed_us + operand_mb(im, x) * pc.us_per_mb) * 1e-6; };
     switch (x.kernel) {
     case K_GEMM: {
@@ -211,18 +262,21 @@ double price(const CalibratedImpl& im, const Topology& topo, const Op& op, const
         // parts (flags): bit 0 delta, bit 1 dK / dV, bit 2 dQ; 0 means all three
         const int parts = (x.flags & 7) ? (x.flags & 7) : 7;
         double t = c.attn_bwd_fixed_us;
-        if (parts & 2) {
-            // one CTA per (kv tile, kv group) sweeping the group's heads, or per query head when that grid fits the SMs
-            const bool split = rep > 1 && B * nkv * nq < c.sms && B * nh * nq <= c.sms;
-            const double longest = (split ? 1.0 : rep) * nq;
-            t += std::max(B * nh * tri / c.sms, longest) * c.attn_dkdv_step_us;
+        // dK / dV: one CTA per (kv tile, kv group) sweeping the group's heads, or per query head when that grid fits the SMs
+        const bool split = rep > 1 && B * nkv * nq < c.sms && B * nh * nq <= c.sms;
+        const double steps = B * nh * tri / c.sms, longest = (split ? 1.0 : rep) * nq;
+        if ((parts & 6) == 6 && longest > kBothParts * steps) t += longest * c.attn_dkdv_step_us;      // one launch: dQ's CTAs run beside the longest
+        else {
+            if (parts & 2) t += std::max(steps, (parts & 4) ? 0.0 : longest) * c.attn_dkdv_step_us;
+            if (parts & 4) t += std::max(steps, (parts & 2) ? 0.0 : nq) * c.attn_dq_step_us;
         }
-        if (parts & 4) t += std::max(B * nh * tri / c.sms, nq) * c.attn_dq_step_us;
         *share = std::min(1.0, B * nh * nq / c.sms);
         return t * 1e-6;
     }
     case K_RMSNORM_FWD: return point(c.rmsnorm_fwd);
-    case K_RMSNORM_BWD: return point(c.rmsnorm_bwd);
+    case K_RMSNORM_BWD:
+        if (joined.how == CalibratedImpl::Joined::kNormSweep) return std::max(0.0, point(c.rmsnorm_bwd) - c.dg_sums_us * 1e-6) + joined.sums * c.dg_sums_us * 1e-6;
+        return point(c.rmsnorm_bwd);
     case K_ROPE: return point(c.rope);
     case K_SWIGLU_FWD: case K_SWIGLU_BWD: return point(c.swiglu);
     case K_ADAMW: return point(c.adamw);
@@ -281,7 +335,32 @@ int calibrated_load_plan(Backend* be, const Plan& plan, const std::string&, uint
     im->exec = plan.exec;
     im->tensors = plan.tensors;
     im->capacity_x100 = plan.train.moe_capacity_factor_x100 ? plan.train.moe_capacity_factor_x100 : 200;
+    im->joined.assign(plan.exec.size(), {});
+    if (plan.exec.empty()) return OK;
+    using Joined = CalibratedImpl::Joined;
+    const std::vector<uint8_t> joins = find_joins(plan);
+    LaunchWalk walk(plan, joins, true, true, im->c.sms);
+    for (Joined& j : im->joined) j.how = Joined::kNothing;
+    uint32_t sweep = 0;
+    for (Launch l; walk.next(&l);) {
+        if (l.what == Launch::kEvent) continue;
+        if (l.what == Launch::kNormSums) {
+            ++im->joined[sweep].sums;
+            continue;
+        }
+        const uint32_t at = plan.ops[l.op].exec - 1;
+        Joined& j = im->joined[at];
+        j.how = l.what == Launch::kTwoProducts ? Joined::kTwoProducts : l.what == Launch::kSwiglu ? Joined::kSwiglu : l.what == Launch::kRotated ? Joined::kRotated
+                : l.what == Launch::kNormSweep ? Joined::kNormSweep : Joined::kRecord;
+        if (l.what == Launch::kTwoProducts) j.next = plan.ops[l.op + 1].exec - 1;
+        if (l.what == Launch::kNormSweep) sweep = at;
+    }
     return OK;
+}
+
+void calibrated_price_launches(Backend* be, bool on) {
+    auto* im = static_cast<CalibratedImpl*>(be->impl);
+    im->join = on && im->c.joins && im->joined.size() == im->exec.size();
 }
 
 void calibrated_destroy(Backend* be) {
@@ -332,6 +411,7 @@ Backend* backend_calibrated_create(const char* calibration_path, std::string* wh
     be->op_seconds = calibrated_op_seconds;
     be->op_sm_share = calibrated_sm_share;
     be->load_plan = calibrated_load_plan;
+    be->price_launches = calibrated_price_launches;
     be->run_step = nullptr;
     be->snapshot = nullptr;
     be->restore = nullptr;

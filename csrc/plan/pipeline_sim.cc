@@ -114,6 +114,7 @@ int replay_pipeline(const std::vector<const Plan*>& stages, const Topology& topo
         const std::vector<int> peer = p2p_peers(p);
         if (be->load_plan)      // a backend that prices by kernel record binds the stage's exec table first
             if (int rc = be->load_plan(be, p, std::string(), p.hdr.global_rank, p.hdr.world_size); rc != OK) return fail(rc, "backend refused the plan of stage " + std::to_string(s));
+        if (be->price_launches) be->price_launches(be, !out->want_trace);
         std::vector<int64_t> event(p.hdr.num_events ? p.hdr.num_events : 1, -1);
         std::vector<int64_t>& last = tails[s];
         const CommGroup* by_id[16] = {};

@@ -109,6 +109,7 @@ static int price_table(cai_context* ctx) {
     const Plan& p = ctx->plan;
     ctx->replay.clear();
     ctx->replay.reserve(p.ops.size());
+    if (ctx->be->price_launches) ctx->be->price_launches(ctx->be, !ctx->trace_on);
     const CommGroup* by_id[16] = {};
     for (const CommGroup& c : p.groups)
         if (c.group_id < 16) by_id[c.group_id] = &c;      // later entries win, as a linear search for the last match does
@@ -335,6 +336,7 @@ int cai_train_step(cai_context_t* ctx, const cai_batch_t* batch) {
 }
 
 int cai_trace_enable(cai_context_t* ctx, int on) {
+    if (ctx->trace_on != (on != 0)) ctx->replay.clear();      // priced again: a traced step runs every record by itself
     ctx->trace_on = on != 0;
     if (!on) ctx->trace.clear();
     return OK;

@@ -608,7 +608,7 @@ int replay(cai_exec* ex) {
         if (ex->used[s]) cudaStreamWaitEvent(ex->streams[s], ex->fork_ev, 0);
     ex->launches = 0;
     const bool traced = ex->trace_on && !ex->use_graph;
-    LaunchWalk walk(*ex, ex->joins, !traced && !ex->debug_bounds, ex->sm_limit_hi <= 0);
+    LaunchWalk walk(*ex, ex->joins, !traced && !ex->debug_bounds, ex->sm_limit_hi <= 0, sm_count(ex->device));
     for (Launch l; walk.next(&l);) {
         if (l.what == Launch::kNormSums) {
             const int rc = launch_sums(ex, *l.sums);
@@ -780,7 +780,7 @@ CAI_API int cai_plan_launches(const void* plan_bytes, size_t nbytes, int join, i
     cai_exec ex;
     if (!read_tables(&ex, plan_bytes, nbytes)) return CAI_K_BAD_ARG;
     ex.joins = find_joins(ex);
-    LaunchWalk walk(ex, ex.joins, join != 0, join != 0);
+    LaunchWalk walk(ex, ex.joins, join != 0, join != 0, 148);
     int n = 0;
     for (Launch l; walk.next(&l); ++n)
         if (n < capacity) {

@@ -2,7 +2,7 @@
 //
 // The plan names every operation. A replay joins neighbours on one stream, leaves out what nobody reads and lets the last sums of
 // RMSNorm backward wait for each other. Which ones follows from the plan's records and the bytes that they name, so it is decided here, without a
-// GPU: the executor carries the list out, and cai_plan_launches shows it.
+// GPU: the executor carries the list out, the calibrated backend prices it, and cai_plan_launches shows it.
 #pragma once
 
 #include <algorithm>
@@ -11,6 +11,8 @@
 #include <vector>
 
 #include "../kernels/cai_kernels.h"
+#include "../kernels/norm_form.h"
+#include "../kernels/pair_form.h"
 #include "../plan/plan.h"
 
 namespace cai {
@@ -81,7 +83,7 @@ inline bool projection_with_swiglu(const Plan& p, const ExecOp& x, const ExecOp&
     const Bytes act = rows_of(p, y.t[1], M, F, 2);
     if (act.meets(operand_a(p, x)) || act.meets(operand_b(p, x)) || act.meets(result_c(p, x))) return false;
     return p.tensors[y.t[0]].offset == p.tensors[x.t[2]].offset && y.i[0] == M && 2 * F == x.i[1] && pitch(p, x.t[2]) == x.i[1] && pitch(p, y.t[1]) == F &&
-           F % 128 != 0 && cai_gemm_bf16_swiglu_pays(M, F, x.i[2]);
+           F % 128 != 0 && pair_swiglu_pays(M, F, x.i[2]);
 }
 
 // Whether two records next to each other are an attention backward and the inverse rotary embedding of its result. The table is read while other rows of
@@ -202,7 +204,8 @@ struct Launch {
 // in other forms than those of single records (false under a limit on the SMs).
 class LaunchWalk {
 public:
-    LaunchWalk(const Plan& plan, const std::vector<uint8_t>& joins, bool join, bool products) : p_(plan), joins_(joins), join_(join), products_(products) {}
+    LaunchWalk(const Plan& plan, const std::vector<uint8_t>& joins, bool join, bool products, int sms)
+        : p_(plan), joins_(joins), join_(join), products_(products), sms_(sms) {}
     bool next(Launch* l) {
         for (; at_ < p_.ops.size(); ++at_) {
             const Op& op = p_.ops[at_];
@@ -214,7 +217,7 @@ public:
             const ExecOp& x = p_.exec[op.exec - 1];
             if (how == kUnread && join_ && !gather_) continue;
             if (x.kernel == K_RMSNORM_BWD && join_) {
-                const int parts = cai_rmsnorm_bwd_partial_rows(x.i[0], x.i[1]);
+                const int parts = rmsnorm_partial_rows(x.i[0], x.i[1], sms_);
                 const bool form = parts > 0 && has_tensor(p_, x.t[5]) && static_cast<uint64_t>(parts) * x.i[1] * sizeof(float) <= tensor_bytes(p_, x.t[6]).hi - tensor_bytes(p_, x.t[6]).lo;
                 if (form && waiting_.add(p_, op, x, parts)) {
                     l->sums = &waiting_;
@@ -248,6 +251,7 @@ private:
     const Plan& p_;
     const std::vector<uint8_t>& joins_;
     const bool join_, products_;
+    const int sms_;
     size_t at_ = 0;
     bool gather_ = false;
     WaitingSums waiting_, out_;
