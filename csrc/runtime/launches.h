@@ -216,7 +216,8 @@ public:
             if (!op.exec) continue;
             const ExecOp& x = p_.exec[op.exec - 1];
             if (how == kUnread && join_ && !gather_) continue;
-            if (x.kernel == K_RMSNORM_BWD && join_) {
+            // (a product that carries a gather writes more than its record names: behind a gather no sum waits)
+            if (x.kernel == K_RMSNORM_BWD && join_ && !gather_) {
                 const int parts = rmsnorm_partial_rows(x.i[0], x.i[1], sms_);
                 const bool form = parts > 0 && has_tensor(p_, x.t[5]) && static_cast<uint64_t>(parts) * x.i[1] * sizeof(float) <= tensor_bytes(p_, x.t[6]).hi - tensor_bytes(p_, x.t[6]).lo;
                 if (form && waiting_.add(p_, op, x, parts)) {

@@ -255,3 +255,18 @@ def test_only_activations_are_left_out(tmp_path):
     t, = result
     for tclass, name in enumerate(planlib.TCLASSES):
         assert bool(left_out(moved(pf, t, tclass=tclass))) == (name == "activation"), name
+
+
+def test_no_sum_waits_behind_a_gather(tmp_path):
+    """The product a gather rides in writes the gathered parameters, which its record does not name. The compiler puts it right behind the gather's record; here
+    a norm comes in between."""
+    pf = plans(tmp_path, "tiny_mp.cfg", 2, "comm = fused\nzero_stage = 3")[0]
+    record = lambda i: pf.exec[pf.ops[i].exec - 1]
+    gather = next(i for i, op in enumerate(pf.ops) if op.exec and record(i).kernel == K["fsdp_ag_gemm"] and record(i).flags & 1)
+    assert record(gather + 1).kernel == K["gemm"]
+    norm = next(i for i in range(gather, len(pf.ops)) if pf.ops[i].exec and record(i).kernel == K["rmsnorm_bwd"])
+    assert (NORM_SWEEP, norm) in [(w, i) for w, i, _, _ in launches(pf.raw)] and pf.ops[norm].stream_id == pf.ops[gather].stream_id
+    pf.ops[gather + 1].exec, pf.ops[norm].exec = pf.ops[norm].exec, pf.ops[gather + 1].exec
+    at = ctypes.sizeof(planlib.PlanHeader) + ctypes.sizeof(pf.tensors) + ctypes.sizeof(pf.groups)
+    steps = [(w, i) for w, i, _, _ in launches(pf.raw[:at] + bytes(pf.ops) + pf.raw[at + ctypes.sizeof(pf.ops):])]
+    assert (RECORD, gather + 1) in steps
