@@ -344,3 +344,26 @@ def test_swiglu_of_any_width(M, K, F):
     assert torch.allclose(gu[:M].float(), want.float(), rtol=2.0 ** -7, atol=1e-2)
     assert bool((gu[M] == 5.0).all()) and bool((act[M] == 5.0).all())
     assert ops.device_status() == 0
+
+
+# The gate / up projection with SwiGLU over ragged slabs (the C entry): live rows as without slabs, bit for bit, and nothing in halves of tiles past a count.
+@pytest.mark.parametrize("slabs,seg_rows,F,K", [(4, 256, 128, 64), (3, 384, 384, 264), (8, 128, 256, 1000)])
+@pytest.mark.parametrize("kind", ["none", "full", "edges", "random"])
+def test_swiglu_of_ragged_rows(slabs, seg_rows, F, K, kind):
+    import ctypes
+    from cai_b200 import ops
+    g = torch.Generator().manual_seed(slabs + F)
+    counts = {"none": torch.zeros(slabs), "full": torch.full((slabs,), seg_rows), "edges": torch.tensor([1, 128, 129, seg_rows - 1, 127, 0, 64, 2])[:slabs],
+              "random": torch.randint(0, seg_rows + 1, (slabs,), generator=g)}[kind].to(torch.int32)
+    M, c = slabs * seg_rows, counts.cuda()
+    x, w = torch.randn(M, K, generator=g).to(torch.bfloat16).cuda(), (torch.randn(2 * F, K, generator=g) * 0.1).to(torch.bfloat16).cuda()
+    gu, act = torch.full((M, 2 * F), 5.0, device="cuda", dtype=torch.bfloat16), torch.full((M, F), 5.0, device="cuda", dtype=torch.bfloat16)
+    p, q = [ctypes.c_void_p(t.data_ptr()) for t in (x, w, gu, act)], ctypes.c_longlong
+    assert ops.lib().cai_gemm_bf16_seg(*p, M, 2 * F, K, q(K), q(K), q(2 * F), q(F), 0, 0, ops.EPI_SWIGLU, ctypes.c_float(1.0), ctypes.c_void_p(c.data_ptr()),
+                                       seg_rows, 1, 0, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+    want_gu, want_act = ops.gemm_swiglu(x, w)
+    for s, n in enumerate(counts.tolist()):
+        for got, want in ((gu, want_gu), (act, want_act)):
+            got, want = got[s * seg_rows:(s + 1) * seg_rows], want[s * seg_rows:(s + 1) * seg_rows]
+            assert torch.equal(got[:n], want[:n]) and bool((got[(n + 127) // 128 * 128:] == 5.0).all())
+    assert ops.device_status() == 0
