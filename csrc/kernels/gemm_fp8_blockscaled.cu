@@ -245,7 +245,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
 // paying its waits under the other's MMAs. What is left is the chain of the epilogue warps (wait, read, add, hand back; a satisfied wait or a read of shared
 // memory takes some 200 cycles beside the operand reads) and the round trip to the issuing warps. So: the MMAs of a k-block come in two halves of
 // 128 columns with barriers of their own, each read by four warps, 128 columns a thread (eight warps of 232 registers, the launch's 168 and what the
-// other warpgroup gives up; sixteen warps of 64 columns had 112 and spilled); two reads are in flight per wait; the next part is asked
+// other warpgroup gives up; sixteen warps of 64 columns had 112; 20 bytes a thread are spilled, 32 with sixteen warps); two reads are in flight per wait; the next part is asked
 // for before the last additions, without blocking; scales come in eight k-blocks at a time and are read and multiplied four at a time. Cycles per
 // k-block, sixteen warps and whole k-blocks / now: 965 / 820 with two pairs at work, 1100 / 983 with 72. us, bursts of 50: 2000 x 4096 x 14336
 // 131 / 118, 9472 x 4096 x 4096 176 / 158 (one CTA per tile 145 for the former); with results that leave by TMA through boxes of shared memory,
